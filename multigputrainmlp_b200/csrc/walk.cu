@@ -2,13 +2,17 @@
 // (seed, epoch, step, rank, sample): native/cuda/random_walk_kernel.cu:7-64 and
 // native/src/random_walk_cpu.cpp:32-66. Integer-only; HBM traffic is 100 bytes per sample.
 //
-// One thread walks one sample. The 18 move permutations live in shared memory; each thread keeps its two 72-byte
-// state buffers in shared memory as words of four positions, words of neighbouring threads next to each other:
-// byte gathers of a warp then fall into 32 different banks and a move writes 18 words per thread instead of 72 bytes.
-// The kernel is one warp's chain of instructions, as deep as the longest walk (about 775 instructions per move, three
-// quarters of them the 72 byte gathers), so moves are applied two at a time: every CTA first composes the 18 x 18 pairs
-// of permutations in shared memory (26 KB), the walk draws its moves one by one as the generator prescribes and gathers
-// once per pair.
+// The moves of a walk must be drawn one after the other (the generator never repeats the previous move, so what a draw means
+// depends on the one before), but they need not be applied to the state one after the other: new[i] = old[move[i]] for
+// every move makes the final value of position i target[m_1[m_2[... m_d[i] ...]]], a chain of lookups that starts at i and
+// never touches the other positions. So a CTA works in two phases: one thread per sample draws the moves of its walk, then
+// all threads trace positions, four per thread (one word of the record), eighteen threads per sample. While the moves are
+// drawn the other warps compose the 18 x 18 pairs of permutations in shared memory, which halves the length of every trace.
+// The states of the generator form a chain of their own whatever the moves are, so the drawing loop takes one state per
+// turn and both remainders of it, and decides afterwards what they were for: no lane waits for another's repeated move.
+// What bounds it: that chain at small batches, the lookups in shared memory at large ones. Before, one thread carried the
+// 72-byte state of a sample through every pair of moves and the repeated-move branch was taken by nearly every warp: 30 us
+// at 1 024 samples and 41 us at 53 248 (depths 1..29), now 7 us and 26 us.
 // The generator's `rng % bound` on the full 64-bit state is computed exactly with 32-bit multiplies
 // (x mod b = ((hi mod b) * (2^32 mod b) + lo mod b) mod b, each step by a multiply-high with ceil(2^32 / b) and one
 // correction), which is several times cheaper than a 64-bit remainder.
@@ -18,8 +22,9 @@
 
 namespace {
 
-constexpr int kWalkThreads = 128;
-constexpr int kStateWords = MGT_STATE_STORAGE_LEN / 4;  // 20 words hold the 72 positions (and the 8 pad bytes)
+constexpr uint32_t kWalkThreads = 512;
+constexpr uint32_t kWalkBlockMoves = 32;  // moves drawn between two trace phases; a longer walk takes several rounds
+constexpr uint32_t kStateWords = MGT_STATE_STORAGE_LEN / 4;  // 20 words hold the 72 positions (and the 8 pad bytes)
 
 __host__ __device__ inline uint64_t Mix64(uint64_t x) {
     x += 0x9e3779b97f4a7c15ULL;
@@ -44,28 +49,41 @@ __device__ inline uint32_t Mod32(uint32_t n, const Bound& q) {
     uint32_t r = n - __umulhi(n, q.magic) * q.b;  // the quotient estimate is exact or one too large
     return r >= q.b ? r + q.b : r;
 }
-// rng = Mix64(rng); value = rng % bound on the full 64-bit state
-__device__ inline uint32_t NextBounded(uint64_t* state, const Bound& q) {
-    *state = Mix64(*state);
-    const uint64_t x = *state;
+// x % bound on the full 64 bits
+__device__ inline uint32_t Mod64(uint64_t x, const Bound& q) {
     if (q.b <= 1U) return 0U;  // (a bound of 0 is a division by zero in the reference; never reached with valid configurations)
     if (q.magic == 0U) return static_cast<uint32_t>(x % q.b);
     const uint32_t h = Mod32(static_cast<uint32_t>(x >> 32), q), l = Mod32(static_cast<uint32_t>(x), q);
     return Mod32(h * q.r32 + l, q);
 }
 
+// The same for the bounds of the drawing loop (at most MGT_MOVE_COUNT), without a branch: a remainder that came out
+// negative wraps to a large number and is then larger than itself plus b.
+__device__ inline uint32_t SmallMod32(uint32_t n, const Bound& q) {
+    const uint32_t r = n - __umulhi(n, q.magic) * q.b;
+    return q.b <= 1U ? 0U : min(r, r + q.b);
+}
+__device__ inline uint32_t SmallMod64(uint64_t x, const Bound& q) {
+    const uint32_t h = SmallMod32(static_cast<uint32_t>(x >> 32), q), l = SmallMod32(static_cast<uint32_t>(x), q);
+    return SmallMod32(h * q.r32 + l, q);
+}
+
+template <uint32_t kWalkSamples>
 __global__ void __launch_bounds__(kWalkThreads)
 RandomWalkKernel(mgt_random_walk_config_t config, uint64_t base_seed, uint64_t epoch, uint64_t step, uint32_t global_rank,
                  const mgt_train_state_t* __restrict__ moves, const mgt_train_state_t* __restrict__ target,
                  mgt_train_state_t* __restrict__ states, float* __restrict__ labels, mgt_walk_meta_t* __restrict__ meta) {
     __shared__ __align__(4) uint8_t s_moves[MGT_MOVE_COUNT * MGT_STATE_STORAGE_LEN];  // pad positions map to themselves
-    // s_pairs[a][b][i] = moves[a][moves[b][i]]: "move a, then move b" as one gather (new[i] = old[move[i]] twice)
+    // s_pairs[a][b][i] = moves[a][moves[b][i]]: "move a, then move b" as one lookup
     __shared__ __align__(4) uint8_t s_pairs[MGT_MOVE_COUNT * MGT_MOVE_COUNT * MGT_STATE_STORAGE_LEN];
-    __shared__ uint32_t s_state[2][kStateWords][kWalkThreads];
+    __shared__ uint32_t s_target[kStateWords];
+    __shared__ __align__(4) uint8_t s_seq[kWalkSamples][kWalkBlockMoves];  // the moves of this round, in the order drawn
+    __shared__ uint8_t s_count[kWalkSamples];                              // and how many
+    __shared__ uint32_t s_state[kWalkSamples][kStateWords];                // only used by walks longer than one round
 
     const uint32_t tid = threadIdx.x;
     // Word wd of a record: the given bytes for positions below state_len. For a move (`as_move`) a pad position maps to
-    // itself, and so does a source position outside the record - a malformed table must not make the gathers below index
+    // itself, and so does a source position outside the record - a malformed table must not make the lookups below index
     // outside the shared arrays; for a state the pad bytes are zero.
     auto keep_valid = [&](uint32_t given, uint32_t wd, bool as_move) -> uint32_t {
         uint32_t out = 0;
@@ -81,93 +99,121 @@ RandomWalkKernel(mgt_random_walk_config_t config, uint64_t base_seed, uint64_t e
     };
     // the records are 80 bytes long and the arrays come from the device allocator: whole words can be read
     constexpr uint32_t kMoveWords = MGT_MOVE_COUNT * kStateWords;
-    for (uint32_t i = tid; i < kMoveWords; i += kWalkThreads) {
-        const uint32_t mv = i / kStateWords, wd = i - mv * kStateWords;
-        const uint32_t given = mv < config.move_count ? reinterpret_cast<const uint32_t*>(moves[mv].v)[wd] : 0U;
-        const uint32_t identity = 0x03020100U + wd * 0x04040404U;  // moves the puzzle does not have: never drawn, kept well-formed
-        reinterpret_cast<uint32_t*>(s_moves)[i] = mv < config.move_count ? keep_valid(given, wd, true) : identity;
-    }
-    {
-        const uint32_t* tw = reinterpret_cast<const uint32_t*>(target->v);
-#pragma unroll
-        for (uint32_t wd = 0; wd < kStateWords; ++wd) s_state[0][wd][tid] = keep_valid(__ldg(tw + wd), wd, false);
-    }
-    __syncthreads();
-    // compose the pairs: one word (four positions) per item; pairs with a move the puzzle does not have are never read
-    for (uint32_t i = tid; i < MGT_MOVE_COUNT * kMoveWords; i += kWalkThreads) {
-        const uint32_t wd = i % kStateWords, ab = i / kStateWords;
-        const uint32_t a = ab / MGT_MOVE_COUNT, b = ab - a * MGT_MOVE_COUNT;
-        if (a >= config.move_count || b >= config.move_count) continue;
-        const uint32_t inner = reinterpret_cast<const uint32_t*>(s_moves + b * MGT_STATE_STORAGE_LEN)[wd];
-        const uint8_t* outer = s_moves + a * MGT_STATE_STORAGE_LEN;
-        uint32_t packed = 0;
-#pragma unroll
-        for (uint32_t k = 0; k < 4U; ++k) packed |= static_cast<uint32_t>(outer[(inner >> (8U * k)) & 0xFFU]) << (8U * k);
-        reinterpret_cast<uint32_t*>(s_pairs)[i] = packed;
-    }
-    __syncthreads();
-
-    const uint32_t sample = blockIdx.x * kWalkThreads + tid;
-    const bool active = sample < config.sample_count;
-
-    uint64_t rng = base_seed;
-    rng ^= Mix64(epoch + 0x100000001b3ULL);
-    rng ^= Mix64(step + 0x9e3779b97f4a7c15ULL);
-    rng ^= Mix64(static_cast<uint64_t>(global_rank) << 32);
-    rng ^= Mix64(sample);
-
-    const Bound span = MakeBound(config.k_max - config.k_min + 1U), all_moves = MakeBound(config.move_count), other_moves = MakeBound(config.move_count - 1U);
-    const uint32_t depth = active ? config.k_min + NextBounded(&rng, span) : 0U;
-    const uint32_t words = (config.state_len + 3U) / 4U;
-    uint32_t last_move = config.move_count;
-    uint32_t cur = 0;
-    // the generator's next move (native/cuda/random_walk_kernel.cu:40-47: never the previous move again)
-    auto draw = [&]() -> uint32_t {
-        uint32_t move = NextBounded(&rng, all_moves);
-        if (last_move != config.move_count && move == last_move) {
-            move = Mod32(move + 1U + NextBounded(&rng, other_moves), all_moves);
+    const bool drawer = tid < kWalkSamples;
+    if (!drawer) {
+        constexpr uint32_t kHelpers = kWalkThreads - kWalkSamples;
+        for (uint32_t i = tid - kWalkSamples; i < kMoveWords; i += kHelpers) {
+            const uint32_t mv = i / kStateWords, wd = i - mv * kStateWords;
+            const uint32_t given = mv < config.move_count ? reinterpret_cast<const uint32_t*>(moves[mv].v)[wd] : 0U;
+            const uint32_t identity = 0x03020100U + wd * 0x04040404U;  // moves the puzzle does not have: never drawn, kept well-formed
+            reinterpret_cast<uint32_t*>(s_moves)[i] = mv < config.move_count ? keep_valid(given, wd, true) : identity;
         }
-        last_move = move;
-        return move;
-    };
-    // new[i] = old[def[i]] for the whole state
-    auto apply = [&](const uint8_t* def_bytes) {
-        const uint32_t* def = reinterpret_cast<const uint32_t*>(def_bytes);
-        const uint8_t* src = reinterpret_cast<const uint8_t*>(&s_state[cur][0][0]);
-        for (uint32_t wd = 0; wd < words; ++wd) {
-            const uint32_t from = def[wd];  // four source positions
+        if (tid - kWalkSamples < kStateWords) s_target[tid - kWalkSamples] = keep_valid(__ldg(reinterpret_cast<const uint32_t*>(target->v) + (tid - kWalkSamples)), tid - kWalkSamples, false);
+        asm volatile("bar.sync 1, %0;" ::"n"(kHelpers) : "memory");
+        // compose the pairs: one word (four positions) per item; pairs with a move the puzzle does not have are never read
+        for (uint32_t i = tid - kWalkSamples; i < MGT_MOVE_COUNT * kMoveWords; i += kHelpers) {
+            const uint32_t wd = i % kStateWords, ab = i / kStateWords;
+            const uint32_t a = ab / MGT_MOVE_COUNT, b = ab - a * MGT_MOVE_COUNT;
+            if (a >= config.move_count || b >= config.move_count) continue;
+            const uint32_t inner = reinterpret_cast<const uint32_t*>(s_moves + b * MGT_STATE_STORAGE_LEN)[wd];
+            const uint8_t* outer = s_moves + a * MGT_STATE_STORAGE_LEN;
             uint32_t packed = 0;
 #pragma unroll
-            for (uint32_t k = 0; k < 4U; ++k) {
-                const uint32_t pos = (from >> (8U * k)) & 0xFFU;
-                packed |= static_cast<uint32_t>(src[((pos >> 2) * kWalkThreads + tid) * 4U + (pos & 3U)]) << (8U * k);
-            }
-            s_state[cur ^ 1U][wd][tid] = packed;
+            for (uint32_t k = 0; k < 4U; ++k) packed |= static_cast<uint32_t>(outer[(inner >> (8U * k)) & 0xFFU]) << (8U * k);
+            reinterpret_cast<uint32_t*>(s_pairs)[i] = packed;
         }
-        cur ^= 1U;
-    };
-    uint32_t d = 0;
-    for (; d + 2U <= depth; d += 2U) {
-        const uint32_t first = draw(), second = draw();
-        apply(s_pairs + (first * MGT_MOVE_COUNT + second) * MGT_STATE_STORAGE_LEN);
     }
-    if (d < depth) apply(s_moves + draw() * MGT_STATE_STORAGE_LEN);
-    if (active) {
-        // the 80-byte record (pad bytes zero) as five 16-byte stores
-        uint4* dst = reinterpret_cast<uint4*>(states + sample);
-#pragma unroll
-        for (int q = 0; q < kStateWords / 4; ++q) {
-            uint32_t wv[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const uint32_t wd = q * 4 + k;
-                uint32_t x = wd < words ? s_state[cur][wd][tid] : 0U;
-                const uint32_t first = wd * 4U;  // positions at or beyond state_len are padding
-                if (first + 4U > config.state_len) x &= first >= config.state_len ? 0U : (0xFFFFFFFFU >> (8U * (first + 4U - config.state_len)));
-                wv[k] = x;
+
+    const uint32_t first_sample = blockIdx.x * kWalkSamples;
+    const uint32_t sample = first_sample + tid;  // of a drawing thread
+    uint64_t rng = 0;
+    uint32_t depth = 0, left = 0, last_move = config.move_count;
+    Bound all_moves{}, other_moves{};
+    if (drawer) {
+        rng = base_seed;
+        rng ^= Mix64(epoch + 0x100000001b3ULL);
+        rng ^= Mix64(step + 0x9e3779b97f4a7c15ULL);
+        rng ^= Mix64(static_cast<uint64_t>(global_rank) << 32);
+        rng ^= Mix64(sample);
+        const Bound span = MakeBound(config.k_max - config.k_min + 1U);
+        all_moves = MakeBound(config.move_count);
+        other_moves = MakeBound(config.move_count - 1U);
+        rng = Mix64(rng);
+        depth = sample < config.sample_count ? config.k_min + Mod64(rng, span) : 0U;
+        left = depth;
+    }
+    uint32_t repeated = 0U;  // 1: the last state drew the previous move again, the next one picks among the others
+    const uint32_t rounds = (config.k_max + kWalkBlockMoves - 1U) / kWalkBlockMoves;  // k_max >= 1
+    for (uint32_t round = 0; round < rounds; ++round) {
+        if (drawer) {
+            const uint32_t now = min(left, kWalkBlockMoves);
+            left -= now;
+            // native/cuda/random_walk_kernel.cu:40-47: a draw equal to the previous move is replaced by one of the others,
+            // picked by the generator's next state
+            // Software pipeline: while turn n decides what its state was for, the remainders of state n + 1 and the state
+            // n + 2 are on their way, so a turn takes about as long as one step of the state chain.
+            uint64_t cur = Mix64(rng), ahead = Mix64(cur);
+            uint32_t plain = SmallMod64(cur, all_moves), other = SmallMod64(cur, other_moves);
+            for (uint32_t done = 0; done < now;) {
+                const uint64_t ahead2 = Mix64(ahead);
+                const uint32_t plain1 = SmallMod64(ahead, all_moves), other1 = SmallMod64(ahead, other_moves);
+                const bool emit = repeated != 0U || plain != last_move;
+                const uint32_t replaced = last_move + 1U + other;  // below 2 * move_count
+                last_move = repeated != 0U ? (replaced >= config.move_count ? replaced - config.move_count : replaced) : plain;  // (when nothing is emitted plain is last_move)
+                repeated = emit ? 0U : 1U;
+                s_seq[tid][done] = static_cast<uint8_t>(last_move);  // (overwritten by the next turn when this one emits nothing)
+                done += emit ? 1U : 0U;
+                rng = cur;
+                cur = ahead; ahead = ahead2; plain = plain1; other = other1;
             }
-            dst[q] = make_uint4(wv[0], wv[1], wv[2], wv[3]);
+            s_count[tid] = static_cast<uint8_t>(now);
         }
+        __syncthreads();
+        const bool final_round = round + 1U == rounds;
+        constexpr uint32_t kItems = kWalkSamples * kStateWords, kPerThread = (kItems + kWalkThreads - 1U) / kWalkThreads;
+        uint32_t result[kPerThread];
+#pragma unroll
+        for (uint32_t r = 0; r < kPerThread; ++r) {
+            const uint32_t item = tid + r * kWalkThreads;
+            const uint32_t ls = item / kStateWords, wd = item - ls * kStateWords;
+            uint32_t packed = 0;
+            result[r] = 0U;
+            if (item >= kItems || first_sample + ls >= config.sample_count) continue;
+            if (wd * 4U < config.state_len) {
+                const uint32_t count = s_count[ls];
+                uint32_t pos[4];
+                const uint32_t odd = (count & 1U) ? s_seq[ls][count - 1U] * MGT_STATE_STORAGE_LEN : 0U;
+#pragma unroll
+                for (uint32_t k = 0; k < 4U; ++k) {
+                    pos[k] = wd * 4U + k;
+                    if (count & 1U) pos[k] = s_moves[odd + pos[k]];
+                }
+                for (uint32_t j = count / 2U; j > 0U; --j) {
+                    const uint32_t both = reinterpret_cast<const uint16_t*>(s_seq[ls])[j - 1U];
+                    const uint8_t* pair = s_pairs + ((both & 0xFFU) * MGT_MOVE_COUNT + (both >> 8)) * MGT_STATE_STORAGE_LEN;
+#pragma unroll
+                    for (uint32_t k = 0; k < 4U; ++k) pos[k] = pair[pos[k]];
+                }
+                const uint8_t* old = reinterpret_cast<const uint8_t*>(round == 0U ? s_target : s_state[ls]);
+#pragma unroll
+                for (uint32_t k = 0; k < 4U; ++k) {
+                    const bool pad = wd * 4U + k >= config.state_len;  // the pad bytes of a record are zero
+                    packed |= (pad ? 0U : static_cast<uint32_t>(old[pos[k]])) << (8U * k);
+                }
+            }
+            if (final_round) reinterpret_cast<uint32_t*>(states + first_sample + ls)[wd] = packed;
+            result[r] = packed;
+        }
+        if (!final_round) {
+            __syncthreads();  // every trace of this round has read the old states
+#pragma unroll
+            for (uint32_t r = 0; r < kPerThread; ++r) {
+                const uint32_t item = tid + r * kWalkThreads;
+                if (item < kItems) s_state[item / kStateWords][item % kStateWords] = result[r];
+            }
+        }
+    }
+    if (drawer && sample < config.sample_count) {
         labels[sample] = static_cast<float>(depth);
         mgt_walk_meta_t m;
         m.depth = depth;
@@ -206,15 +252,22 @@ mgt_status_t mgt_launch_random_walk(const mgt_random_walk_config_t* config, uint
         device_states == nullptr || device_labels == nullptr || device_meta == nullptr) {
         return MGT_INVALID_CONFIG;
     }
-    // the kernel reads moves and target as words and writes a state record as five 16-byte vectors
+    // the kernel reads moves and target as words and writes a state record as words (16 bytes is what the other kernels want)
     if ((reinterpret_cast<uintptr_t>(device_moves) & 3U) != 0 || (reinterpret_cast<uintptr_t>(device_target) & 3U) != 0 ||
         (reinterpret_cast<uintptr_t>(device_states) & 15U) != 0 || (reinterpret_cast<uintptr_t>(device_labels) & 3U) != 0 ||
         (reinterpret_cast<uintptr_t>(device_meta) & 7U) != 0) {
         return MGT_INVALID_CONFIG;
     }
-    const uint32_t blocks = (config->sample_count + kWalkThreads - 1U) / kWalkThreads;
-    RandomWalkKernel<<<blocks, kWalkThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-        *config, base_seed, epoch, step, global_rank, device_moves, device_target, device_states, device_labels, device_meta);
+    // Up to 32 samples for each of 148 SMs a CTA takes 32: one word of positions per thread, the shortest path. Beyond that
+    // 128 per CTA, so that the pair table is composed a quarter as often (three CTAs share an SM).
+    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    if (config->sample_count <= 148U * 32U) {
+        RandomWalkKernel<32><<<(config->sample_count + 31U) / 32U, kWalkThreads, 0, st>>>(
+            *config, base_seed, epoch, step, global_rank, device_moves, device_target, device_states, device_labels, device_meta);
+    } else {
+        RandomWalkKernel<128><<<(config->sample_count + 127U) / 128U, kWalkThreads, 0, st>>>(
+            *config, base_seed, epoch, step, global_rank, device_moves, device_target, device_states, device_labels, device_meta);
+    }
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
 }
 

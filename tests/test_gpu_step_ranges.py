@@ -1,0 +1,102 @@
+"""GPU parity at the sizes where a kernel's split or a rule of the dispatch changes: edges of tiles, remainders, the smallest
+and largest of a range. The walk generator bit-exactly and the loss + gradient against the oracle, as in the other suites."""
+import numpy as np
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+if not torch.cuda.is_available():
+    pytest.skip("needs a CUDA device", allow_module_level=True)
+
+import multigputrainmlp_b200 as mgt  # noqa: E402
+from helpers import rel_l2  # noqa: E402
+from oracle import MlpShape  # noqa: E402
+from oracle.binding import WALK_META_DTYPE  # noqa: E402
+
+DEV = "cuda:0"
+
+
+def random_puzzle(state_len, move_count, seed):
+    """Random permutations (they do not commute, so the order of the moves shows) on `state_len` positions."""
+    rng = np.random.default_rng(seed)
+    moves = np.zeros((18, 80), np.uint8)
+    for i in range(move_count):
+        moves[i, :state_len] = rng.permutation(state_len)
+    target = np.zeros(80, np.uint8)
+    target[:state_len] = np.arange(state_len)
+    return moves, target
+
+
+# samples around a CTA's 32 and the step to 128 (4 736), depths around a drawing round's 32 moves, record lengths that end inside a word
+@pytest.mark.parametrize("n,k_min,k_max,state_len,move_count", [(1, 1, 1, 72, 18), (31, 1, 2, 72, 18), (32, 31, 32, 72, 18), (33, 32, 33, 70, 18),
+                                                                 (4737, 1, 29, 72, 18),
+                                                                 (200, 1, 64, 71, 3), (130, 60, 65, 17, 2), (100, 90, 200, 72, 18)])
+def test_walk_rounds_and_edges(oracle, n, k_min, k_max, state_len, move_count):
+    moves, target = random_puzzle(state_len, move_count, n)
+    d_states = torch.full((n, 80), 255, dtype=torch.uint8, device=DEV)
+    labels, meta = torch.zeros(n, device=DEV), torch.zeros(n, 16, dtype=torch.uint8, device=DEV)
+    cfg = mgt.RandomWalkKernelConfig(n, k_min, k_max, move_count, state_len, 80)
+    assert mgt.launch_random_walk_kernel(cfg, 77, 1, 5, 3, torch.from_numpy(moves).to(DEV), torch.from_numpy(target).to(DEV), d_states, labels, meta) == 0
+    st, want, depth, want_meta = oracle.random_walks(moves, target, seed=77, epoch=1, step=5, rank=3, k_min=k_min, k_max=k_max, samples=n,
+                                                     move_count=move_count, state_len=state_len)
+    assert st == 0
+    assert np.array_equal(d_states.cpu().numpy(), want) and np.array_equal(labels.cpu().numpy(), depth)
+    assert np.array_equal(meta.cpu().numpy().view(WALK_META_DTYPE).reshape(-1), want_meta)
+
+
+def loss_grad_case(oracle, dims, n, *, seed=1, scale=0.03, mirror=True, options=None, flags=(True, True), tol=1e-3, section_tol=3e-3, coherent=False):
+    """One loss + gradient launch on a walk batch against the oracle's model of the same data flow, whole and by section."""
+    shape = MlpShape(*dims)
+    length, values = shape.state_len, shape.state_value_pad
+    moves, target = random_puzzle(length, 18, seed)
+    target[:length] = np.arange(length) * values // length
+    _, states, depth, _ = oracle.random_walks(moves, target, seed=seed, epoch=0, step=0, rank=0, k_min=1, k_max=29, samples=n, state_len=length)
+    labels = np.ascontiguousarray(np.repeat(depth.reshape(-1, 1), shape.output_dim, axis=1).astype(np.float32))
+    w = (np.random.default_rng(seed).standard_normal(shape.param_count) * scale).astype(np.float32)
+    c = mgt.CudaMlpShape(*dims)
+    half_ig, half_lin = flags
+    engine = mgt.Engine(0)
+    try:
+        if options:
+            assert engine.set_train_options(**options) == 0
+        dw = torch.from_numpy(w).to(DEV)
+        loss = torch.zeros(1, device=DEV)
+        grad = torch.full((shape.param_count,), float("nan"), device=DEV)
+        floats = mgt.mlp_loss_grad_workspace_floats(c, n, 1, half_ig, half_lin)
+        ws = torch.full((floats,), float("nan"), device=DEV)
+        results = []
+        for _ in range(3):  # the same call again must give the same bits, whatever the library keeps between calls
+            grad.fill_(float("nan"))
+            st = engine.launch_mlp_loss_grad(c, dw, dw.half() if mirror else None, torch.from_numpy(states).to(DEV), torch.from_numpy(labels).to(DEV), n, loss, grad,
+                                             ws, floats, use_half_input_grad=half_ig, use_half_linear=half_lin)
+            assert st == 0 and engine.check()[0] == 0
+            results.append((float(loss.item()), grad.cpu().numpy()))
+    finally:
+        engine.close()
+    for other in results[1:]:
+        assert other[0] == results[0][0] and np.array_equal(other[1], results[0][1])
+    got_loss, got = results[0]
+    if options or flags == (False, True):
+        st, want_loss, want, _ = oracle.loss_grad_ex(shape, w, states, labels, half_linear=half_lin, half_input_grad=half_ig, **(options or {}))
+    elif half_lin:
+        st, want_loss, want = oracle.loss_grad_mixed(shape, w, states, labels)
+    else:
+        st, want_loss, want = oracle.loss_grad(shape, w, states, labels)
+    assert st == 0 and np.isfinite(got).all()
+    assert abs(got_loss - want_loss) <= tol * abs(want_loss)
+    assert rel_l2(got, want) <= tol, rel_l2(got, want)
+    table = length * values * shape.hd1
+    hidden = table + shape.hd1
+    tower = hidden + shape.hd1 * shape.hd2 + shape.hd2
+    head = shape.param_count - shape.hd2 * shape.output_dim - shape.output_dim
+    for name, lo, hi in (("table", 0, table), ("input bias", table, hidden), ("hidden", hidden, tower), ("tower", tower, head), ("head", head, shape.param_count)):
+        if hi > lo and np.abs(want[lo:hi]).max() > 0:
+            assert rel_l2(got[lo:hi], want[lo:hi]) <= section_tol, (name, rel_l2(got[lo:hi], want[lo:hi]))
+    return got_loss, got
+
+
+# widths of the fused residual tower that are not multiples of its 32-column chunks, with and without the caller's fp16 copy
+@pytest.mark.parametrize("hd2,n,mirror", [(8, 130, True), (31, 127, False), (33, 129, False), (72, 300, True), (200, 257, True), (250, 128, False), (255, 400, True)])
+def test_residual_tower_widths(oracle, hd2, n, mirror):
+    loss_grad_case(oracle, (72, 72, 48, hd2, 3, 1), n, mirror=mirror)
