@@ -878,9 +878,10 @@ mgt_status_t GemmBackpropInputRows(mgt_engine* e, cudaStream_t st, const __half*
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
 }
 
-// The residual tower in one launch per direction; see tower_chain.cuh. Shapes it takes: hd2 a multiple of 32 up to 256.
+// The residual tower in one launch per direction; see tower_chain.cuh. Shapes it takes: hd2 up to 256 (a tile's state and
+// product need two TMEM columns per hidden unit).
 bool ChainEligible(const mgt_engine* e, const mgt_mlp_shape_t& s) {
-    return s.residual_blocks > 0 && s.hd2 % 32U == 0 && s.hd2 >= 32U && s.hd2 <= 256U && !e->layered_tower;
+    return s.residual_blocks > 0 && s.hd2 <= 256U && !e->layered_tower;
 }
 
 template <bool BWD>
@@ -896,7 +897,7 @@ mgt_status_t LaunchChain(mgt_engine* e, cudaStream_t st, const __half* w_first, 
         }
     }
     CUtensorMap tw, ts, tt;
-    MGT_MAP(e->Map3D(&tw, w_first, a.H, a.H, 2ULL * a.R, w_pitch, w_layer_stride_bytes, 64, BWD ? a.H : 64));
+    MGT_MAP(e->Map3D(&tw, w_first, a.H, a.H, 2ULL * a.R, w_pitch, w_layer_stride_bytes, 64, BWD ? (a.H + 31U) & ~31U : 64));
     // the tapes as stacks of [samples][H] matrices; a store box is one operand panel: 64 columns x 128 rows
     MGT_MAP(e->Map3D(&ts, a.tape_s, a.H, a.samples, tape_s_entries, a.ld_s, a.tape_s_stride * 2, 64, 128));
     MGT_MAP(e->Map3D(&tt, a.tape_t, a.H, a.samples, tape_t_entries, a.ld_t, a.tape_t_stride * 2, 64, 128));
