@@ -78,6 +78,8 @@ struct Workspace {
 
 constexpr uint32_t kHeadBlocks = 296;   // two CTAs per SM on a 148-SM part
 constexpr uint32_t kHeadThreads = 256;
+// per CTA: { grad W_out, grad b_out, loss, column sums of dz } with one output, { loss, column sums of dz, grad b_out } with more
+inline uint64_t HeadPartialFloats(const mgt_mlp_shape_t& s) { return s.output_dim == 1U ? 2ULL * s.hd2 + 2ULL : (uint64_t)s.hd2 + 1ULL + s.output_dim; }
 
 // The scratch for per-CTA partial sums is sized by the SM count: never below the B200's 148, so that the size the
 // query reports (it has no engine, it asks the current device) covers the launch on any sm_100 part.
@@ -133,7 +135,7 @@ Workspace PlanWorkspace(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm_count,
     w.partial_floats = p1 > p2 ? p1 : p2;
     w.off_partial = take(w.partial_floats * 4);
     w.head_blocks = kHeadBlocks;
-    w.off_head = take((uint64_t)kHeadBlocks * (2ULL * s.hd2 + 2) * 4);
+    w.off_head = take((uint64_t)kHeadBlocks * HeadPartialFloats(s) * 4);
     // per-warp column sums: one slot per residual dX GEMM (2R of them)
     const uint64_t chain_tiles = (B + 127) / 128;
     const uint64_t slot_rows = (uint64_t)sm_count * 16 > chain_tiles * 4 ? (uint64_t)sm_count * 16 : chain_tiles * 4;  // up to 16 epilogue warps per CTA
@@ -302,6 +304,7 @@ template <int BN> using CfgDw = GemmCfg<BN, 1, true, BSource::kTmaMN, Epi::kPart
 template <int BN, Epi EPI> using CfgFwdRows = GemmCfg<BN, 1, true, BSource::kTmaMN, EPI, 3, 3>;        // a1T[K][M] x W[K][N]
 template <int BN> using CfgDwRows = GemmCfg<BN, 1, false, BSource::kTmaMN, Epi::kPartialF32, 3, 3>;    // a1T[M][K] x dz[K][N]
 using CfgDxRows = GemmCfg<256, 1, false, BSource::kTmaK, Epi::kMaskRowsumF16, 4, 4>;                   // W[M][K] x dz[N][K] -> dz1T[M][N]
+using CfgDxRowsF32 = GemmCfg<256, 1, false, BSource::kTmaK, Epi::kMaskRowsumF32, 4, 4>;                // the same -> dz1[N][M] in fp32
 template <int BN> using CfgDwG = GemmCfg<BN, 1, true, BSource::kTmaMN, Epi::kPartialF32, 3, 3, false, true>; // R stacked act^T x dz
 // Two 256-column accumulators per unit (all of TMEM) and a two-stage one-hot ring. Measured alternatives at p888: 2 x 192
 // columns with a three-stage ring 1.44 ms, one double-buffered 256-column accumulator (epilogue under the next unit's
@@ -502,7 +505,6 @@ ReduceRowsGroupedKernel(const float* __restrict__ src, uint32_t rows, uint32_t c
 // partials[CTA][2*H2+2] = { grad W_out[H2], grad b_out, loss, column sums of dz[H2] } and are added
 // in a fixed order by ReduceRowsKernel.
 constexpr int kHeadMaxPerLane = MGT_MAX_HD2 / 32;
-constexpr size_t kHeadStagedSmemLimit = 160U * 1024U;  // dynamic shared memory of HeadOutNKernel with staged weights (two CTAs per SM at up to 96 KB)
 __global__ void __launch_bounds__(kHeadThreads)
 HeadOut1Kernel(const float* __restrict__ w_out, const float* __restrict__ b_out, const float* __restrict__ labels, const float* __restrict__ x,
                uint32_t p_f32, uint32_t B, uint32_t H2, float* __restrict__ dzf, __half* __restrict__ dz_h, uint32_t p_dz, float* __restrict__ partials,
@@ -557,7 +559,7 @@ HeadOut1Kernel(const float* __restrict__ w_out, const float* __restrict__ b_out,
                 const float d = xv[q] > 0.0f ? wreg[q] * dy : 0.0f;
                 dacc[q] += d;
                 dzf[(uint64_t)b * p_f32 + j] = d;
-                reinterpret_cast<uint16_t*>(dz_h)[(uint64_t)b * p_dz + j] = ptx::to_operand(d, bf16);
+                if (dz_h != nullptr) reinterpret_cast<uint16_t*>(dz_h)[(uint64_t)b * p_dz + j] = ptx::to_operand(d, bf16);
             }
         }
     }
@@ -575,82 +577,256 @@ HeadOut1Kernel(const float* __restrict__ w_out, const float* __restrict__ b_out,
     }
 }
 
-// Output head for output_dim > 1 (native/cuda/mlp_backward.cu:1341-1363): 16-bit operands, fp32 accumulate, dy rounded to
-// the operand format for the two products that follow. kCrossEntropy = false: the reference's MSE against the labels.
-// kCrossEntropy = true (no counterpart in the reference): the outputs are per-depth logits, class = depth - 1 (the labels
-// carry the walk depth in every output slot), loss = mean over the batch of -log softmax(y)[class],
-// dy = (softmax(y) - onehot(class)) / B. One warp per sample, plain SIMT (B x OUT x H2 multiply-adds twice). kStageW: the
-// output weights are converted once per CTA into shared memory ([H2][OUT | 1] floats: rows for the forward product, a
-// lane per row without bank conflicts for the backward one); read from global memory instead, the lane-per-row access of
-// the backward product touches 32 sectors per instruction and the kernel is bound by L2 (5.4 ms instead of 0.5 ms at
-// batch 131072, hd2 512, 29 outputs).
-template <bool kCrossEntropy, bool kStageW>
+// ---- output head for output_dim > 1 (native/cuda/mlp_backward.cu:1341-1363) -------------------------------------------
+// 16-bit operands, fp32 accumulate, dy rounded to the operand format for the two products that follow; kF32: fp32 operands
+// throughout. kCrossEntropy = false: the reference's MSE against the labels. kCrossEntropy = true (no counterpart in the
+// reference): the outputs are per-depth logits, class = depth - 1 (the labels carry the walk depth in every output slot),
+// loss = mean over the batch of -log softmax(y)[class], dy = (softmax(y) - onehot(class)) / B.
+// Both kernels leave one row of partial sums per CTA: { loss, column sums of dz[H2], column sums of dy[OUT] }.
+struct HeadArgs {
+    const void* w_out;       // [H2][p_wout] operand format, or fp32
+    uint32_t p_wout;
+    const float* b_out;
+    const float* labels;
+    const __half* x_h;       // operand copy of x (unused with kF32)
+    uint32_t p_act;
+    const float* x_f32;
+    uint32_t p_f32;
+    uint32_t B, H2, OUT;
+    float* dy;
+    __half* dy_h;            // (unused with kF32)
+    uint32_t p_dy;
+    float* dzf;
+    __half* dz_h;            // (unused with kF32)
+    uint32_t p_dz;
+    float* partials;
+    bool bf16;
+};
+
+// dL/dy of one sample, a lane per output (and every 32nd): y and dy in `row` (the logits come in, the operand of the two
+// products goes out), the plain dy to memory. Adds the sample's loss term to `loss` and its dy to `dyb`, if kept there.
+template <bool kCrossEntropy, bool kF32, int kKept>
+__device__ __forceinline__ void HeadLossRow(const HeadArgs& a, uint32_t b, float inv_n, float* row, uint32_t lane, float& loss, float (&dyb)[kKept]) {
+    float mx = -3.0e38f, log_sum = 0.0f;
+    uint32_t cls = 0;
+    if (kCrossEntropy) {
+        for (uint32_t o = lane; o < a.OUT; o += 32) mx = fmaxf(mx, row[o]);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFU, mx, o));
+        float sum = 0.0f;
+        for (uint32_t o = lane; o < a.OUT; o += 32) sum += expf(row[o] - mx);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFU, sum, o);
+        log_sum = logf(sum) + mx;
+        // a depth outside 1..OUT cannot come from the walk generator with k_max <= OUT; clamp instead of reading out of bounds
+        const int c = __float2int_rn(a.labels[(uint64_t)b * a.OUT]) - 1;
+        cls = static_cast<uint32_t>(c < 0 ? 0 : (c >= static_cast<int>(a.OUT) ? static_cast<int>(a.OUT) - 1 : c));
+    }
+#pragma unroll 1
+    for (uint32_t o = lane, i = 0; o < a.OUT; o += 32, ++i) {
+        const float y = row[o];
+        float d;
+        if (kCrossEntropy) {
+            d = (expf(y - log_sum) - (o == cls ? 1.0f : 0.0f)) * inv_n;
+            if (o == cls) loss += (log_sum - y) * inv_n;
+        } else {
+            const float diff = y - a.labels[(uint64_t)b * a.OUT + o];
+            d = 2.0f * diff * inv_n;
+            loss += diff * diff * inv_n;
+        }
+        a.dy[(uint64_t)b * a.OUT + o] = d;
+        if (kF32) {
+            row[o] = d;
+        } else {
+            const uint16_t dh = ptx::to_operand(d, a.bf16);
+            reinterpret_cast<uint16_t*>(a.dy_h)[(uint64_t)b * a.p_dy + o] = dh;
+            row[o] = ptx::from_operand(dh, a.bf16);
+        }
+#pragma unroll
+        for (int q = 0; q < kKept; ++q) dyb[q] += static_cast<int>(i) == q ? d : 0.0f;
+    }
+}
+
+// Up to 64 outputs: a CTA takes 64 samples at a time. Forward as a small register-tiled product (a thread: four samples x
+// OP / 16 outputs) from x staged 64 columns at a time and the weights staged once; the loss by a warp per sample; backward
+// with a thread per hidden column, its OP weights in registers, so that dy is read as broadcast vectors and rows of dz are
+// written whole. Bound by HBM: x in the operand format and in fp32 (the ReLU mask), dz in both. One warp per sample with a
+// scalar read of x and of a weight for every multiply-add was bound by the load pipe: 1.83 ms at batch 131 072, hd2 512, 29
+// outputs, now 0.70 ms.
+constexpr uint32_t kHeadTile = 64;
+template <int OP>
+constexpr size_t HeadTileSmem(uint32_t H2) { return ((size_t)H2 * OP + 64U * (kHeadTile + 4U) + kHeadTile * OP) * sizeof(float); }
+template <int OP, bool kCrossEntropy, bool kF32>
 __global__ void __launch_bounds__(kHeadThreads)
-HeadOutNKernel(const __half* __restrict__ w_out_h, uint32_t p_wout, const float* __restrict__ b_out, const float* __restrict__ labels,
-               const __half* __restrict__ x_h, uint32_t p_act, const float* __restrict__ x_f32, uint32_t p_f32, uint32_t B, uint32_t H2, uint32_t OUT,
-               float* __restrict__ dy, __half* __restrict__ dy_h, uint32_t p_dy, float* __restrict__ dzf, __half* __restrict__ dz_h, uint32_t p_dz,
-               float* __restrict__ partials, bool bf16) {
-    extern __shared__ float s_dyn[];  // per warp: OUT floats (logits, then rounded dy); then the staged weights
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31U;
-    const uint32_t warps_total = gridDim.x * (kHeadThreads / 32);
-    float* s_dy = s_dyn + warp * OUT;
-    const uint16_t* wq = reinterpret_cast<const uint16_t*>(w_out_h);
-    const uint32_t outp = OUT | 1U;
-    float* w_s = s_dyn + (kHeadThreads / 32) * OUT;
-    if (kStageW) {
-        for (uint32_t i = threadIdx.x; i < H2 * OUT; i += kHeadThreads) {
-            const uint32_t j = i / OUT, o = i % OUT;
-            w_s[j * outp + o] = ptx::from_operand(wq[(uint64_t)j * p_wout + o], bf16);
+HeadTileKernel(const __grid_constant__ HeadArgs a) {
+    extern __shared__ __align__(16) float s_head[];
+    constexpr uint32_t NO = OP / 16, XP = kHeadTile + 4U;
+    float* ws = s_head;                                // [H2][OP]
+    float* xs = ws + (size_t)a.H2 * OP;                // [64 columns][XP]: x of the tile, transposed
+    float* ys = xs + 64U * XP;                         // [64 samples][OP]
+    const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31U;
+    for (uint32_t i = t; i < a.H2 * OP; i += kHeadThreads) {
+        const uint32_t j = i / OP, o = i % OP;
+        float w = 0.0f;
+        if (o < a.OUT) w = kF32 ? static_cast<const float*>(a.w_out)[(uint64_t)j * a.p_wout + o] : ptx::from_operand(static_cast<const uint16_t*>(a.w_out)[(uint64_t)j * a.p_wout + o], a.bf16);
+        ws[i] = w;
+    }
+    const float inv_n = 1.0f / static_cast<float>(kCrossEntropy ? (uint64_t)a.B : (uint64_t)a.B * a.OUT);
+    float loss = 0.0f, dyb[2] = {0.0f, 0.0f};
+    const uint32_t hj = min(kHeadThreads, (a.H2 + 31U) & ~31U), groups = kHeadThreads / hj, jg = t / hj, jl = t % hj;
+    float dacc[2] = {0.0f, 0.0f};
+    const uint32_t tiles = (a.B + kHeadTile - 1U) / kHeadTile;
+    for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const uint32_t b0 = tile * kHeadTile;
+        float acc[4][NO] = {};
+        const uint32_t og = t % 16U, sg = t / 16U;
+        for (uint32_t j0 = 0; j0 < a.H2; j0 += 64U) {
+            // a thread stages sixteen columns of one sample; consecutive lanes take consecutive samples
+            const uint32_t s = t % kHeadTile, jb = (t / kHeadTile) * 16U;
+            __syncthreads();
+#pragma unroll
+            for (uint32_t q = 0; q < 2U; ++q) {
+                const uint32_t j = j0 + jb + q * 8U;
+                float v[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] = 0.0f;
+                if (b0 + s < a.B && j < a.H2) {
+                    if (kF32) {
+#pragma unroll
+                        for (uint32_t e = 0; e < 8U; ++e)
+                            if (j + e < a.H2) v[e] = __ldg(a.x_f32 + (uint64_t)(b0 + s) * a.p_f32 + j + e);
+                    } else {
+                        // (rows are padded to eight elements; what lies past H2 meets nothing: the product stops at H2)
+                        const uint4 u = *reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(a.x_h) + (uint64_t)(b0 + s) * a.p_act + j);
+                        const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) {
+                            v[2 * e] = ptx::from_operand(static_cast<uint16_t>(w4[e] & 0xFFFFU), a.bf16);
+                            v[2 * e + 1] = ptx::from_operand(static_cast<uint16_t>(w4[e] >> 16), a.bf16);
+                        }
+                    }
+                }
+#pragma unroll
+                for (uint32_t e = 0; e < 8U; ++e) xs[(jb + q * 8U + e) * XP + s] = v[e];
+            }
+            __syncthreads();
+            const uint32_t jn = min(64U, a.H2 - j0);
+#pragma unroll 8
+            for (uint32_t j = 0; j < jn; ++j) {
+                const float4 x4 = *reinterpret_cast<const float4*>(xs + j * XP + sg * 4U);
+                const float* w = ws + (size_t)(j0 + j) * OP + og * NO;
+#pragma unroll
+                for (uint32_t n = 0; n < NO; ++n) {
+                    acc[0][n] += x4.x * w[n];
+                    acc[1][n] += x4.y * w[n];
+                    acc[2][n] += x4.z * w[n];
+                    acc[3][n] += x4.w * w[n];
+                }
+            }
+        }
+#pragma unroll
+        for (uint32_t n = 0; n < NO; ++n) {
+            const uint32_t o = og * NO + n;
+            const float bias = o < a.OUT ? __ldg(a.b_out + o) : 0.0f;
+#pragma unroll
+            for (uint32_t i = 0; i < 4U; ++i) ys[(sg * 4U + i) * OP + o] = acc[i][n] + bias;
         }
         __syncthreads();
+        for (uint32_t i = 0; i < kHeadTile / (kHeadThreads / 32U); ++i) {
+            const uint32_t s = warp * (kHeadTile / (kHeadThreads / 32U)) + i;
+            if (b0 + s >= a.B) break;
+            HeadLossRow<kCrossEntropy, kF32, 2>(a, b0 + s, inv_n, ys + s * OP, lane, loss, dyb);
+        }
+        __syncthreads();
+        if (jg < groups) {
+            for (uint32_t cb = 0; cb < 2U; ++cb) {
+                const uint32_t j = jl + cb * kHeadThreads;
+                if (j >= a.H2) break;
+                float w[OP];
+#pragma unroll
+                for (int o = 0; o < OP; o += 4) {
+                    const float4 w4 = *reinterpret_cast<const float4*>(ws + (size_t)j * OP + o);
+                    w[o] = w4.x; w[o + 1] = w4.y; w[o + 2] = w4.z; w[o + 3] = w4.w;
+                }
+                const uint32_t rows = min(kHeadTile, a.B - b0);
+                float sum = 0.0f;
+#pragma unroll 4
+                for (uint32_t s = jg; s < rows; s += groups) {
+                    const uint64_t b = b0 + s;
+                    const float x = __ldg(a.x_f32 + b * a.p_f32 + j);
+                    float d = 0.0f;
+#pragma unroll
+                    for (int o = 0; o < OP; o += 4) {
+                        const float4 g = *reinterpret_cast<const float4*>(ys + s * OP + o);
+                        d += g.x * w[o];
+                        d += g.y * w[o + 1];
+                        d += g.z * w[o + 2];
+                        d += g.w * w[o + 3];
+                    }
+                    d = x > 0.0f ? d : 0.0f;
+                    sum += d;
+                    a.dzf[b * a.p_f32 + j] = d;
+                    if (!kF32) reinterpret_cast<uint16_t*>(a.dz_h)[b * a.p_dz + j] = ptx::to_operand(d, a.bf16);
+                }
+                dacc[cb] += sum;
+            }
+        }
+        // (outputs past OUT: their weights are zero, and ys holds acc + bias = 0 there)
     }
-    auto weight = [&](uint32_t j, uint32_t o) -> float { return kStageW ? w_s[j * outp + o] : ptx::from_operand(wq[(uint64_t)j * p_wout + o], bf16); };
-    const float inv_n = 1.0f / static_cast<float>(kCrossEntropy ? (uint64_t)B : (uint64_t)B * OUT);
-    float loss = 0.0f;
+    __syncthreads();
+    // partial sums of the CTA, in a fixed order: warps for the loss and dy, sample groups for the columns
+    float* red = xs;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xFFFFFFFFU, loss, o);
+    if (lane == 0) red[warp] = loss;
+    red[8U + warp * 64U + lane] = dyb[0];
+    red[8U + warp * 64U + 32U + lane] = dyb[1];
+    float* cols = red + 8U + 8U * 64U;  // [groups][H2], groups * H2 <= 512
+    if (jg < groups) {
+        if (jl < a.H2) cols[jg * a.H2 + jl] = dacc[0];
+        if (jl + kHeadThreads < a.H2) cols[jl + kHeadThreads] = dacc[1];
+    }
+    __syncthreads();
+    float* out = a.partials + (uint64_t)blockIdx.x * (1U + a.H2 + a.OUT);
+    for (uint32_t i = t; i < 1U + a.H2 + a.OUT; i += kHeadThreads) {
+        float sum = 0.0f;
+        if (i == 0U) {
+            for (uint32_t w = 0; w < 8U; ++w) sum += red[w];
+        } else if (i <= a.H2) {
+            for (uint32_t g = 0; g < groups; ++g) sum += cols[g * a.H2 + i - 1U];
+        } else {
+            for (uint32_t w = 0; w < 8U; ++w) sum += red[8U + w * 64U + i - 1U - a.H2];
+        }
+        out[i] = sum;
+    }
+}
+
+// More than 64 outputs: one warp per sample, plain SIMT. Column sums of dy are left to HeadOutNBiasGradKernel.
+template <bool kCrossEntropy, bool kF32>
+__global__ void __launch_bounds__(kHeadThreads)
+HeadOutNKernel(const __grid_constant__ HeadArgs a) {
+    extern __shared__ float s_dyn[];  // per warp: OUT floats (logits, then rounded dy)
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31U;
+    const uint32_t warps_total = gridDim.x * (kHeadThreads / 32), H2 = a.H2, OUT = a.OUT;
+    float* s_dy = s_dyn + warp * OUT;
+    auto weight = [&](uint32_t j, uint32_t o) -> float {
+        return kF32 ? static_cast<const float*>(a.w_out)[(uint64_t)j * a.p_wout + o] : ptx::from_operand(static_cast<const uint16_t*>(a.w_out)[(uint64_t)j * a.p_wout + o], a.bf16);
+    };
+    const float inv_n = 1.0f / static_cast<float>(kCrossEntropy ? (uint64_t)a.B : (uint64_t)a.B * OUT);
+    float loss = 0.0f, none[1] = {0.0f};
     float dacc[kHeadMaxPerLane];
 #pragma unroll
     for (int q = 0; q < kHeadMaxPerLane; ++q) dacc[q] = 0.0f;
-    for (uint32_t b = blockIdx.x * (kHeadThreads / 32) + warp; b < B; b += warps_total) {
-        const uint16_t* row = reinterpret_cast<const uint16_t*>(x_h) + (uint64_t)b * p_act;
-        float mx = -3.0e38f;
+    for (uint32_t b = blockIdx.x * (kHeadThreads / 32) + warp; b < a.B; b += warps_total) {
+        const uint16_t* row = reinterpret_cast<const uint16_t*>(a.x_h) + (uint64_t)b * a.p_act;
+        const float* row_f = a.x_f32 + (uint64_t)b * a.p_f32;
         for (uint32_t o = lane; o < OUT; o += 32) {
             float acc = 0.0f;
-            for (uint32_t j = 0; j < H2; ++j) acc += ptx::from_operand(row[j], bf16) * weight(j, o);
-            const float y = acc + b_out[o];
-            s_dy[o] = y;
-            mx = fmaxf(mx, y);
+            for (uint32_t j = 0; j < H2; ++j) acc += (kF32 ? row_f[j] : ptx::from_operand(row[j], a.bf16)) * weight(j, o);
+            s_dy[o] = acc + a.b_out[o];
         }
-        float log_sum = 0.0f;
-        uint32_t cls = 0;
-        if (kCrossEntropy) {
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFU, mx, o));
-            __syncwarp();
-            float sum = 0.0f;
-            for (uint32_t o = lane; o < OUT; o += 32) sum += expf(s_dy[o] - mx);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFU, sum, o);
-            log_sum = logf(sum) + mx;
-            // a depth outside 1..OUT cannot come from the walk generator with k_max <= OUT; clamp instead of reading out of bounds
-            const int c = __float2int_rn(labels[(uint64_t)b * OUT]) - 1;
-            cls = static_cast<uint32_t>(c < 0 ? 0 : (c >= static_cast<int>(OUT) ? static_cast<int>(OUT) - 1 : c));
-        }
-        for (uint32_t o = lane; o < OUT; o += 32) {
-            const float y = s_dy[o];
-            float d;
-            if (kCrossEntropy) {
-                d = (expf(y - log_sum) - (o == cls ? 1.0f : 0.0f)) * inv_n;
-                if (o == cls) loss += (log_sum - y) * inv_n;
-            } else {
-                const float diff = y - labels[(uint64_t)b * OUT + o];
-                d = 2.0f * diff * inv_n;
-                loss += diff * diff * inv_n;
-            }
-            dy[(uint64_t)b * OUT + o] = d;
-            const uint16_t dh = ptx::to_operand(d, bf16);
-            reinterpret_cast<uint16_t*>(dy_h)[(uint64_t)b * p_dy + o] = dh;
-            s_dy[o] = ptx::from_operand(dh, bf16);
-        }
+        __syncwarp();
+        HeadLossRow<kCrossEntropy, kF32, 1>(a, b, inv_n, s_dy, lane, loss, none);
         __syncwarp();
 #pragma unroll
         for (int q = 0; q < kHeadMaxPerLane; ++q) {
@@ -658,10 +834,10 @@ HeadOutNKernel(const __half* __restrict__ w_out_h, uint32_t p_wout, const float*
             if (j < H2) {
                 float acc = 0.0f;
                 for (uint32_t o = 0; o < OUT; ++o) acc += s_dy[o] * weight(j, o);
-                const float d = x_f32[(uint64_t)b * p_f32 + j] > 0.0f ? acc : 0.0f;
+                const float d = row_f[j] > 0.0f ? acc : 0.0f;
                 dacc[q] += d;
-                dzf[(uint64_t)b * p_f32 + j] = d;
-                reinterpret_cast<uint16_t*>(dz_h)[(uint64_t)b * p_dz + j] = ptx::to_operand(d, bf16);
+                a.dzf[(uint64_t)b * a.p_f32 + j] = d;
+                if (!kF32) reinterpret_cast<uint16_t*>(a.dz_h)[(uint64_t)b * a.p_dz + j] = ptx::to_operand(d, a.bf16);
             }
         }
         __syncwarp();
@@ -679,7 +855,32 @@ HeadOutNKernel(const __half* __restrict__ w_out_h, uint32_t p_wout, const float*
     for (uint32_t j = threadIdx.x; j < H2 + 1; j += kHeadThreads) {
         float sum = 0.0f;
         for (int wi = 0; wi < kHeadThreads / 32; ++wi) sum += s_part[wi][j];
-        partials[(uint64_t)blockIdx.x * (H2 + 1) + j] = sum;
+        a.partials[(uint64_t)blockIdx.x * (1U + H2 + OUT) + j] = sum;
+    }
+}
+
+// The partial rows of the head with several outputs: item 0 -> loss, items [1, H2] -> the bias gradient of the layer below,
+// items (H2, H2 + OUT] -> grad b_out. Same order of additions as ReduceRowsKernel.
+__global__ void __launch_bounds__(256)
+ReduceHeadNKernel(const float* __restrict__ src, uint32_t rows, uint32_t H2, uint32_t row_floats, uint32_t items, float* __restrict__ loss, float* __restrict__ bias_below,
+                  float* __restrict__ grad_b) {
+    __shared__ float s_part[32][kReduceCols + 1];
+    const uint32_t cl = threadIdx.x & (kReduceCols - 1U), g = threadIdx.x / kReduceCols;
+    const uint32_t c = blockIdx.x * kReduceCols + cl;
+    float sum = 0.0f;
+    if (c < items) {
+#pragma unroll 4
+        for (uint32_t r = g; r < rows; r += 32U) sum += src[(uint64_t)r * row_floats + c];
+    }
+    s_part[g][cl] = sum;
+    __syncthreads();
+    if (g == 0 && c < items) {
+        float total = s_part[0][cl];
+#pragma unroll
+        for (int q = 1; q < 32; ++q) total += s_part[q][cl];
+        if (c == 0U) *loss = total;
+        else if (c <= H2) bias_below[c - 1U] = total;
+        else grad_b[c - 1U - H2] = total;
     }
 }
 
@@ -697,6 +898,31 @@ HeadOutNBiasGradKernel(const float* __restrict__ dy, uint32_t B, uint32_t OUT, f
         __syncthreads();
     }
     if (threadIdx.x == 0) grad_b[o] = s_sum[0];
+}
+
+// Output layer with several outputs, its loss and the gradient entering the layer below, enqueued; all gradients of the head
+// except W_out's, which is a product over the batch.
+template <bool kCrossEntropy, bool kF32>
+mgt_status_t LaunchHeadN(mgt_engine* e, cudaStream_t st, const HeadArgs& a, float* loss, float* bias_below, float* grad_b) {
+    const bool tiled = a.OUT <= 64U;
+    const uint32_t tiles = tiled ? (a.B + kHeadTile - 1U) / kHeadTile : (a.B + 7U) / 8U;
+    const uint32_t grid = tiles < kHeadBlocks ? tiles : kHeadBlocks;
+    auto run = [&](auto kernel, size_t smem) -> bool {
+        if (smem > 48U * 1024U && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return false;
+        kernel<<<grid, kHeadThreads, smem, st>>>(a);
+        return true;
+    };
+    bool ok;
+    if (a.OUT <= 16U) ok = run(HeadTileKernel<16, kCrossEntropy, kF32>, HeadTileSmem<16>(a.H2));
+    else if (a.OUT <= 32U) ok = run(HeadTileKernel<32, kCrossEntropy, kF32>, HeadTileSmem<32>(a.H2));
+    else if (tiled) ok = run(HeadTileKernel<64, kCrossEntropy, kF32>, HeadTileSmem<64>(a.H2));
+    else ok = run(HeadOutNKernel<kCrossEntropy, kF32>, (kHeadThreads / 32) * a.OUT * sizeof(float));
+    if (!ok) return MGT_CUDA_FAILURE;
+    const uint32_t items = tiled ? 1U + a.H2 + a.OUT : 1U + a.H2;
+    ReduceHeadNKernel<<<(items + kReduceCols - 1U) / kReduceCols, 256, 0, st>>>(a.partials, grid, a.H2, 1U + a.H2 + a.OUT, items, loss, bias_below, grad_b);
+    if (!tiled) HeadOutNBiasGradKernel<<<a.OUT, 256, 0, st>>>(a.dy, a.B, a.OUT, grad_b);
+    e->launches += tiled ? 2 : 3;
+    return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
 }
 
 inline uint32_t GridFor(uint64_t items, uint32_t threads, int sm_count) {
@@ -886,18 +1112,19 @@ mgt_status_t GemmGradWeightsRows(mgt_engine* e, cudaStream_t st, const __half* a
 
 // dxT[N_in x samples] = (W[N_in x K] * dz[samples x K]^T) * [mask bit]: the hidden layer's dX with its wide side as rows; the
 // mask words are the ones the embedding forward wrote beside its activation.
-// Row sums of the result (the bias gradient of the layer below) are reduced into bias_grad[N_in] in a fixed order.
+// Row sums of the result (the bias gradient of the layer below) are reduced into bias_grad[N_in] in a fixed order. With
+// dx_f32 the result goes there instead, in fp32 and with one row per sample.
 mgt_status_t GemmBackpropInputRows(mgt_engine* e, cudaStream_t st, const __half* w, uint32_t w_pitch, const __half* dz, uint32_t dz_pitch, uint32_t samples,
-                                   uint32_t in_dim, uint32_t out_dim, uint32_t* mask_bits, uint32_t ld_bits, __half* dx_t, uint32_t t_pitch, float* rowsum,
+                                   uint32_t in_dim, uint32_t out_dim, uint32_t* mask_bits, uint32_t ld_bits, __half* dx_t, uint32_t t_pitch, float* dx_f32, uint32_t f32_pitch, float* rowsum,
                                    uint64_t rowsum_rows, float* bias_grad) {
     GemmArgs a = BaseArgs(in_dim, samples, out_dim, CfgDxRows::BN, 1);
     const uint64_t rows = (uint64_t)a.n_tiles * CfgDxRows::EPI_STRIDE;
     if (rows > rowsum_rows) return MGT_CAPACITY_EXCEEDED;
-    a.bits = mask_bits; a.ld_bits = ld_bits; a.out_f16 = dx_t; a.ld_f16 = t_pitch; a.rowsum = rowsum;
+    a.bits = mask_bits; a.ld_bits = ld_bits; a.out_f16 = dx_t; a.ld_f16 = t_pitch; a.out_f32 = dx_f32; a.ld_f32 = f32_pitch; a.rowsum = rowsum;
     CUtensorMap ta, tb;
     MGT_MAP(e->Map(&ta, w, out_dim, in_dim, w_pitch, 64, 128));
     MGT_MAP(e->Map(&tb, dz, out_dim, samples, dz_pitch, 64, CfgDxRows::BN));
-    MGT_TRY(LaunchGemm<CfgDxRows>(e, ta, tb, a, st));
+    MGT_TRY(dx_f32 != nullptr ? LaunchGemm<CfgDxRowsF32>(e, ta, tb, a, st) : LaunchGemm<CfgDxRows>(e, ta, tb, a, st));
     ReduceRowsKernel<<<(in_dim + kReduceCols - 1) / kReduceCols, 256, 0, st>>>(rowsum, (uint32_t)rows, in_dim, 0, in_dim, bias_grad);
     ++e->launches;
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
@@ -935,112 +1162,170 @@ mgt_status_t LaunchChain(mgt_engine* e, cudaStream_t st, const __half* w_first, 
 }
 
 // ---- the fp32 data flow (use_half_linear == 0), mlp_backward.cu:1273-1510 without the fp16 copies -----------------
+// Every activation and every gradient w.r.t. a pre-activation is kept (as in the tensor-core flow), so that the weight
+// gradients of all blocks are two grouped products at the end. Rows are padded to four floats.
 struct Fp32Workspace {
-    uint64_t a1, x, r1, z, y, dy, d0, d1, dz1, lossp, total;  // float offsets
+    uint32_t p1, p2;
+    uint64_t a1, x, r1, dz2, dz1t, dz1, dy, head, partial, colsum, colsum_slot, colsum_in, lists, total;  // float offsets
 };
-Fp32Workspace PlanFp32(const mgt_mlp_shape_t& s, uint32_t B) {
+struct DwPlan {
+    fp32path::SgemmTile tile;
+    uint32_t splits;
+};
+// Weight gradients: few tiles, a long sum over the batch. Enough K splits for eight CTAs of the middle tile per SM, as long as
+// a split keeps 256 samples (16 products of 224 x 224 over 8 192 samples: 3, 6, 9 splits 428, 380, 365 us).
+DwPlan PlanDw(uint32_t M, uint32_t N, uint32_t K, uint32_t groups, uint32_t sm) {
+    DwPlan p{M > 32U && N > 32U ? fp32path::SgemmTile::kMiddle : fp32path::SgemmTile::kSmall, 1U};
+    const uint32_t t = fp32path::SgemmTileRows(p.tile);
+    const uint64_t tiles = (uint64_t)((M + t - 1) / t) * ((N + t - 1) / t) * groups;
+    const uint64_t want = (8ULL * sm + tiles - 1) / tiles, most = K / 256U > 0U ? K / 256U : 1U;
+    p.splits = (uint32_t)(want < most ? want : most);
+    return p;
+}
+Fp32Workspace PlanFp32(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm) {
     Fp32Workspace w{};
     uint64_t off = 0;
     auto take = [&](uint64_t n) { const uint64_t at = off; off += (n + 63) & ~63ULL; return at; };
-    const uint64_t bh2 = (uint64_t)B * s.hd2, bh1 = (uint64_t)B * s.hd1;
+    w.p1 = (uint32_t)RoundUp(s.hd1, 4);
+    w.p2 = (uint32_t)RoundUp(s.hd2, 4);
+    const uint64_t bh2 = (uint64_t)B * w.p2, bh1 = (uint64_t)B * w.p1, r = s.residual_blocks > 0 ? s.residual_blocks : 1ULL;
     w.a1 = take(bh1);
     w.x = take(bh2 * (s.residual_blocks + 1ULL));
-    w.r1 = take(bh2 * (s.residual_blocks > 0 ? s.residual_blocks : 1ULL));
-    w.z = take(bh2);
-    w.y = take((uint64_t)B * s.output_dim);
-    w.dy = take((uint64_t)B * s.output_dim);
-    w.d0 = take(bh2);
-    w.d1 = take(bh2);
+    w.r1 = take(bh2 * r);
+    w.dz2 = take(bh2 * (s.residual_blocks + 1ULL));
+    w.dz1t = take(bh2 * r);
     w.dz1 = take(bh1);
-    w.lossp = take(1024);
+    w.dy = take((uint64_t)B * s.output_dim);
+    w.head = take((uint64_t)kHeadBlocks * HeadPartialFloats(s));
+    auto planes = [&](uint32_t M, uint32_t N, uint32_t groups) { return (uint64_t)PlanDw(M, N, B, groups, sm).splits * groups * M * N; };
+    const uint64_t p_hidden = planes(s.hd1, s.hd2, 1), p_block = planes(s.hd2, s.hd2, (uint32_t)r), p_out = planes(s.hd2, s.output_dim, 1);
+    w.partial = take(std::max(p_hidden, std::max(p_block, p_out)));
+    w.colsum_slot = (uint64_t)((B + 31U) / 32U) * s.hd2;  // one row per tile of at least 32 samples
+    w.colsum = take(w.colsum_slot * 2 * r);
+    w.colsum_in = take((uint64_t)((B + 31U) / 32U) * s.hd1);
+    w.lists = take(fp32path::EmbeddingGradListWords(B, s.state_len, s.state_value_pad));
     w.total = off + 64;
     return w;
 }
-uint64_t Fp32WorkspaceFloats(const mgt_mlp_shape_t& s, uint32_t B) { return PlanFp32(s, B).total; }
+uint64_t Fp32WorkspaceFloats(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm) { return PlanFp32(s, B, sm).total; }
 
 template <class F>
 mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float* w, const uint8_t* states, const float* labels, uint32_t B, float* loss,
                             float* grad, float* workspace, bool half_ig, mgt_backward_profile_t* profile, F&& notify, cudaStream_t st) {
     using namespace mgt::fp32path;
-    const Fp32Workspace ws = PlanFp32(s, B);
+    const uint32_t sm = PlanSmCount(e->sm_count);
+    const Fp32Workspace ws = PlanFp32(s, B, sm);
     float* base = reinterpret_cast<float*>(RoundUp(reinterpret_cast<uintptr_t>(workspace), 256));
-    const uint32_t H1 = s.hd1, H2 = s.hd2, R = s.residual_blocks, OUT = s.output_dim, L = s.state_len, V = s.state_value_pad;
-    const uint64_t bh2 = (uint64_t)B * H2, bh1 = (uint64_t)B * H1;
+    const uint32_t H1 = s.hd1, H2 = s.hd2, R = s.residual_blocks, OUT = s.output_dim, L = s.state_len, V = s.state_value_pad, p1 = ws.p1, p2 = ws.p2;
+    const uint64_t bh2 = (uint64_t)B * p2;
     float* a1 = base + ws.a1;
     auto x = [&](uint32_t k) { return base + ws.x + bh2 * k; };
     auto r1 = [&](uint32_t k) { return base + ws.r1 + bh2 * k; };
-    float *z = base + ws.z, *y = base + ws.y, *dy = base + ws.dy, *d0 = base + ws.d0, *d1 = base + ws.d1, *dz1 = base + ws.dz1, *lossp = base + ws.lossp;
-    const int sm = e->sm_count;
-    auto blocks = [&](uint64_t n) { return GridFor(n, 256, sm); };
+    auto dz2 = [&](uint32_t k) { return base + ws.dz2 + bh2 * k; };    // [0] hidden layer, [k + 1] fc2 of block k
+    auto dz1t = [&](uint32_t k) { return base + ws.dz1t + bh2 * k; };  // fc1 of block k
+    float *dy = base + ws.dy, *dz1 = base + ws.dz1, *partial = base + ws.partial, *colsum = base + ws.colsum;
+    const SgemmTile tile_h2 = PickSgemmTile(B, H2, 1, sm), tile_h1 = PickSgemmTile(B, H1, 1, sm);
+    const uint32_t rows_h2 = (B + SgemmTileRows(tile_h2) - 1U) / SgemmTileRows(tile_h2), rows_h1 = (B + SgemmTileRows(tile_h1) - 1U) / SgemmTileRows(tile_h1);
     auto ok = [&]() { return cudaGetLastError() == cudaSuccess; };
-    auto colsum = [&](const float* src, uint32_t cols, float* dst) {
-        ColumnSumKernel<<<(cols + 7) / 8, 256, 0, st>>>(src, B, cols, dst);
+    // out[B x N] = act[B x K] W[K x N] + bias, ReLU (with the residual added before it)
+    auto forward = [&](const float* act, uint32_t ld_act, uint32_t K, const float* weight, const float* bias, const float* res, float* out) {
+        SgemmArgs a{};
+        a.A = act; a.lda = ld_act; a.B = weight; a.ldb = H2; a.C = out; a.ldc = p2; a.M = B; a.N = H2; a.K = K; a.splits = 1; a.bias = bias; a.add = res; a.ld_add = p2; a.relu = 1U;
         ++e->launches;
+        return Sgemm<false, false>(st, a, 1, tile_h2) == cudaSuccess;
+    };
+    // out[B x N] = (dz[B x H2] W[N x H2]^T (+ skip)) * [act > 0], with its column sums per tile
+    auto backward = [&](const float* dz, const float* weight, uint32_t N, const float* skip, const float* act, uint32_t ld, float* out, float* sums, SgemmTile tile) {
+        SgemmArgs a{};
+        a.A = dz; a.lda = p2; a.B = weight; a.ldb = H2; a.C = out; a.ldc = ld; a.M = B; a.N = N; a.K = H2; a.splits = 1; a.add = skip; a.ld_add = ld; a.mask = act; a.ld_mask = ld;
+        a.colsum = sums;
+        ++e->launches;
+        return Sgemm<false, true>(st, a, 1, tile) == cudaSuccess;
+    };
+    // grad_g[M x N] = act_g^T dz_g over the batch
+    auto weight_grad = [&](const float* act, uint32_t ld_act, uint64_t act_stride, uint32_t M, const float* dz, uint32_t ld_dz, uint64_t dz_stride, uint32_t N, uint32_t groups,
+                           float* out, uint64_t out_stride) {
+        const DwPlan plan = PlanDw(M, N, B, groups, sm);
+        SgemmArgs a{};
+        a.A = act; a.lda = ld_act; a.stride_a = act_stride; a.B = dz; a.ldb = ld_dz; a.stride_b = dz_stride; a.M = M; a.N = N; a.K = B; a.splits = plan.splits;
+        a.C = plan.splits > 1U ? partial : out; a.ldc = N; a.stride_c = out_stride;
+        if (Sgemm<true, false>(st, a, groups, plan.tile) != cudaSuccess) return false;
+        ++e->launches;
+        if (plan.splits > 1U) {
+            const uint64_t count = (uint64_t)M * N;
+            const dim3 grid(GridFor(count, 256, e->sm_count) / (groups > 4 ? 4 : 1) + 1, groups);
+            ReducePartialsGroupedKernel<<<grid, 256, 0, st>>>(partial, plan.splits, count, out, out_stride);
+            ++e->launches;
+        }
+        return ok();
     };
     StageTimer timer{e, st, profile};
     if (!timer.Start()) return MGT_CUDA_FAILURE;
 
-    InputForwardKernel<<<blocks(bh1), 256, 0, st>>>(states, w, w + InputBias(s), B, L, V, H1, a1);
+    if (EmbeddingForward(st, states, w, w + InputBias(s), B, L, V, H1, a1, p1, sm) != cudaSuccess) return MGT_CUDA_FAILURE;
     ++e->launches;
-    if (!ok() || !timer.Mark(profile ? &profile->input_forward_ms : nullptr)) return MGT_CUDA_FAILURE;
-    // hidden layer and residual blocks (y = x W, weights row-major [in][out])
-    if (Sgemm<false, false>(st, B, H2, H1, a1, H1, w + HiddenWeight(s), H2, z, H2) != cudaSuccess) return MGT_CUDA_FAILURE;
-    BiasReluKernel<<<blocks(bh2), 256, 0, st>>>(z, w + HiddenBias(s), nullptr, H2, bh2, x(0));
-    e->launches += 2;
-    if (!ok() || !timer.Mark(profile ? &profile->hidden_forward_ms : nullptr)) return MGT_CUDA_FAILURE;
+    if (!timer.Mark(profile ? &profile->input_forward_ms : nullptr)) return MGT_CUDA_FAILURE;
+    if (!forward(a1, p1, H1, w + HiddenWeight(s), w + HiddenBias(s), nullptr, x(0))) return MGT_CUDA_FAILURE;
+    if (!timer.Mark(profile ? &profile->hidden_forward_ms : nullptr)) return MGT_CUDA_FAILURE;
     for (uint32_t k = 0; k < R; ++k) {
-        if (Sgemm<false, false>(st, B, H2, H2, x(k), H2, w + Fc1W(s, k), H2, z, H2) != cudaSuccess) return MGT_CUDA_FAILURE;
-        BiasReluKernel<<<blocks(bh2), 256, 0, st>>>(z, w + Fc1B(s, k), nullptr, H2, bh2, r1(k));
-        if (Sgemm<false, false>(st, B, H2, H2, r1(k), H2, w + Fc2W(s, k), H2, z, H2) != cudaSuccess) return MGT_CUDA_FAILURE;
-        BiasReluKernel<<<blocks(bh2), 256, 0, st>>>(z, w + Fc2B(s, k), x(k), H2, bh2, x(k + 1));
-        e->launches += 4;
+        if (!forward(x(k), p2, H2, w + Fc1W(s, k), w + Fc1B(s, k), nullptr, r1(k)) || !forward(r1(k), p2, H2, w + Fc2W(s, k), w + Fc2B(s, k), x(k), x(k + 1U))) return MGT_CUDA_FAILURE;
     }
-    if (!ok() || !timer.Mark(profile ? &profile->residual_forward_ms : nullptr)) return MGT_CUDA_FAILURE;
-    // output layer, loss, dL/dy, gradients of the output layer, gradient entering the tower
-    const uint64_t by = (uint64_t)B * OUT;
-    if (Sgemm<false, false>(st, B, OUT, H2, x(R), H2, w + OutputWeight(s), OUT, y, OUT) != cudaSuccess) return MGT_CUDA_FAILURE;
-    AddBiasKernel<<<blocks(by), 256, 0, st>>>(y, w + OutputBias(s), OUT, by);
-    const uint32_t loss_blocks = (uint32_t)(blocks(by) < 1024 ? blocks(by) : 1024);
-    LossKernel<<<loss_blocks, 256, 0, st>>>(y, labels, by, 1.0f / (float)by, dy, lossp);
-    FinishLossKernel<<<1, 32, 0, st>>>(lossp, loss_blocks, loss);
-    if (Sgemm<true, false>(st, H2, OUT, B, x(R), H2, dy, OUT, grad + OutputWeight(s), OUT) != cudaSuccess) return MGT_CUDA_FAILURE;
-    colsum(dy, OUT, grad + OutputBias(s));
-    if (Sgemm<false, true>(st, B, H2, OUT, dy, OUT, w + OutputWeight(s), OUT, d0, H2) != cudaSuccess) return MGT_CUDA_FAILURE;
-    e->launches += 6;
+    if (!timer.Mark(profile ? &profile->residual_forward_ms : nullptr)) return MGT_CUDA_FAILURE;
+    // output layer, loss, and the masked gradient entering the tower with its column sums
+    float* head_bias_dst = grad + (R > 0 ? Fc2B(s, R - 1) : HiddenBias(s));
+    if (OUT == 1U) {
+        const uint32_t grid = (B + 7U) / 8U < kHeadBlocks ? (B + 7U) / 8U : kHeadBlocks;
+        HeadOut1Kernel<<<grid, kHeadThreads, 0, st>>>(w + OutputWeight(s), w + OutputBias(s), labels, x(R), p2, B, H2, dz2(R), nullptr, 0, base + ws.head, false);
+        ReduceHeadKernel<<<(2 * H2 + 2 + kReduceCols - 1) / kReduceCols, 256, 0, st>>>(base + ws.head, grid, H2, grad + OutputWeight(s), loss, head_bias_dst);
+        e->launches += 2;
+    } else {
+        const HeadArgs h{w + OutputWeight(s), OUT, w + OutputBias(s), labels, nullptr, 0, x(R), p2, B, H2, OUT, dy, nullptr, 0, dz2(R), nullptr, 0, base + ws.head, false};
+        MGT_TRY(LaunchHeadN<false, true>(e, st, h, loss, head_bias_dst, grad + OutputBias(s)));
+        if (!weight_grad(x(R), p2, 0, H2, dy, OUT, 0, OUT, 1, grad + OutputWeight(s), 0)) return MGT_CUDA_FAILURE;
+    }
+    if (!ok()) return MGT_CUDA_FAILURE;
     MGT_TRY(notify(OutputWeight(s), (uint64_t)H2 * OUT + OUT));
-    if (!ok() || !timer.Mark(profile ? &profile->output_ms : nullptr)) return MGT_CUDA_FAILURE;
-    // residual blocks backward: d0 holds dL/dx_{k+1}
+    if (!timer.Mark(profile ? &profile->output_ms : nullptr)) return MGT_CUDA_FAILURE;
+    // input gradients down the tower and through the hidden layer
     for (uint32_t rb = R; rb > 0; --rb) {
         const uint32_t k = rb - 1U;
-        MaskKernel<float><<<blocks(bh2), 256, 0, st>>>(d0, nullptr, x(k + 1), H2, H2, bh2, false, d0);  // dz2, in place
-        colsum(d0, H2, grad + Fc2B(s, k));
-        if (Sgemm<true, false>(st, H2, H2, B, r1(k), H2, d0, H2, grad + Fc2W(s, k), H2) != cudaSuccess) return MGT_CUDA_FAILURE;
-        if (Sgemm<false, true>(st, B, H2, H2, d0, H2, w + Fc2W(s, k), H2, z, H2) != cudaSuccess) return MGT_CUDA_FAILURE;
-        MGT_TRY(notify(Fc2W(s, k), (uint64_t)H2 * H2 + H2));  // after the last reader of W2_k
-        MaskKernel<float><<<blocks(bh2), 256, 0, st>>>(z, nullptr, r1(k), H2, H2, bh2, false, d1);       // dz1 of the block
-        colsum(d1, H2, grad + Fc1B(s, k));
-        if (Sgemm<true, false>(st, H2, H2, B, x(k), H2, d1, H2, grad + Fc1W(s, k), H2) != cudaSuccess) return MGT_CUDA_FAILURE;
-        if (Sgemm<false, true>(st, B, H2, H2, d1, H2, w + Fc1W(s, k), H2, z, H2) != cudaSuccess) return MGT_CUDA_FAILURE;
-        MGT_TRY(notify(Fc1W(s, k), (uint64_t)H2 * H2 + H2));
-        AddIntoKernel<<<blocks(bh2), 256, 0, st>>>(d0, z, bh2);  // dL/dx_k = dz2 + dz1 W1^T
-        e->launches += 7;
+        if (!backward(dz2(k + 1U), w + Fc2W(s, k), H2, nullptr, r1(k), p2, dz1t(k), colsum + ws.colsum_slot * k, tile_h2) ||
+            !backward(dz1t(k), w + Fc1W(s, k), H2, dz2(k + 1U), x(k), p2, dz2(k), colsum + ws.colsum_slot * (R + k), tile_h2)) return MGT_CUDA_FAILURE;
+    }
+    if (!timer.Mark(profile ? &profile->residual_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
+    if (!backward(dz2(0), w + HiddenWeight(s), H1, nullptr, a1, p1, dz1, base + ws.colsum_in, tile_h1)) return MGT_CUDA_FAILURE;
+    // the input-bias gradient sums the fp32 dz1 (mlp_backward.cu:1505)
+    ReduceRowsKernel<<<(H1 + kReduceCols - 1) / kReduceCols, 256, 0, st>>>(base + ws.colsum_in, rows_h1, H1, 0, H1, grad + InputBias(s));
+    ++e->launches;
+    if (half_ig) {
+        RoundHalfKernel<<<GridFor((uint64_t)B * p1, 256, e->sm_count), 256, 0, st>>>(dz1, (uint64_t)B * p1);
+        ++e->launches;
+    }
+    if (!ok() || !timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
+    if (EmbeddingGrad(st, states, dz1, p1, B, L, V, H1, reinterpret_cast<uint32_t*>(base + ws.lists), grad) != cudaSuccess) return MGT_CUDA_FAILURE;
+    e->launches += 2;
+    if (!timer.Mark(profile ? &profile->input_grad_ms : nullptr)) return MGT_CUDA_FAILURE;
+    // weight gradients of all blocks and of the hidden layer, bias gradients from the column sums
+    if (R > 0) {
+        if (!weight_grad(r1(0), p2, bh2, H2, dz2(1), p2, bh2, H2, R, grad + Fc2W(s, 0), BlockParams(s)) ||
+            !weight_grad(x(0), p2, bh2, H2, dz1t(0), p2, bh2, H2, R, grad + Fc1W(s, 0), BlockParams(s))) return MGT_CUDA_FAILURE;
+        ReduceDestinations dst{};
+        for (uint32_t k = 0; k < R; ++k) {
+            dst.offset[k] = Fc1B(s, k);
+            dst.offset[R + k] = k > 0 ? Fc2B(s, k - 1) : HiddenBias(s);
+        }
+        ReduceRowsGroupedKernel<<<dim3((H2 + kReduceCols - 1) / kReduceCols, 2 * R), 256, 0, st>>>(colsum, rows_h2, H2, ws.colsum_slot, grad, dst);
+        ++e->launches;
+        for (uint32_t rb = R; rb > 0; --rb) {
+            MGT_TRY(notify(Fc2W(s, rb - 1U), (uint64_t)H2 * H2 + H2));
+            MGT_TRY(notify(Fc1W(s, rb - 1U), (uint64_t)H2 * H2 + H2));
+        }
     }
     if (!ok() || !timer.Mark(profile ? &profile->residual_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
-    // hidden layer backward
-    MaskKernel<float><<<blocks(bh2), 256, 0, st>>>(d0, nullptr, x(0), H2, H2, bh2, false, d0);  // dzh
-    colsum(d0, H2, grad + HiddenBias(s));
-    if (Sgemm<true, false>(st, H1, H2, B, a1, H1, d0, H2, grad + HiddenWeight(s), H2) != cudaSuccess) return MGT_CUDA_FAILURE;
-    if (Sgemm<false, true>(st, B, H1, H2, d0, H2, w + HiddenWeight(s), H2, dz1, H1) != cudaSuccess) return MGT_CUDA_FAILURE;
+    if (!weight_grad(a1, p1, 0, H1, dz2(0), p2, 0, H2, 1, grad + HiddenWeight(s), 0)) return MGT_CUDA_FAILURE;
     MGT_TRY(notify(HiddenWeight(s), (uint64_t)H1 * H2 + H2));
-    MaskKernel<float><<<blocks(bh1), 256, 0, st>>>(dz1, nullptr, a1, H1, H1, bh1, false, dz1);
-    colsum(dz1, H1, grad + InputBias(s));  // the reference sums the fp32 dz1 (mlp_backward.cu:1505)
-    if (half_ig) MaskKernel<float><<<blocks(bh1), 256, 0, st>>>(dz1, nullptr, a1, H1, H1, bh1, true, dz1);  // fp16 operand of the embedding gradient
-    e->launches += 5;
-    if (!ok() || !timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
-    EmbeddingGradKernel<float><<<dim3(L, (H1 + 63) / 64), 128, 2ULL * V * 64 * sizeof(float), st>>>(states, dz1, H1, B, V, H1, grad);
-    ++e->launches;
+    if (!timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
     MGT_TRY(notify(0, (uint64_t)L * V * H1 + H1));
-    if (!ok() || !timer.Mark(profile ? &profile->input_grad_ms : nullptr)) return MGT_CUDA_FAILURE;
     return MGT_OK;
 }
 
@@ -1132,14 +1417,18 @@ mgt_status_t mgt_engine_check(mgt_engine_t* e, void* stream, int32_t* out_device
     return MGT_OK;
 }
 
+// The fp32 operand of the table gradient behind the tensor-core workspace: dz1 [samples][hd1], rows padded to four floats,
+// then the sample lists of its classes (and slack to align the start).
+static uint64_t Fp32TableFloats(const mgt_mlp_shape_t& s, uint32_t B) {
+    return (uint64_t)B * RoundUp(s.hd1, 4) + fp32path::EmbeddingGradListWords(B, s.state_len, s.state_value_pad) + 64;
+}
+
 static uint64_t WorkspaceFloats(const mgt_mlp_shape_t* shape, uint32_t sample_count, uint32_t chunks, int32_t use_half_input_grad, int32_t use_half_linear,
                                 bool batch_norm) {
     if (!ValidShape(shape) || sample_count == 0 || chunks == 0) return 0;
-    if (!use_half_linear) return batch_norm ? 0 : Fp32WorkspaceFloats(*shape, sample_count);
+    if (!use_half_linear) return batch_norm ? 0 : Fp32WorkspaceFloats(*shape, sample_count, CurrentDeviceSmCount());
     const Workspace w = PlanWorkspace(*shape, sample_count, CurrentDeviceSmCount(), batch_norm);
-    // fp32 embedding-gradient operand: da1 and dz1 [samples][hd1] in fp32 behind the tensor-core workspace
-    const uint64_t extra = use_half_input_grad ? 0 : 2ULL * sample_count * shape->hd1;
-    return (w.total_bytes + 3) / 4 + extra + (extra ? 256 : 0);
+    return (w.total_bytes + 3) / 4 + (use_half_input_grad ? 0 : Fp32TableFloats(*shape, sample_count));
 }
 
 uint64_t mgt_mlp_loss_grad_workspace_floats(const mgt_mlp_shape_t* shape, uint32_t sample_count, uint32_t chunks,
@@ -1189,7 +1478,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     e->bf16_now = half_lin && e->options.operand_format == MGT_OPERAND_BF16;
     if (!half_lin) {
         // fp32 linear layers: the CUDA-core path (fp32_path.cuh); half_ig only selects the rounding of its embedding-gradient operand
-        if (workspace_floats < Fp32WorkspaceFloats(s, B)) return MGT_CAPACITY_EXCEEDED;
+        if (workspace_floats < Fp32WorkspaceFloats(s, B, PlanSmCount(e->sm_count))) return MGT_CAPACITY_EXCEEDED;
         uint32_t id = 0;
         auto tell = [&](uint64_t off, uint64_t count) -> mgt_status_t {
             if (ready == nullptr) return MGT_OK;
@@ -1199,12 +1488,11 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
                               static_cast<cudaStream_t>(stream_v));
     }
     const Workspace ws = PlanWorkspace(s, B, PlanSmCount(e->sm_count), bnorm);
-    const uint64_t f32_extra = half_ig ? 0 : 2ULL * B * s.hd1;  // da1, dz1 in fp32 for the fp32 embedding gradient
-    if (workspace_floats < (ws.total_bytes + 3) / 4 + f32_extra + (f32_extra ? 256 : 0)) return MGT_CAPACITY_EXCEEDED;
+    if (workspace_floats < (ws.total_bytes + 3) / 4 + (half_ig ? 0 : Fp32TableFloats(s, B))) return MGT_CAPACITY_EXCEEDED;
     cudaStream_t st = static_cast<cudaStream_t>(stream_v);
     uint8_t* base = reinterpret_cast<uint8_t*>(RoundUp(reinterpret_cast<uintptr_t>(workspace), 1024));
-    float* da1_f32 = reinterpret_cast<float*>(RoundUp(reinterpret_cast<uintptr_t>(workspace + (ws.total_bytes + 3) / 4), 256));  // behind the tensor-core workspace
-    float* dz1_f32 = da1_f32 + (uint64_t)B * s.hd1;
+    float* dz1_f32 = reinterpret_cast<float*>(RoundUp(reinterpret_cast<uintptr_t>(workspace + (ws.total_bytes + 3) / 4), 256));  // behind the tensor-core workspace
+    const uint32_t p_dz1_f32 = (uint32_t)RoundUp(s.hd1, 4);
     __half* a1_h = reinterpret_cast<__half*>(base + ws.off_a1);
     auto x_h = [&](uint32_t k) { return reinterpret_cast<__half*>(base + ws.off_x + ws.x_stride * k); };
     auto r1_h = [&](uint32_t k) { return reinterpret_cast<__half*>(base + ws.off_r1 + ws.r1_stride * k); };
@@ -1382,24 +1670,9 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     } else {
         float* dy = reinterpret_cast<float*>(base + ws.off_dy);
         __half* dy_h = reinterpret_cast<__half*>(base + ws.off_dyh);
-        const size_t warp_smem = (kHeadThreads / 32) * OUT * sizeof(float);
-        const size_t staged_smem = warp_smem + (size_t)H2 * (OUT | 1U) * sizeof(float);
-        const bool stage_w = staged_smem <= kHeadStagedSmemLimit;
-        const bool ce = e->options.loss_kind == MGT_LOSS_CROSS_ENTROPY;
-        auto launch_head = [&](auto kernel, size_t smem) -> bool {
-            if (smem > 48U * 1024U && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kHeadStagedSmemLimit) != cudaSuccess) return false;
-            kernel<<<kHeadBlocks, kHeadThreads, smem, st>>>(hw.wout, hw.pout, w + OutputBias(s), labels, x_h(R), ws.p_act, x_f32, ws.p_f32, B, H2, OUT, dy, dy_h, ws.p_wout,
-                                                           dzf, dz_cur, ws.p_dz, head_partial, e->bf16_now);
-            return true;
-        };
-        const bool launched = stage_w ? (ce ? launch_head(HeadOutNKernel<true, true>, staged_smem) : launch_head(HeadOutNKernel<false, true>, staged_smem))
-                                      : (ce ? launch_head(HeadOutNKernel<true, false>, warp_smem) : launch_head(HeadOutNKernel<false, false>, warp_smem));
-        if (!launched) return MGT_CUDA_FAILURE;
-        ReduceRowsKernel<<<1, 256, 0, st>>>(head_partial, kHeadBlocks, H2 + 1, 0, 1, loss);
-        ReduceRowsKernel<<<(H2 + kReduceCols - 1) / kReduceCols, 256, 0, st>>>(head_partial, kHeadBlocks, H2 + 1, 1, H2, head_bias_dst);
-        HeadOutNBiasGradKernel<<<OUT, 256, 0, st>>>(dy, B, OUT, grad + OutputBias(s));
-        e->launches += 4;
-        if (cudaGetLastError() != cudaSuccess) return MGT_CUDA_FAILURE;
+        const HeadArgs h{hw.wout, hw.pout, w + OutputBias(s), labels, x_h(R), ws.p_act, x_f32, ws.p_f32, B, H2, OUT, dy, dy_h, ws.p_wout, dzf, dz_cur, ws.p_dz, head_partial, e->bf16_now};
+        MGT_TRY(e->options.loss_kind == MGT_LOSS_CROSS_ENTROPY ? LaunchHeadN<true, false>(e, st, h, loss, head_bias_dst, grad + OutputBias(s))
+                                                               : LaunchHeadN<false, false>(e, st, h, loss, head_bias_dst, grad + OutputBias(s)));
         // grad W_out = x_R^T * dy (16-bit operands, fp32 accumulate, mlp_backward.cu:1349-1354): the split-K weight-gradient GEMM
         MGT_TRY(GemmGradWeights(e, st, x_h(R), ws.p_act, dy_h, ws.p_wout, B, H2, OUT, partial, ws.partial_floats, grad + OutputWeight(s)));
     }
@@ -1443,31 +1716,19 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     // ---- hidden layer backward, dX part (mlp_backward.cu:1417-1438): dz_tape(0) = dcur * [x0 > 0]
     dz_cur = dz_tape(0);
     if (bnorm) MGT_TRY(bn_backward(0, grad + HiddenBias(s)));
-    if (half_ig) {
-        // dz1T = (Wh * dzh^T) * [pre-activation of a1 > 0], the input-bias gradient from its row sums
-        MGT_TRY(GemmBackpropInputRows(e, st, hw.wh, hw.p2, dz_cur, ws.p_dz, B, H1, H2, reinterpret_cast<uint32_t*>(base + ws.off_bits_h1), ws.ld_bits_h1, dz1_h,
-                                      ws.p_bt, reinterpret_cast<float*>(base + ws.off_rowsum), ws.rowsum_rows, grad + InputBias(s)));
-    } else {
-        // --input-grad-fp16 0: the embedding gradient wants dz1 in fp32 (mlp_backward.cu:1433-1504, float one-hot GEMM).
-        // da1 from the same fp16 operands with fp32 accumulation, masked in fp32, then the table gradient on CUDA cores.
-        using namespace mgt::fp32path;
-        const uint64_t bh1 = (uint64_t)B * H1;
-        if (Sgemm<false, true>(st, B, H1, H2, dz_cur, ws.p_dz, hw.wh, hw.p2, da1_f32, H1) != cudaSuccess) return MGT_CUDA_FAILURE;
-        MaskKernel<__half><<<GridFor(bh1, 256, e->sm_count), 256, 0, st>>>(da1_f32, nullptr, a1_h, H1, ws.p_bt, bh1, false, dz1_f32, true);
-        ColumnSumKernel<<<(H1 + 7) / 8, 256, 0, st>>>(dz1_f32, B, H1, grad + InputBias(s));
-        e->launches += 3;
-        if (cudaGetLastError() != cudaSuccess) return MGT_CUDA_FAILURE;
-    }
+    // dz1T = (Wh * dzh^T) * [pre-activation of a1 > 0], the input-bias gradient from its row sums. With --input-grad-fp16 0 the
+    // embedding gradient wants dz1 in fp32 (mlp_backward.cu:1433-1504, float one-hot GEMM): the same product of fp16 operands
+    // with fp32 accumulation, written unrounded as rows of samples.
+    MGT_TRY(GemmBackpropInputRows(e, st, hw.wh, hw.p2, dz_cur, ws.p_dz, B, H1, H2, reinterpret_cast<uint32_t*>(base + ws.off_bits_h1), ws.ld_bits_h1, dz1_h,
+                                  ws.p_bt, half_ig ? nullptr : dz1_f32, p_dz1_f32, reinterpret_cast<float*>(base + ws.off_rowsum), ws.rowsum_rows, grad + InputBias(s)));
     if (!timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
 
     // ---- embedding gradient: grad W_in = onehot^T * dz1  (mlp_backward.cu:1440-1504); the input-bias
     // gradient (mlp_backward.cu:1505) is the column sum written by the GEMM above
     if (!half_ig) {
-        using namespace mgt::fp32path;
-        EmbeddingGradKernel<float><<<dim3(s.state_len, (H1 + 63) / 64), 128, 2ULL * s.state_value_pad * 64 * sizeof(float), st>>>(
-            reinterpret_cast<const uint8_t*>(states), dz1_f32, H1, B, s.state_value_pad, H1, grad);
-        ++e->launches;
-        if (cudaGetLastError() != cudaSuccess) return MGT_CUDA_FAILURE;
+        if (fp32path::EmbeddingGrad(st, reinterpret_cast<const uint8_t*>(states), dz1_f32, p_dz1_f32, B, s.state_len, s.state_value_pad, H1,
+                                    reinterpret_cast<uint32_t*>(dz1_f32 + (uint64_t)B * p_dz1_f32), grad) != cudaSuccess) return MGT_CUDA_FAILURE;
+        e->launches += 2;
     } else {
         const uint32_t unit_rows = CfgEmbGrad::NACC * CfgEmbGrad::BN;
         GemmArgs a = BaseArgs(H1, IN, B, unit_rows, 1);

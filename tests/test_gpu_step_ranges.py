@@ -100,3 +100,26 @@ def loss_grad_case(oracle, dims, n, *, seed=1, scale=0.03, mirror=True, options=
 @pytest.mark.parametrize("hd2,n,mirror", [(8, 130, True), (31, 127, False), (33, 129, False), (72, 300, True), (200, 257, True), (250, 128, False), (255, 400, True)])
 def test_residual_tower_widths(oracle, hd2, n, mirror):
     loss_grad_case(oracle, (72, 72, 48, hd2, 3, 1), n, mirror=mirror)
+
+
+# fp32 linear layers: the three tile sizes of the products, K splits, sizes that are no multiples of four, several outputs
+@pytest.mark.parametrize("dims,n", [((72, 72, 40, 24, 2, 1), 70), ((72, 72, 37, 19, 1, 1), 33), ((20, 6, 200, 136, 3, 1), 1500), ((72, 72, 132, 68, 2, 3), 517),
+                                     ((30, 30, 64, 40, 0, 5), 300), ((12, 5, 516, 260, 1, 1), 9700)])
+def test_fp32_linears_over_tiles(oracle, dims, n):
+    loss_grad_case(oracle, dims, n, flags=(False, False), tol=1e-5, section_tol=2e-5)
+
+
+# fp32 table gradient behind fp16 linears: classes without samples, one class per position, many samples per class
+@pytest.mark.parametrize("dims,n,mirror", [((72, 72, 36, 40, 1, 1), 45, True), ((54, 6, 130, 64, 2, 1), 1000, True), ((16, 1, 33, 24, 1, 2), 257, False)])
+def test_fp32_table_gradient(oracle, dims, n, mirror):
+    loss_grad_case(oracle, dims, n, flags=(False, True), mirror=mirror)
+
+
+# output head: the widths of its tile (16, 32, 64) and the per-sample form beyond them, tiles of 64 samples
+@pytest.mark.parametrize("outputs,hd2,n", [(2, 16, 64), (16, 300, 65), (17, 40, 63), (32, 272, 200), (33, 24, 130), (64, 512, 70), (65, 48, 96)])
+@pytest.mark.parametrize("cross_entropy", [False, True])
+def test_output_head_widths(oracle, outputs, hd2, n, cross_entropy):
+    dims = (72, 72, 48, hd2, 1, outputs)
+    if cross_entropy and outputs < 29:
+        pytest.skip("a class per depth")
+    loss_grad_case(oracle, dims, n, options=dict(cross_entropy=True) if cross_entropy else None, tol=2e-3, section_tol=5e-3)
