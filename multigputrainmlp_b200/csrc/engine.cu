@@ -12,6 +12,7 @@
 //   * activations are kept once (fp16 tape + one in-place fp32 residual stream).
 #include "../../include/mgt_b200.h"
 #include "batch_norm.cuh"
+#include "embedding_gather.cuh"
 #include "fp32_path.cuh"
 #include "tower_chain.cuh"
 #include "umma_gemm.cuh"
@@ -72,6 +73,10 @@ struct Workspace {
     uint64_t partial_floats, head_blocks;
     // batch normalisation (only planned when it is on): fp32 pre-activations of the R+1 normalised layers, their saved
     // mean / rstd, partial sums of the reductions, the statistics vector when the caller gives no exchange buffer
+    // the embedding layer by gathering rows instead of one-hot GEMMs (sample lists of the table gradient, dz1 as rows of samples)
+    bool gather_fwd, gather_grad;
+    uint32_t p_dz1_rows;
+    uint64_t off_lists;
     uint64_t off_bn_z, bn_z_stride, off_bn_save, off_bn_partial, off_bn_stats;
     uint64_t total_bytes;
 };
@@ -91,6 +96,23 @@ inline uint32_t CurrentDeviceSmCount() {
         return 148U;
     }
     return PlanSmCount(sms);
+}
+
+// Which form the embedding layer takes, by estimated microseconds (fitted to a B200; within a fifth over the range). Gathering
+// adds about 8 (forward) or 6.7 (gradient) values a picosecond, after a few us of start-up and, in the backward direction, the
+// sort of the samples. The one-hot GEMMs run in waves of 128 x 512 tiles, one per SM: so many us for the tile's start and
+// epilogue and 0.7 us a K chunk of 64 - several times that where a position has fewer than 64 classes and every chunk holds
+// many ones of a row.
+struct EmbeddingForms { bool gather_fwd, gather_grad; };
+EmbeddingForms PickEmbeddingForms(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm) {
+    const double sums = (double)B * s.state_len * s.hd1;
+    const bool few_classes = s.state_value_pad < 64U;
+    const uint64_t in = (uint64_t)s.state_len * s.state_value_pad, m_tiles = (s.hd1 + 127U) / 128U;
+    const double fwd_us = (double)((m_tiles * ((B + 511ULL) / 512ULL) + sm - 1) / sm) * (12.0 + (double)((in + 64U) / 64U) * (few_classes ? 5.0 : 0.72));
+    const uint64_t tiles = m_tiles * ((in + 511ULL) / 512ULL), waves1 = (tiles + sm - 1) / sm, waves2 = (2 * tiles + sm - 1) / sm;
+    const double chunks = B / 64.0, chunk_us = few_classes ? 3.3 : 0.70;
+    const double grad_us = waves2 < 2 * waves1 ? (double)waves2 * (15.0 + 0.5 * chunks * chunk_us) + (double)in * s.hd1 * 4.0 / 5.0e6 : (double)waves1 * (15.0 + chunks * chunk_us);
+    return {4.0 + sums / 8.0e6 < fwd_us, 8.0 + B * 0.0019 + sums / 6.7e6 < grad_us};
 }
 
 Workspace PlanWorkspace(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm_count, bool batch_norm = false) {
@@ -121,7 +143,12 @@ Workspace PlanWorkspace(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm_count,
     w.dz_stride = RoundUp((uint64_t)B * w.p_dz * 2, 1024);
     w.off_dz2 = take(w.dz_stride * (w.R + 1));
     w.off_dz1t = take(w.dz_stride * (w.R > 0 ? w.R : 1));
-    w.off_dz1 = take(hidden_act_bytes);
+    const EmbeddingForms forms = PickEmbeddingForms(s, B, sm_count);
+    w.gather_fwd = forms.gather_fwd;
+    w.gather_grad = forms.gather_grad;
+    w.p_dz1_rows = (uint32_t)RoundUp(s.hd1, 8);
+    w.off_dz1 = take(std::max<uint64_t>(hidden_act_bytes, forms.gather_grad ? (uint64_t)B * w.p_dz1_rows * 2 : 0));
+    w.off_lists = take(forms.gather_grad ? gather::ListWords(B, s.state_len, s.state_value_pad) * 4 : 0);
     // split-K partials: at most one CTA wave of [128 x 256] fp32 tiles plus slack for tile padding
     const uint64_t hidden_units = (uint64_t)((s.hd1 + 127) / 128) * ((s.hd2 + 255) / 256);
     const uint64_t resid_units = (uint64_t)((s.hd2 + 127) / 128) * ((s.hd2 + 255) / 256);
@@ -305,6 +332,7 @@ template <int BN, Epi EPI> using CfgFwdRows = GemmCfg<BN, 1, true, BSource::kTma
 template <int BN> using CfgDwRows = GemmCfg<BN, 1, false, BSource::kTmaMN, Epi::kPartialF32, 3, 3>;    // a1T[M][K] x dz[K][N]
 using CfgDxRows = GemmCfg<256, 1, false, BSource::kTmaK, Epi::kMaskRowsumF16, 4, 4>;                   // W[M][K] x dz[N][K] -> dz1T[M][N]
 using CfgDxRowsF32 = GemmCfg<256, 1, false, BSource::kTmaK, Epi::kMaskRowsumF32, 4, 4>;                // the same -> dz1[N][M] in fp32
+using CfgDxRowsF16T = GemmCfg<256, 1, false, BSource::kTmaK, Epi::kMaskRowsumF16T, 4, 4>;               // the same -> dz1[N][M]
 template <int BN> using CfgDwG = GemmCfg<BN, 1, true, BSource::kTmaMN, Epi::kPartialF32, 3, 3, false, true>; // R stacked act^T x dz
 // Two 256-column accumulators per unit (all of TMEM) and a two-stage one-hot ring. Measured alternatives at p888: 2 x 192
 // columns with a three-stage ring 1.44 ms, one double-buffered 256-column accumulator (epilogue under the next unit's
@@ -1113,18 +1141,20 @@ mgt_status_t GemmGradWeightsRows(mgt_engine* e, cudaStream_t st, const __half* a
 // dxT[N_in x samples] = (W[N_in x K] * dz[samples x K]^T) * [mask bit]: the hidden layer's dX with its wide side as rows; the
 // mask words are the ones the embedding forward wrote beside its activation.
 // Row sums of the result (the bias gradient of the layer below) are reduced into bias_grad[N_in] in a fixed order. With
-// dx_f32 the result goes there instead, in fp32 and with one row per sample.
+// dx_f32 the result goes there instead, in fp32 and with one row per sample; with dx_rows it goes to dx_t in the operand format
+// with one row per sample.
 mgt_status_t GemmBackpropInputRows(mgt_engine* e, cudaStream_t st, const __half* w, uint32_t w_pitch, const __half* dz, uint32_t dz_pitch, uint32_t samples,
-                                   uint32_t in_dim, uint32_t out_dim, uint32_t* mask_bits, uint32_t ld_bits, __half* dx_t, uint32_t t_pitch, float* dx_f32, uint32_t f32_pitch, float* rowsum,
+                                   uint32_t in_dim, uint32_t out_dim, uint32_t* mask_bits, uint32_t ld_bits, __half* dx_t, uint32_t t_pitch, float* dx_f32, uint32_t f32_pitch, bool dx_rows, uint32_t dx_rows_pitch, float* rowsum,
                                    uint64_t rowsum_rows, float* bias_grad) {
     GemmArgs a = BaseArgs(in_dim, samples, out_dim, CfgDxRows::BN, 1);
     const uint64_t rows = (uint64_t)a.n_tiles * CfgDxRows::EPI_STRIDE;
     if (rows > rowsum_rows) return MGT_CAPACITY_EXCEEDED;
     a.bits = mask_bits; a.ld_bits = ld_bits; a.out_f16 = dx_t; a.ld_f16 = t_pitch; a.out_f32 = dx_f32; a.ld_f32 = f32_pitch; a.rowsum = rowsum;
+    if (dx_rows) a.ld_f16 = dx_rows_pitch;
     CUtensorMap ta, tb;
     MGT_MAP(e->Map(&ta, w, out_dim, in_dim, w_pitch, 64, 128));
     MGT_MAP(e->Map(&tb, dz, out_dim, samples, dz_pitch, 64, CfgDxRows::BN));
-    MGT_TRY(dx_f32 != nullptr ? LaunchGemm<CfgDxRowsF32>(e, ta, tb, a, st) : LaunchGemm<CfgDxRows>(e, ta, tb, a, st));
+    MGT_TRY(dx_f32 != nullptr ? LaunchGemm<CfgDxRowsF32>(e, ta, tb, a, st) : (dx_rows ? LaunchGemm<CfgDxRowsF16T>(e, ta, tb, a, st) : LaunchGemm<CfgDxRows>(e, ta, tb, a, st)));
     ReduceRowsKernel<<<(in_dim + kReduceCols - 1) / kReduceCols, 256, 0, st>>>(rowsum, (uint32_t)rows, in_dim, 0, in_dim, bias_grad);
     ++e->launches;
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
@@ -1203,7 +1233,7 @@ Fp32Workspace PlanFp32(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm) {
     w.colsum_slot = (uint64_t)((B + 31U) / 32U) * s.hd2;  // one row per tile of at least 32 samples
     w.colsum = take(w.colsum_slot * 2 * r);
     w.colsum_in = take((uint64_t)((B + 31U) / 32U) * s.hd1);
-    w.lists = take(fp32path::EmbeddingGradListWords(B, s.state_len, s.state_value_pad));
+    w.lists = take(gather::ListWords(B, s.state_len, s.state_value_pad));
     w.total = off + 64;
     return w;
 }
@@ -1420,7 +1450,7 @@ mgt_status_t mgt_engine_check(mgt_engine_t* e, void* stream, int32_t* out_device
 // The fp32 operand of the table gradient behind the tensor-core workspace: dz1 [samples][hd1], rows padded to four floats,
 // then the sample lists of its classes (and slack to align the start).
 static uint64_t Fp32TableFloats(const mgt_mlp_shape_t& s, uint32_t B) {
-    return (uint64_t)B * RoundUp(s.hd1, 4) + fp32path::EmbeddingGradListWords(B, s.state_len, s.state_value_pad) + 64;
+    return (uint64_t)B * RoundUp(s.hd1, 4) + gather::ListWords(B, s.state_len, s.state_value_pad) + 64;
 }
 
 static uint64_t WorkspaceFloats(const mgt_mlp_shape_t* shape, uint32_t sample_count, uint32_t chunks, int32_t use_half_input_grad, int32_t use_half_linear,
@@ -1600,7 +1630,16 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     }
 
     // ---- embedding forward: a1 = relu([onehot | 1] * [W_in ; b_in])  (mlp_backward.cu:755-832)
-    {
+    if (ws.gather_fwd) {
+        auto run = [&](auto kernel) {
+            kernel<<<dim3((B + 31U) / 32U, (H1 + 63U) / 64U), 256 * gather::kForwardSplit, 0, st>>>(
+                reinterpret_cast<const uint8_t*>(states), reinterpret_cast<const uint16_t*>(hw.in_table), hw.p1, B, s.state_len, s.state_value_pad, H1,
+                reinterpret_cast<uint16_t*>(a1_h), ws.p_bt, reinterpret_cast<uint32_t*>(base + ws.off_bits_h1), ws.ld_bits_h1);
+        };
+        if (e->bf16_now) run(gather::ForwardKernel<gather::kForwardSplit, true>); else run(gather::ForwardKernel<gather::kForwardSplit, false>);
+        ++e->launches;
+        if (cudaGetLastError() != cudaSuccess) return MGT_CUDA_FAILURE;
+    } else {
         GemmArgs a = BaseArgs(H1, B, IN + 1, CfgEmbFwd::NACC * CfgEmbFwd::BN, 1);
         a.out_f16 = a1_h; a.ld_f16 = ws.p_bt;
         a.bits = reinterpret_cast<uint32_t*>(base + ws.off_bits_h1); a.ld_bits = ws.ld_bits_h1;
@@ -1720,7 +1759,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     // embedding gradient wants dz1 in fp32 (mlp_backward.cu:1433-1504, float one-hot GEMM): the same product of fp16 operands
     // with fp32 accumulation, written unrounded as rows of samples.
     MGT_TRY(GemmBackpropInputRows(e, st, hw.wh, hw.p2, dz_cur, ws.p_dz, B, H1, H2, reinterpret_cast<uint32_t*>(base + ws.off_bits_h1), ws.ld_bits_h1, dz1_h,
-                                  ws.p_bt, half_ig ? nullptr : dz1_f32, p_dz1_f32, reinterpret_cast<float*>(base + ws.off_rowsum), ws.rowsum_rows, grad + InputBias(s)));
+                                  ws.p_bt, half_ig ? nullptr : dz1_f32, p_dz1_f32, half_ig && ws.gather_grad, ws.p_dz1_rows, reinterpret_cast<float*>(base + ws.off_rowsum), ws.rowsum_rows, grad + InputBias(s)));
     if (!timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
 
     // ---- embedding gradient: grad W_in = onehot^T * dz1  (mlp_backward.cu:1440-1504); the input-bias
@@ -1729,6 +1768,21 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
         if (fp32path::EmbeddingGrad(st, reinterpret_cast<const uint8_t*>(states), dz1_f32, p_dz1_f32, B, s.state_len, s.state_value_pad, H1,
                                     reinterpret_cast<uint32_t*>(dz1_f32 + (uint64_t)B * p_dz1_f32), grad) != cudaSuccess) return MGT_CUDA_FAILURE;
         e->launches += 2;
+    } else if (ws.gather_grad) {
+        uint32_t* order = reinterpret_cast<uint32_t*>(base + ws.off_lists);
+        uint32_t* first = order + (uint64_t)s.state_len * B;
+        gather::SortByClassKernel<<<s.state_len, 1024, 0, st>>>(reinterpret_cast<const uint8_t*>(states), B, s.state_value_pad, order, first);
+        const bool vec = (H1 & 3U) == 0U && (reinterpret_cast<uintptr_t>(grad) & 15U) == 0U;
+        auto run = [&](auto kernel, uint32_t rows_per_cta) {
+            kernel<<<dim3((IN + rows_per_cta - 1U) / rows_per_cta, (H1 + 63U) / 64U), 256, 0, st>>>(order, first, reinterpret_cast<const uint16_t*>(dz1_h), ws.p_dz1_rows, B,
+                                                                                               s.state_len, s.state_value_pad, H1, grad, vec);
+        };
+        // a group of lanes per table row, four groups where that leaves fewer than 16 warps for an SM
+        const bool few = (uint64_t)IN * ((H1 + 63U) / 64U) < 64ULL * e->sm_count;
+        if (few) { if (e->bf16_now) run(gather::GradKernel<4, true>, 8U); else run(gather::GradKernel<4, false>, 8U); }
+        else { if (e->bf16_now) run(gather::GradKernel<1, true>, 32U); else run(gather::GradKernel<1, false>, 32U); }
+        e->launches += 2;
+        if (cudaGetLastError() != cudaSuccess) return MGT_CUDA_FAILURE;
     } else {
         const uint32_t unit_rows = CfgEmbGrad::NACC * CfgEmbGrad::BN;
         GemmArgs a = BaseArgs(H1, IN, B, unit_rows, 1);

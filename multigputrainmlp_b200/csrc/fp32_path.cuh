@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "embedding_gather.cuh"
+
 namespace mgt {
 namespace fp32path {
 
@@ -340,51 +342,6 @@ inline cudaError_t EmbeddingForward(cudaStream_t st, const uint8_t* states, cons
     return cudaGetLastError();
 }
 
-// The samples of each position in the order of their class there (stable, so sums over a class keep the sample order):
-// order[p][first[p][v] .. first[p][v+1]) = samples with class v at position p. One CTA per position: every warp counts the
-// classes of its own stretch of samples, the counts are scanned class by class, and the same sweep places the samples.
-__global__ void __launch_bounds__(1024)
-SortByClassKernel(const uint8_t* __restrict__ states, uint32_t B, uint32_t V, uint32_t* __restrict__ order, uint32_t* __restrict__ first) {
-    __shared__ uint32_t count[32][80];
-    __shared__ uint32_t base[81];
-    const uint32_t p = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31U;
-    for (uint32_t v = lane; v < 80U; v += 32U) count[warp][v] = 0U;
-    __syncwarp();
-    const uint32_t stretch = ((B + 31U) / 32U + 31U) / 32U * 32U;
-    const uint32_t lo = min(B, warp * stretch), hi = min(B, lo + stretch);
-    for (uint32_t s = lo; s < hi; s += 32U) {
-        const uint32_t v = s + lane < hi ? states[static_cast<uint64_t>(s + lane) * 80U + p] : 0xFFU;
-        const uint32_t same = __match_any_sync(0xFFFFFFFFU, v);
-        if (v < V && lane == static_cast<uint32_t>(__ffs(static_cast<int>(same))) - 1U) count[warp][v] += static_cast<uint32_t>(__popc(same));
-        __syncwarp();
-    }
-    __syncthreads();
-    if (threadIdx.x < V) {
-        uint32_t sum = 0;
-        for (uint32_t w = 0; w < 32U; ++w) {
-            const uint32_t c = count[w][threadIdx.x];
-            count[w][threadIdx.x] = sum;
-            sum += c;
-        }
-        base[threadIdx.x + 1U] = sum;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        base[0] = 0U;
-        for (uint32_t v = 1; v <= V; ++v) base[v] += base[v - 1U];
-    }
-    __syncthreads();
-    if (threadIdx.x <= V) first[p * (V + 1U) + threadIdx.x] = base[threadIdx.x];
-    for (uint32_t s = lo; s < hi; s += 32U) {
-        const uint32_t v = s + lane < hi ? states[static_cast<uint64_t>(s + lane) * 80U + p] : 0xFFU;
-        const uint32_t same = __match_any_sync(0xFFFFFFFFU, v);
-        if (v < V) order[static_cast<uint64_t>(p) * B + base[v] + count[warp][v] + static_cast<uint32_t>(__popc(same & ((1U << lane) - 1U)))] = s + lane;
-        __syncwarp();
-        if (v < V && lane == static_cast<uint32_t>(__ffs(static_cast<int>(same))) - 1U) count[warp][v] += static_cast<uint32_t>(__popc(same));
-        __syncwarp();
-    }
-}
-
 // Table gradient: grad[p*V + v][h] = sum of dz1[s][h] over the samples with class v at position p (zero where there are
 // none), in sample order. A warp owns one table row and 32 * W columns and adds the listed rows of dz1, eight loads in flight;
 // the column blocks are the slow grid dimension, so the slice of dz1 in use stays in L2. Bound by L2: every dz1 row is read
@@ -424,12 +381,11 @@ EmbeddingGradKernel(const uint32_t* __restrict__ order, const uint32_t* __restri
     if (W == 4) *reinterpret_cast<float4*>(dst) = make_float4(acc[0], acc[1 % W], acc[2 % W], acc[3 % W]);
     else dst[0] = acc[0];
 }
-// `lists`: L * B + L * (V + 1) words of scratch
-inline uint64_t EmbeddingGradListWords(uint32_t B, uint32_t L, uint32_t V) { return static_cast<uint64_t>(L) * B + static_cast<uint64_t>(L) * (V + 1U); }
+// `lists`: gather::ListWords words of scratch
 inline cudaError_t EmbeddingGrad(cudaStream_t st, const uint8_t* states, const float* dz1, uint32_t ld, uint32_t B, uint32_t L, uint32_t V, uint32_t H1,
                                  uint32_t* lists, float* grad_table) {
     uint32_t* first = lists + static_cast<uint64_t>(L) * B;
-    SortByClassKernel<<<L, 1024, 0, st>>>(states, B, V, lists, first);
+    gather::SortByClassKernel<<<L, 1024, 0, st>>>(states, B, V, lists, first);
     const bool quads = (H1 & 3U) == 0U && (ld & 3U) == 0U && (reinterpret_cast<uintptr_t>(grad_table) & 15U) == 0U;
     const uint32_t cols = quads ? 128U : 32U;
     const dim3 grid((L * V + 7U) / 8U, (H1 + cols - 1U) / cols);

@@ -39,6 +39,7 @@ enum class Epi : int {
                            // per output column of the layer; the sign words are the ReLU mask the backward pass needs)
     kMaskRowsumF16,        // out_f16[m][n] = acc * [bit n of bits[m]]; rowsum[(n tile, warp of the quadrant)][m] = sum over the warp's columns
     kMaskRowsumF32,        // the same values unrounded and transposed: out_f32[n][m] (the lanes of a warp write 32 neighbouring columns of one row)
+    kMaskRowsumF16T,       // ... in the operand format: out_f16[n][m]
 };
 
 struct GemmArgs {
@@ -108,7 +109,7 @@ struct GemmCfg {
     static constexpr int EPI_TILE_PITCH = 36;
     // per epilogue warp: a padded 32x32 fp32 tile, 32 words of ReLU-mask bits and four rows of column-sum accumulators
     // (the embedding epilogues write transposed and need no staging)
-    static constexpr int EPI_WARP_BYTES = (kOneHot || EPI_ == Epi::kMaskRowsumF16 || EPI_ == Epi::kMaskRowsumF32) ? 0 : (32 * EPI_TILE_PITCH * 4 + 128 + 4 * 32 * 4);
+    static constexpr int EPI_WARP_BYTES = (kOneHot || EPI_ == Epi::kMaskRowsumF16 || EPI_ == Epi::kMaskRowsumF32 || EPI_ == Epi::kMaskRowsumF16T) ? 0 : (32 * EPI_TILE_PITCH * 4 + 128 + 4 * 32 * 4);
     static constexpr int EPI_STAGE_BYTES = EPI_WARPS * EPI_WARP_BYTES;
     static constexpr int SMEM_BYTES = 1024 + SA_ * A_STAGE_BYTES + SB_ * B_STAGE_BYTES + 256 + EPI_STAGE_BYTES;
     static_assert(BN_ % 16 == 0 && BN_ >= 16 && BN_ <= 256, "UMMA N");
@@ -467,7 +468,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                 tc_fence_before();
                 mbar_arrive(&acc_empty[ab]);
             }
-        } else if constexpr (Cfg::EPI == Epi::kMaskRowsumF16 || Cfg::EPI == Epi::kMaskRowsumF32) {
+        } else if constexpr (Cfg::EPI == Epi::kMaskRowsumF16 || Cfg::EPI == Epi::kMaskRowsumF32 || Cfg::EPI == Epi::kMaskRowsumF16T) {
             // D and the output have a row per TMEM lane and the warp's 32 columns side by side in that row: 64 bytes per lane,
             // written as four 16-byte vectors straight from registers; the mask of a chunk is one word per lane; the row
             // sum is a sum over the lane's own registers. (Full 32-byte sectors; whole rows per warp are not needed.)
@@ -514,11 +515,14 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                     for (int j = 0; j < 32; ++j) v[j] = ((mw[ci] >> j) & 1U) ? __uint_as_float(r[j]) : 0.0f;
 #pragma unroll
                     for (int j = 0; j < 32; ++j) row_sum += v[j];  // (columns past N were masked with zeros above)
-                    if (Cfg::EPI == Epi::kMaskRowsumF32) {
+                    if (Cfg::EPI == Epi::kMaskRowsumF32 || Cfg::EPI == Epi::kMaskRowsumF16T) {
                         if (m_ok) {
 #pragma unroll
-                            for (int j = 0; j < 32; ++j)
-                                if (static_cast<uint32_t>(j) < valid) args.out_f32[static_cast<uint64_t>(n0 + j) * args.ld_f32 + m] = v[j];
+                            for (int j = 0; j < 32; ++j) {
+                                if (static_cast<uint32_t>(j) >= valid) continue;
+                                if (Cfg::EPI == Epi::kMaskRowsumF32) args.out_f32[static_cast<uint64_t>(n0 + j) * args.ld_f32 + m] = v[j];
+                                else reinterpret_cast<uint16_t*>(args.out_f16)[static_cast<uint64_t>(n0 + j) * args.ld_f16 + m] = to_operand(v[j], args.bf16 != 0U);
+                            }
                         }
                     } else if (m_ok) {
                         uint16_t* dst = reinterpret_cast<uint16_t*>(args.out_f16) + static_cast<uint64_t>(m) * args.ld_f16 + n0;

@@ -123,3 +123,14 @@ def test_output_head_widths(oracle, outputs, hd2, n, cross_entropy):
     if cross_entropy and outputs < 29:
         pytest.skip("a class per depth")
     loss_grad_case(oracle, dims, n, options=dict(cross_entropy=True) if cross_entropy else None, tol=2e-3, section_tol=5e-3)
+
+
+# embedding layer by gathering rows: samples around a CTA's 32 and 128, columns around its 64 and the vectors of eight, few
+# classes, a single position; the last one lies beyond the rule's border and takes the one-hot GEMMs
+@pytest.mark.parametrize("dims,n,mirror", [((72, 72, 64, 16, 1, 1), 31, True), ((72, 72, 65, 24, 1, 1), 33, False), ((54, 6, 136, 32, 1, 1), 129, True), ((1, 3, 40, 8, 1, 1), 65, True),
+                                            ((72, 72, 200, 40, 1, 1), 2100, True), ((30, 30, 1100, 48, 1, 1), 4200, True), ((7, 64, 4096, 16, 0, 1), 9000, True)])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_embedding_forms(oracle, dims, n, mirror, bf16):
+    if n > 4000 and bf16:
+        pytest.skip("the oracle takes long; the form is the same")
+    loss_grad_case(oracle, dims, n, mirror=mirror, options=dict(bf16=True) if bf16 else None, tol=8e-3 if bf16 else 1e-3, section_tol=2e-2 if bf16 else 3e-3)
