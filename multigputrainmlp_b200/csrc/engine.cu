@@ -14,6 +14,7 @@
 #include "batch_norm.cuh"
 #include "embedding_gather.cuh"
 #include "fp32_path.cuh"
+#include "onehot_pair.cuh"
 #include "tower_chain.cuh"
 #include "umma_gemm.cuh"
 
@@ -24,6 +25,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <mutex>
 #include <unordered_map>
@@ -98,21 +100,52 @@ inline uint32_t CurrentDeviceSmCount() {
     return PlanSmCount(sms);
 }
 
-// Which form the embedding layer takes, by estimated microseconds (fitted to a B200; within a fifth over the range). Gathering
-// adds about 8 (forward) or 6.7 (gradient) values a picosecond, after a few us of start-up and, in the backward direction, the
-// sort of the samples. The one-hot GEMMs run in waves of 128 x 512 tiles, one per SM: so many us for the tile's start and
-// epilogue and 0.7 us a K chunk of 64 - several times that where a position has fewer than 64 classes and every chunk holds
-// many ones of a row.
+// ---- the embedding layer: one-hot GEMMs for CTA pairs (onehot_pair.cuh) or gathered rows (embedding_gather.cuh) -------------
+// How the pairs cut their work, and an estimate of what it takes in microseconds (fitted to a B200, within a fifth or so).
+struct PairPlan {
+    uint32_t workers, tile_cols, n_tiles, row_len;
+    uint64_t line;
+    bool shared_tiles;  // gradient: two pairs add into some tiles, the result has to be zeroed before
+    double us;
+};
+// Forward: every pair an equal number of 64-column steps of the line; below four full pieces per pair the pieces of a row tile
+// instead (a stretch across a row tile's end is one piece more).
+PairPlan PlanPairForward(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm) {
+    PairPlan p{};
+    const uint32_t m_tiles = (s.hd1 + 255U) / 256U, pairs = sm / 2U, k_chunks = (s.state_len * s.state_value_pad + 64U) / 64U;
+    const bool by_tile = m_tiles <= pairs && B <= 2048U * (pairs / m_tiles);
+    p.row_len = (B + 63U) / 64U * 64U;
+    p.line = (uint64_t)m_tiles * p.row_len;
+    p.workers = (uint32_t)std::min<uint64_t>(by_tile ? m_tiles * (pairs / m_tiles) : pairs, p.line / 64U);
+    const double cols = (double)p.line / p.workers, pieces = std::ceil(cols / 512.0) + (by_tile ? 0.0 : 0.5);
+    p.us = 12.0 + pieces * (k_chunks * std::max(700.0, 2.0 * cols / pieces + 25.0) + 6000.0) / 1845.0;
+    return p;
+}
+// Gradient: tiles of up to 512 columns - the more columns, the fewer times A is read; with few classes the synthesis is what
+// takes the time, so narrower ones as long as there are pairs for them. Stretches of at least a tile for every pair; with fewer
+// tiles than pairs whole tiles, or halves where they all fit.
+PairPlan PlanPairGrad(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm) {
+    PairPlan p{};
+    const uint32_t m_tiles = (s.hd1 + 255U) / 256U, pairs = sm / 2U, k_chunks = (B + 63U) / 64U, rows = s.state_len * s.state_value_pad;
+    p.n_tiles = (rows + 511U) / 512U;
+    if (s.state_value_pad < 64U) p.n_tiles = std::max(p.n_tiles, std::min((rows + 63U) / 64U, pairs / 2U / m_tiles));
+    p.tile_cols = ((rows + p.n_tiles - 1U) / p.n_tiles + 31U) & ~31U;
+    p.n_tiles = (rows + p.tile_cols - 1U) / p.tile_cols;
+    const uint32_t tiles = m_tiles * p.n_tiles;
+    p.workers = tiles >= pairs ? pairs : (2U * tiles <= pairs && k_chunks >= 2U ? 2U * tiles : tiles);
+    p.line = (uint64_t)tiles * k_chunks;
+    p.shared_tiles = tiles % p.workers != 0U;
+    const double share = (double)tiles / p.workers;
+    p.us = 12.0 + (share * k_chunks * std::max(1100.0, 2.0 * p.tile_cols + 230.0) + (share > 1.0 ? share + 1.0 : 1.0) * 27000.0) / 1845.0 +
+           (p.shared_tiles ? 3.0 + (double)rows * s.hd1 * 4.0 / 6.0e6 : 0.0);
+    return p;
+}
+// Gathering adds about 8 (forward) or 6.7 (gradient) values a picosecond, after a few us of start-up and, in the backward
+// direction, the sort of the samples.
 struct EmbeddingForms { bool gather_fwd, gather_grad; };
 EmbeddingForms PickEmbeddingForms(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm) {
     const double sums = (double)B * s.state_len * s.hd1;
-    const bool few_classes = s.state_value_pad < 64U;
-    const uint64_t in = (uint64_t)s.state_len * s.state_value_pad, m_tiles = (s.hd1 + 127U) / 128U;
-    const double fwd_us = (double)((m_tiles * ((B + 511ULL) / 512ULL) + sm - 1) / sm) * (12.0 + (double)((in + 64U) / 64U) * (few_classes ? 5.0 : 0.72));
-    const uint64_t tiles = m_tiles * ((in + 511ULL) / 512ULL), waves1 = (tiles + sm - 1) / sm, waves2 = (2 * tiles + sm - 1) / sm;
-    const double chunks = B / 64.0, chunk_us = few_classes ? 3.3 : 0.70;
-    const double grad_us = waves2 < 2 * waves1 ? (double)waves2 * (15.0 + 0.5 * chunks * chunk_us) + (double)in * s.hd1 * 4.0 / 5.0e6 : (double)waves1 * (15.0 + chunks * chunk_us);
-    return {4.0 + sums / 8.0e6 < fwd_us, 8.0 + B * 0.0019 + sums / 6.7e6 < grad_us};
+    return {4.0 + sums / 8.0e6 < PlanPairForward(s, B, sm).us, 8.0 + B * 0.0019 + sums / 6.7e6 < PlanPairGrad(s, B, sm).us};
 }
 
 Workspace PlanWorkspace(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm_count, bool batch_norm = false) {
@@ -265,8 +298,10 @@ struct mgt_engine {
         return true;
     }
 
-    // fp16 2-D tensor map with 128-byte swizzle: `inner` contiguous elements per row, `outer` rows.
-    bool Map(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t pitch_elems, uint32_t box_inner, uint32_t box_outer) {
+    // fp16 2-D tensor map: `inner` contiguous elements per row, `outer` rows; the swizzle spans a box row (128 bytes, or 64 with
+    // a box of 32 elements).
+    bool Map(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t pitch_elems, uint32_t box_inner, uint32_t box_outer,
+             CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
         const mgt::MapKey key{base, inner, outer, pitch_elems, box_inner, box_outer};
         std::lock_guard<std::mutex> lock(mu);
         auto it = maps.find(key);
@@ -278,7 +313,7 @@ struct mgt_engine {
         const cuuint32_t elem[2] = {1, 1};
         CUtensorMap m;
         const CUresult r = encode(&m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(base), dims, strides, box, elem,
-                                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) return false;
         if (maps.size() > 4096) maps.clear();
@@ -319,32 +354,43 @@ mgt_status_t LaunchGemm(mgt_engine* e, const CUtensorMap& ta, const CUtensorMap&
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
 }
 
+template <bool GRAD>
+mgt_status_t LaunchPair(mgt_engine* e, const CUtensorMap& ta, const CUtensorMap& to, PairArgs args, cudaStream_t stream) {
+    static std::mutex attr_mu;
+    static bool attr_done[64] = {};
+    if (e->device < 0 || e->device >= 64) return MGT_INVALID_CONFIG;
+    {
+        std::lock_guard<std::mutex> lock(attr_mu);
+        if (!attr_done[e->device]) {
+            if (cudaFuncSetAttribute(onehot_pair_kernel<GRAD>, cudaFuncAttributeMaxDynamicSharedMemorySize, PairCfg<GRAD>::SMEM_BYTES) != cudaSuccess) return MGT_CUDA_FAILURE;
+            attr_done[e->device] = true;
+        }
+    }
+    args.status = e->status_word;
+    args.bf16 = e->bf16_now ? 1U : 0U;
+    onehot_pair_kernel<GRAD><<<2U * args.workers, PairCfg<GRAD>::THREADS, PairCfg<GRAD>::SMEM_BYTES, stream>>>(ta, to, args);
+    ++e->launches;
+    return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
+}
+
 // Tile configurations. BN = 224 serves the p888 residual width without padded MMA columns.
-template <int BN, Epi EPI> using CfgFwd = GemmCfg<BN, 1, false, BSource::kTmaMN, EPI, 3, 3>;   // act[K-major] x W[K][N]
-template <int BN, Epi EPI> using CfgDx = GemmCfg<BN, 1, false, BSource::kTmaK, EPI, 3, 3>;     // dz[K-major] x W[N][K]
+template <int BN, Epi EPI> using CfgFwd = GemmCfg<BN, false, BSource::kTmaMN, EPI, 3, 3>;   // act[K-major] x W[K][N]
+template <int BN, Epi EPI> using CfgDx = GemmCfg<BN, false, BSource::kTmaK, EPI, 3, 3>;     // dz[K-major] x W[N][K]
 // B-stationary forms for reductions of at most 256 (the residual width): weights stay in shared memory
-template <int BN, Epi EPI> using CfgFwdS = GemmCfg<BN, 1, false, BSource::kTmaMN, EPI, 3, 4, true>;
-template <int BN, Epi EPI> using CfgDxS = GemmCfg<BN, 1, false, BSource::kTmaK, EPI, 3, 4, true>;
-template <int BN> using CfgDw = GemmCfg<BN, 1, true, BSource::kTmaMN, Epi::kPartialF32, 3, 3>; // act^T x dz
+template <int BN, Epi EPI> using CfgFwdS = GemmCfg<BN, false, BSource::kTmaMN, EPI, 3, 4, true>;
+template <int BN, Epi EPI> using CfgDxS = GemmCfg<BN, false, BSource::kTmaK, EPI, 3, 4, true>;
+template <int BN> using CfgDw = GemmCfg<BN, true, BSource::kTmaMN, Epi::kPartialF32, 3, 3>; // act^T x dz
 // The hidden layer with its wide side (hd1) as rows: a1 and dz1 are kept as [hd1][samples], the way the two embedding GEMMs
 // produce and consume them, so that their epilogues and the hidden dX epilogue move 64 contiguous bytes per lane
-template <int BN, Epi EPI> using CfgFwdRows = GemmCfg<BN, 1, true, BSource::kTmaMN, EPI, 3, 3>;        // a1T[K][M] x W[K][N]
-template <int BN> using CfgDwRows = GemmCfg<BN, 1, false, BSource::kTmaMN, Epi::kPartialF32, 3, 3>;    // a1T[M][K] x dz[K][N]
-using CfgDxRows = GemmCfg<256, 1, false, BSource::kTmaK, Epi::kMaskRowsumF16, 4, 4>;                   // W[M][K] x dz[N][K] -> dz1T[M][N]
-using CfgDxRowsF32 = GemmCfg<256, 1, false, BSource::kTmaK, Epi::kMaskRowsumF32, 4, 4>;                // the same -> dz1[N][M] in fp32
-using CfgDxRowsF16T = GemmCfg<256, 1, false, BSource::kTmaK, Epi::kMaskRowsumF16T, 4, 4>;               // the same -> dz1[N][M]
-template <int BN> using CfgDwG = GemmCfg<BN, 1, true, BSource::kTmaMN, Epi::kPartialF32, 3, 3, false, true>; // R stacked act^T x dz
-// Two 256-column accumulators per unit (all of TMEM) and a two-stage one-hot ring. Measured alternatives at p888: 2 x 192
-// columns with a three-stage ring 1.44 ms, one double-buffered 256-column accumulator (epilogue under the next unit's
-// MMAs, but the table tile re-read twice as often) 1.37 ms, this form 1.14 ms: the K loop already issues MMAs back to back.
-using CfgEmbFwd = GemmCfg<256, 2, true, BSource::kOneHotFwd, Epi::kEmbFwdRows, 4, 2>;   // table[K][M] x onehot -> a1T[M][N]
-using CfgEmbGrad = GemmCfg<256, 2, false, BSource::kOneHotGrad, Epi::kEmbGrad, 4, 2>;    // dz1T[M][K] x onehot -> grad[N][M]
-// (One accumulator per unit with two units in flight - the epilogue of one draining under the MMAs of the next, operand
-// ring four deep - was measured at p888: forward 1.40 ms against 1.22 ms, gradient 1.56 ms against 1.13 ms. A K chunk
-// costs about a thousand cycles in hand-overs whatever it feeds, so it should feed eight MMAs, not four.)
-using CfgDbgKK = GemmCfg<256, 1, false, BSource::kTmaK, Epi::kPartialF32, 3, 3>;
-using CfgDbgKM = GemmCfg<256, 1, false, BSource::kTmaMN, Epi::kPartialF32, 3, 3>;
-using CfgDbgMK = GemmCfg<256, 1, true, BSource::kTmaK, Epi::kPartialF32, 3, 3>;
+template <int BN, Epi EPI> using CfgFwdRows = GemmCfg<BN, true, BSource::kTmaMN, EPI, 3, 3>;        // a1T[K][M] x W[K][N]
+template <int BN> using CfgDwRows = GemmCfg<BN, false, BSource::kTmaMN, Epi::kPartialF32, 3, 3>;    // a1T[M][K] x dz[K][N]
+using CfgDxRows = GemmCfg<256, false, BSource::kTmaK, Epi::kMaskRowsumF16, 4, 4>;                   // W[M][K] x dz[N][K] -> dz1T[M][N]
+using CfgDxRowsF32 = GemmCfg<256, false, BSource::kTmaK, Epi::kMaskRowsumF32, 4, 4>;                // the same -> dz1[N][M] in fp32
+using CfgDxRowsF16T = GemmCfg<256, false, BSource::kTmaK, Epi::kMaskRowsumF16T, 4, 4>;               // the same -> dz1[N][M]
+template <int BN> using CfgDwG = GemmCfg<BN, true, BSource::kTmaMN, Epi::kPartialF32, 3, 3, false, true>; // R stacked act^T x dz
+using CfgDbgKK = GemmCfg<256, false, BSource::kTmaK, Epi::kPartialF32, 3, 3>;
+using CfgDbgKM = GemmCfg<256, false, BSource::kTmaMN, Epi::kPartialF32, 3, 3>;
+using CfgDbgMK = GemmCfg<256, true, BSource::kTmaK, Epi::kPartialF32, 3, 3>;
 
 inline uint32_t PickBN(uint32_t n) { return n <= 224 ? 224U : 256U; }
 
@@ -1640,13 +1686,17 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
         ++e->launches;
         if (cudaGetLastError() != cudaSuccess) return MGT_CUDA_FAILURE;
     } else {
-        GemmArgs a = BaseArgs(H1, B, IN + 1, CfgEmbFwd::NACC * CfgEmbFwd::BN, 1);
+        PairArgs a{};
+        a.M = H1; a.N = B; a.K = IN + 1U; a.k_chunks = (IN + 64U) / 64U;
+        const PairPlan plan = PlanPairForward(s, B, (uint32_t)e->sm_count);
+        a.row_len = plan.row_len; a.line = plan.line; a.workers = plan.workers;
         a.out_f16 = a1_h; a.ld_f16 = ws.p_bt;
         a.bits = reinterpret_cast<uint32_t*>(base + ws.off_bits_h1); a.ld_bits = ws.ld_bits_h1;
         a.states = reinterpret_cast<const uint8_t*>(states); a.state_len = s.state_len; a.value_pad = s.state_value_pad; a.samples = B; a.in_rows = IN;
-        CUtensorMap ta;
+        CUtensorMap ta, to;
         MGT_MAP(e->Map(&ta, hw.in_table, H1, IN + 1, hw.p1, 64, 64));
-        MGT_TRY(LaunchGemm<CfgEmbFwd>(e, ta, ta, a, st));
+        MGT_MAP(e->Map(&to, a1_h, B, H1, ws.p_bt, 32, 32, CU_TENSOR_MAP_SWIZZLE_64B));
+        MGT_TRY(LaunchPair<false>(e, ta, to, a, st));
     }
     if (!timer.Mark(profile ? &profile->input_forward_ms : nullptr)) return MGT_CUDA_FAILURE;
 
@@ -1784,22 +1834,16 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
         e->launches += 2;
         if (cudaGetLastError() != cudaSuccess) return MGT_CUDA_FAILURE;
     } else {
-        const uint32_t unit_rows = CfgEmbGrad::NACC * CfgEmbGrad::BN;
-        GemmArgs a = BaseArgs(H1, IN, B, unit_rows, 1);
-        const uint64_t tiles = (uint64_t)a.m_tiles * a.n_tiles;
-        // Two splits keep fp32 atomics order-independent (0 + a + b == 0 + b + a); use them when one
-        // split would leave a large part of the last wave idle.
-        const uint64_t waves1 = (tiles + e->sm_count - 1) / e->sm_count;
-        const uint64_t waves2 = (2 * tiles + e->sm_count - 1) / e->sm_count;
-        const uint32_t splits = (a.k_chunks >= 2 && waves2 < 2 * waves1) ? 2U : 1U;
-        a = BaseArgs(H1, IN, B, unit_rows, splits);
+        PairArgs a{};
+        a.M = H1; a.N = IN; a.K = B; a.k_chunks = (B + 63U) / 64U;
+        const PairPlan plan = PlanPairGrad(s, B, (uint32_t)e->sm_count);
+        a.n_tiles = plan.n_tiles; a.tile_cols = plan.tile_cols; a.workers = plan.workers; a.line = plan.line;
         a.out_f32 = grad; a.ld_f32 = H1;
         a.states = reinterpret_cast<const uint8_t*>(states); a.state_len = s.state_len; a.value_pad = s.state_value_pad; a.samples = B;
-        a.in_rows = 0xFFFFFFFFU;  // no all-ones row in this direction
-        if (a.splits > 1 && cudaMemsetAsync(grad, 0, (uint64_t)IN * H1 * sizeof(float), st) != cudaSuccess) return MGT_CUDA_FAILURE;
+        if (plan.shared_tiles && cudaMemsetAsync(grad, 0, (uint64_t)IN * H1 * sizeof(float), st) != cudaSuccess) return MGT_CUDA_FAILURE;
         CUtensorMap ta;
         MGT_MAP(e->Map(&ta, dz1_h, B, H1, ws.p_bt, 64, 128));
-        MGT_TRY(LaunchGemm<CfgEmbGrad>(e, ta, ta, a, st));
+        MGT_TRY(LaunchPair<true>(e, ta, ta, a, st));
     }
     // table and input bias are complete: tell a caller who asked to hear of it before the weight-gradient GEMMs are enqueued
     if (e->early_fn != nullptr && e->early_fn(e->early_user, 2U * R + 2U, 0, InputBias(s) + H1, stream_v) != MGT_OK) return MGT_CUDA_FAILURE;

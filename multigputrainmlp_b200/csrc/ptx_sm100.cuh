@@ -58,12 +58,14 @@ constexpr uint64_t kWaitLimitNs = 1000ULL * 1000ULL * 1000ULL;
 
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* cta_abort, int code) {
     if (mbar_try_wait(bar, parity)) return true;
-    const uint64_t start = global_timer_ns();
+    uint64_t start = 0;
     uint32_t spins = 0;
     while (!mbar_try_wait(bar, parity)) {
         if ((++spins & 63U) == 0U) {
             if (*cta_abort != 0) return false;
-            if (global_timer_ns() - start > kWaitLimitNs) {
+            const uint64_t now = global_timer_ns();  // (read for the first time after 64 polls: it costs more than most waits)
+            if (start == 0) start = now;
+            if (now - start > kWaitLimitNs) {
                 *cta_abort = code;
                 return false;
             }
@@ -87,12 +89,14 @@ __device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
 }
 __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, volatile int* cta_abort, int code) {
     if (mbar_test_wait(bar, parity)) return true;
-    const uint64_t start = global_timer_ns();
+    uint64_t start = 0;
     uint32_t spins = 0;
     while (!mbar_test_wait(bar, parity)) {
         if ((++spins & 1023U) == 0U) {
             if (*cta_abort != 0) return false;
-            if (global_timer_ns() - start > kWaitLimitNs) {
+            const uint64_t now = global_timer_ns();
+            if (start == 0) start = now;
+            if (now - start > kWaitLimitNs) {
                 *cta_abort = code;
                 return false;
             }

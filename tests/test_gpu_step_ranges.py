@@ -134,3 +134,10 @@ def test_embedding_forms(oracle, dims, n, mirror, bf16):
     if n > 4000 and bf16:
         pytest.skip("the oracle takes long; the form is the same")
     loss_grad_case(oracle, dims, n, mirror=mirror, options=dict(bf16=True) if bf16 else None, tol=8e-3 if bf16 else 1e-3, section_tol=2e-2 if bf16 else 3e-3)
+
+
+# one-hot GEMMs for CTA pairs: ragged rows, columns and K on both sides, tiles shared by two pairs and whole ones; 64 classes and
+# more (single places set and cleared), and few classes (rows written whole)
+@pytest.mark.parametrize("dims,n", [((72, 72, 1000, 16, 0, 1), 9001), ((54, 6, 4090, 16, 0, 1), 9000)])
+def test_one_hot_pairs(oracle, dims, n):
+    loss_grad_case(oracle, dims, n)
