@@ -80,18 +80,39 @@ __device__ __forceinline__ float warp_column_sums(float (&v)[32], uint32_t lane)
     return v[0];
 }
 
-// 32 floats -> 16 packed half2 words (round to nearest even) and the "value is positive" bit of each element. The bit
-// is taken from the fp32 value, as the reference takes its ReLU masks (mlp_backward.cu:944-1025 compare the fp32 copies):
-// a positive value too small for fp16 rounds to +0 in the operand but still lets its gradient through.
-__device__ __forceinline__ uint32_t pack_halfs(const float (&v)[32], uint32_t (&h)[16], bool bf16) {
+// The "is positive" bit of each of 32 values, taken from the fp32 value as the reference takes its ReLU masks
+// (mlp_backward.cu:944-1025 compare the fp32 copies): a positive value too small for fp16 rounds to +0 in the operand but still
+// lets its gradient through. Two instructions a value: for anything but -0 the sign bit of 0 - v (as integers) is set exactly
+// when v > 0, and a funnel shift collects it. The values are ReLU results, which are never -0 or NaN.
+__device__ __forceinline__ uint32_t positive_bits(const uint32_t (&v)[32]) {
     uint32_t bits = 0;
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-        h[i] = ptx::pack_operand_pair(v[2 * i], v[2 * i + 1], bf16);
-        bits |= (v[2 * i] > 0.0f ? 1U : 0U) << (2 * i);
-        bits |= (v[2 * i + 1] > 0.0f ? 1U : 0U) << (2 * i + 1);
-    }
+    for (int j = 31; j >= 0; --j) bits = __funnelshift_l(0U - v[j], bits, 1);
     return bits;
+}
+
+// 32 floats -> 16 packed words of the operand format (round to nearest even)
+__device__ __forceinline__ void pack_operands(const uint32_t (&v)[32], uint32_t (&h)[16], bool bf16) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) h[i] = ptx::pack_operand_pair(__uint_as_float(v[2 * i]), __uint_as_float(v[2 * i + 1]), bf16);
+}
+
+// v = ReLU(v + b) for 32 values, the additions two per instruction (each rounded as on its own)
+__device__ __forceinline__ void add_bias_relu(uint32_t (&v)[32], const float* b) {
+    const ulonglong2* p = reinterpret_cast<const ulonglong2*>(b);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const ulonglong2 f = p[q];
+        uint64_t x, y;
+        asm("mov.b64 %0, {%1, %2};" : "=l"(x) : "r"(v[4 * q]), "r"(v[4 * q + 1]));
+        asm("mov.b64 %0, {%1, %2};" : "=l"(y) : "r"(v[4 * q + 2]), "r"(v[4 * q + 3]));
+        asm("add.rn.f32x2 %0, %0, %1;" : "+l"(x) : "l"(f.x));
+        asm("add.rn.f32x2 %0, %0, %1;" : "+l"(y) : "l"(f.y));
+        asm("mov.b64 {%0, %1}, %2;" : "=r"(v[4 * q]), "=r"(v[4 * q + 1]) : "l"(x));
+        asm("mov.b64 {%0, %1}, %2;" : "=r"(v[4 * q + 2]), "=r"(v[4 * q + 3]) : "l"(y));
+    }
+#pragma unroll
+    for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(fmaxf(__uint_as_float(v[j]), 0.0f));
 }
 
 }  // namespace detail
@@ -295,17 +316,6 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                 __syncwarp();
             }
         };
-        auto add_bias_relu = [&](float (&v)[32], uint32_t ci) {
-            const float4* b = reinterpret_cast<const float4*>(bias_slots + (par * WPW + ci) * 32U);
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                const float4 f = b[q];
-                v[4 * q] = fmaxf(v[4 * q] + f.x, 0.0f);
-                v[4 * q + 1] = fmaxf(v[4 * q + 1] + f.y, 0.0f);
-                v[4 * q + 2] = fmaxf(v[4 * q + 2] + f.z, 0.0f);
-                v[4 * q + 3] = fmaxf(v[4 * q + 3] + f.w, 0.0f);
-            }
-        };
         auto store_words = [&](uint32_t* dst, const uint32_t (&wd)[4]) {
             if (WPW == 4U) *reinterpret_cast<uint4*>(dst) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
             else *reinterpret_cast<uint2*>(dst) = make_uint2(wd[0], wd[1]);
@@ -319,9 +329,15 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                 wd[0] = m.x; wd[1] = m.y;
             }
         };
-        auto apply_mask = [&](float (&v)[32], uint32_t bits) {
+        auto apply_mask = [&](uint32_t (&v)[32], uint32_t bits) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = ((bits >> j) & 1U) ? v[j] : 0.0f;
+            for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(((bits >> j) & 1U) ? __uint_as_float(v[j]) : 0.0f);
+        };
+        auto column_sums = [&](const uint32_t (&raw)[32]) {
+            float v[32];
+#pragma unroll
+            for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
+            return detail::warp_column_sums(v, lane);
         };
 
         uint32_t uses = 0;
@@ -358,7 +374,8 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                     for (int j = 0; j < 32; ++j) raw[j] = __float_as_uint(v[j]);
                     tmem_st_32x32(tmem_base + lane_addr + kStateCol + cc * 32U, raw);
                     uint32_t h[16];
-                    words[ci] = detail::pack_halfs(v, h, args.bf16 != 0U);
+                    detail::pack_operands(raw, h, args.bf16 != 0U);
+                    if (!BWD) words[ci] = detail::positive_bits(raw);
                     store_operand(act_s, cc, h);
                     tmem_st_wait();
                     publish(&ready_s[cc >> 1]);
@@ -385,17 +402,15 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                         uint32_t raw[32];
                         tmem_ld_32x32(tmem_base + lane_addr + cc * 32U, raw);
                         tmem_ld_wait();
-                        float v[32];
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
-                        if (BWD) apply_mask(v, mwords[ci]);
-                        else add_bias_relu(v, ci);
                         uint32_t h[16];
-                        words[ci] = detail::pack_halfs(v, h, args.bf16 != 0U);
+                        if (BWD) apply_mask(raw, mwords[ci]);
+                        else detail::add_bias_relu(raw, bias_slots + (par * WPW + ci) * 32U);
+                        detail::pack_operands(raw, h, args.bf16 != 0U);
                         store_operand(act_t, cc, h);
                         publish(&ready_t[cc >> 1]);
+                        if (!BWD) words[ci] = detail::positive_bits(raw);
                         if (BWD) {
-                            const float total = detail::warp_column_sums(v, lane);
+                            const float total = column_sums(raw);
                             if (cc * 32U + lane < H) args.colsum[k * args.colsum_stride + (static_cast<uint64_t>(tile) * 4U + quad) * H + cc * 32U + lane] = total;
                         }
                     }
@@ -419,32 +434,28 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                         uint32_t raw[32];
                         tmem_ld_32x32(tmem_base + lane_addr + kStateCol + cc * 32U, raw);
                         tmem_ld_wait();
-                        float v[32];
-#pragma unroll
-                        for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
-                        if (BWD) apply_mask(v, mwords[ci]);
-                        else add_bias_relu(v, ci);
                         uint32_t h[16];
-                        words[ci] = detail::pack_halfs(v, h, args.bf16 != 0U);
+                        if (BWD) apply_mask(raw, mwords[ci]);
+                        else detail::add_bias_relu(raw, bias_slots + (par * WPW + ci) * 32U);
+                        detail::pack_operands(raw, h, args.bf16 != 0U);
                         if (!last) {
-#pragma unroll
-                            for (int j = 0; j < 32; ++j) raw[j] = __float_as_uint(v[j]);
                             tmem_st_32x32(tmem_base + lane_addr + kStateCol + cc * 32U, raw);
                             store_operand(act_s, cc, h);
                             tmem_st_wait();
                             publish(&ready_s[cc >> 1]);
                         }
+                        if (!BWD) words[ci] = detail::positive_bits(raw);
                         if (row_ok && last) {  // no MMA consumes the last S of a tile, so no panel store either
                             store_tape(tape_row, cc, h);
                             if (!BWD) {
                                 float4* dst = reinterpret_cast<float4*>(args.state_f32 + row * args.ld_f32 + cc * 32U);
 #pragma unroll
                                 for (int q = 0; q < 8; ++q)
-                                    if (cc * 32U + 4U * q < args.ld_f32) dst[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+                                    if (cc * 32U + 4U * q < args.ld_f32) dst[q] = make_float4(__uint_as_float(raw[4 * q]), __uint_as_float(raw[4 * q + 1]), __uint_as_float(raw[4 * q + 2]), __uint_as_float(raw[4 * q + 3]));
                             }
                         }
                         if (BWD) {
-                            const float total = detail::warp_column_sums(v, lane);
+                            const float total = column_sums(raw);
                             if (cc * 32U + lane < H) args.colsum[(R + k) * args.colsum_stride + (static_cast<uint64_t>(tile) * 4U + quad) * H + cc * 32U + lane] = total;
                         }
                     }
