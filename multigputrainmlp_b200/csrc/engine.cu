@@ -16,6 +16,7 @@
 #include "fp32_path.cuh"
 #include "onehot_pair.cuh"
 #include "tower_chain.cuh"
+#include "tower_wide.cuh"
 #include "umma_gemm.cuh"
 
 #include <cuda.h>
@@ -206,7 +207,7 @@ Workspace PlanWorkspace(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm_count,
     w.off_rowsum = take(w.rowsum_rows * s.hd1 * 4);
     w.ld_bits_h1 = (uint32_t)RoundUp((B + 31) / 32, 8);  // (32-byte rows)
     w.off_bits_h1 = take((uint64_t)s.hd1 * w.ld_bits_h1 * 4);
-    w.bits_stride = chain_tiles * 128 * 8;
+    w.bits_stride = chain_tiles * 128 * (s.hd2 > 256U ? 16 : 8);  // words: one per 32 of 256 columns, twice that in the wide tower
     w.off_bits = take(w.bits_stride * 4 * (2 * w.R + 1));
     // internal fp16 weight copy (used when the caller's mirror cannot be addressed by TMA as it lies)
     const uint64_t wint_halfs = (uint64_t)(w.IN + 1) * w.p_w1 + (uint64_t)s.hd1 * w.p_w2 + 2ULL * w.R * s.hd2 * w.p_w2 + (uint64_t)s.hd2 * w.p_wout;
@@ -1206,10 +1207,10 @@ mgt_status_t GemmBackpropInputRows(mgt_engine* e, cudaStream_t st, const __half*
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
 }
 
-// The residual tower in one launch per direction; see tower_chain.cuh. Shapes it takes: hd2 up to 256 (a tile's state and
-// product need two TMEM columns per hidden unit).
+// The residual tower in one launch per direction. hd2 up to 256: tower_chain.cuh, a CTA per tile of 128 samples (the tile's
+// state and product take two TMEM columns per hidden unit). Up to the largest width, 512: tower_wide.cuh, a pair of CTAs per tile.
 bool ChainEligible(const mgt_engine* e, const mgt_mlp_shape_t& s) {
-    return s.residual_blocks > 0 && s.hd2 <= 256U && !e->layered_tower;
+    return s.residual_blocks > 0 && !e->layered_tower;
 }
 
 template <bool BWD>
@@ -1220,19 +1221,23 @@ mgt_status_t LaunchChain(mgt_engine* e, cudaStream_t st, const __half* w_first, 
     {
         std::lock_guard<std::mutex> lock(attr_mu);
         if (e->device >= 0 && e->device < 64 && !attr_done[e->device]) {
-            if (cudaFuncSetAttribute(tower_chain_kernel<BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ChainCfg::SMEM_BYTES) != cudaSuccess) return MGT_CUDA_FAILURE;
+            if (cudaFuncSetAttribute(tower_chain_kernel<BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, ChainCfg::SMEM_BYTES) != cudaSuccess ||
+                cudaFuncSetAttribute(tower_wide_kernel<BWD>, cudaFuncAttributeMaxDynamicSharedMemorySize, WideCfg::SMEM_BYTES) != cudaSuccess) return MGT_CUDA_FAILURE;
             attr_done[e->device] = true;
         }
     }
+    const bool wide = a.H > 256U;
     CUtensorMap tw, ts, tt;
-    MGT_MAP(e->Map3D(&tw, w_first, a.H, a.H, 2ULL * a.R, w_pitch, w_layer_stride_bytes, 64, BWD ? (a.H + 31U) & ~31U : 64));
+    // (backward: a box of weight rows for the columns of one CTA)
+    MGT_MAP(e->Map3D(&tw, w_first, a.H, a.H, 2ULL * a.R, w_pitch, w_layer_stride_bytes, 64, !BWD ? 64U : (wide ? (a.H + 127U) / 128U * 64U : (a.H + 31U) & ~31U)));
     // the tapes as stacks of [samples][H] matrices; a store box is one operand panel: 64 columns x 128 rows
     MGT_MAP(e->Map3D(&ts, a.tape_s, a.H, a.samples, tape_s_entries, a.ld_s, a.tape_s_stride * 2, 64, 128));
     MGT_MAP(e->Map3D(&tt, a.tape_t, a.H, a.samples, tape_t_entries, a.ld_t, a.tape_t_stride * 2, 64, 128));
     a.status = e->status_word;
     a.bf16 = e->bf16_now ? 1U : 0U;
-    const uint32_t grid = a.tiles < (uint32_t)e->sm_count ? a.tiles : (uint32_t)e->sm_count;
-    tower_chain_kernel<BWD><<<grid, ChainCfg::THREADS, ChainCfg::SMEM_BYTES, st>>>(tw, ts, tt, a);
+    const uint32_t units = wide ? (uint32_t)e->sm_count / 2U : (uint32_t)e->sm_count, grid = a.tiles < units ? a.tiles : units;
+    if (wide) tower_wide_kernel<BWD><<<2U * grid, WideCfg::THREADS, WideCfg::SMEM_BYTES, st>>>(tw, ts, tt, a);
+    else tower_chain_kernel<BWD><<<grid, ChainCfg::THREADS, ChainCfg::SMEM_BYTES, st>>>(tw, ts, tt, a);
     ++e->launches;
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
 }

@@ -141,3 +141,11 @@ def test_embedding_forms(oracle, dims, n, mirror, bf16):
 @pytest.mark.parametrize("dims,n", [((72, 72, 1000, 16, 0, 1), 9001), ((54, 6, 4090, 16, 0, 1), 9000)])
 def test_one_hot_pairs(oracle, dims, n):
     loss_grad_case(oracle, dims, n)
+
+
+# residual tower for pairs of CTAs (hd2 above 256): unequal halves, a second half of one chunk, whole panels, ragged tiles
+@pytest.mark.parametrize("hd2,n,mirror", [(257, 130, False), (264, 128, True), (320, 129, True), (390, 300, False), (512, 257, True)])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_wide_residual_tower(oracle, hd2, n, mirror, bf16):
+    loss_grad_case(oracle, (72, 72, 48, hd2, 3, 1), n, scale=0.02, mirror=mirror, options=dict(bf16=True) if bf16 else None, tol=8e-3 if bf16 else 1e-3,
+                   section_tol=2e-2 if bf16 else 3e-3)
