@@ -114,18 +114,24 @@ __device__ __forceinline__ void tmem_alloc(uint32_t* smem_holder, uint32_t colum
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t columns) {
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(columns) : "memory");
 }
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// (predicated for a converged warp: see ptx::umma_f16)
+__device__ __forceinline__ void umma_f16(uint32_t lead, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead)
         : "memory");
 }
 // arrives on the barrier at this offset in both CTAs once every MMA issued so far by this thread has completed
-__device__ __forceinline__ void umma_commit_both(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(ptx::smem_u32(bar)), "h"(static_cast<uint16_t>(3))
-                 : "memory");
+__device__ __forceinline__ void umma_commit_both(uint32_t lead, uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %2, 0;\n\t"
+        "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+        ::"r"(ptx::smem_u32(bar)), "h"(static_cast<uint16_t>(3)), "r"(lead)
+        : "memory");
 }
 
 // One piece of a pair's stretch: 256 rows from mt * 256, columns [n0, n0 + cols), K chunks [c0, c1).
@@ -242,11 +248,12 @@ onehot_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------- MMA issuer: one thread of the pair ---------------
-        if (lane == 0 && rank == 0U) {
+        if (rank == 0U) {
+            const uint32_t lead = elect_one();
             uint32_t it = 0, unit = 0;
             bool ok = true;
             while (ok && pieces.next(p)) {
-                if (!mbar_wait_spin(acc_empty, (unit & 1U) ^ 1U, cta_abort, kAbortMmaWait)) { ok = false; break; }
+                if (!mbar_wait_warp(acc_empty, (unit & 1U) ^ 1U, cta_abort, kAbortMmaWait)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t cols0 = min(256U, p.cols), cols1 = p.cols - cols0;
                 const uint32_t idesc0 = make_idesc_f16(256, cols0, !GRAD, false, args.bf16 != 0U);
@@ -254,7 +261,7 @@ onehot_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
                 for (uint32_t c = p.c0; c < p.c1; ++c, ++it) {
                     const uint32_t s = it % ST;
                     // (one wait and one commit a chunk: with separate rings for A and B, two of each, a chunk took 170 cycles more)
-                    if (!mbar_wait_spin(&full[s], (it / ST) & 1U, cta_abort, kAbortMmaWait)) { ok = false; break; }
+                    if (!mbar_wait_warp(&full[s], (it / ST) & 1U, cta_abort, kAbortMmaWait)) { ok = false; break; }
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(smem + s * PairCfg<GRAD>::STAGE_BYTES), b_addr = a_addr + PairCfg<GRAD>::A_BYTES;
                     const uint32_t k_left = args.K - c * 64U;
@@ -266,17 +273,17 @@ onehot_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
                     const uint32_t first = c > p.c0 ? 1U : 0U;
                     if (ksteps == 4U && cols1 != 0U) {
 #pragma unroll
-                        for (uint32_t kk = 0; kk < 4U; ++kk) pair::umma_f16(tmem_base, a_desc + kk * kStepA, b_desc0 + kk * kStepB, idesc0, kk == 0U ? first : 1U);
+                        for (uint32_t kk = 0; kk < 4U; ++kk) pair::umma_f16(lead, tmem_base, a_desc + kk * kStepA, b_desc0 + kk * kStepB, idesc0, kk == 0U ? first : 1U);
 #pragma unroll
-                        for (uint32_t kk = 0; kk < 4U; ++kk) pair::umma_f16(tmem_base + 256U, a_desc + kk * kStepA, b_desc1 + kk * kStepB, idesc1, kk == 0U ? first : 1U);
+                        for (uint32_t kk = 0; kk < 4U; ++kk) pair::umma_f16(lead, tmem_base + 256U, a_desc + kk * kStepA, b_desc1 + kk * kStepB, idesc1, kk == 0U ? first : 1U);
                     } else {
-                        for (uint32_t kk = 0; kk < ksteps; ++kk) pair::umma_f16(tmem_base, a_desc + kk * kStepA, b_desc0 + kk * kStepB, idesc0, kk == 0U ? first : 1U);
+                        for (uint32_t kk = 0; kk < ksteps; ++kk) pair::umma_f16(lead, tmem_base, a_desc + kk * kStepA, b_desc0 + kk * kStepB, idesc0, kk == 0U ? first : 1U);
                         if (cols1 != 0U)
-                            for (uint32_t kk = 0; kk < ksteps; ++kk) pair::umma_f16(tmem_base + 256U, a_desc + kk * kStepA, b_desc1 + kk * kStepB, idesc1, kk == 0U ? first : 1U);
+                            for (uint32_t kk = 0; kk < ksteps; ++kk) pair::umma_f16(lead, tmem_base + 256U, a_desc + kk * kStepA, b_desc1 + kk * kStepB, idesc1, kk == 0U ? first : 1U);
                     }
-                    pair::umma_commit_both(&empty[s]);
+                    pair::umma_commit_both(lead, &empty[s]);
                 }
-                if (ok) pair::umma_commit_both(acc_full);
+                if (ok) pair::umma_commit_both(lead, acc_full);
                 ++unit;
             }
         }

@@ -105,6 +105,32 @@ __device__ __forceinline__ bool mbar_wait_spin(uint64_t* bar, uint32_t parity, v
     return true;
 }
 
+// For a whole warp, which stays converged: the vote makes the answer the same for all lanes, and known to be.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* cta_abort, int code) {
+    if (__all_sync(0xFFFFFFFFU, mbar_try_wait(bar, parity))) return true;
+    uint64_t start = 0;
+    uint32_t spins = 0;
+    while (!__all_sync(0xFFFFFFFFU, mbar_try_wait(bar, parity))) {
+        if ((++spins & 63U) == 0U) {
+            const uint64_t now = global_timer_ns();
+            if (start == 0) start = now;
+            if (__any_sync(0xFFFFFFFFU, *cta_abort != 0)) return false;
+            if (__any_sync(0xFFFFFFFFU, now - start > kWaitLimitNs)) {
+                *cta_abort = code;
+                return false;
+            }
+        }
+    }
+    return true;
+}
+
+// true in one lane of a converged warp
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t lead;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xFFFFFFFF;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(lead));
+    return lead;
+}
+
 // Named barrier over `threads` threads (a multiple of 32); id 0 is __syncthreads' own barrier.
 __device__ __forceinline__ void named_bar_sync(uint32_t id, uint32_t threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
@@ -168,18 +194,28 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t columns) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// D[tmem] (+)= A[smem] * B[smem], fp16 inputs, fp32 accumulate, issued by ONE thread.
-__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+// D[tmem] (+)= A[smem] * B[smem], 16-bit inputs, fp32 accumulate, issued by the lane of the warp whose `lead` is set.
+//
+// The whole issuing warp runs the loop around its MMAs, waits included, and the instructions that one thread has to issue are
+// predicated. Descriptors and addresses are then uniform values to the compiler; inside a branch that a single lane takes each
+// has to be moved to a uniform register on its own. A chunk of four MMAs of 128 x 128 x 16 (256 cycles), a commit and one
+// wait on a barrier that is already open: 472 cycles in a one-lane loop, 316 with the waits of the whole warp, 256 like this.
+__device__ __forceinline__ void umma_f16(uint32_t lead, uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\t"
+        "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+        ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(lead)
         : "memory");
 }
 // Arrives on the mbarrier once every UMMA issued so far by this thread has completed.
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void umma_commit(uint32_t lead, uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %1, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(lead)
+        : "memory");
 }
 
 // 32 lanes x 32 consecutive 32-bit columns: thread t of the warp receives lane (base_lane + t).
@@ -192,6 +228,17 @@ __device__ __forceinline__ void tmem_ld_32x32(uint32_t taddr, uint32_t (&r)[32])
           "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
           "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
           "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr)
+        : "memory");
+}
+// 16 lanes x 32 consecutive columns: thread t receives, for columns 8 q + 2 (t % 4) + {0, 1}, row t / 4 in r[4 q], r[4 q + 1] and
+// row t / 4 + 8 in r[4 q + 2], r[4 q + 3].
+__device__ __forceinline__ void tmem_ld_16x256(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.16x256b.x4.b32 "
+        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
+          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
         : "r"(taddr)
         : "memory");
 }

@@ -205,7 +205,8 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------- UMMA issuer --------------------------------------
-        if (lane == 0) {
+        {
+            const uint32_t lead = elect_one();
             const uint32_t idesc = make_idesc_f16(128, HP, false, !BWD, args.bf16 != 0U);
             uint32_t it = 0, uses = 0;
             bool ok = true;
@@ -217,16 +218,15 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                         const uint32_t d_addr = tmem_base + (half ? kStateCol : 0U);
                         for (uint32_t c = 0; c < KC; ++c, ++it) {
                             const uint32_t s = it % SW, ph = (it / SW) & 1U;
-                            // (the issuing thread polls its barriers: waking from a suspended wait costs more than the hand-over itself)
-                            if (!mbar_wait_spin(&ready[c], uses & 1U, cta_abort, kAbortChainWait)) { ok = false; break; }
-                            if (!mbar_wait_spin(&w_full[s], ph, cta_abort, kAbortChainWait)) { ok = false; break; }
+                            if (!mbar_wait_warp(&ready[c], uses & 1U, cta_abort, kAbortChainWait)) { ok = false; break; }
+                            if (!mbar_wait_warp(&w_full[s], ph, cta_abort, kAbortChainWait)) { ok = false; break; }
                             tc_fence_after();
                             const uint32_t a_addr = a_base + c * 16384U;
                             const uint32_t b_addr = smem_u32(w_ring + s * ChainCfg::W_STAGE_BYTES);
                             const uint32_t k_left = H - c * 64U;
                             const uint32_t ksteps = k_left >= 64U ? 4U : (k_left + 15U) / 16U;
                             // descriptors of the chunk's first K step; a later step only moves the start address (units of 16
-                            // bytes, no carry out of the field). One thread issues everything: the full chunk is unrolled.
+                            // bytes, no carry out of the field).
                             const uint64_t a_desc0 = make_smem_desc(a_addr, 16U, 1024U);
                             const uint64_t b_desc0 = BWD ? make_smem_desc(b_addr, 16U, 1024U) : make_smem_desc(b_addr, 8192U, 1024U);
                             constexpr uint64_t kStepA = 32U / 16U, kStepB = BWD ? 32U / 16U : 2048U / 16U;
@@ -234,19 +234,19 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                             const uint32_t first = (half != 0U || c > 0U) ? 1U : 0U;
                             if (ksteps == 4U) {
 #pragma unroll
-                                for (uint32_t kk = 0; kk < 4U; ++kk) umma_f16(d_addr, a_desc0 + kk * kStepA, b_desc0 + kk * kStepB, idesc, kk == 0U ? first : 1U);
+                                for (uint32_t kk = 0; kk < 4U; ++kk) umma_f16(lead, d_addr, a_desc0 + kk * kStepA, b_desc0 + kk * kStepB, idesc, kk == 0U ? first : 1U);
                             } else {
-                                for (uint32_t kk = 0; kk < ksteps; ++kk) umma_f16(d_addr, a_desc0 + kk * kStepA, b_desc0 + kk * kStepB, idesc, kk == 0U ? first : 1U);
+                                for (uint32_t kk = 0; kk < ksteps; ++kk) umma_f16(lead, d_addr, a_desc0 + kk * kStepA, b_desc0 + kk * kStepB, idesc, kk == 0U ? first : 1U);
                             }
-                            umma_commit(&w_empty[s]);
+                            umma_commit(lead, &w_empty[s]);
                         }
                         // the epilogue this commit releases overwrites the operand the PREVIOUS phase read and stored
                         bulk_wait_read_all();
-                        if (ok) umma_commit(&mma_done[half]);
+                        if (ok) umma_commit(lead, &mma_done[half]);
                         // Each operand panel is also a 64-column slice of a tape entry: T of this block, or the S the previous
                         // block produced (the S a tile starts with is on its tape already). Issued here, after the commit,
                         // the stores cost the MMA stream nothing.
-                        if (ok && (half != 0U || kb > 0U)) {
+                        if (ok && lead && (half != 0U || kb > 0U)) {
                             const uint32_t k = BWD ? R - 1U - kb : kb;
                             const uint32_t entry = half ? k : (BWD ? k + 1U : k);
                             for (uint32_t c = 0; c < KC; ++c)

@@ -35,9 +35,13 @@ struct WideCfg {
 namespace detail {
 
 // arrives on the barrier at this offset in both CTAs of the cluster once every MMA of this CTA issued so far has completed
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(ptx::smem_u32(bar)), "h"(static_cast<uint16_t>(3))
-                 : "memory");
+__device__ __forceinline__ void umma_commit_pair(uint32_t lead, uint64_t* bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.b32 q, %2, 0;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+        ::"r"(ptx::smem_u32(bar)), "h"(static_cast<uint16_t>(3)), "r"(lead)
+        : "memory");
 }
 // shared memory of this CTA -> shared memory of another, bytes counted on a barrier there
 __device__ __forceinline__ void copy_to_cluster(uint32_t dst_cluster, uint32_t src, uint32_t bytes, uint32_t bar_cluster) {
@@ -140,7 +144,8 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------- UMMA issuer --------------------------------------
-        if (lane == 0) {
+        {
+            const uint32_t lead = elect_one();
             const uint32_t idesc = make_idesc_f16(128, NC * 32U, false, !BWD, args.bf16 != 0U);
             uint32_t it = 0, step = 0;
             bool ok = true;
@@ -150,20 +155,19 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
                         const uint32_t a_base = smem_u32(act);
                         const uint32_t d_addr = tmem_base + (half ? kStateCol : 0U);
                         for (uint32_t c = 0; c < KC; ++c)
-                            if (!mine(c)) mbar_arrive_expect_tx(&ready[c], 16384U);
+                            if (lead && !mine(c)) mbar_arrive_expect_tx(&ready[c], 16384U);
                         for (uint32_t i = 0; i < KC; ++i, ++it) {
                             const uint32_t c = chunk_at(i);
                             const uint32_t s = it % SW, ph = (it / SW) & 1U;
-                            // (the issuing thread polls its barriers: waking from a suspended wait costs more than the hand-over itself)
-                            if (!mbar_wait_spin(&ready[c], step & 1U, cta_abort, kAbortChainWait)) { ok = false; break; }
-                            if (!mbar_wait_spin(&w_full[s], ph, cta_abort, kAbortChainWait)) { ok = false; break; }
+                            if (!mbar_wait_warp(&ready[c], step & 1U, cta_abort, kAbortChainWait)) { ok = false; break; }
+                            if (!mbar_wait_warp(&w_full[s], ph, cta_abort, kAbortChainWait)) { ok = false; break; }
                             tc_fence_after();
                             const uint32_t a_addr = a_base + c * 16384U;
                             const uint32_t b_addr = smem_u32(w_ring + s * WideCfg::W_STAGE_BYTES);
                             const uint32_t k_left = H - c * 64U;
                             const uint32_t ksteps = k_left >= 64U ? 4U : (k_left + 15U) / 16U;
                             // descriptors of the chunk's first K step; a later step only moves the start address (units of 16
-                            // bytes, no carry out of the field). One thread issues everything: the full chunk is unrolled.
+                            // bytes, no carry out of the field).
                             const uint64_t a_desc0 = make_smem_desc(a_addr, 16U, 1024U);
                             const uint64_t b_desc0 = BWD ? make_smem_desc(b_addr, 16U, 1024U) : make_smem_desc(b_addr, 8192U, 1024U);
                             constexpr uint64_t kStepA = 32U / 16U, kStepB = BWD ? 32U / 16U : 2048U / 16U;
@@ -171,13 +175,13 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
                             const uint32_t first = (half != 0U || i > 0U) ? 1U : 0U;
                             if (ksteps == 4U) {
 #pragma unroll
-                                for (uint32_t kk = 0; kk < 4U; ++kk) umma_f16(d_addr, a_desc0 + kk * kStepA, b_desc0 + kk * kStepB, idesc, kk == 0U ? first : 1U);
+                                for (uint32_t kk = 0; kk < 4U; ++kk) umma_f16(lead, d_addr, a_desc0 + kk * kStepA, b_desc0 + kk * kStepB, idesc, kk == 0U ? first : 1U);
                             } else {
-                                for (uint32_t kk = 0; kk < ksteps; ++kk) umma_f16(d_addr, a_desc0 + kk * kStepA, b_desc0 + kk * kStepB, idesc, kk == 0U ? first : 1U);
+                                for (uint32_t kk = 0; kk < ksteps; ++kk) umma_f16(lead, d_addr, a_desc0 + kk * kStepA, b_desc0 + kk * kStepB, idesc, kk == 0U ? first : 1U);
                             }
-                            umma_commit(&w_empty[s]);
+                            umma_commit(lead, &w_empty[s]);
                         }
-                        if (ok) detail::umma_commit_pair(&mma_done[half]);
+                        if (ok) detail::umma_commit_pair(lead, &mma_done[half]);
                     }
                 }
             }

@@ -298,7 +298,8 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         __syncwarp();
     } else if (warp == 1) {
         // ------------------------------- UMMA issuer --------------------------------------
-        if (lane == 0) {
+        {
+            const uint32_t lead = elect_one();
             const uint32_t idesc = make_idesc_f16(BM, BN, Cfg::A_MN, Cfg::B_MN, args.bf16 != 0U);
             uint32_t it = 0, unit_iter = 0;
             bool ok = true;
@@ -307,16 +308,15 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                 decode(unit, mt, nt, sp);
                 const uint32_t c0 = chunk_begin(sp), c1 = chunk_begin(sp + 1);
                 const uint32_t ab = unit_iter % ACC_BUFS, aph = (unit_iter / ACC_BUFS) & 1U;
-                if (!mbar_wait_spin(&acc_empty[ab], aph ^ 1U, cta_abort, kAbortMmaWait)) { ok = false; break; }
+                if (!mbar_wait_warp(&acc_empty[ab], aph ^ 1U, cta_abort, kAbortMmaWait)) { ok = false; break; }
                 tc_fence_after();
                 const uint32_t d_base = tmem_base + ab * Cfg::ACC_COLS;
                 for (uint32_t c = c0; c < c1; ++c, ++it) {
                     const uint32_t sa = it % SA, pa = (it / SA) & 1U;
                     const uint32_t sb = Cfg::BSTAT ? (c - c0) : it % SB, pb = Cfg::BSTAT ? 0U : (it / SB) & 1U;
-                    // (the issuing thread polls its barriers: waking from a suspended wait costs more than the hand-over itself)
-                    if (!mbar_wait_spin(&full_a[sa], pa, cta_abort, kAbortMmaWait)) { ok = false; break; }
+                    if (!mbar_wait_warp(&full_a[sa], pa, cta_abort, kAbortMmaWait)) { ok = false; break; }
                     if (!Cfg::BSTAT || unit == blockIdx.x) {
-                        if (!mbar_wait_spin(&full_b[sb], pb, cta_abort, kAbortMmaWait)) { ok = false; break; }
+                        if (!mbar_wait_warp(&full_b[sb], pb, cta_abort, kAbortMmaWait)) { ok = false; break; }
                     }
                     tc_fence_after();
                     const uint32_t a_addr = smem_u32(a_ring + sa * Cfg::A_STAGE_BYTES);
@@ -324,22 +324,22 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                     const uint32_t k_left = args.K - c * 64U;
                     const uint32_t ksteps = k_left >= 64U ? 4U : (k_left + 15U) / 16U;
                     // Descriptors of the chunk's first K step; a later step only moves the start address (bits [0,14) in
-                    // units of 16 bytes, no carry: shared-memory addresses are below 2^18). One thread issues everything,
-                    // so the fewer dependent instructions stand between two MMAs the better: the full chunk is unrolled.
+                    // units of 16 bytes, no carry: shared-memory addresses are below 2^18). The fewer
+                    // dependent instructions stand between two MMAs the better: the full chunk is unrolled.
                     constexpr uint64_t kStepA = Cfg::A_MN ? 2048U / 16U : 32U / 16U, kStepB = Cfg::B_MN ? 2048U / 16U : 32U / 16U;
                     const uint64_t a_desc0 = Cfg::A_MN ? make_smem_desc(a_addr, 8192U, 1024U) : make_smem_desc(a_addr, 16U, 1024U);
                     const uint32_t first = c > c0 ? 1U : 0U;
                     const uint64_t b_desc0 = Cfg::B_MN ? make_smem_desc(b_addr, 8192U, 1024U) : make_smem_desc(b_addr, 16U, 1024U);
                     if (ksteps == 4U) {
 #pragma unroll
-                        for (uint32_t kk = 0; kk < 4U; ++kk) umma_f16(d_base, a_desc0 + kk * kStepA, b_desc0 + kk * kStepB, idesc, kk == 0U ? first : 1U);
+                        for (uint32_t kk = 0; kk < 4U; ++kk) umma_f16(lead, d_base, a_desc0 + kk * kStepA, b_desc0 + kk * kStepB, idesc, kk == 0U ? first : 1U);
                     } else {
-                        for (uint32_t kk = 0; kk < ksteps; ++kk) umma_f16(d_base, a_desc0 + kk * kStepA, b_desc0 + kk * kStepB, idesc, kk == 0U ? first : 1U);
+                        for (uint32_t kk = 0; kk < ksteps; ++kk) umma_f16(lead, d_base, a_desc0 + kk * kStepA, b_desc0 + kk * kStepB, idesc, kk == 0U ? first : 1U);
                     }
-                    umma_commit(&empty_a[sa]);
-                    if (!Cfg::BSTAT) umma_commit(&empty_b[sb]);
+                    umma_commit(lead, &empty_a[sa]);
+                    if (!Cfg::BSTAT) umma_commit(lead, &empty_b[sb]);
                 }
-                if (ok) umma_commit(&acc_full[ab]);
+                if (ok) umma_commit(lead, &acc_full[ab]);
             }
         }
         __syncwarp();
