@@ -58,26 +58,37 @@ struct ChainCfg {
     static constexpr int SW = 3;                    // weight ring stages
     static constexpr int ACT_BYTES = 4 * 16384;     // one operand: up to four 64-column panels of 128 rows x 128 bytes
     static constexpr int W_STAGE_BYTES = 32768;
-    static constexpr int SMEM_BYTES = 1024 + 2 * ACT_BYTES + SW * W_STAGE_BYTES + 256 + 1024;  // + barriers + bias slices
+    static constexpr int SMEM_BYTES = 2 * ACT_BYTES + SW * W_STAGE_BYTES + 256 + 2048;  // + barriers + bias slices
     static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 };
 
 namespace detail {
 
-// Sum over the 32 lanes of a warp of each of 32 per-lane values: afterwards lane L holds the sum of v[L] over
-// all lanes (a fixed tree, so the result does not depend on timing). Destroys v.
-__device__ __forceinline__ float warp_column_sums(float (&v)[32], uint32_t lane) {
+// Sums over the 32 rows of a TMEM lane quadrant of 32 consecutive columns; the lane's column is returned, a fixed tree. Read in the
+// 16x256b form a thread has four rows of eight columns, so that seven shuffles finish the sum (a row a thread: 31).
+__device__ __forceinline__ float column_sums(uint32_t taddr, uint32_t lane, uint32_t* column) {
+    uint32_t a[16], b[16];
+    ptx::tmem_ld_16x256(taddr, a);
+    ptx::tmem_ld_16x256(taddr + (16U << 16), b);
+    ptx::tmem_ld_wait();
+    float s[8];  // columns 8 q + 2 (lane % 4) + e at 2 q + e
 #pragma unroll
-    for (int w = 16; w >= 1; w >>= 1) {
-        const bool hi = (lane & static_cast<uint32_t>(w)) != 0U;
+    for (int i = 0; i < 8; ++i) {
+        const int j = (i >> 1) * 4 + (i & 1);
+        s[i] = (__uint_as_float(a[j]) + __uint_as_float(a[j + 2])) + (__uint_as_float(b[j]) + __uint_as_float(b[j + 2]));
+    }
+#pragma unroll
+    for (int w = 4; w >= 1; w >>= 1) {  // lane bits 4, 3, 2
+        const bool hi = (lane & static_cast<uint32_t>(4 * w)) != 0U;
 #pragma unroll
         for (int j = 0; j < w; ++j) {
-            const float send = hi ? v[j] : v[j + w];
-            const float keep = hi ? v[j + w] : v[j];
-            v[j] = keep + __shfl_xor_sync(0xFFFFFFFFU, send, w);
+            const float send = hi ? s[j] : s[j + w];
+            const float keep = hi ? s[j + w] : s[j];
+            s[j] = keep + __shfl_xor_sync(0xFFFFFFFFU, send, 4 * w);
         }
     }
-    return v[0];
+    *column = ((lane >> 4) & 1U) * 16U + ((lane >> 3) & 1U) * 8U + ((lane & 3U) << 1) + ((lane >> 2) & 1U);
+    return s[0];
 }
 
 // The "is positive" bit of each of 32 values, taken from the fp32 value as the reference takes its ReLU masks
@@ -125,9 +136,8 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
     constexpr int SW = ChainCfg::SW;
     constexpr uint32_t kStateCol = 256;  // first TMEM column of S
 
-    extern __shared__ uint8_t smem_raw[];
-    const uint32_t raw_addr = smem_u32(smem_raw);
-    uint8_t* smem = smem_raw + (((raw_addr + 1023U) & ~1023U) - raw_addr);
+    extern __shared__ __align__(1024) uint8_t tower_smem[];
+    uint8_t* smem = tower_smem;
     uint8_t* act_s = smem;                           // fp16 copy of S, the A operand of the first MMA of a block
     uint8_t* act_t = smem + ChainCfg::ACT_BYTES;     // fp16 T, the A operand of the second
     uint8_t* w_ring = smem + 2 * ChainCfg::ACT_BYTES;
@@ -139,7 +149,7 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
     uint64_t* mma_done = ready_t + 4;   // [2] D complete / S complete
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(mma_done + 2);
     volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_holder + 1);
-    float* bias_slots = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);  // [warps per quadrant][chunks per warp][32]
+    float* bias_slots = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);  // [products of a block][warps per quadrant][chunks per warp][32]
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31U;
     const uint32_t H = args.H, R = args.R;
@@ -295,24 +305,17 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
             __syncwarp();
             if (lane == 0) mbar_arrive(bar);
         };
-        // Bias of a layer: each lane fetches one value per chunk of its warp before the warp waits for the MMAs (the
-        // load flies during the wait); after the wait the values go through a shared-memory slot so that every
-        // thread can read all 32 of a chunk as broadcast vectors. The warps of one quadrant set share slots and write
-        // identical values; a slot is rewritten only after the MMAs that needed every warp's previous epilogue.
-        float bias_reg[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        auto fetch_bias = [&](uint32_t layer) {
+        // Bias of a layer: before the warp waits for the MMAs each lane fetches one value per chunk of its warp into a shared-memory
+        // slot, so that every thread can read all 32 of a chunk as broadcast vectors. The warps of one quadrant set share
+        // slots and write identical values; a slot is rewritten two products later, after MMAs that needed every warp's
+        // epilogue in between.
+        auto stage_bias = [&](uint32_t layer) {
             if (!BWD) {
 #pragma unroll
                 for (uint32_t ci = 0; ci < WPW; ++ci) {
                     const uint32_t cc = par + SUBS * ci;
-                    bias_reg[ci] = cc * 32U + lane < H ? __ldg(args.bias + layer * args.bias_stride + cc * 32U + lane) : 0.0f;
+                    bias_slots[(layer & 1U) * 256U + (par * WPW + ci) * 32U + lane] = cc * 32U + lane < H ? __ldg(args.bias + layer * args.bias_stride + cc * 32U + lane) : 0.0f;
                 }
-            }
-        };
-        auto stage_bias = [&]() {
-            if (!BWD) {
-#pragma unroll
-                for (uint32_t ci = 0; ci < WPW; ++ci) bias_slots[(par * WPW + ci) * 32U + lane] = bias_reg[ci];
                 __syncwarp();
             }
         };
@@ -333,11 +336,18 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(((bits >> j) & 1U) ? __uint_as_float(v[j]) : 0.0f);
         };
-        auto column_sums = [&](const uint32_t (&raw)[32]) {
-            float v[32];
+        // bias sums of a product (its columns from `taddr` on), when the panels are handed on
+        auto column_sums = [&](uint32_t taddr, uint32_t tile, uint32_t slot) {
+            tmem_st_wait();
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
-            return detail::warp_column_sums(v, lane);
+            for (uint32_t ci = 0; ci < WPW; ++ci) {
+                const uint32_t cc = par + SUBS * ci;
+                if (cc >= NC) break;
+                uint32_t j;
+                const float total = detail::column_sums(taddr + cc * 32U, lane, &j);
+                const uint32_t col = cc * 32U + j;
+                if (col < H) args.colsum[slot * args.colsum_stride + (static_cast<uint64_t>(tile) * 4U + quad) * H + col] = total;
+            }
         };
 
         uint32_t uses = 0;
@@ -391,10 +401,9 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                     uint32_t mwords[4] = {0, 0, 0, 0};
                     if (BWD) load_words(args.bits_t + k * args.bits_stride + bits_row, mwords);
                     uint32_t words[4] = {0, 0, 0, 0};  // the first WPW are used
-                    fetch_bias(2U * k);
+                    stage_bias(2U * k);
                     if (!warp_wait(&mma_done[0], uses & 1U)) { ok = false; break; }
                     tc_fence_after();
-                    stage_bias();
 #pragma unroll
                     for (uint32_t ci = 0; ci < WPW; ++ci) {
                         const uint32_t cc = par + SUBS * ci;
@@ -403,17 +412,18 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                         tmem_ld_32x32(tmem_base + lane_addr + cc * 32U, raw);
                         tmem_ld_wait();
                         uint32_t h[16];
-                        if (BWD) apply_mask(raw, mwords[ci]);
-                        else detail::add_bias_relu(raw, bias_slots + (par * WPW + ci) * 32U);
+                        if (BWD) {
+                            apply_mask(raw, mwords[ci]);
+                            tmem_st_32x32(tmem_base + lane_addr + cc * 32U, raw);  // (for the column sums)
+                        } else {
+                            detail::add_bias_relu(raw, bias_slots + (par * WPW + ci) * 32U);
+                        }
                         detail::pack_operands(raw, h, args.bf16 != 0U);
                         store_operand(act_t, cc, h);
                         publish(&ready_t[cc >> 1]);
                         if (!BWD) words[ci] = detail::positive_bits(raw);
-                        if (BWD) {
-                            const float total = column_sums(raw);
-                            if (cc * 32U + lane < H) args.colsum[k * args.colsum_stride + (static_cast<uint64_t>(tile) * 4U + quad) * H + cc * 32U + lane] = total;
-                        }
                     }
+                    if (BWD) column_sums(tmem_base + lane_addr, tile, k);
                     if (!BWD) store_words(args.bits_t + k * args.bits_stride + bits_row, words);
                 }
                 // ================= second epilogue: new S =================
@@ -421,10 +431,9 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                     uint32_t mwords[4] = {0, 0, 0, 0};
                     if (BWD) load_words(args.bits_s + k * args.bits_stride + bits_row, mwords);
                     uint32_t words[4] = {0, 0, 0, 0};  // the first WPW are used
-                    fetch_bias(2U * k + 1U);
+                    stage_bias(2U * k + 1U);
                     if (!warp_wait(&mma_done[1], uses & 1U)) { ok = false; break; }
                     tc_fence_after();
-                    stage_bias();
                     const uint32_t entry = BWD ? k : k + 1U;
                     __half* tape_row = args.tape_s + entry * args.tape_s_stride + row * args.ld_s;
 #pragma unroll
@@ -436,10 +445,10 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                         tmem_ld_wait();
                         uint32_t h[16];
                         if (BWD) apply_mask(raw, mwords[ci]);
-                        else detail::add_bias_relu(raw, bias_slots + (par * WPW + ci) * 32U);
+                        else detail::add_bias_relu(raw, bias_slots + 256U + (par * WPW + ci) * 32U);
                         detail::pack_operands(raw, h, args.bf16 != 0U);
+                        if (BWD || !last) tmem_st_32x32(tmem_base + lane_addr + kStateCol + cc * 32U, raw);
                         if (!last) {
-                            tmem_st_32x32(tmem_base + lane_addr + kStateCol + cc * 32U, raw);
                             store_operand(act_s, cc, h);
                             tmem_st_wait();
                             publish(&ready_s[cc >> 1]);
@@ -454,11 +463,8 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                                     if (cc * 32U + 4U * q < args.ld_f32) dst[q] = make_float4(__uint_as_float(raw[4 * q]), __uint_as_float(raw[4 * q + 1]), __uint_as_float(raw[4 * q + 2]), __uint_as_float(raw[4 * q + 3]));
                             }
                         }
-                        if (BWD) {
-                            const float total = column_sums(raw);
-                            if (cc * 32U + lane < H) args.colsum[(R + k) * args.colsum_stride + (static_cast<uint64_t>(tile) * 4U + quad) * H + cc * 32U + lane] = total;
-                        }
                     }
+                    if (BWD) column_sums(tmem_base + lane_addr + kStateCol, tile, R + k);
                     if (!BWD) store_words(args.bits_s + (k + 1U) * args.bits_stride + bits_row, words);
                     if (last) tc_fence_before();  // the next tile's state load overwrites the TMEM columns read here
                 }

@@ -28,7 +28,7 @@ struct WideCfg {
     static constexpr int SW = 3;                    // weight ring stages
     static constexpr int ACT_BYTES = 8 * 16384;     // the operand: up to eight 64-column panels of 128 rows x 128 bytes
     static constexpr int W_STAGE_BYTES = 32768;
-    static constexpr int SMEM_BYTES = 1024 + ACT_BYTES + SW * W_STAGE_BYTES + 256 + 1024;  // + barriers + bias slices
+    static constexpr int SMEM_BYTES = ACT_BYTES + SW * W_STAGE_BYTES + 256 + 2048;  // + barriers + bias slices
     static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 };
 
@@ -58,9 +58,8 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
     constexpr int SW = WideCfg::SW;
     constexpr uint32_t kStateCol = 256;  // first TMEM column of S
 
-    extern __shared__ uint8_t smem_raw[];
-    const uint32_t raw_addr = smem_u32(smem_raw);
-    uint8_t* smem = smem_raw + (((raw_addr + 1023U) & ~1023U) - raw_addr);
+    extern __shared__ __align__(1024) uint8_t tower_smem[];
+    uint8_t* smem = tower_smem;
     uint8_t* act = smem;                            // the A operand of the MMA at hand: S or T rounded, all H columns
     uint8_t* w_ring = smem + WideCfg::ACT_BYTES;
     uint64_t* bars = reinterpret_cast<uint64_t*>(w_ring + SW * WideCfg::W_STAGE_BYTES);
@@ -70,7 +69,7 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
     uint64_t* mma_done = ready + 8;     // [2] D / S complete in both CTAs and the operand's panels stored
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(mma_done + 2);
     volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_holder + 1);
-    float* bias_slots = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);  // [warps per quadrant][chunks per warp][32]
+    float* bias_slots = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);  // [products of a block][warps per quadrant][chunks per warp][32]
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31U;
     const uint32_t H = args.H, R = args.R, rank = pair::cluster_rank();
@@ -205,10 +204,11 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
                             if (!mbar_wait_spin(&ready[c], step & 1U, cta_abort, kAbortChainWait)) { ok = false; break; }
                             const uint32_t src = smem_u32(act + c * 16384U);
                             detail::copy_to_cluster(pair::map_to(src, rank ^ 1U), src, 16384U, pair::map_to(smem_u32(&ready[c]), rank ^ 1U));
-                            if (half != 0U || kb > 0U)
+                        }
+                        if (ok && (half != 0U || kb > 0U))  // (behind the copies: the other CTA waits for them)
+                            for (uint32_t c = p0; c < p0 + PC; ++c)
                                 tma_store_3d(half ? &tma_tape_t : &tma_tape_s, act + c * 16384U, static_cast<int32_t>(c * 64U), static_cast<int32_t>(tile * 128U),
                                              static_cast<int32_t>(entry));
-                        }
                         bulk_commit_group();
                         bulk_wait_read_all();  // the epilogue that follows overwrites the panels
                         if (ok) mbar_arrive(&mma_done[half]);
@@ -253,24 +253,17 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
             __syncwarp();
             if (lane == 0) mbar_arrive(bar);
         };
-        // Bias of a layer: each lane fetches one value per chunk of its warp before the warp waits for the MMAs (the
-        // load flies during the wait); after the wait the values go through a shared-memory slot so that every
-        // thread can read all 32 of a chunk as broadcast vectors. The warps of one quadrant set share slots and write
-        // identical values; a slot is rewritten only after the MMAs that needed every warp's previous epilogue.
-        float bias_reg[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-        auto fetch_bias = [&](uint32_t layer) {
+        // Bias of a layer: before the warp waits for the MMAs each lane fetches one value per chunk of its warp into a shared-memory
+        // slot, so that every thread can read all 32 of a chunk as broadcast vectors. The warps of one quadrant set share
+        // slots and write identical values; a slot is rewritten two products later, after MMAs that needed every warp's
+        // epilogue in between.
+        auto stage_bias = [&](uint32_t layer) {
             if (!BWD) {
 #pragma unroll
                 for (uint32_t ci = 0; ci < WPW; ++ci) {
                     const uint32_t cc = par + SUBS * ci;
-                    bias_reg[ci] = col0 + cc * 32U + lane < H ? __ldg(args.bias + layer * args.bias_stride + col0 + cc * 32U + lane) : 0.0f;
+                    bias_slots[(layer & 1U) * 256U + (par * WPW + ci) * 32U + lane] = col0 + cc * 32U + lane < H ? __ldg(args.bias + layer * args.bias_stride + col0 + cc * 32U + lane) : 0.0f;
                 }
-            }
-        };
-        auto stage_bias = [&]() {
-            if (!BWD) {
-#pragma unroll
-                for (uint32_t ci = 0; ci < WPW; ++ci) bias_slots[(par * WPW + ci) * 32U + lane] = bias_reg[ci];
                 __syncwarp();
             }
         };
@@ -291,11 +284,18 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = ((bits >> j) & 1U) ? v[j] : 0U;
         };
-        auto column_sums = [&](const uint32_t (&raw)[32]) {
-            float v[32];
+        // bias sums of a product (its columns from `taddr` on), when the panels are handed on
+        auto column_sums = [&](uint32_t taddr, uint32_t tile, uint32_t slot) {
+            tmem_st_wait();
 #pragma unroll
-            for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(raw[j]);
-            return detail::warp_column_sums(v, lane);
+            for (uint32_t ci = 0; ci < WPW; ++ci) {
+                const uint32_t cc = par + SUBS * ci;
+                if (cc >= NC) break;
+                uint32_t j;
+                const float total = detail::column_sums(taddr + cc * 32U, lane, &j);
+                const uint32_t col = col0 + cc * 32U + j;
+                if (col < H) args.colsum[slot * args.colsum_stride + (static_cast<uint64_t>(tile) * 4U + quad) * H + col] = total;
+            }
         };
 
         uint32_t uses = 0;
@@ -349,10 +349,9 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
                     uint32_t mwords[4] = {0, 0, 0, 0};
                     if (BWD) load_words(args.bits_t + k * args.bits_stride + bits_row, mwords);
                     uint32_t words[4] = {0, 0, 0, 0};  // the first WPW are used
-                    fetch_bias(2U * k);
+                    stage_bias(2U * k);
                     if (!warp_wait(&mma_done[0], uses & 1U)) { ok = false; break; }
                     tc_fence_after();
-                    stage_bias();
 #pragma unroll
                     for (uint32_t ci = 0; ci < WPW; ++ci) {
                         const uint32_t cc = par + SUBS * ci;
@@ -361,17 +360,18 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
                         tmem_ld_32x32(tmem_base + lane_addr + cc * 32U, raw);
                         tmem_ld_wait();
                         uint32_t h[16];
-                        if (BWD) apply_mask(raw, mwords[ci]);
-                        else detail::add_bias_relu(raw, bias_slots + (par * WPW + ci) * 32U);
+                        if (BWD) {
+                            apply_mask(raw, mwords[ci]);
+                            tmem_st_32x32(tmem_base + lane_addr + cc * 32U, raw);  // (for the column sums)
+                        } else {
+                            detail::add_bias_relu(raw, bias_slots + (par * WPW + ci) * 32U);
+                        }
                         detail::pack_operands(raw, h, args.bf16 != 0U);
                         store_operand(cc, h);
                         publish(&ready[p0 + (cc >> 1)]);
                         if (!BWD) words[ci] = detail::positive_bits(raw);
-                        if (BWD) {
-                            const float total = column_sums(raw);
-                            if (col0 + cc * 32U + lane < H) args.colsum[k * args.colsum_stride + (static_cast<uint64_t>(tile) * 4U + quad) * H + col0 + cc * 32U + lane] = total;
-                        }
                     }
+                    if (BWD) column_sums(tmem_base + lane_addr, tile, k);
                     if (!BWD) store_words(args.bits_t + k * args.bits_stride + bits_row, words);
                 }
                 // ================= second epilogue: new S =================
@@ -379,10 +379,9 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
                     uint32_t mwords[4] = {0, 0, 0, 0};
                     if (BWD) load_words(args.bits_s + k * args.bits_stride + bits_row, mwords);
                     uint32_t words[4] = {0, 0, 0, 0};  // the first WPW are used
-                    fetch_bias(2U * k + 1U);
+                    stage_bias(2U * k + 1U);
                     if (!warp_wait(&mma_done[1], uses & 1U)) { ok = false; break; }
                     tc_fence_after();
-                    stage_bias();
                     const uint32_t entry = BWD ? k : k + 1U;
                     __half* tape_row = args.tape_s + entry * args.tape_s_stride + row * args.ld_s;
 #pragma unroll
@@ -394,10 +393,10 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
                         tmem_ld_wait();
                         uint32_t h[16];
                         if (BWD) apply_mask(raw, mwords[ci]);
-                        else detail::add_bias_relu(raw, bias_slots + (par * WPW + ci) * 32U);
+                        else detail::add_bias_relu(raw, bias_slots + 256U + (par * WPW + ci) * 32U);
                         detail::pack_operands(raw, h, args.bf16 != 0U);
+                        if (BWD || !last) tmem_st_32x32(tmem_base + lane_addr + kStateCol + cc * 32U, raw);
                         if (!last) {
-                            tmem_st_32x32(tmem_base + lane_addr + kStateCol + cc * 32U, raw);
                             store_operand(cc, h);
                             tmem_st_wait();
                             publish(&ready[p0 + (cc >> 1)]);
@@ -412,11 +411,8 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
                                     if (col0 + cc * 32U + 4U * q < args.ld_f32) dst[q] = make_float4(__uint_as_float(raw[4 * q]), __uint_as_float(raw[4 * q + 1]), __uint_as_float(raw[4 * q + 2]), __uint_as_float(raw[4 * q + 3]));
                             }
                         }
-                        if (BWD) {
-                            const float total = column_sums(raw);
-                            if (col0 + cc * 32U + lane < H) args.colsum[(R + k) * args.colsum_stride + (static_cast<uint64_t>(tile) * 4U + quad) * H + col0 + cc * 32U + lane] = total;
-                        }
                     }
+                    if (BWD) column_sums(tmem_base + lane_addr + kStateCol, tile, R + k);
                     if (!BWD) store_words(args.bits_s + (k + 1U) * args.bits_stride + bits_row, words);
                     if (last) tc_fence_before();  // the next tile's state load overwrites the TMEM columns read here
                 }
