@@ -225,23 +225,23 @@ onehot_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
 
     if (warp == 0) {
         // ------------------------------- TMA producer: this CTA's 128 rows of A -----------
-        if (lane == 0) {
-            uint32_t it = 0;
-            bool ok = true;
-            while (ok && pieces.next(p)) {
-                const int32_t m = static_cast<int32_t>(p.mt * 256U + rank * 128U);
-                for (uint32_t c = p.c0; c < p.c1; ++c, ++it) {
-                    const uint32_t s = it % ST;
-                    if (!mbar_wait_spin(&empty[s], ((it / ST) & 1U) ^ 1U, cta_abort, kAbortProducerWait)) { ok = false; break; }
-                    uint8_t* dst = smem + s * PairCfg<GRAD>::STAGE_BYTES;
-                    const uint32_t bar = pair::map_to(smem_u32(&full[s]), 0);
-                    if (rank == 0U) mbar_arrive_expect_tx(&full[s], 2U * PairCfg<GRAD>::A_BYTES);
-                    if (GRAD) {
-                        pair::tma_load_2d(dst, &tma_a, static_cast<int32_t>(c * 64U), m, bar);
-                    } else {
-                        pair::tma_load_2d(dst, &tma_a, m, static_cast<int32_t>(c * 64U), bar);
-                        pair::tma_load_2d(dst + 8192, &tma_a, m + 64, static_cast<int32_t>(c * 64U), bar);
-                    }
+        const uint32_t lead = elect_one();
+        uint32_t it = 0;
+        bool ok = true;
+        while (ok && pieces.next(p)) {
+            const int32_t m = static_cast<int32_t>(p.mt * 256U + rank * 128U);
+            for (uint32_t c = p.c0; c < p.c1; ++c, ++it) {
+                const uint32_t s = it % ST;
+                if (!mbar_wait_warp(&empty[s], ((it / ST) & 1U) ^ 1U, cta_abort, kAbortProducerWait)) { ok = false; break; }
+                if (!lead) continue;
+                uint8_t* dst = smem + s * PairCfg<GRAD>::STAGE_BYTES;
+                const uint32_t bar = pair::map_to(smem_u32(&full[s]), 0);
+                if (rank == 0U) mbar_arrive_expect_tx(&full[s], 2U * PairCfg<GRAD>::A_BYTES);
+                if (GRAD) {
+                    pair::tma_load_2d(dst, &tma_a, static_cast<int32_t>(c * 64U), m, bar);
+                } else {
+                    pair::tma_load_2d(dst, &tma_a, m, static_cast<int32_t>(c * 64U), bar);
+                    pair::tma_load_2d(dst + 8192, &tma_a, m + 64, static_cast<int32_t>(c * 64U), bar);
                 }
             }
         }

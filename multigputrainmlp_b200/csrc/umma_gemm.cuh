@@ -189,6 +189,8 @@ __global__ void __launch_bounds__(Cfg::THREADS, 1)
 umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const GemmArgs args) {
     using namespace ptx;
     constexpr int BM = Cfg::BM, BN = Cfg::BN, SA = Cfg::SA, SB = Cfg::SB;
+    // equal rings of A and B advance together: one barrier pair a stage
+    constexpr bool kJoint = !Cfg::BSTAT && SA == SB;
     constexpr int ACC_BUFS = Cfg::ACC_BUFS;
 
     extern __shared__ uint8_t smem_raw[];
@@ -252,44 +254,49 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 
     if (warp == 0) {
         // ------------------------------- TMA producer -------------------------------------
-        if (lane == 0) {
-            uint32_t it = 0;
-            bool ok = true;
-            for (uint32_t unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x) {
-                uint32_t mt, nt, sp;
-                decode(unit, mt, nt, sp);
-                const uint32_t c0 = chunk_begin(sp), c1 = chunk_begin(sp + 1);
-                for (uint32_t c = c0; c < c1; ++c, ++it) {
-                    const uint32_t sa = it % SA, pa = (it / SA) & 1U;
-                    if (!mbar_wait_spin(&empty_a[sa], pa ^ 1U, cta_abort, kAbortProducerWait)) { ok = false; break; }
+        // (a whole converged warp, as the issuer's: in one lane's loop the waits, expectations and six loads of a chunk of
+        // 128 x 256 took twice its 512 cycles of MMAs)
+        const uint32_t lead = elect_one();
+        uint32_t it = 0;
+        bool ok = true;
+        for (uint32_t unit = blockIdx.x; unit < total_units && ok; unit += gridDim.x) {
+            uint32_t mt, nt, sp;
+            decode(unit, mt, nt, sp);
+            const uint32_t c0 = chunk_begin(sp), c1 = chunk_begin(sp + 1);
+            const int32_t m0 = static_cast<int32_t>(mt * BM), n0 = static_cast<int32_t>(nt * BN), z = Cfg::GROUPED ? static_cast<int32_t>(group_of(unit)) : 0;
+            for (uint32_t c = c0; c < c1; ++c, ++it) {
+                const uint32_t sa = it % SA, pa = (it / SA) & 1U;
+                const int32_t k0 = static_cast<int32_t>(c * 64);
+                if (!mbar_wait_warp(&empty_a[sa], pa ^ 1U, cta_abort, kAbortProducerWait)) { ok = false; break; }
+                if (lead) {
                     uint8_t* a_dst = a_ring + sa * Cfg::A_STAGE_BYTES;
-                    mbar_arrive_expect_tx(&full_a[sa], Cfg::A_STAGE_BYTES);
+                    mbar_arrive_expect_tx(&full_a[sa], Cfg::A_STAGE_BYTES + (kJoint ? Cfg::B_STAGE_BYTES : 0));
                     if (Cfg::GROUPED) {
-                        const int32_t g = static_cast<int32_t>(group_of(unit));
-                        tma_load_3d(a_dst, &tma_a, static_cast<int32_t>(mt * BM), static_cast<int32_t>(c * 64), g, &full_a[sa]);
-                        tma_load_3d(a_dst + 8192, &tma_a, static_cast<int32_t>(mt * BM + 64), static_cast<int32_t>(c * 64), g, &full_a[sa]);
+                        tma_load_3d(a_dst, &tma_a, m0, k0, z, &full_a[sa]);
+                        tma_load_3d(a_dst + 8192, &tma_a, m0 + 64, k0, z, &full_a[sa]);
                     } else if (Cfg::A_MN) {
-                        tma_load_2d(a_dst, &tma_a, static_cast<int32_t>(mt * BM), static_cast<int32_t>(c * 64), &full_a[sa]);
-                        tma_load_2d(a_dst + 8192, &tma_a, static_cast<int32_t>(mt * BM + 64), static_cast<int32_t>(c * 64), &full_a[sa]);
+                        tma_load_2d(a_dst, &tma_a, m0, k0, &full_a[sa]);
+                        tma_load_2d(a_dst + 8192, &tma_a, m0 + 64, k0, &full_a[sa]);
                     } else {
-                        tma_load_2d(a_dst, &tma_a, static_cast<int32_t>(c * 64), static_cast<int32_t>(mt * BM), &full_a[sa]);
+                        tma_load_2d(a_dst, &tma_a, k0, m0, &full_a[sa]);
                     }
-                    if (!Cfg::BSTAT || unit == blockIdx.x) {
-                        // B-stationary: chunk c of B lives in stage c for the whole kernel, loaded with the first unit
-                        const uint32_t sb = Cfg::BSTAT ? (c - c0) : it % SB, pb = Cfg::BSTAT ? 0U : (it / SB) & 1U;
-                        if (!Cfg::BSTAT && !mbar_wait_spin(&empty_b[sb], pb ^ 1U, cta_abort, kAbortProducerWait)) { ok = false; break; }
+                }
+                if (!Cfg::BSTAT || unit == blockIdx.x) {
+                    // B-stationary: chunk c of B lives in stage c for the whole kernel, loaded with the first unit
+                    const uint32_t sb = Cfg::BSTAT ? (c - c0) : it % SB, pb = Cfg::BSTAT ? 0U : (it / SB) & 1U;
+                    if (!Cfg::BSTAT && !kJoint && !mbar_wait_warp(&empty_b[sb], pb ^ 1U, cta_abort, kAbortProducerWait)) { ok = false; break; }
+                    if (lead) {
                         uint8_t* b_dst = b_ring + sb * Cfg::B_STAGE_BYTES;
-                        mbar_arrive_expect_tx(&full_b[sb], Cfg::B_STAGE_BYTES);
-                        const int32_t n0 = static_cast<int32_t>(nt * BN), k0 = static_cast<int32_t>(c * 64);
+                        uint64_t* full = kJoint ? &full_a[sa] : &full_b[sb];
+                        if (!kJoint) mbar_arrive_expect_tx(full, Cfg::B_STAGE_BYTES);
                         if (Cfg::GROUPED) {
-                            const int32_t z = static_cast<int32_t>(group_of(unit));
 #pragma unroll
-                            for (int g = 0; g < Cfg::N_GROUPS; ++g) tma_load_3d(b_dst + g * 8192, &tma_b, n0 + g * 64, k0, z, &full_b[sb]);
+                            for (int g = 0; g < Cfg::N_GROUPS; ++g) tma_load_3d(b_dst + g * 8192, &tma_b, n0 + g * 64, k0, z, full);
                         } else if (Cfg::B_MN) {
 #pragma unroll
-                            for (int g = 0; g < Cfg::N_GROUPS; ++g) tma_load_2d(b_dst + g * 8192, &tma_b, n0 + g * 64, k0, &full_b[sb]);
+                            for (int g = 0; g < Cfg::N_GROUPS; ++g) tma_load_2d(b_dst + g * 8192, &tma_b, n0 + g * 64, k0, full);
                         } else {
-                            tma_load_2d(b_dst, &tma_b, k0, n0, &full_b[sb]);
+                            tma_load_2d(b_dst, &tma_b, k0, n0, full);
                         }
                     }
                 }
@@ -315,7 +322,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                     const uint32_t sa = it % SA, pa = (it / SA) & 1U;
                     const uint32_t sb = Cfg::BSTAT ? (c - c0) : it % SB, pb = Cfg::BSTAT ? 0U : (it / SB) & 1U;
                     if (!mbar_wait_warp(&full_a[sa], pa, cta_abort, kAbortMmaWait)) { ok = false; break; }
-                    if (!Cfg::BSTAT || unit == blockIdx.x) {
+                    if (!kJoint && (!Cfg::BSTAT || unit == blockIdx.x)) {
                         if (!mbar_wait_warp(&full_b[sb], pb, cta_abort, kAbortMmaWait)) { ok = false; break; }
                     }
                     tc_fence_after();
@@ -337,7 +344,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                         for (uint32_t kk = 0; kk < ksteps; ++kk) umma_f16(lead, d_base, a_desc0 + kk * kStepA, b_desc0 + kk * kStepB, idesc, kk == 0U ? first : 1U);
                     }
                     umma_commit(lead, &empty_a[sa]);
-                    if (!Cfg::BSTAT) umma_commit(lead, &empty_b[sb]);
+                    if (!Cfg::BSTAT && !kJoint) umma_commit(lead, &empty_b[sb]);
                 }
                 if (ok) umma_commit(lead, &acc_full[ab]);
             }
