@@ -260,6 +260,10 @@ struct mgt_engine {
     std::unordered_map<mgt::MapKey, CUtensorMap, mgt::MapKeyHash> maps;
     std::mutex mu;
     cudaEvent_t ev_last = nullptr, ev_now = nullptr;
+    // a second stream for the weight gradients of small batches (SideBranch), and the events that tie it to the caller's
+    cudaStream_t side = nullptr;
+    cudaEvent_t ev_side[3] = {nullptr, nullptr, nullptr};
+    std::mutex side_mu;  // an event is recorded and waited for in one piece
     uint64_t launches = 0;  // kernels launched through this engine (host-side count)
     bool layered_tower = false;  // MGT_RESIDUAL_PATH=layered: per-layer GEMMs instead of the fused residual-tower kernels (both are tested)
     mgt_gradient_ready_fn early_fn = nullptr;  // mgt_engine_set_early_range_hook
@@ -1006,6 +1010,34 @@ inline uint32_t GridFor(uint64_t items, uint32_t threads, int sm_count) {
     return (uint32_t)(want < 1 ? 1 : (want < cap ? want : cap));
 }
 
+// Work of the backward pass on the engine's second stream, beside the caller's: from Fork() on, until the object ends (on every
+// path, so that the caller's stream is never ahead of it).
+struct SideBranch {
+    mgt_engine* e;
+    cudaStream_t main;
+    bool open = false;
+
+    bool Tie(int event, cudaStream_t from, cudaStream_t to) {
+        std::lock_guard<std::mutex> lock(e->side_mu);
+        return cudaEventRecord(e->ev_side[event], from) == cudaSuccess && cudaStreamWaitEvent(to, e->ev_side[event], 0) == cudaSuccess;
+    }
+    bool Fork() {
+        {
+            std::lock_guard<std::mutex> lock(e->side_mu);
+            if (e->side == nullptr && cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking) != cudaSuccess) return false;
+            for (cudaEvent_t& ev : e->ev_side)
+                if (ev == nullptr && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return false;
+        }
+        return open = Tie(0, main, e->side);
+    }
+    bool Join() {
+        const bool was = open;
+        open = false;
+        return !was || Tie(2, e->side, main);
+    }
+    ~SideBranch() { Join(); }
+};
+
 struct StageTimer {
     mgt_engine* e;
     cudaStream_t stream;
@@ -1478,6 +1510,9 @@ mgt_status_t mgt_engine_destroy(mgt_engine_t* e) {
     if (e == nullptr) return MGT_OK;
     if (e->ev_last) cudaEventDestroy(e->ev_last);
     if (e->ev_now) cudaEventDestroy(e->ev_now);
+    for (cudaEvent_t ev : e->ev_side)
+        if (ev) cudaEventDestroy(ev);
+    if (e->side) cudaStreamDestroy(e->side);
     if (e->status_word) cudaFree(e->status_word);
     delete e;
     return MGT_OK;
@@ -1810,6 +1845,24 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     // ---- hidden layer backward, dX part (mlp_backward.cu:1417-1438): dz_tape(0) = dcur * [x0 > 0]
     dz_cur = dz_tape(0);
     if (bnorm) MGT_TRY(bn_backward(0, grad + HiddenBias(s)));
+    // Small batches: the weight gradients run beside the dX products and the embedding gradient, on the second stream. Neither
+    // branch fills the SMs there (the dX product has fewer than two tiles an SM), and every launch is a gap: 9 001 samples of
+    // hd1 1000, hd2 200, 8 blocks 510 -> 453 us a step, 1 024 of hd1 256, hd2 64, 2 blocks 134 -> 114. With more tiles each
+    // kernel has the whole chip anyway, and beyond some 16 000 samples of a small model the gradient's gathers lose more to
+    // the shared memory of the GEMMs beside them than they gain (54 025 of hd1 88: 611 -> 660 us). Below eight tiles the host is
+    // what a pass waits for, and the events would only add to that. Not with callers that are told of finished ranges
+    // or time the stages: they rely on the order.
+    const uint64_t dx_tiles = (uint64_t)((H1 + 127U) / 128U) * ((B + 255U) / 256U);
+    SideBranch branch{e, st};
+    if (dx_tiles >= 8U && dx_tiles < 2ULL * e->sm_count && B <= 16384U && ready == nullptr && e->early_fn == nullptr && profile == nullptr && !branch.Fork()) return MGT_CUDA_FAILURE;
+    cudaStream_t st_dw = branch.open ? e->side : st;
+    uint32_t* order = reinterpret_cast<uint32_t*>(base + ws.off_lists);
+    uint32_t* first = order + (uint64_t)s.state_len * B;
+    auto sort_classes = [&](cudaStream_t stream) {
+        gather::SortByClassKernel<<<s.state_len, 1024, 0, stream>>>(reinterpret_cast<const uint8_t*>(states), B, s.state_value_pad, order, first);
+        ++e->launches;
+    };
+    if (branch.open && half_ig && ws.gather_grad) sort_classes(e->side);
     // dz1T = (Wh * dzh^T) * [pre-activation of a1 > 0], the input-bias gradient from its row sums. With --input-grad-fp16 0 the
     // embedding gradient wants dz1 in fp32 (mlp_backward.cu:1433-1504, float one-hot GEMM): the same product of fp16 operands
     // with fp32 accumulation, written unrounded as rows of samples.
@@ -1824,19 +1877,18 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
                                     reinterpret_cast<uint32_t*>(dz1_f32 + (uint64_t)B * p_dz1_f32), grad) != cudaSuccess) return MGT_CUDA_FAILURE;
         e->launches += 2;
     } else if (ws.gather_grad) {
-        uint32_t* order = reinterpret_cast<uint32_t*>(base + ws.off_lists);
-        uint32_t* first = order + (uint64_t)s.state_len * B;
-        gather::SortByClassKernel<<<s.state_len, 1024, 0, st>>>(reinterpret_cast<const uint8_t*>(states), B, s.state_value_pad, order, first);
         const bool vec = (H1 & 3U) == 0U && (reinterpret_cast<uintptr_t>(grad) & 15U) == 0U;
         auto run = [&](auto kernel, uint32_t rows_per_cta) {
             kernel<<<dim3((IN + rows_per_cta - 1U) / rows_per_cta, (H1 + 63U) / 64U), 256, 0, st>>>(order, first, reinterpret_cast<const uint16_t*>(dz1_h), ws.p_dz1_rows, B,
                                                                                                s.state_len, s.state_value_pad, H1, grad, vec);
         };
+        if (!branch.open) sort_classes(st);
+        else if (!branch.Tie(1, e->side, st)) return MGT_CUDA_FAILURE;  // (of the branch only the sort is enqueued yet)
         // a group of lanes per table row, four groups where that leaves fewer than 16 warps for an SM
         const bool few = (uint64_t)IN * ((H1 + 63U) / 64U) < 64ULL * e->sm_count;
         if (few) { if (e->bf16_now) run(gather::GradKernel<4, true>, 8U); else run(gather::GradKernel<4, false>, 8U); }
         else { if (e->bf16_now) run(gather::GradKernel<1, true>, 32U); else run(gather::GradKernel<1, false>, 32U); }
-        e->launches += 2;
+        ++e->launches;
         if (cudaGetLastError() != cudaSuccess) return MGT_CUDA_FAILURE;
     } else {
         PairArgs a{};
@@ -1856,9 +1908,9 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
 
     if (R > 0) {
         // weight gradients of all blocks: two grouped split-K GEMMs (fc2: r1_k^T dz2_k, fc1: x_k^T dz1_k)
-        MGT_TRY(GemmGradWeightsGrouped(e, st, r1_h(0), ws.p_act, ws.r1_stride, dz_tape(1), ws.p_dz, ws.dz_stride, R, B, H2, H2, partial,
+        MGT_TRY(GemmGradWeightsGrouped(e, st_dw, r1_h(0), ws.p_act, ws.r1_stride, dz_tape(1), ws.p_dz, ws.dz_stride, R, B, H2, H2, partial,
                                        ws.partial_floats, grad + Fc2W(s, 0), BlockParams(s)));
-        MGT_TRY(GemmGradWeightsGrouped(e, st, x_h(0), ws.p_act, ws.x_stride, dz1_tape(0), ws.p_dz, ws.dz_stride, R, B, H2, H2, partial,
+        MGT_TRY(GemmGradWeightsGrouped(e, st_dw, x_h(0), ws.p_act, ws.x_stride, dz1_tape(0), ws.p_dz, ws.dz_stride, R, B, H2, H2, partial,
                                        ws.partial_floats, grad + Fc1W(s, 0), BlockParams(s)));
         // bias gradients: column sums of dz1_k -> b1_k, of the dz each fc1 GEMM produced -> b2_{k-1} (hidden bias for k = 0)
         ReduceDestinations dst{};
@@ -1867,7 +1919,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
             dst.offset[R + k] = k > 0 ? Fc2B(s, k - 1) : HiddenBias(s);
         }
         // (with batch normalisation b2_k and the hidden bias got their gradients from the normalisation's backward pass)
-        ReduceRowsGroupedKernel<<<dim3((H2 + kReduceCols - 1) / kReduceCols, bnorm ? R : 2 * R), 256, 0, st>>>(colsum, colsum_rows, H2, ws.colsum_slot_floats, grad, dst);
+        ReduceRowsGroupedKernel<<<dim3((H2 + kReduceCols - 1) / kReduceCols, bnorm ? R : 2 * R), 256, 0, st_dw>>>(colsum, colsum_rows, H2, ws.colsum_slot_floats, grad, dst);
         ++e->launches;
         if (cudaGetLastError() != cudaSuccess) return MGT_CUDA_FAILURE;
         for (uint32_t rb = R; rb > 0; --rb) {
@@ -1879,7 +1931,8 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
 
     // ---- hidden layer backward, dW part; every kernel that reads the hidden weights was enqueued long before, so a caller
     // may update the range in place as soon as it is announced
-    MGT_TRY(GemmGradWeightsRows(e, st, a1_h, ws.p_bt, dz_cur, ws.p_dz, B, H1, H2, partial, ws.partial_floats, grad + HiddenWeight(s)));
+    MGT_TRY(GemmGradWeightsRows(e, st_dw, a1_h, ws.p_bt, dz_cur, ws.p_dz, B, H1, H2, partial, ws.partial_floats, grad + HiddenWeight(s)));
+    if (!branch.Join()) return MGT_CUDA_FAILURE;
     MGT_TRY(notify(HiddenWeight(s), (uint64_t)H1 * H2 + H2));
     if (!timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
     MGT_TRY(notify(0, InputBias(s) + H1));

@@ -149,3 +149,9 @@ def test_one_hot_pairs(oracle, dims, n):
 def test_wide_residual_tower(oracle, hd2, n, mirror, bf16):
     loss_grad_case(oracle, (72, 72, 48, hd2, 3, 1), n, scale=0.02, mirror=mirror, options=dict(bf16=True) if bf16 else None, tol=8e-3 if bf16 else 1e-3,
                    section_tol=2e-2 if bf16 else 3e-3)
+
+
+# weight gradients on the second stream: eight dX tiles or more; the embedding gradient by gathering and by the one-hot product
+@pytest.mark.parametrize("dims,n", [((72, 72, 896, 40, 2, 1), 96), ((72, 72, 897, 40, 2, 1), 96), ((54, 6, 1024, 64, 1, 3), 513), ((72, 72, 1032, 33, 0, 1), 257)])
+def test_weight_gradients_beside_the_embedding_gradient(oracle, dims, n):
+    loss_grad_case(oracle, dims, n, scale=0.02)
