@@ -31,6 +31,7 @@ VARIANTS = {
 }
 SEED = 1234
 LR = 1e-4
+TIMED_BLOCKS = 4
 
 
 def run(args) -> dict:
@@ -142,17 +143,22 @@ def run(args) -> dict:
     st, code = engine.check()
     assert st == 0, f"device status {code}"
     launches0 = engine.launch_count + other[0] + (backend.launch_count if backend else 0) + (stats_backend.launch_count if stats_backend else 0)
-    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    barrier()
-    e0.record()
-    for s in range(args.steps):
-        step(warmup + s)
-    e1.record()
-    barrier()
-    ms = torch.tensor([e0.elapsed_time(e1) / args.steps], device=dev)
-    if world > 1:
-        dist.all_reduce(ms, op=dist.ReduceOp.MAX)
-    ms_step = float(ms.item())
+    # the steps are timed in several blocks, the line has the median: a block of a few steps is a few milliseconds
+    block_ms, done = [], warmup
+    for _ in range(TIMED_BLOCKS):
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        barrier()
+        e0.record()
+        for s in range(args.steps):
+            step(done + s)
+        e1.record()
+        barrier()
+        done += args.steps
+        ms = torch.tensor([e0.elapsed_time(e1) / args.steps], device=dev)
+        if world > 1:
+            dist.all_reduce(ms, op=dist.ReduceOp.MAX)
+        block_ms.append(float(ms.item()))
+    ms_step = float(np.median(block_ms))
     launches = engine.launch_count + other[0] + (backend.launch_count if backend else 0) + (stats_backend.launch_count if stats_backend else 0) - launches0
     for b in (backend, stats_backend):
         if b is not None:
@@ -160,7 +166,7 @@ def run(args) -> dict:
             assert st == 0, f"communicator status {code}"
     final_loss = float(loss.item())
     prof = mgt.BackwardProfile()
-    step(warmup + args.steps, profile=prof)
+    step(done, profile=prof)
     torch.cuda.synchronize()
     stage_ms = {n: round(getattr(prof, n), 4) for n, _ in prof._fields_}
     # replicas must still agree (N > 1): the same two checksums of the weights on every rank
@@ -179,7 +185,7 @@ def run(args) -> dict:
         "config": {"workload": v["workload"], "variant": args.variant, "batch_per_rank": batch, **v["shape"], "batch_norm": bool(nbn),
                    "loss": "cross_entropy" if v["cross_entropy"] else "mse", "weight_decay": v["weight_decay"], "parallelism": f"dp{world}",
                    "l2": "inputs larger than L2 (activation tapes of several GB per step)"},
-        "gpu_launches": int(launches), "stage_ms": stage_ms, "final_loss": final_loss, "replicas_identical": replicas_identical,
+        "timed_blocks": TIMED_BLOCKS, "gpu_launches": int(launches), "stage_ms": stage_ms, "final_loss": final_loss, "replicas_identical": replicas_identical,
         "step_tflops_algorithmic": flop * batch / (ms_step * 1e-3) / 1e12,
         "workspace_gb": ws_floats * 4 / 1e9,
     }
