@@ -1024,7 +1024,11 @@ struct SideBranch {
     bool Fork() {
         {
             std::lock_guard<std::mutex> lock(e->side_mu);
-            if (e->side == nullptr && cudaStreamCreateWithFlags(&e->side, cudaStreamNonBlocking) != cudaSuccess) return false;
+            // (ahead of the caller's stream where both have blocks to place: the embedding gradient then ends the pass with the
+            // whole chip; 3 001 samples of p888 550 -> 523 us a step)
+            int least = 0, greatest = 0;
+            if (e->side == nullptr && (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess ||
+                                       cudaStreamCreateWithPriority(&e->side, cudaStreamNonBlocking, greatest) != cudaSuccess)) return false;
             for (cudaEvent_t& ev : e->ev_side)
                 if (ev == nullptr && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return false;
         }
@@ -1847,14 +1851,13 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     if (bnorm) MGT_TRY(bn_backward(0, grad + HiddenBias(s)));
     // Small batches: the weight gradients run beside the dX products and the embedding gradient, on the second stream. Neither
     // branch fills the SMs there (the dX product has fewer than two tiles an SM), and every launch is a gap: 9 001 samples of
-    // hd1 1000, hd2 200, 8 blocks 510 -> 453 us a step, 1 024 of hd1 256, hd2 64, 2 blocks 134 -> 114. With more tiles each
-    // kernel has the whole chip anyway, and beyond some 16 000 samples of a small model the gradient's gathers lose more to
-    // the shared memory of the GEMMs beside them than they gain (54 025 of hd1 88: 611 -> 660 us). Below eight tiles the host is
-    // what a pass waits for, and the events would only add to that. Not with callers that are told of finished ranges
-    // or time the stages: they rely on the order.
+    // hd1 1000, hd2 200, 8 blocks 510 -> 453 us a step, 1 024 of hd1 256, hd2 64, 2 blocks 134 -> 114, 64 of hd1 8, hd2 8
+    // 99 -> 89. With more tiles each kernel has the whole chip anyway, and beyond some 16 000 samples of a small model the
+    // gradient's gathers lose more to the shared memory of the GEMMs beside them than they gain (54 025 of hd1 88: 611 ->
+    // 660 us). Not with callers that are told of finished ranges or time the stages: they rely on the order.
     const uint64_t dx_tiles = (uint64_t)((H1 + 127U) / 128U) * ((B + 255U) / 256U);
     SideBranch branch{e, st};
-    if (dx_tiles >= 8U && dx_tiles < 2ULL * e->sm_count && B <= 16384U && ready == nullptr && e->early_fn == nullptr && profile == nullptr && !branch.Fork()) return MGT_CUDA_FAILURE;
+    if (dx_tiles < 2ULL * e->sm_count && B <= 16384U && ready == nullptr && e->early_fn == nullptr && profile == nullptr && !branch.Fork()) return MGT_CUDA_FAILURE;
     cudaStream_t st_dw = branch.open ? e->side : st;
     uint32_t* order = reinterpret_cast<uint32_t*>(base + ws.off_lists);
     uint32_t* first = order + (uint64_t)s.state_len * B;
