@@ -43,7 +43,8 @@ EMB_EXEC_FLOP_PER_CANDIDATE = 2 * (72 * 72 + 1) * 2560  # what the one-hot GEMM 
 # this run: the source is named in the output next to the figure)
 EMB_FWD_DRAM_BYTES_PER_LAUNCH = 268_568_064
 EMB_FWD_DRAM_SOURCE = ("ncu dram__bytes_read.sum + dram__bytes_write.sum, one launch at batch 53248 (32.9 MB read + 235.7 MB written: "
-                       "the [hd1][B] activation and its sign words), single-pass capture of 2026-11-25, profiles/training_step_p888_launch_list.md")
+                       "the [hd1][B] activation and its sign words; captured on the single-CTA form of the kernel, the operands and results are the same), "
+                       "profiles/training_step_p888_launch_list.md")
 README_P888_FLAGS = ["--batch-size", "53248", "--k-min", "1", "--k-max", "29", "--hd1", "2556", "--hd2", "218", "--nrd", "16",
                      "--input-grad-fp16", "1", "--input-grad-position-tile", "36", "--linear-fp16", "1", "--write-artifacts", "0",
                      "--allreduce-bucket-bytes", "4194304"]  # the reference README's p888 command (README.md:48-64)
@@ -565,7 +566,7 @@ def main():
     algo_tflops = EMB_ALGO_FLOP_PER_CANDIDATE * batch / (emb * 1e-3) / 1e12
     exec_tflops = EMB_EXEC_FLOP_PER_CANDIDATE * batch / (emb * 1e-3) / 1e12
     roofline = {
-        "kernel": "umma_gemm_kernel<one-hot forward> (embedding layer)", "bound": "tensor", "achieved": algo_tflops,
+        "kernel": "onehot_pair_kernel<forward> (embedding layer)", "bound": "tensor", "achieved": algo_tflops,
         "peak": peaks["tflops_burst"], "unit": "TFLOP/s", "frac": algo_tflops / peaks["tflops_burst"],
         "traffic": EMB_FWD_DRAM_BYTES_PER_LAUNCH if batch == BATCH else None,
         "traffic_source": EMB_FWD_DRAM_SOURCE if batch == BATCH else None,
@@ -579,7 +580,7 @@ def main():
     tower_fwd_bytes = batch * (224 * 4 + 16 * 2 * 224 * 2 + 17 * 32 + 224 * 4)   # state in, 32 fp16 tape entries, sign bits, state out
     hidden_fwd_bytes = batch * (2560 * 2 + 224 * 4 + 224 * 2) + 2560 * 224 * 2    # a1 in, x fp32 + fp16 out, weights
     roofline_other = [
-        {"kernel": "umma_gemm_kernel<one-hot gradient> (embedding table gradient)", "bound": "tensor", "ms_per_launch": grad_t,
+        {"kernel": "onehot_pair_kernel<gradient> (embedding table gradient)", "bound": "tensor", "ms_per_launch": grad_t,
          "achieved": EMB_ALGO_FLOP_PER_CANDIDATE * batch / (grad_t * 1e-3) / 1e12, "executed_tflops": 2 * 72 * 72 * 2560 * batch / (grad_t * 1e-3) / 1e12,
          "peak": peaks["tflops_burst"], "unit": "TFLOP/s", "executed_frac": 2 * 72 * 72 * 2560 * batch / (grad_t * 1e-3) / 1e12 / peaks["tflops_burst"]},
         {"kernel": "tower_chain_kernel<forward> (16 residual blocks)", "bound": "hbm", "ms_per_launch": stage_ms["residual_forward_ms"],
