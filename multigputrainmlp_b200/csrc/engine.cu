@@ -252,6 +252,68 @@ struct MapKeyHash {
 }  // namespace
 }  // namespace mgt
 
+namespace mgt {
+// A second stream and the events that tie it to the caller's. Taken by an engine's first pass that wants one and given back when
+// the engine goes: the pool keeps at most kPooled per device (a program that makes engines one after the other would pay 0.1 ms
+// each for new ones).
+struct SideStream {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t events[3] = {nullptr, nullptr, nullptr};
+};
+class SidePool {
+    static constexpr size_t kPooled = 4;
+    std::mutex mu;
+    std::vector<SideStream> idle[64];
+
+public:
+    static SidePool& Get() {
+        static SidePool* pool = new SidePool();  // (never destroyed: the CUDA runtime may be gone before it)
+        return *pool;
+    }
+    bool Take(int device, SideStream* out) {
+        if (device < 0 || device >= 64) return false;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (!idle[device].empty()) {
+                *out = idle[device].back();
+                idle[device].pop_back();
+                return true;
+            }
+        }
+        // (ahead of the caller's stream where both have blocks to place: the embedding gradient then ends the pass with the whole
+        // chip; 3 001 samples of p888 550 -> 523 us a step)
+        SideStream s;
+        int least = 0, greatest = 0;
+        bool ok = cudaDeviceGetStreamPriorityRange(&least, &greatest) == cudaSuccess && cudaStreamCreateWithPriority(&s.stream, cudaStreamNonBlocking, greatest) == cudaSuccess;
+        for (cudaEvent_t& ev : s.events) ok = ok && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) == cudaSuccess;
+        if (!ok) {
+            Destroy(s);
+            return false;
+        }
+        *out = s;
+        return true;
+    }
+    void GiveBack(int device, const SideStream& s) {
+        if (s.stream == nullptr) return;
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (idle[device].size() < kPooled) {
+                idle[device].push_back(s);
+                return;
+            }
+        }
+        Destroy(s);
+    }
+
+private:
+    static void Destroy(const SideStream& s) {
+        for (cudaEvent_t ev : s.events)
+            if (ev) cudaEventDestroy(ev);
+        if (s.stream) cudaStreamDestroy(s.stream);
+    }
+};
+}  // namespace mgt
+
 struct mgt_engine {
     int device = 0;
     int sm_count = 148;
@@ -260,10 +322,8 @@ struct mgt_engine {
     std::unordered_map<mgt::MapKey, CUtensorMap, mgt::MapKeyHash> maps;
     std::mutex mu;
     cudaEvent_t ev_last = nullptr, ev_now = nullptr;
-    // a second stream for the weight gradients of small batches (SideBranch), and the events that tie it to the caller's
-    cudaStream_t side = nullptr;
-    cudaEvent_t ev_side[3] = {nullptr, nullptr, nullptr};
-    std::mutex side_mu;  // an event is recorded and waited for in one piece
+    mgt::SideStream side;  // for the weight gradients of small batches (SideBranch)
+    std::mutex side_mu;    // an event is recorded and waited for in one piece
     uint64_t launches = 0;  // kernels launched through this engine (host-side count)
     bool layered_tower = false;  // MGT_RESIDUAL_PATH=layered: per-layer GEMMs instead of the fused residual-tower kernels (both are tested)
     mgt_gradient_ready_fn early_fn = nullptr;  // mgt_engine_set_early_range_hook
@@ -1019,25 +1079,19 @@ struct SideBranch {
 
     bool Tie(int event, cudaStream_t from, cudaStream_t to) {
         std::lock_guard<std::mutex> lock(e->side_mu);
-        return cudaEventRecord(e->ev_side[event], from) == cudaSuccess && cudaStreamWaitEvent(to, e->ev_side[event], 0) == cudaSuccess;
+        return cudaEventRecord(e->side.events[event], from) == cudaSuccess && cudaStreamWaitEvent(to, e->side.events[event], 0) == cudaSuccess;
     }
     bool Fork() {
         {
             std::lock_guard<std::mutex> lock(e->side_mu);
-            // (ahead of the caller's stream where both have blocks to place: the embedding gradient then ends the pass with the
-            // whole chip; 3 001 samples of p888 550 -> 523 us a step)
-            int least = 0, greatest = 0;
-            if (e->side == nullptr && (cudaDeviceGetStreamPriorityRange(&least, &greatest) != cudaSuccess ||
-                                       cudaStreamCreateWithPriority(&e->side, cudaStreamNonBlocking, greatest) != cudaSuccess)) return false;
-            for (cudaEvent_t& ev : e->ev_side)
-                if (ev == nullptr && cudaEventCreateWithFlags(&ev, cudaEventDisableTiming) != cudaSuccess) return false;
+            if (e->side.stream == nullptr && !SidePool::Get().Take(e->device, &e->side)) return false;
         }
-        return open = Tie(0, main, e->side);
+        return open = Tie(0, main, e->side.stream);
     }
     bool Join() {
         const bool was = open;
         open = false;
-        return !was || Tie(2, e->side, main);
+        return !was || Tie(2, e->side.stream, main);
     }
     ~SideBranch() { Join(); }
 };
@@ -1514,9 +1568,7 @@ mgt_status_t mgt_engine_destroy(mgt_engine_t* e) {
     if (e == nullptr) return MGT_OK;
     if (e->ev_last) cudaEventDestroy(e->ev_last);
     if (e->ev_now) cudaEventDestroy(e->ev_now);
-    for (cudaEvent_t ev : e->ev_side)
-        if (ev) cudaEventDestroy(ev);
-    if (e->side) cudaStreamDestroy(e->side);
+    SidePool::Get().GiveBack(e->device, e->side);
     if (e->status_word) cudaFree(e->status_word);
     delete e;
     return MGT_OK;
@@ -1858,14 +1910,14 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     const uint64_t dx_tiles = (uint64_t)((H1 + 127U) / 128U) * ((B + 255U) / 256U);
     SideBranch branch{e, st};
     if (dx_tiles < 2ULL * e->sm_count && B <= 16384U && ready == nullptr && e->early_fn == nullptr && profile == nullptr && !branch.Fork()) return MGT_CUDA_FAILURE;
-    cudaStream_t st_dw = branch.open ? e->side : st;
+    cudaStream_t st_dw = branch.open ? e->side.stream : st;
     uint32_t* order = reinterpret_cast<uint32_t*>(base + ws.off_lists);
     uint32_t* first = order + (uint64_t)s.state_len * B;
     auto sort_classes = [&](cudaStream_t stream) {
         gather::SortByClassKernel<<<s.state_len, 1024, 0, stream>>>(reinterpret_cast<const uint8_t*>(states), B, s.state_value_pad, order, first);
         ++e->launches;
     };
-    if (branch.open && half_ig && ws.gather_grad) sort_classes(e->side);
+    if (branch.open && half_ig && ws.gather_grad) sort_classes(e->side.stream);
     // dz1T = (Wh * dzh^T) * [pre-activation of a1 > 0], the input-bias gradient from its row sums. With --input-grad-fp16 0 the
     // embedding gradient wants dz1 in fp32 (mlp_backward.cu:1433-1504, float one-hot GEMM): the same product of fp16 operands
     // with fp32 accumulation, written unrounded as rows of samples.
@@ -1886,7 +1938,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
                                                                                                s.state_len, s.state_value_pad, H1, grad, vec);
         };
         if (!branch.open) sort_classes(st);
-        else if (!branch.Tie(1, e->side, st)) return MGT_CUDA_FAILURE;  // (of the branch only the sort is enqueued yet)
+        else if (!branch.Tie(1, e->side.stream, st)) return MGT_CUDA_FAILURE;  // (of the branch only the sort is enqueued yet)
         // a group of lanes per table row, four groups where that leaves fewer than 16 warps for an SM
         const bool few = (uint64_t)IN * ((H1 + 63U) / 64U) < 64ULL * e->sm_count;
         if (few) { if (e->bf16_now) run(gather::GradKernel<4, true>, 8U); else run(gather::GradKernel<4, false>, 8U); }
