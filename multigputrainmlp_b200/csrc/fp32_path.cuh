@@ -72,17 +72,17 @@ __device__ __forceinline__ float4 LoadQuad(const float* __restrict__ p, uint32_t
 
 // A CTA computes a BM x BN tile, a thread TM x TN of it; KG groups of threads share the tile's K chunks and are added in
 // shared memory at the end (small problems: the K loop of one tile is the critical path). Operands are staged through
-// registers into double-buffered shared memory, 16 deep, one barrier per chunk. Bound by the fp32 pipes: with pairs of
+// registers into double-buffered shared memory, BK deep, one barrier per chunk. Bound by the fp32 pipes: with pairs of
 // rows in one fma.rn.f32x2 the inner loop needs TM * TN / 2 of them, TN duplications and (TM + TN) / 4 vector reads.
 // (The first version of this path read scalars through a 4 x 4 tile without prefetch and never split K: the 34 weight
 // gradients of p888 at 8 192 samples took 45.2 ms, now 1.1 ms.)
-template <int BM, int BN, int TM, int TN, int KG, bool TA, bool TB>
+template <int BM, int BN, int TM, int TN, int KG, int BK, bool TA, bool TB>
 __global__ void __launch_bounds__((BM / TM) * (BN / TN) * KG)
 SgemmKernel(const __grid_constant__ SgemmArgs a) {
-    constexpr uint32_t NT = (BM / TM) * (BN / TN), BK = 16;
+    constexpr uint32_t NT = (BM / TM) * (BN / TN);
     constexpr uint32_t QA = BM * BK / 4 / NT, QB = BN * BK / 4 / NT;  // float4 loads per thread and chunk
     constexpr uint32_t LDA = BM + 4, LDB = BN + 4;
-    static_assert(QA >= 1 && QB >= 1 && QA * NT * 4 == BM * BK && QB * NT * 4 == BN * BK, "whole quads per thread");
+    static_assert(QA >= 1 && QB >= 1 && QA * NT * 4 == BM * BK && QB * NT * 4 == BN * BK && BK % 16 == 0, "whole quads per thread");
     __shared__ __align__(16) float As[KG][2][BK][LDA];
     __shared__ __align__(16) float Bs[KG][2][BK][LDB];
     const uint32_t group_k = threadIdx.x / NT, tid = threadIdx.x % NT;
@@ -96,6 +96,9 @@ SgemmKernel(const __grid_constant__ SgemmArgs a) {
     const uint32_t c_end = static_cast<uint32_t>(static_cast<uint64_t>(split + 1U) * chunks / a.splits);
     const uint32_t turns = (c_end - c_begin + KG - 1U) / KG;
 
+    // quad q of an operand with K inside: 16 columns of K at a time, four lanes to a row of them
+    auto k_of = [](uint32_t q, uint32_t rows) { return q / (rows * 4U) * 16U + (q % 4U) * 4U; };
+    auto row_of = [](uint32_t q, uint32_t rows) { return q % (rows * 4U) / 4U; };
     float4 qa[QA], qb[QB];
     auto fetch = [&](uint32_t turn) {
         const uint32_t c = c_begin + turn * KG + group_k;
@@ -104,17 +107,17 @@ SgemmKernel(const __grid_constant__ SgemmArgs a) {
         for (uint32_t i = 0; i < QA; ++i) {
             const uint32_t q = tid + i * NT;
             if (TA) qa[i] = LoadQuad<false>(A, a.lda, a.M, K, m0 + (q % (BM / 4)) * 4U, c * BK + q / (BM / 4), a.vec_a);
-            else qa[i] = LoadQuad<true>(A, a.lda, a.M, K, m0 + q / (BK / 4), c * BK + (q % (BK / 4)) * 4U, a.vec_a);
+            else qa[i] = LoadQuad<true>(A, a.lda, a.M, K, m0 + row_of(q, BM), c * BK + k_of(q, BM), a.vec_a);
         }
 #pragma unroll
         for (uint32_t i = 0; i < QB; ++i) {
             const uint32_t q = tid + i * NT;
-            if (TB) qb[i] = LoadQuad<true>(B, a.ldb, a.N, K, n0 + q / (BK / 4), c * BK + (q % (BK / 4)) * 4U, a.vec_b);
+            if (TB) qb[i] = LoadQuad<true>(B, a.ldb, a.N, K, n0 + row_of(q, BN), c * BK + k_of(q, BN), a.vec_b);
             else qb[i] = LoadQuad<false>(B, a.ldb, a.N, K, n0 + (q % (BN / 4)) * 4U, c * BK + q / (BN / 4), a.vec_b);
         }
     };
-    // An operand with K inside is transposed on its way into shared memory: the four scalars of a quad go to four K rows. Its
-    // rows 8..15 hold the columns with bit 3 flipped, so that the quads of eight rows meet in 32 different banks.
+    // An operand with K inside is transposed on its way into shared memory: the four scalars of a quad go to four K rows. Rows
+    // 8..15 of every 16 hold the columns with bit 3 flipped, so that the quads of eight rows meet in 32 different banks.
     auto stage = [&](uint32_t buf) {
 #pragma unroll
         for (uint32_t i = 0; i < QA; ++i) {
@@ -122,7 +125,7 @@ SgemmKernel(const __grid_constant__ SgemmArgs a) {
             if (TA) {
                 *reinterpret_cast<float4*>(&As[group_k][buf][q / (BM / 4)][(q % (BM / 4)) * 4U]) = qa[i];
             } else {
-                const uint32_t k = (q % (BK / 4)) * 4U, r = (q / (BK / 4)) ^ (k & 8U);
+                const uint32_t k = k_of(q, BM), r = row_of(q, BM) ^ (k & 8U);
                 As[group_k][buf][k][r] = qa[i].x; As[group_k][buf][k + 1][r] = qa[i].y; As[group_k][buf][k + 2][r] = qa[i].z; As[group_k][buf][k + 3][r] = qa[i].w;
             }
         }
@@ -132,7 +135,7 @@ SgemmKernel(const __grid_constant__ SgemmArgs a) {
             if (!TB) {
                 *reinterpret_cast<float4*>(&Bs[group_k][buf][q / (BN / 4)][(q % (BN / 4)) * 4U]) = qb[i];
             } else {
-                const uint32_t k = (q % (BK / 4)) * 4U, r = (q / (BK / 4)) ^ (k & 8U);
+                const uint32_t k = k_of(q, BN), r = row_of(q, BN) ^ (k & 8U);
                 Bs[group_k][buf][k][r] = qb[i].x; Bs[group_k][buf][k + 1][r] = qb[i].y; Bs[group_k][buf][k + 2][r] = qb[i].z; Bs[group_k][buf][k + 3][r] = qb[i].w;
             }
         }
@@ -149,7 +152,7 @@ SgemmKernel(const __grid_constant__ SgemmArgs a) {
     for (uint32_t turn = 0; turn < turns; ++turn) {
         const uint32_t buf = turn & 1U;
         if (turn + 1U < turns) fetch(turn + 1U);
-#pragma unroll
+#pragma unroll 16
         for (uint32_t k = 0; k < BK; ++k) {
             uint64_t av[TM / 2];
             float bv[TN];
@@ -255,7 +258,11 @@ SgemmKernel(const __grid_constant__ SgemmArgs a) {
 
 // Tile choice. The large tile has the best ratio of multiply-adds to shared-memory reads but needs two waves of the 148 SMs
 // to balance; the middle one (four CTAs per SM) covers the rest of the range; below one CTA per SM the K loop of a single
-// tile is what takes the time, so small tiles with four K groups.
+// tile is what takes the time, so small tiles. Gradients split K over four groups of threads there. The forward product (neither
+// operand transposed) adds in the order of k whatever its tile: its results decide the ReLUs, and every other order opens or
+// closes one here and there, which moves the gradient by up to 1e-4, where a gradient product's own order moves it by 1e-7. So one
+// K group, and chunks of 64 to keep loads in flight (a step of 1 024 samples, hd1 256, hd2 64, 2 blocks 186 us with four groups,
+// 195 us like this).
 enum class SgemmTile { kLarge, kMiddle, kSmall };
 inline uint32_t SgemmTileRows(SgemmTile t) { return t == SgemmTile::kLarge ? 128U : (t == SgemmTile::kMiddle ? 64U : 32U); }
 inline SgemmTile PickSgemmTile(uint32_t M, uint32_t N, uint64_t batches, uint32_t sm_count) {
@@ -273,9 +280,10 @@ inline cudaError_t Sgemm(cudaStream_t st, SgemmArgs a, uint32_t groups, SgemmTil
     a.vec_b = SgemmAligned(a.B, a.ldb, a.stride_b);
     const uint32_t t = SgemmTileRows(tile);
     const dim3 grid((a.N + t - 1) / t, (a.M + t - 1) / t, groups * a.splits);
-    if (tile == SgemmTile::kLarge) SgemmKernel<128, 128, 8, 8, 1, TA, TB><<<grid, 256, 0, st>>>(a);
-    else if (tile == SgemmTile::kMiddle) SgemmKernel<64, 64, 8, 4, 1, TA, TB><<<grid, 128, 0, st>>>(a);
-    else SgemmKernel<32, 32, 4, 4, 4, TA, TB><<<grid, 256, 0, st>>>(a);
+    if (tile == SgemmTile::kLarge) SgemmKernel<128, 128, 8, 8, 1, 16, TA, TB><<<grid, 256, 0, st>>>(a);
+    else if (tile == SgemmTile::kMiddle) SgemmKernel<64, 64, 8, 4, 1, 16, TA, TB><<<grid, 128, 0, st>>>(a);
+    else if constexpr (!TA && !TB) SgemmKernel<32, 32, 4, 4, 1, 64, TA, TB><<<grid, 64, 0, st>>>(a);
+    else SgemmKernel<32, 32, 4, 4, 4, 16, TA, TB><<<grid, 256, 0, st>>>(a);
     return cudaGetLastError();
 }
 

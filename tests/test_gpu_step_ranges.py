@@ -109,6 +109,63 @@ def test_fp32_linears_over_tiles(oracle, dims, n):
     loss_grad_case(oracle, dims, n, flags=(False, False), tol=1e-5, section_tol=2e-5)
 
 
+def multiply_in_order(x, w):
+    """x w in fp32, one multiply-add after the other along k (the product of two floats is exact in double)."""
+    acc = np.zeros((x.shape[0], w.shape[1]), np.float32)
+    x, w = x.astype(np.float64), w.astype(np.float64)
+    for k in range(w.shape[0]):
+        acc = (x[:, k:k + 1] * w[k] + acc).astype(np.float32)
+    return acc
+
+
+# The forward products of the fp32 path add in the order of k whatever their tile: another order opens or closes a ReLU here and
+# there, and with it the path of a whole gradient. With a batch of one sample every activation can be read back to the bit: a
+# weight's gradient is the rounded product of the activation below it and of its unit's bias gradient.
+@pytest.mark.parametrize("dims", [(18, 6, 64, 48, 6, 1), (18, 6, 200, 33, 3, 1), (72, 72, 1032, 230, 2, 1), (5, 3, 17, 300, 1, 1), (5, 3, 16, 8, 1, 1)])
+def test_fp32_forward_adds_in_order(oracle, dims):
+    shape = MlpShape(*dims)
+    length, values, h1, h2, blocks = dims[:5]
+    c = mgt.CudaMlpShape(*dims)
+    floats = mgt.mlp_loss_grad_workspace_floats(c, 1, 1, False, False)
+    ws, loss, grad = torch.empty(floats, device=DEV), torch.zeros(1, device=DEV), torch.zeros(shape.param_count, device=DEV)
+    std = [0.8 / length ** 0.5, 0.05, (2 / h1) ** 0.5, 0.05] + [(2 / h2) ** 0.5, 0.05, (2 / h2) ** 0.5, 0.02] * blocks + [h2 ** -0.5, 0.1]
+    sizes = [(length * values, h1), (h1,), (h1, h2), (h2,)] + [(h2, h2), (h2,)] * (2 * blocks) + [(h2,), (1,)]
+
+    def split(flat):
+        ends = np.cumsum([int(np.prod(size)) for size in sizes])
+        return [part.reshape(size) for part, size in zip(np.split(flat, ends[:-1]), sizes)]
+    engine = mgt.Engine(0)
+    try:
+        for seed in range(4):
+            moves, target = random_puzzle(length, 18, seed)
+            target[:length] = np.arange(length) * values // length
+            _, state, depth, _ = oracle.random_walks(moves, target, seed=seed, epoch=0, step=0, rank=0, k_min=1, k_max=29, samples=1, state_len=length)
+            rng = np.random.default_rng(seed)
+            w = np.concatenate([rng.standard_normal(int(np.prod(size))) * s for size, s in zip(sizes, std)]).astype(np.float32)
+            st = engine.launch_mlp_loss_grad(c, torch.from_numpy(w).to(DEV), None, torch.from_numpy(state).to(DEV), torch.from_numpy(depth).to(DEV), 1, loss, grad, ws,
+                                             floats, use_half_input_grad=False, use_half_linear=False)
+            assert st == 0 and engine.check()[0] == 0
+            part, g = split(w), split(grad.cpu().numpy())
+            a = part[1][None].copy()
+            for p in range(length):
+                a += part[0][p * values + int(state[0, p])]
+            a = np.maximum(a, np.float32(0))
+            layers = [(a, 2)]
+            x = np.maximum(multiply_in_order(a, part[2]) + part[3], np.float32(0))
+            for b in range(4, 4 + 4 * blocks, 4):
+                r = np.maximum(multiply_in_order(x, part[b]) + part[b + 1], np.float32(0))
+                layers += [(x, b), (r, b + 2)]
+                x = np.maximum((multiply_in_order(r, part[b + 2]) + part[b + 3]) + x, np.float32(0))
+            layers.append((x, 4 + 4 * blocks))
+            for act, i in layers:
+                bias = g[i + 1]
+                assert np.count_nonzero(act) and np.count_nonzero(bias)
+                want = act[0] * bias[0] if i == 4 + 4 * blocks else act[0][:, None] * bias
+                assert np.array_equal(g[i], want), (seed, i)
+    finally:
+        engine.close()
+
+
 # fp32 table gradient behind fp16 linears: classes without samples, one class per position, many samples per class
 @pytest.mark.parametrize("dims,n,mirror", [((72, 72, 36, 40, 1, 1), 45, True), ((54, 6, 130, 64, 2, 1), 1000, True), ((16, 1, 33, 24, 1, 2), 257, False)])
 def test_fp32_table_gradient(oracle, dims, n, mirror):
