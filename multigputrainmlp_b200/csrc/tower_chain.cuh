@@ -152,7 +152,8 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
     uint64_t* ready_s = w_empty + SW;   // [4] K chunk c of act_s is written
     uint64_t* ready_t = ready_s + 4;    // [4]
     uint64_t* mma_done = ready_t + 4;   // [2] D complete / S complete
-    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(mma_done + 2);
+    uint64_t* sums_done = mma_done + 2; // [2] backward: every epilogue warp has read its bias sums out of D / out of S
+    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(sums_done + 2);
     volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_holder + 1);
     float* bias_slots = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);  // [products of a block][warps per quadrant][chunks per warp][32]
 
@@ -175,6 +176,8 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
         }
         mbar_init(&mma_done[0], 1);
         mbar_init(&mma_done[1], 1);
+        mbar_init(&sums_done[0], ChainCfg::EPI_WARPS);
+        mbar_init(&sums_done[1], ChainCfg::EPI_WARPS);
         *cta_abort = 0;
         fence_barrier_init();
         prefetch_tensormap(&tma_w);
@@ -228,6 +231,9 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
             for (uint32_t tile = blockIdx.x; tile < args.tiles && ok; tile += gridDim.x) {
                 for (uint32_t kb = 0; kb < R && ok; ++kb, ++uses) {
                     for (uint32_t half = 0; half < 2U && ok; ++half) {
+                        // The bias sums of the last product into this D (or S) are read after its panels are handed on, and the
+                        // first K chunk of this product may be in before a warp with other columns has read its own.
+                        if (BWD && !mbar_wait_warp(&sums_done[half], (uses & 1U) ^ 1U, cta_abort, kAbortChainWait)) { ok = false; break; }
                         uint64_t* ready = half ? ready_t : ready_s;
                         const uint32_t a_base = smem_u32(half ? act_t : act_s);
                         const uint32_t d_addr = tmem_base + (half ? kStateCol : 0U);
@@ -341,8 +347,8 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = __float_as_uint(((bits >> j) & 1U) ? __uint_as_float(v[j]) : 0.0f);
         };
-        // bias sums of a product (its columns from `taddr` on), when the panels are handed on
-        auto column_sums = [&](uint32_t taddr, uint32_t tile, uint32_t slot) {
+        // bias sums of a product (its columns from `taddr` on), when the panels are handed on; `done`: the columns may be overwritten
+        auto column_sums = [&](uint32_t taddr, uint32_t tile, uint32_t slot, uint64_t* done) {
             tmem_st_wait();
 #pragma unroll
             for (uint32_t ci = 0; ci < WPW; ++ci) {
@@ -353,6 +359,9 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                 const uint32_t col = cc * 32U + j;
                 if (col < H) args.colsum[slot * args.colsum_stride + (static_cast<uint64_t>(tile) * 4U + quad) * H + col] = total;
             }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(done);
         };
 
         uint32_t uses = 0;
@@ -428,7 +437,7 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                         publish(&ready_t[cc >> 1]);
                         if (!BWD) words[ci] = detail::positive_bits(raw);
                     }
-                    if (BWD) column_sums(tmem_base + lane_addr, tile, k);
+                    if (BWD) column_sums(tmem_base + lane_addr, tile, k, &sums_done[0]);
                     if (!BWD) store_words(args.bits_t + k * args.bits_stride + bits_row, words);
                 }
                 // ================= second epilogue: new S =================
@@ -469,7 +478,7 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                             }
                         }
                     }
-                    if (BWD) column_sums(tmem_base + lane_addr + kStateCol, tile, R + k);
+                    if (BWD) column_sums(tmem_base + lane_addr + kStateCol, tile, R + k, &sums_done[1]);
                     if (!BWD) store_words(args.bits_s + (k + 1U) * args.bits_stride + bits_row, words);
                     if (last) tc_fence_before();  // the next tile's state load overwrites the TMEM columns read here
                 }

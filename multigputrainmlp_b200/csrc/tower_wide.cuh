@@ -67,7 +67,8 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
     uint64_t* w_empty = w_full + SW;
     uint64_t* ready = w_empty + SW;     // [8] K chunk c of the operand is there: own chunks from the epilogue, the others by copy
     uint64_t* mma_done = ready + 8;     // [2] D / S complete in both CTAs and the operand's panels stored
-    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(mma_done + 2);
+    uint64_t* sums_done = mma_done + 2; // [2] backward: every epilogue warp has read its bias sums out of D / out of S
+    uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(sums_done + 2);
     volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_holder + 1);
     float* bias_slots = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(bars) + 256);  // [products of a block][warps per quadrant][chunks per warp][32]
 
@@ -95,6 +96,8 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
         }
         mbar_init(&mma_done[0], 3);  // the commits of both CTAs and the storing warp
         mbar_init(&mma_done[1], 3);
+        mbar_init(&sums_done[0], WideCfg::EPI_WARPS);
+        mbar_init(&sums_done[1], WideCfg::EPI_WARPS);
         *cta_abort = 0;
         fence_barrier_init();
         prefetch_tensormap(&tma_w);
@@ -151,6 +154,8 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
             for (uint32_t tile = cluster; tile < args.tiles && ok; tile += clusters) {
                 for (uint32_t kb = 0; kb < R && ok; ++kb) {
                     for (uint32_t half = 0; half < 2U && ok; ++half, ++step) {
+                        // (the bias sums are read after the panels are handed on, and a panel may be in before they are: see tower_chain.cuh)
+                        if (BWD && !mbar_wait_warp(&sums_done[half], ((step >> 1) & 1U) ^ 1U, cta_abort, kAbortChainWait)) { ok = false; break; }
                         const uint32_t a_base = smem_u32(act);
                         const uint32_t d_addr = tmem_base + (half ? kStateCol : 0U);
                         for (uint32_t c = 0; c < KC; ++c)
@@ -284,8 +289,8 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = ((bits >> j) & 1U) ? v[j] : 0U;
         };
-        // bias sums of a product (its columns from `taddr` on), when the panels are handed on
-        auto column_sums = [&](uint32_t taddr, uint32_t tile, uint32_t slot) {
+        // bias sums of a product (its columns from `taddr` on), when the panels are handed on; `done`: the columns may be overwritten
+        auto column_sums = [&](uint32_t taddr, uint32_t tile, uint32_t slot, uint64_t* done) {
             tmem_st_wait();
 #pragma unroll
             for (uint32_t ci = 0; ci < WPW; ++ci) {
@@ -296,6 +301,9 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
                 const uint32_t col = col0 + cc * 32U + j;
                 if (col < H) args.colsum[slot * args.colsum_stride + (static_cast<uint64_t>(tile) * 4U + quad) * H + col] = total;
             }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(done);
         };
 
         uint32_t uses = 0;
@@ -371,7 +379,7 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
                         publish(&ready[p0 + (cc >> 1)]);
                         if (!BWD) words[ci] = detail::positive_bits(raw);
                     }
-                    if (BWD) column_sums(tmem_base + lane_addr, tile, k);
+                    if (BWD) column_sums(tmem_base + lane_addr, tile, k, &sums_done[0]);
                     if (!BWD) store_words(args.bits_t + k * args.bits_stride + bits_row, words);
                 }
                 // ================= second epilogue: new S =================
@@ -412,7 +420,7 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
                             }
                         }
                     }
-                    if (BWD) column_sums(tmem_base + lane_addr + kStateCol, tile, R + k);
+                    if (BWD) column_sums(tmem_base + lane_addr + kStateCol, tile, R + k, &sums_done[1]);
                     if (!BWD) store_words(args.bits_s + (k + 1U) * args.bits_stride + bits_row, words);
                     if (last) tc_fence_before();  // the next tile's state load overwrites the TMEM columns read here
                 }

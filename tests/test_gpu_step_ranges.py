@@ -212,3 +212,36 @@ def test_wide_residual_tower(oracle, hd2, n, mirror, bf16):
 @pytest.mark.parametrize("dims,n", [((72, 72, 896, 40, 2, 1), 96), ((72, 72, 897, 40, 2, 1), 96), ((54, 6, 1024, 64, 1, 3), 513), ((72, 72, 1032, 33, 0, 1), 257)])
 def test_weight_gradients_beside_the_embedding_gradient(oracle, dims, n):
     loss_grad_case(oracle, dims, n, scale=0.02)
+
+
+# Bias sums of the backward tower with two and three tiles to a CTA (or pair), whose products follow one another into the same
+# tensor memory: the same bits every time, and the layer-by-layer path's sums up to fp16 roundings that fall the other way.
+@pytest.mark.parametrize("hd2,n", [(64, 37965), (160, 37965), (256, 40000), (272, 19021), (512, 19021)])
+def test_tower_bias_sums_over_tiles(oracle, monkeypatch, hd2, n):
+    dims = (8, 8, 32, hd2, 3, 1)
+    shape = MlpShape(*dims)
+    moves, target = random_puzzle(8, 18, 3)
+    _, states, depth, _ = oracle.random_walks(moves, target, seed=3, epoch=0, step=0, rank=0, k_min=1, k_max=29, samples=n, state_len=8)
+    w = torch.from_numpy((np.random.default_rng(3).standard_normal(shape.param_count) * 0.05).astype(np.float32)).to(DEV)
+    d_states, labels = torch.from_numpy(states).to(DEV), torch.from_numpy(depth).to(DEV)
+    c = mgt.CudaMlpShape(*dims)
+    floats = mgt.mlp_loss_grad_workspace_floats(c, n)
+    ws, loss = torch.empty(floats, device=DEV), torch.zeros(1, device=DEV)
+    grads = []
+    for path in ("fused", "layered"):
+        monkeypatch.setenv("MGT_RESIDUAL_PATH", path)
+        engine = mgt.Engine(0)
+        try:
+            for _ in range(4 if path == "fused" else 1):
+                grad = torch.full((shape.param_count,), float("nan"), device=DEV)
+                assert engine.launch_mlp_loss_grad(c, w, w.half(), d_states, labels, n, loss, grad, ws, floats) == 0
+                assert engine.check()[0] == 0
+                grads.append(grad.cpu().numpy())
+        finally:
+            engine.close()
+    for other in grads[1:4]:
+        assert np.array_equal(other, grads[0])
+    first = 64 * 32 + 32 + 32 * hd2 + hd2
+    for layer in range(6):
+        lo = first + layer * (hd2 * hd2 + hd2) + hd2 * hd2
+        assert rel_l2(grads[0][lo:lo + hd2], grads[4][lo:lo + hd2]) <= 1e-3, layer
