@@ -149,7 +149,10 @@ EmbeddingForms PickEmbeddingForms(const mgt_mlp_shape_t& s, uint32_t B, uint32_t
     return {4.0 + sums / 8.0e6 < PlanPairForward(s, B, sm).us, 8.0 + B * 0.0019 + sums / 6.7e6 < PlanPairGrad(s, B, sm).us};
 }
 
-Workspace PlanWorkspace(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm_count, bool batch_norm = false) {
+// No term may fall with a larger batch: a caller sizes its scratch for the largest batch and runs smaller ones in it. So what a
+// form of the embedding layer needs is planned whichever form this batch takes (288 bytes a sample of 72 positions). half_ig: the
+// table gradient is the 16-bit one (the fp32 one keeps its lists behind this workspace).
+Workspace PlanWorkspace(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm_count, bool half_ig, bool batch_norm = false) {
     Workspace w{};
     w.B = B; w.H1 = s.hd1; w.H2 = s.hd2; w.R = s.residual_blocks; w.OUT = s.output_dim;
     w.IN = s.state_len * s.state_value_pad;
@@ -181,8 +184,8 @@ Workspace PlanWorkspace(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm_count,
     w.gather_fwd = forms.gather_fwd;
     w.gather_grad = forms.gather_grad;
     w.p_dz1_rows = (uint32_t)RoundUp(s.hd1, 8);
-    w.off_dz1 = take(std::max<uint64_t>(hidden_act_bytes, forms.gather_grad ? (uint64_t)B * w.p_dz1_rows * 2 : 0));
-    w.off_lists = take(forms.gather_grad ? gather::ListWords(B, s.state_len, s.state_value_pad) * 4 : 0);
+    w.off_dz1 = take(std::max<uint64_t>(hidden_act_bytes, half_ig ? (uint64_t)B * w.p_dz1_rows * 2 : 0));
+    w.off_lists = take(half_ig ? gather::ListWords(B, s.state_len, s.state_value_pad) * 4 : 0);
     // split-K partials: at most one CTA wave of [128 x 256] fp32 tiles plus slack for tile padding
     const uint64_t hidden_units = (uint64_t)((s.hd1 + 127) / 128) * ((s.hd2 + 255) / 256);
     const uint64_t resid_units = (uint64_t)((s.hd2 + 127) / 128) * ((s.hd2 + 255) / 256);
@@ -1590,16 +1593,17 @@ mgt_status_t mgt_engine_check(mgt_engine_t* e, void* stream, int32_t* out_device
 }
 
 // The fp32 operand of the table gradient behind the tensor-core workspace: dz1 [samples][hd1], rows padded to four floats,
-// then the sample lists of its classes (and slack to align the start).
+// then the sample lists of its classes (and slack: to align the start, and for the rounding of what the 16-bit gradient plans
+// instead, so that scratch of this size does for either).
 static uint64_t Fp32TableFloats(const mgt_mlp_shape_t& s, uint32_t B) {
-    return (uint64_t)B * RoundUp(s.hd1, 4) + gather::ListWords(B, s.state_len, s.state_value_pad) + 64;
+    return (uint64_t)B * RoundUp(s.hd1, 4) + gather::ListWords(B, s.state_len, s.state_value_pad) + 64 + 512;
 }
 
 static uint64_t WorkspaceFloats(const mgt_mlp_shape_t* shape, uint32_t sample_count, uint32_t chunks, int32_t use_half_input_grad, int32_t use_half_linear,
                                 bool batch_norm) {
     if (!ValidShape(shape) || sample_count == 0 || chunks == 0) return 0;
     if (!use_half_linear) return batch_norm ? 0 : Fp32WorkspaceFloats(*shape, sample_count, CurrentDeviceSmCount());
-    const Workspace w = PlanWorkspace(*shape, sample_count, CurrentDeviceSmCount(), batch_norm);
+    const Workspace w = PlanWorkspace(*shape, sample_count, CurrentDeviceSmCount(), use_half_input_grad != 0, batch_norm);
     return (w.total_bytes + 3) / 4 + (use_half_input_grad ? 0 : Fp32TableFloats(*shape, sample_count));
 }
 
@@ -1659,7 +1663,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
         return LaunchFp32Path(e, s, w, reinterpret_cast<const uint8_t*>(states), labels, B, loss, grad, workspace, half_ig != 0, profile, tell,
                               static_cast<cudaStream_t>(stream_v));
     }
-    const Workspace ws = PlanWorkspace(s, B, PlanSmCount(e->sm_count), bnorm);
+    const Workspace ws = PlanWorkspace(s, B, PlanSmCount(e->sm_count), half_ig != 0, bnorm);
     if (workspace_floats < (ws.total_bytes + 3) / 4 + (half_ig ? 0 : Fp32TableFloats(s, B))) return MGT_CAPACITY_EXCEEDED;
     cudaStream_t st = static_cast<cudaStream_t>(stream_v);
     uint8_t* base = reinterpret_cast<uint8_t*>(RoundUp(reinterpret_cast<uintptr_t>(workspace), 1024));

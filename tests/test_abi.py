@@ -49,6 +49,22 @@ def test_host_side_validation_without_gpu():
     assert mgt.validate_adamw_kernel_config(mgt.AdamWKernelConfig(8, 1, 1e-3, weight_decay=-1.0)) == 1
 
 
+def test_workspace_never_shrinks_with_the_batch():
+    # scratch sized for the largest batch has to do for every smaller one, on both sides of every rule that picks a kernel by size
+    import multigputrainmlp_b200 as mgt
+    spans = [((72, 72, 2560, 224, 16, 1), range(3500, 3800)), ((72, 72, 1000, 200, 8, 29), range(7200, 7600)), ((54, 54, 512, 64, 2, 1), range(16600, 16800)),
+             ((54, 6, 1024, 256, 4, 1), range(1, 4000, 37)), ((72, 72, 333, 77, 3, 1), range(1, 40000, 401)), ((16, 1, 33, 24, 0, 2), range(1, 300))]
+    for dims, batches in spans:
+        shape = mgt.CudaMlpShape(*dims)
+        for half_ig, half_lin, bn in ((True, True, False), (False, True, False), (True, True, True), (False, False, False), (True, False, False)):
+            sizes = [mgt.mlp_loss_grad_workspace_floats(shape, b, 1, half_ig, half_lin, batch_norm=bn) for b in batches]
+            assert sizes[0] > 0
+            assert all(x <= y for x, y in zip(sizes, sizes[1:])), (dims, half_ig, half_lin, bn)
+        # and what is asked for with the fp32 table gradient does for the 16-bit one
+        for b in batches:
+            assert mgt.mlp_loss_grad_workspace_floats(shape, b, 1, False, True) >= mgt.mlp_loss_grad_workspace_floats(shape, b, 1, True, True)
+
+
 def test_walk_launch_refuses_misaligned_arrays_before_any_launch():
     # host-side argument checks only: nothing reaches the device (there is none here)
     import multigputrainmlp_b200 as mgt
