@@ -1042,6 +1042,30 @@ HeadOutNBiasGradKernel(const float* __restrict__ dy, uint32_t B, uint32_t OUT, f
     if (threadIdx.x == 0) grad_b[o] = s_sum[0];
 }
 
+// The dynamic shared memory a kernel may take is an attribute that every thread of the process shares: it is set once per device,
+// to all that is left beside the kernel's static arrays, never to what this launch needs (another thread's launch may want more
+// at that moment, and a kernel with static arrays needs it set below 48 KB too).
+template <void (*kKernel)(HeadArgs)>
+bool LaunchHeadKernel(int device, uint32_t grid, size_t smem, cudaStream_t st, const HeadArgs& a) {
+    static std::mutex attr_mu;
+    static size_t most[64] = {};
+    if (device < 0 || device >= 64) return false;
+    {
+        std::lock_guard<std::mutex> lock(attr_mu);
+        if (most[device] == 0) {
+            cudaFuncAttributes attr{};
+            int limit = 0;
+            if (cudaFuncGetAttributes(&attr, kKernel) != cudaSuccess || cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess) return false;
+            const size_t left = static_cast<size_t>(limit) - attr.sharedSizeBytes;
+            if (cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(left)) != cudaSuccess) return false;
+            most[device] = left;
+        }
+        if (smem > most[device]) return false;
+    }
+    kKernel<<<grid, kHeadThreads, smem, st>>>(a);
+    return true;
+}
+
 // Output layer with several outputs, its loss and the gradient entering the layer below, enqueued; all gradients of the head
 // except W_out's, which is a product over the batch.
 template <bool kCrossEntropy, bool kF32>
@@ -1049,16 +1073,11 @@ mgt_status_t LaunchHeadN(mgt_engine* e, cudaStream_t st, const HeadArgs& a, floa
     const bool tiled = a.OUT <= 64U;
     const uint32_t tiles = tiled ? (a.B + kHeadTile - 1U) / kHeadTile : (a.B + 7U) / 8U;
     const uint32_t grid = tiles < kHeadBlocks ? tiles : kHeadBlocks;
-    auto run = [&](auto kernel, size_t smem) -> bool {
-        if (smem > 48U * 1024U && cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return false;
-        kernel<<<grid, kHeadThreads, smem, st>>>(a);
-        return true;
-    };
     bool ok;
-    if (a.OUT <= 16U) ok = run(HeadTileKernel<16, kCrossEntropy, kF32>, HeadTileSmem<16>(a.H2));
-    else if (a.OUT <= 32U) ok = run(HeadTileKernel<32, kCrossEntropy, kF32>, HeadTileSmem<32>(a.H2));
-    else if (tiled) ok = run(HeadTileKernel<64, kCrossEntropy, kF32>, HeadTileSmem<64>(a.H2));
-    else ok = run(HeadOutNKernel<kCrossEntropy, kF32>, (kHeadThreads / 32) * a.OUT * sizeof(float));
+    if (a.OUT <= 16U) ok = LaunchHeadKernel<HeadTileKernel<16, kCrossEntropy, kF32>>(e->device, grid, HeadTileSmem<16>(a.H2), st, a);
+    else if (a.OUT <= 32U) ok = LaunchHeadKernel<HeadTileKernel<32, kCrossEntropy, kF32>>(e->device, grid, HeadTileSmem<32>(a.H2), st, a);
+    else if (tiled) ok = LaunchHeadKernel<HeadTileKernel<64, kCrossEntropy, kF32>>(e->device, grid, HeadTileSmem<64>(a.H2), st, a);
+    else ok = LaunchHeadKernel<HeadOutNKernel<kCrossEntropy, kF32>>(e->device, grid, (kHeadThreads / 32) * a.OUT * sizeof(float), st, a);
     if (!ok) return MGT_CUDA_FAILURE;
     const uint32_t items = tiled ? 1U + a.H2 + a.OUT : 1U + a.H2;
     ReduceHeadNKernel<<<(items + kReduceCols - 1U) / kReduceCols, 256, 0, st>>>(a.partials, grid, a.H2, 1U + a.H2 + a.OUT, items, loss, bias_below, grad_b);

@@ -1,5 +1,7 @@
 """GPU parity at the sizes where a kernel's split or a rule of the dispatch changes: edges of tiles, remainders, the smallest
 and largest of a range. The walk generator bit-exactly and the loss + gradient against the oracle, as in the other suites."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -180,6 +182,40 @@ def test_output_head_widths(oracle, outputs, hd2, n, cross_entropy):
     if cross_entropy and outputs < 29:
         pytest.skip("a class per depth")
     loss_grad_case(oracle, dims, n, options=dict(cross_entropy=True) if cross_entropy else None, tol=2e-3, section_tol=5e-3)
+
+
+# four threads, an engine and a stream each, whose heads are one kernel with different amounts of shared memory
+def test_output_heads_in_several_threads():
+    failed = []
+
+    def steps(hd2):
+        c = mgt.CudaMlpShape(8, 8, 16, hd2, 0, 29)
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            w = torch.zeros(c.param_count, device=DEV)
+            states, labels = torch.zeros(64, 80, dtype=torch.uint8, device=DEV), torch.ones(64 * 29, device=DEV)
+            floats = mgt.mlp_loss_grad_workspace_floats(c, 64)
+            ws, loss, grad = torch.empty(floats, device=DEV), torch.zeros(1, device=DEV), torch.zeros_like(w)
+            engine = mgt.Engine(0)
+            for _ in range(1500):
+                status = engine.launch_mlp_loss_grad(c, w, None, states, labels, 64, loss, grad, ws, floats, stream=stream)
+                if status != 0:
+                    failed.append((hd2, status))
+                    break
+            stream.synchronize()
+            engine.close()
+    threads = [threading.Thread(target=steps, args=(hd2,)) for hd2 in (512, 224, 512, 224)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed
+
+
+# outputs around the limit of shared memory that a kernel gets without asking, counting the static array beside it
+@pytest.mark.parametrize("outputs", [1000, 1030, 1600])
+def test_many_outputs(oracle, outputs):
+    loss_grad_case(oracle, (8, 8, 16, 24, 1, outputs), 70, tol=2e-3, section_tol=5e-3)
 
 
 # embedding layer by gathering rows: samples around a CTA's 32 and 128, columns around its 64 and the vectors of eight, few
