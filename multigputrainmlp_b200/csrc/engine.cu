@@ -256,13 +256,24 @@ struct MapKeyHash {
 }  // namespace mgt
 
 namespace mgt {
-// A second stream and the events that tie it to the caller's. Taken by an engine's first pass that wants one and given back when
-// the engine goes: the pool keeps at most kPooled per device (a program that makes engines one after the other would pay 0.1 ms
-// each for new ones).
+// A second stream and the events that tie it to the caller's. Taken by an engine's first pass on a stream that wants one and given
+// back when the engine goes: the pool keeps kPooled idle ones per device (a program that makes engines one after the other would
+// pay 0.1 ms each for new ones). A stream that a capture still holds is neither handed out nor destroyed.
 struct SideStream {
     cudaStream_t stream = nullptr;
     cudaEvent_t events[3] = {nullptr, nullptr, nullptr};
 };
+// 0: the stream is not being captured, ~0: it cannot be told or the capture is invalid, else the id of the capture
+inline unsigned long long CaptureOf(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    if (cudaStreamGetCaptureInfo(stream, &status, &id) != cudaSuccess) {
+        cudaGetLastError();
+        return ~0ULL;
+    }
+    if (status == cudaStreamCaptureStatusNone) return 0;
+    return status == cudaStreamCaptureStatusActive ? id + 1U : ~0ULL;
+}
 class SidePool {
     static constexpr size_t kPooled = 4;
     std::mutex mu;
@@ -273,16 +284,19 @@ public:
         static SidePool* pool = new SidePool();  // (never destroyed: the CUDA runtime may be gone before it)
         return *pool;
     }
-    bool Take(int device, SideStream* out) {
+    // make = false: only an idle one (nothing is created while a stream is being captured)
+    bool Take(int device, bool make, SideStream* out) {
         if (device < 0 || device >= 64) return false;
         {
             std::lock_guard<std::mutex> lock(mu);
-            if (!idle[device].empty()) {
-                *out = idle[device].back();
-                idle[device].pop_back();
+            for (size_t i = idle[device].size(); i-- > 0;) {
+                if (CaptureOf(idle[device][i].stream) != 0) continue;
+                *out = idle[device][i];
+                idle[device].erase(idle[device].begin() + static_cast<ptrdiff_t>(i));
                 return true;
             }
         }
+        if (!make) return false;
         // (ahead of the caller's stream where both have blocks to place: the embedding gradient then ends the pass with the whole
         // chip; 3 001 samples of p888 550 -> 523 us a step)
         SideStream s;
@@ -300,7 +314,7 @@ public:
         if (s.stream == nullptr) return;
         {
             std::lock_guard<std::mutex> lock(mu);
-            if (idle[device].size() < kPooled) {
+            if (idle[device].size() < kPooled || CaptureOf(s.stream) != 0) {
                 idle[device].push_back(s);
                 return;
             }
@@ -325,8 +339,14 @@ struct mgt_engine {
     std::unordered_map<mgt::MapKey, CUtensorMap, mgt::MapKeyHash> maps;
     std::mutex mu;
     cudaEvent_t ev_last = nullptr, ev_now = nullptr;
-    mgt::SideStream side;  // for the weight gradients of small batches (SideBranch)
-    std::mutex side_mu;    // an event is recorded and waited for in one piece
+    // second streams for the weight gradients of small batches (SideBranch), one for each of the streams this engine was called on
+    struct SideOf {
+        cudaStream_t main;
+        mgt::SideStream side;
+    };
+    std::vector<SideOf> sides;
+    size_t side_turn = 0;
+    std::mutex side_mu;    // of the two above; and an event is recorded and waited for in one piece
     uint64_t launches = 0;  // kernels launched through this engine (host-side count)
     bool layered_tower = false;  // MGT_RESIDUAL_PATH=layered: per-layer GEMMs instead of the fused residual-tower kernels (both are tested)
     mgt_gradient_ready_fn early_fn = nullptr;  // mgt_engine_set_early_range_hook
@@ -1092,28 +1112,55 @@ inline uint32_t GridFor(uint64_t items, uint32_t threads, int sm_count) {
     return (uint32_t)(want < 1 ? 1 : (want < cap ? want : cap));
 }
 
-// Work of the backward pass on the engine's second stream, beside the caller's: from Fork() on, until the object ends (on every
-// path, so that the caller's stream is never ahead of it).
+// Work of the backward pass on a second stream, beside the caller's: from Fork() on, until the object ends (on every path, so that
+// the caller's stream is never ahead of it). Every stream the engine is called on has a second one of its own: on a shared one a
+// step would wait for the step of another stream. (Beyond kSides streams they do share; only the time differs.) Fork() may find no
+// second stream - none can be made, or a capture of other streams holds it - and then all work stays on the caller's, with the same
+// bits.
 struct SideBranch {
+    static constexpr size_t kSides = 4;
     mgt_engine* e;
     cudaStream_t main;
+    SideStream side{};
     bool open = false;
 
+    bool TieLocked(int event, cudaStream_t from, cudaStream_t to) {
+        return cudaEventRecord(side.events[event], from) == cudaSuccess && cudaStreamWaitEvent(to, side.events[event], 0) == cudaSuccess;
+    }
     bool Tie(int event, cudaStream_t from, cudaStream_t to) {
         std::lock_guard<std::mutex> lock(e->side_mu);
-        return cudaEventRecord(e->side.events[event], from) == cudaSuccess && cudaStreamWaitEvent(to, e->side.events[event], 0) == cudaSuccess;
+        return TieLocked(event, from, to);
     }
     bool Fork() {
-        {
-            std::lock_guard<std::mutex> lock(e->side_mu);
-            if (e->side.stream == nullptr && !SidePool::Get().Take(e->device, &e->side)) return false;
+        std::lock_guard<std::mutex> lock(e->side_mu);
+        const unsigned long long capture = CaptureOf(main);
+        bool ok = capture != ~0ULL;
+        mgt_engine::SideOf* slot = nullptr;
+        for (auto& known : e->sides)
+            if (ok && known.main == main) slot = &known;
+        if (ok && slot == nullptr && e->sides.size() < kSides) {
+            SideStream taken;
+            if ((ok = SidePool::Get().Take(e->device, capture == 0, &taken))) {
+                e->sides.push_back({main, taken});
+                slot = &e->sides.back();
+            }
+        } else if (ok && slot == nullptr) {
+            slot = &e->sides[e->side_turn++ % kSides];
+            slot->main = main;
         }
-        return open = Tie(0, main, e->side.stream);
+        if (ok) {
+            side = slot->side;
+            const unsigned long long held = CaptureOf(side.stream);
+            ok = held == 0 || held == capture;
+            open = ok && TieLocked(0, main, side.stream);
+        }
+        if (!open) cudaGetLastError();
+        return open;
     }
     bool Join() {
         const bool was = open;
         open = false;
-        return !was || Tie(2, e->side.stream, main);
+        return !was || Tie(2, side.stream, main);
     }
     ~SideBranch() { Join(); }
 };
@@ -1590,7 +1637,7 @@ mgt_status_t mgt_engine_destroy(mgt_engine_t* e) {
     if (e == nullptr) return MGT_OK;
     if (e->ev_last) cudaEventDestroy(e->ev_last);
     if (e->ev_now) cudaEventDestroy(e->ev_now);
-    SidePool::Get().GiveBack(e->device, e->side);
+    for (const auto& known : e->sides) SidePool::Get().GiveBack(e->device, known.side);
     if (e->status_word) cudaFree(e->status_word);
     delete e;
     return MGT_OK;
@@ -1932,15 +1979,15 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     // 660 us). Not with callers that are told of finished ranges or time the stages: they rely on the order.
     const uint64_t dx_tiles = (uint64_t)((H1 + 127U) / 128U) * ((B + 255U) / 256U);
     SideBranch branch{e, st};
-    if (dx_tiles < 2ULL * e->sm_count && B <= 16384U && ready == nullptr && e->early_fn == nullptr && profile == nullptr && !branch.Fork()) return MGT_CUDA_FAILURE;
-    cudaStream_t st_dw = branch.open ? e->side.stream : st;
+    if (dx_tiles < 2ULL * e->sm_count && B <= 16384U && ready == nullptr && e->early_fn == nullptr && profile == nullptr) branch.Fork();
+    cudaStream_t st_dw = branch.open ? branch.side.stream : st;
     uint32_t* order = reinterpret_cast<uint32_t*>(base + ws.off_lists);
     uint32_t* first = order + (uint64_t)s.state_len * B;
     auto sort_classes = [&](cudaStream_t stream) {
         gather::SortByClassKernel<<<s.state_len, 1024, 0, stream>>>(reinterpret_cast<const uint8_t*>(states), B, s.state_value_pad, order, first);
         ++e->launches;
     };
-    if (branch.open && half_ig && ws.gather_grad) sort_classes(e->side.stream);
+    if (branch.open && half_ig && ws.gather_grad) sort_classes(branch.side.stream);
     // dz1T = (Wh * dzh^T) * [pre-activation of a1 > 0], the input-bias gradient from its row sums. With --input-grad-fp16 0 the
     // embedding gradient wants dz1 in fp32 (mlp_backward.cu:1433-1504, float one-hot GEMM): the same product of fp16 operands
     // with fp32 accumulation, written unrounded as rows of samples.
@@ -1961,7 +2008,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
                                                                                                s.state_len, s.state_value_pad, H1, grad, vec);
         };
         if (!branch.open) sort_classes(st);
-        else if (!branch.Tie(1, e->side.stream, st)) return MGT_CUDA_FAILURE;  // (of the branch only the sort is enqueued yet)
+        else if (!branch.Tie(1, branch.side.stream, st)) return MGT_CUDA_FAILURE;  // (of the branch only the sort is enqueued yet)
         // a group of lanes per table row, four groups where that leaves fewer than 16 warps for an SM
         const bool few = (uint64_t)IN * ((H1 + 63U) / 64U) < 64ULL * e->sm_count;
         if (few) { if (e->bf16_now) run(gather::GradKernel<4, true>, 8U); else run(gather::GradKernel<4, false>, 8U); }

@@ -281,3 +281,111 @@ def test_tower_bias_sums_over_tiles(oracle, monkeypatch, hd2, n):
     for layer in range(6):
         lo = first + layer * (hd2 * hd2 + hd2) + hd2 * hd2
         assert rel_l2(grads[0][lo:lo + hd2], grads[4][lo:lo + hd2]) <= 1e-3, layer
+
+
+class SmallStep:
+    """Loss + gradient of a batch that the library spreads over two streams, with scratch of its own."""
+
+    def __init__(self, engine, n=96, dims=(72, 72, 256, 40, 2, 1)):
+        rng = np.random.default_rng(n)
+        self.engine, self.n, self.shape = engine, n, mgt.CudaMlpShape(*dims)
+        self.w = torch.from_numpy((rng.standard_normal(self.shape.param_count) * 0.03).astype(np.float32)).to(DEV)
+        self.states = torch.from_numpy(rng.integers(0, 72, (n, 80), dtype=np.uint8)).to(DEV)
+        self.labels, self.loss, self.grad = torch.ones(n, device=DEV), torch.zeros(1, device=DEV), torch.zeros_like(self.w)
+        self.floats = mgt.mlp_loss_grad_workspace_floats(self.shape, n)
+        self.ws = torch.empty(self.floats, device=DEV)
+        torch.cuda.synchronize()
+
+    def __call__(self, stream=None, one_stream=False):
+        return self.engine.launch_mlp_loss_grad(self.shape, self.w, None, self.states, self.labels, self.n, self.loss, self.grad, self.ws, self.floats, stream=stream,
+                                                gradient_ready=(lambda *a: 0) if one_stream else None)
+
+    def result(self):
+        torch.cuda.synchronize()
+        assert self.engine.check()[0] == 0
+        got = self.grad.cpu().numpy()
+        self.grad.fill_(float("nan"))
+        torch.cuda.synchronize()
+        return got
+
+
+@pytest.fixture
+def small_step():
+    engine = mgt.Engine(0)
+    yield SmallStep(engine)
+    torch.cuda.synchronize()
+    engine.close()
+
+
+def test_steps_on_several_streams_do_not_wait_for_each_other(small_step):
+    other = SmallStep(small_step.engine, 64)
+    assert small_step(one_stream=True) == 0
+    want = small_step.result()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for stream in streams:
+        assert other(stream) == 0 and other.result() is not None  # (modules loaded, second streams made)
+    with torch.cuda.stream(streams[0]):
+        torch.cuda._sleep(1 << 30)  # half a second
+    assert other(streams[0]) == 0
+    late = streams[0].record_event()
+    assert small_step(streams[1]) == 0
+    streams[1].synchronize()
+    assert not late.query()
+    assert np.array_equal(small_step.result(), want)
+    for stream in [torch.cuda.Stream() for _ in range(7)]:  # more streams than the engine keeps second ones for
+        assert small_step(stream) == 0
+    assert np.array_equal(small_step.result(), want)
+
+
+def test_step_beside_a_capture(small_step):
+    assert small_step(one_stream=True) == 0
+    want = small_step.result()
+    other = SmallStep(small_step.engine, 64)
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    assert small_step(stream) == 0 and other() == 0
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+        assert small_step(stream) == 0 and small_step(stream) == 0
+        free = torch.cuda.Stream()
+        assert other(free) == 0  # eager, on another stream, with the capture open
+        free.synchronize()
+    assert np.isfinite(other.result()).all()
+    small_step.result()
+    graph.replay()
+    assert np.array_equal(small_step.result(), want)
+
+
+def test_two_captures_at_once(small_step):
+    other = SmallStep(small_step.engine, 64)
+    assert other(one_stream=True) == 0 and small_step(one_stream=True) == 0
+    want_other, want = other.result(), small_step.result()
+    streams, graphs = [torch.cuda.Stream() for _ in range(2)], [torch.cuda.CUDAGraph() for _ in range(2)]
+    with torch.cuda.stream(streams[0]):
+        graphs[0].capture_begin(capture_error_mode="relaxed")
+        assert small_step(streams[0]) == 0
+    with torch.cuda.stream(streams[1]):
+        graphs[1].capture_begin(capture_error_mode="relaxed")
+        assert other(streams[1]) == 0
+    for stream, graph in zip(streams, graphs):
+        with torch.cuda.stream(stream):
+            graph.capture_end()
+    for graph in graphs:
+        graph.replay()
+    assert np.array_equal(small_step.result(), want) and np.array_equal(other.result(), want_other)
+
+
+def test_first_step_of_an_engine_under_capture():
+    # no idle second stream is left and none is made during a capture: everything on the caller's stream
+    holders = [SmallStep(mgt.Engine(0), 64) for _ in range(6)]
+    for holder in holders:
+        assert holder() == 0
+    step = SmallStep(mgt.Engine(0))
+    assert step(one_stream=True) == 0
+    want = step.result()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        assert step() == 0
+    graph.replay()
+    assert np.array_equal(step.result(), want)
+    for held in holders + [step]:
+        held.engine.close()
