@@ -356,15 +356,17 @@ onehot_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
                     tmem_ld_32x32(tmem_base + ((quad * 32U) << 16) + cc * 32U, r);
                     tmem_ld_wait();
                     const uint32_t valid = n0 < args.N ? min(32U, args.N - n0) : 0U;
-                    if (!m_ok) continue;
-                    float* dst = args.out_f32 + static_cast<uint64_t>(n0) * args.ld_f32 + m;
+                    if (m_ok) {
+                        float* dst = args.out_f32 + static_cast<uint64_t>(n0) * args.ld_f32 + m;
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        if (static_cast<uint32_t>(j) < valid) {
-                            if (shared_tile) atomicAdd(dst, __uint_as_float(r[j])); else *dst = __uint_as_float(r[j]);
+                        for (int j = 0; j < 32; ++j) {
+                            if (static_cast<uint32_t>(j) < valid) {
+                                if (shared_tile) atomicAdd(dst, __uint_as_float(r[j])); else *dst = __uint_as_float(r[j]);
+                            }
+                            dst += args.ld_f32;
                         }
-                        dst += args.ld_f32;
                     }
+                    __syncwarp();  // the next load needs the whole warp
                 }
             }
             tc_fence_before();
