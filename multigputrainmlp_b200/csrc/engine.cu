@@ -237,9 +237,10 @@ struct MapKey {
     const void* base;
     uint64_t inner, outer, pitch;
     uint32_t box_inner, box_outer;
+    CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B;
     uint64_t layers = 0, layer_stride = 0;  // 3-D maps only
     bool operator==(const MapKey& o) const {
-        return base == o.base && inner == o.inner && outer == o.outer && pitch == o.pitch && box_inner == o.box_inner && box_outer == o.box_outer &&
+        return base == o.base && inner == o.inner && outer == o.outer && pitch == o.pitch && box_inner == o.box_inner && box_outer == o.box_outer && swizzle == o.swizzle &&
                layers == o.layers && layer_stride == o.layer_stride;
     }
 };
@@ -247,7 +248,7 @@ struct MapKeyHash {
     size_t operator()(const MapKey& k) const {
         uint64_t h = reinterpret_cast<uint64_t>(k.base);
         auto mix = [&](uint64_t v) { h ^= v + 0x9e3779b97f4a7c15ULL + (h << 6) + (h >> 2); };
-        mix(k.inner); mix(k.outer); mix(k.pitch); mix(k.box_inner); mix(k.box_outer); mix(k.layers); mix(k.layer_stride);
+        mix(k.inner); mix(k.outer); mix(k.pitch); mix(k.box_inner); mix(k.box_outer); mix(k.swizzle); mix(k.layers); mix(k.layer_stride);
         return (size_t)h;
     }
 };
@@ -390,7 +391,7 @@ struct mgt_engine {
     // a box of 32 elements).
     bool Map(CUtensorMap* out, const void* base, uint64_t inner, uint64_t outer, uint64_t pitch_elems, uint32_t box_inner, uint32_t box_outer,
              CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_128B) {
-        const mgt::MapKey key{base, inner, outer, pitch_elems, box_inner, box_outer};
+        const mgt::MapKey key{base, inner, outer, pitch_elems, box_inner, box_outer, swizzle};
         std::lock_guard<std::mutex> lock(mu);
         auto it = maps.find(key);
         if (it != maps.end()) { *out = it->second; return true; }
