@@ -1533,20 +1533,8 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
         if (!backward(dz2(k + 1U), w + Fc2W(s, k), H2, nullptr, r1(k), p2, dz1t(k), colsum + ws.colsum_slot * k, tile_h2) ||
             !backward(dz1t(k), w + Fc1W(s, k), H2, dz2(k + 1U), x(k), p2, dz2(k), colsum + ws.colsum_slot * (R + k), tile_h2)) return MGT_CUDA_FAILURE;
     }
-    if (!timer.Mark(profile ? &profile->residual_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
-    if (!backward(dz2(0), w + HiddenWeight(s), H1, nullptr, a1, p1, dz1, base + ws.colsum_in, tile_h1)) return MGT_CUDA_FAILURE;
-    // the input-bias gradient sums the fp32 dz1 (mlp_backward.cu:1505)
-    ReduceRowsKernel<<<(H1 + kReduceCols - 1) / kReduceCols, 256, 0, st>>>(base + ws.colsum_in, rows_h1, H1, 0, H1, grad + InputBias(s));
-    ++e->launches;
-    if (half_ig) {
-        RoundHalfKernel<<<GridFor((uint64_t)B * p1, 256, e->sm_count), 256, 0, st>>>(dz1, (uint64_t)B * p1);
-        ++e->launches;
-    }
-    if (!ok() || !timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
-    if (EmbeddingGrad(st, states, dz1, p1, B, L, V, H1, reinterpret_cast<uint32_t*>(base + ws.lists), grad) != cudaSuccess) return MGT_CUDA_FAILURE;
-    e->launches += 2;
-    if (!timer.Mark(profile ? &profile->input_grad_ms : nullptr)) return MGT_CUDA_FAILURE;
-    // weight gradients of all blocks and of the hidden layer, bias gradients from the column sums
+    // The weight gradients of all blocks, bias gradients from the column sums, and then those of the hidden layer come before the
+    // table gradient: their ranges are announced as soon as they are enqueued, and a caller's exchange of them runs beside it.
     if (R > 0) {
         if (!weight_grad(r1(0), p2, bh2, H2, dz2(1), p2, bh2, H2, R, grad + Fc2W(s, 0), BlockParams(s)) ||
             !weight_grad(x(0), p2, bh2, H2, dz1t(0), p2, bh2, H2, R, grad + Fc1W(s, 0), BlockParams(s))) return MGT_CUDA_FAILURE;
@@ -1563,10 +1551,21 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
         }
     }
     if (!ok() || !timer.Mark(profile ? &profile->residual_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
+    if (!backward(dz2(0), w + HiddenWeight(s), H1, nullptr, a1, p1, dz1, base + ws.colsum_in, tile_h1)) return MGT_CUDA_FAILURE;
     if (!weight_grad(a1, p1, 0, H1, dz2(0), p2, 0, H2, 1, grad + HiddenWeight(s), 0)) return MGT_CUDA_FAILURE;
     MGT_TRY(notify(HiddenWeight(s), (uint64_t)H1 * H2 + H2));
-    if (!timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
+    // the input-bias gradient sums the fp32 dz1 (mlp_backward.cu:1505)
+    ReduceRowsKernel<<<(H1 + kReduceCols - 1) / kReduceCols, 256, 0, st>>>(base + ws.colsum_in, rows_h1, H1, 0, H1, grad + InputBias(s));
+    ++e->launches;
+    if (half_ig) {
+        RoundHalfKernel<<<GridFor((uint64_t)B * p1, 256, e->sm_count), 256, 0, st>>>(dz1, (uint64_t)B * p1);
+        ++e->launches;
+    }
+    if (!ok() || !timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
+    if (EmbeddingGrad(st, states, dz1, p1, B, L, V, H1, reinterpret_cast<uint32_t*>(base + ws.lists), grad) != cudaSuccess) return MGT_CUDA_FAILURE;
+    e->launches += 2;
     MGT_TRY(notify(0, (uint64_t)L * V * H1 + H1));
+    if (!timer.Mark(profile ? &profile->input_grad_ms : nullptr)) return MGT_CUDA_FAILURE;
     return MGT_OK;
 }
 

@@ -79,6 +79,33 @@ def test_fp32_linears_walk_batch_and_notifications(oracle, engine):
     assert [o[0] for o in order] == list(range(2 * 2 + 3)) and order[-1][1] == 0 and order[-1][2] == 72 * 72 * 96 + 96
 
 
+@pytest.mark.parametrize("half_ig", [False, True])
+def test_fp32_linears_announce_a_range_when_it_is_enqueued(oracle, engine, half_ig):
+    # at every announcement the gradient as it stands on the stream is copied: the announced range is final, and the table, which
+    # comes last, is not written yet - what a caller exchanges at that point runs beside it
+    moves, target = oracle.cyclic_puzzle(72, 18)
+    _, states, labels, _ = oracle.random_walks(moves, target, seed=9, epoch=0, step=0, rank=0, k_min=1, k_max=29, samples=300)
+    dims = (72, 72, 64, 40, 3, 1)
+    cshape = mgt.CudaMlpShape(*dims)
+    w = torch.from_numpy((np.random.default_rng(4).standard_normal(cshape.param_count) * 0.03).astype(np.float32)).to(DEV)
+    floats = mgt.mlp_loss_grad_workspace_floats(cshape, 300, 1, half_ig, False)
+    ws, loss = torch.empty(floats, device=DEV), torch.zeros(1, device=DEV)
+    grad = torch.full((cshape.param_count,), float("nan"), device=DEV)
+    seen = []
+
+    def cb(user, ready_id, off, count, stream):
+        seen.append((off, count, grad.clone()))
+        return 0
+    assert engine.launch_mlp_loss_grad(cshape, w, None, torch.from_numpy(states).to(DEV), torch.from_numpy(labels).to(DEV), 300, loss, grad, ws, floats,
+                                       use_half_input_grad=half_ig, use_half_linear=False, gradient_ready=cb) == 0
+    torch.cuda.synchronize()
+    table = 72 * 72 * 64
+    assert len(seen) == 2 * 3 + 3
+    for off, count, copy in seen:
+        assert torch.equal(copy[off:off + count], grad[off:off + count])
+        assert off == 0 or bool(torch.isnan(copy[:table]).all())
+
+
 def test_fp16_linears_with_fp32_table_gradient(oracle, engine):
     # --input-grad-fp16 0 with fp16 linears (the reference's ctest native_train_input_grad_float_backend)
     moves, target = oracle.cyclic_puzzle(72, 18)
