@@ -143,7 +143,7 @@ RandomWalkKernel(mgt_random_walk_config_t config, uint64_t base_seed, uint64_t e
         left = depth;
     }
     uint32_t repeated = 0U;  // 1: the last state drew the previous move again, the next one picks among the others
-    const uint32_t rounds = (config.k_max + kWalkBlockMoves - 1U) / kWalkBlockMoves;  // k_max >= 1
+    const uint32_t rounds = (config.k_max - 1U) / kWalkBlockMoves + 1U;  // k_max >= 1, up to the largest of 32 bits
     for (uint32_t round = 0; round < rounds; ++round) {
         if (drawer) {
             const uint32_t now = min(left, kWalkBlockMoves);
