@@ -350,6 +350,7 @@ struct mgt_engine {
     std::mutex side_mu;    // of the two above; and an event is recorded and waited for in one piece
     uint64_t launches = 0;  // kernels launched through this engine (host-side count)
     bool layered_tower = false;  // MGT_RESIDUAL_PATH=layered: per-layer GEMMs instead of the fused residual-tower kernels (both are tested)
+    enum { kBySize, kGather, kOneHot } embedding_form = kBySize;  // MGT_EMBEDDING_FORM=gather|onehot: one form of the embedding layer for all sizes (both are tested)
     mgt_gradient_ready_fn early_fn = nullptr;  // mgt_engine_set_early_range_hook
     void* early_user = nullptr;
     mgt_train_options_t options{MGT_OPERAND_FP16, MGT_LOSS_MSE, 0, 1.0e-5f};  // mgt_engine_set_train_options
@@ -1625,6 +1626,8 @@ mgt_status_t mgt_engine_create(int32_t device_id, mgt_engine_t** out_engine) {
     }
     e->encode = reinterpret_cast<EncodeTiledFn>(fn);
     if (const char* path = std::getenv("MGT_RESIDUAL_PATH")) e->layered_tower = std::strcmp(path, "layered") == 0;
+    if (const char* form = std::getenv("MGT_EMBEDDING_FORM"))
+        e->embedding_form = std::strcmp(form, "gather") == 0 ? mgt_engine::kGather : (std::strcmp(form, "onehot") == 0 ? mgt_engine::kOneHot : mgt_engine::kBySize);
     if (cudaMalloc(&e->status_word, sizeof(int)) != cudaSuccess || cudaMemset(e->status_word, 0, sizeof(int)) != cudaSuccess) {
         delete e;
         return MGT_CUDA_FAILURE;
@@ -1729,7 +1732,8 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
         return LaunchFp32Path(e, s, w, reinterpret_cast<const uint8_t*>(states), labels, B, loss, grad, workspace, half_ig != 0, profile, tell,
                               static_cast<cudaStream_t>(stream_v));
     }
-    const Workspace ws = PlanWorkspace(s, B, PlanSmCount(e->sm_count), half_ig != 0, bnorm);
+    Workspace ws = PlanWorkspace(s, B, PlanSmCount(e->sm_count), half_ig != 0, bnorm);
+    if (e->embedding_form != mgt_engine::kBySize) ws.gather_fwd = ws.gather_grad = e->embedding_form == mgt_engine::kGather;
     if (workspace_floats < (ws.total_bytes + 3) / 4 + (half_ig ? 0 : Fp32TableFloats(s, B))) return MGT_CAPACITY_EXCEEDED;
     cudaStream_t st = static_cast<cudaStream_t>(stream_v);
     uint8_t* base = reinterpret_cast<uint8_t*>(RoundUp(reinterpret_cast<uintptr_t>(workspace), 1024));

@@ -48,7 +48,8 @@ def test_walk_rounds_and_edges(oracle, n, k_min, k_max, state_len, move_count):
 
 
 def loss_grad_case(oracle, dims, n, *, seed=1, scale=0.03, mirror=True, options=None, flags=(True, True), tol=1e-3, section_tol=3e-3, coherent=False):
-    """One loss + gradient launch on a walk batch against the oracle's model of the same data flow, whole and by section."""
+    """One loss + gradient launch on a walk batch against the oracle's model of the same data flow, whole and by section. The last
+    of four calls has a callback, which keeps all work on the caller's stream; the first three may use a second one."""
     shape = MlpShape(*dims)
     length, values = shape.state_len, shape.state_value_pad
     moves, target = random_puzzle(length, 18, seed)
@@ -68,11 +69,13 @@ def loss_grad_case(oracle, dims, n, *, seed=1, scale=0.03, mirror=True, options=
         floats = mgt.mlp_loss_grad_workspace_floats(c, n, 1, half_ig, half_lin)
         ws = torch.full((floats,), float("nan"), device=DEV)
         results = []
-        for _ in range(3):  # the same call again must give the same bits, whatever the library keeps between calls
+        for callback in (None, None, None, lambda *a: 0):  # the same call again must give the same bits, whatever the library keeps between calls
             grad.fill_(float("nan"))
+            before = engine.launch_count
             st = engine.launch_mlp_loss_grad(c, dw, dw.half() if mirror else None, torch.from_numpy(states).to(DEV), torch.from_numpy(labels).to(DEV), n, loss, grad,
-                                             ws, floats, use_half_input_grad=half_ig, use_half_linear=half_lin)
+                                             ws, floats, use_half_input_grad=half_ig, use_half_linear=half_lin, gradient_ready=callback)
             assert st == 0 and engine.check()[0] == 0
+            launches = engine.launch_count - before
             results.append((float(loss.item()), grad.cpu().numpy()))
     finally:
         engine.close()
@@ -95,7 +98,7 @@ def loss_grad_case(oracle, dims, n, *, seed=1, scale=0.03, mirror=True, options=
     for name, lo, hi in (("table", 0, table), ("input bias", table, hidden), ("hidden", hidden, tower), ("tower", tower, head), ("head", head, shape.param_count)):
         if hi > lo and np.abs(want[lo:hi]).max() > 0:
             assert rel_l2(got[lo:hi], want[lo:hi]) <= section_tol, (name, rel_l2(got[lo:hi], want[lo:hi]))
-    return got_loss, got
+    return launches
 
 
 # widths of the fused residual tower that are not multiples of its 32-column chunks, with and without the caller's fp16 copy
@@ -218,8 +221,8 @@ def test_many_outputs(oracle, outputs):
     loss_grad_case(oracle, (8, 8, 16, 24, 1, outputs), 70, tol=2e-3, section_tol=5e-3)
 
 
-# embedding layer by gathering rows: samples around a CTA's 32 and 128, columns around its 64 and the vectors of eight, few
-# classes, a single position; the last one lies beyond the rule's border and takes the one-hot GEMMs
+# embedding layer by gathering rows: samples around a CTA's 32, columns around its 64 and the vectors of eight, few classes, a
+# single position, batches towards the rule's border
 @pytest.mark.parametrize("dims,n,mirror", [((72, 72, 64, 16, 1, 1), 31, True), ((72, 72, 65, 24, 1, 1), 33, False), ((54, 6, 136, 32, 1, 1), 129, True), ((1, 3, 40, 8, 1, 1), 65, True),
                                             ((72, 72, 200, 40, 1, 1), 2100, True), ((30, 30, 1100, 48, 1, 1), 4200, True), ((7, 64, 4096, 16, 0, 1), 9000, True)])
 @pytest.mark.parametrize("bf16", [False, True])
@@ -236,6 +239,20 @@ def test_one_hot_pairs(oracle, dims, n):
     loss_grad_case(oracle, dims, n)
 
 
+# both forms of the embedding layer on the same small batches, whatever the rule would pick: table gradients of 110 tiles on 74
+# pairs (stretches that share tiles), of few tiles (halves) and of whole tiles, few classes and 64 or more, ragged sizes, the
+# weight gradients of the blocks beside the table gradient. The gathered gradient has one launch more, the sort.
+@pytest.mark.parametrize("dims,n", [((72, 72, 2560, 24, 1, 1), 130), ((72, 72, 200, 24, 2, 1), 257), ((54, 6, 1030, 24, 1, 1), 300), ((20, 12, 130, 40, 1, 2), 70), ((30, 4, 130, 40, 1, 2), 70),
+                                     ((1, 64, 40, 8, 1, 1), 65), ((7, 64, 4090, 16, 1, 1), 333)])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_embedding_forms_on_one_batch(oracle, monkeypatch, dims, n, bf16):
+    launches = {}
+    for form in ("gather", "onehot"):
+        monkeypatch.setenv("MGT_EMBEDDING_FORM", form)
+        launches[form] = loss_grad_case(oracle, dims, n, scale=0.02, options=dict(bf16=True) if bf16 else None, tol=8e-3 if bf16 else 1e-3, section_tol=2e-2 if bf16 else 3e-3)
+    assert launches["gather"] == launches["onehot"] + 1
+
+
 # residual tower for pairs of CTAs (hd2 above 256): unequal halves, a second half of one chunk, whole panels, ragged tiles
 @pytest.mark.parametrize("hd2,n,mirror", [(257, 130, False), (264, 128, True), (320, 129, True), (390, 300, False), (512, 257, True)])
 @pytest.mark.parametrize("bf16", [False, True])
@@ -244,9 +261,12 @@ def test_wide_residual_tower(oracle, hd2, n, mirror, bf16):
                    section_tol=2e-2 if bf16 else 3e-3)
 
 
-# weight gradients on the second stream: eight dX tiles or more; the embedding gradient by gathering and by the one-hot product
+# weight gradients on the second stream beside the table gradient, by gathering (its sort on that stream too) and by the one-hot
+# product; the last call of a case runs on one stream and has to give the same bits
 @pytest.mark.parametrize("dims,n", [((72, 72, 896, 40, 2, 1), 96), ((72, 72, 897, 40, 2, 1), 96), ((54, 6, 1024, 64, 1, 3), 513), ((72, 72, 1032, 33, 0, 1), 257)])
-def test_weight_gradients_beside_the_embedding_gradient(oracle, dims, n):
+@pytest.mark.parametrize("form", ["gather", "onehot"])
+def test_weight_gradients_beside_the_embedding_gradient(oracle, monkeypatch, dims, n, form):
+    monkeypatch.setenv("MGT_EMBEDDING_FORM", form)
     loss_grad_case(oracle, dims, n, scale=0.02)
 
 
