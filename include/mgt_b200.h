@@ -192,7 +192,8 @@ uint64_t mgt_mlp_loss_grad_workspace_floats(const mgt_mlp_shape_t* shape, uint32
 /* device_weights_half may be NULL (the fp16 mirror is then rebuilt from device_weights each call).
  * input_grad_partial_chunks / positions_per_block / position_tile select among the reference's
  * input-gradient back-ends; they are validated like the reference does and otherwise ignored:
- * this library has one back-end (one-hot operand synthesised in shared memory for tcgen05). */
+ * this library picks between its own two by size (one-hot operand synthesised in shared memory for tcgen05,
+ * or gathered rows). */
 mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* engine, const mgt_mlp_shape_t* shape, const float* device_weights,
                                       const uint16_t* device_weights_half, const mgt_train_state_t* device_states,
                                       const float* device_labels, uint32_t sample_count, float* device_loss,

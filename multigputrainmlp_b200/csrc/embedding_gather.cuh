@@ -1,12 +1,12 @@
 // The embedding layer as what it is, sums of table rows: every sample of the batch picks one row per position, forward adds
 // the picked rows, the table gradient adds the rows of dz1 that picked a table row. 16-bit operands, fp32 sums, the same
-// results as the one-hot GEMMs of umma_gemm.cuh up to the order of the additions.
+// results as the one-hot GEMMs of onehot_pair.cuh up to the order of the additions.
 //
 // Per sample both read L rows of H1 values and do nothing else; the GEMMs multiply by L * V - L zeros per sample to get the
 // tensor cores to do it. Gathering runs at what L2 delivers (measured 20 TB/s: 256-byte and longer row segments, tables and
 // slices that fit L2), scales with the batch from one sample on and does not care how many classes a position has, while a
-// one-hot GEMM needs a wave of 128 x 512 tiles with L * V / 64 K chunks each, 60-75 us for 72 x 72. engine.cu picks the
-// cheaper of the two by size.
+// one-hot GEMM needs a wave of 256 x 512 tiles, two CTAs to each, with L * V / 64 K chunks. engine.cu picks the cheaper of the
+// two by size.
 #pragma once
 
 #include <cuda_fp16.h>
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(256 * SPLIT)
 ForwardKernel(const uint8_t* __restrict__ states, const uint16_t* __restrict__ table, uint32_t ld_table, uint32_t B, uint32_t L, uint32_t V, uint32_t H1,
               uint16_t* __restrict__ a1_t, uint32_t ld, uint32_t* __restrict__ bits, uint32_t ld_bits) {
     constexpr uint32_t kThreads = 256U * SPLIT;
-    constexpr uint32_t NB = SPLIT == 1 ? 6U : 9U;  // loads in flight per thread
+    constexpr uint32_t NB = 9U;  // loads in flight per thread
     __shared__ uint8_t cls[80][32];
     __shared__ float tile[SPLIT][64][33];
     const uint32_t s0 = blockIdx.x * 32U, h0 = blockIdx.y * 64U, t = threadIdx.x, group = (t >> 3) & 31U, part = t >> 8, sub = t & 7U;

@@ -4,7 +4,8 @@
 // accumulation, fp32 master biases for the hidden/residual layers, fp16 mirror for the embedding
 // table and its bias. What differs is how it is computed:
 //   * the embedding layer and its gradient are one-hot GEMMs whose one-hot operand is synthesised
-//     in shared memory from the 80-byte states (never materialised in HBM);
+//     in shared memory from the 80-byte states (never materialised in HBM), or sums of gathered rows
+//     where the batch is small for the GEMMs;
 //   * bias, ReLU, residual add, ReLU-mask and the fp16 down-cast are epilogues of the GEMMs;
 //   * bias gradients are fp32 column sums taken in the epilogue that produces each dz tensor
 //     (the reference sums the fp32 dz, not its fp16 copy: tiny gradients that underflow in fp16
@@ -190,12 +191,10 @@ Workspace PlanWorkspace(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm_count,
     const uint64_t hidden_units = (uint64_t)((s.hd1 + 127) / 128) * ((s.hd2 + 255) / 256);
     const uint64_t resid_units = (uint64_t)((s.hd2 + 127) / 128) * ((s.hd2 + 255) / 256);
     const uint64_t hidden_splits = hidden_units >= sm_count ? 1 : sm_count / hidden_units;
-    const uint64_t resid_splits = resid_units >= sm_count ? 1 : sm_count / resid_units;
     const uint64_t p1 = hidden_splits * (uint64_t)s.hd1 * s.hd2;
     const uint64_t group_units = resid_units * (w.R > 0 ? w.R : 1);
     const uint64_t group_splits = group_units >= sm_count ? 1 : sm_count / group_units;
     const uint64_t p2 = group_splits * (w.R > 0 ? w.R : 1) * (uint64_t)s.hd2 * s.hd2;
-    (void)resid_splits;
     w.partial_floats = p1 > p2 ? p1 : p2;
     w.off_partial = take(w.partial_floats * 4);
     w.head_blocks = kHeadBlocks;

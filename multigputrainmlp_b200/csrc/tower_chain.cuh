@@ -48,7 +48,7 @@ struct ChainArgs {
     __half* tape_t;
     uint64_t tape_t_stride;
     uint32_t ld_t;
-    uint32_t* bits_s;          // ReLU sign bits, entry e at bits_s + e * bits_stride, 8 words per row (tiles*128 rows)
+    uint32_t* bits_s;          // ReLU sign bits, entry e at bits_s + e * bits_stride, 8 words per row (16 in the wide tower; tiles*128 rows)
     uint32_t* bits_t;
     uint64_t bits_stride;
     float* colsum;             // backward: slot j at colsum + j * colsum_stride, [tiles*4][H] partial column sums
@@ -287,6 +287,7 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
         const uint32_t quad = warp & 3U;       // TMEM lanes [32*quad, 32*quad+32)
         constexpr uint32_t SUBS = ChainCfg::EPI_WARPS / 4;  // warps per quadrant
         constexpr uint32_t WPW = 8U / SUBS;                  // 32-column chunks (and sign-bit words) per warp at most
+        static_assert(WPW == 2U, "sign words move as pairs");
         const uint32_t par = ew >> 2;          // this warp takes 32-column chunks par, par+SUBS, ...
         const uint32_t r = quad * 32U + lane;  // row inside the tile
         const uint32_t lane_addr = (quad * 32U) << 16;
@@ -330,18 +331,10 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                 __syncwarp();
             }
         };
-        auto store_words = [&](uint32_t* dst, const uint32_t (&wd)[4]) {
-            if (WPW == 4U) *reinterpret_cast<uint4*>(dst) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
-            else *reinterpret_cast<uint2*>(dst) = make_uint2(wd[0], wd[1]);
-        };
-        auto load_words = [&](const uint32_t* src, uint32_t (&wd)[4]) {
-            if (WPW == 4U) {
-                const uint4 m = *reinterpret_cast<const uint4*>(src);
-                wd[0] = m.x; wd[1] = m.y; wd[2] = m.z; wd[3] = m.w;
-            } else {
-                const uint2 m = *reinterpret_cast<const uint2*>(src);
-                wd[0] = m.x; wd[1] = m.y;
-            }
+        auto store_words = [&](uint32_t* dst, const uint32_t (&wd)[WPW]) { *reinterpret_cast<uint2*>(dst) = make_uint2(wd[0], wd[1]); };
+        auto load_words = [&](const uint32_t* src, uint32_t (&wd)[WPW]) {
+            const uint2 m = *reinterpret_cast<const uint2*>(src);
+            wd[0] = m.x; wd[1] = m.y;
         };
         auto apply_mask = [&](uint32_t (&v)[32], uint32_t bits) {
 #pragma unroll
@@ -373,7 +366,7 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
 
             // ---- load the state: TMEM S, fp16 operand, (forward) sign bits of x_0
             {
-                uint32_t words[4] = {0, 0, 0, 0};  // the first WPW are used
+                uint32_t words[WPW] = {0, 0};
 #pragma unroll
                 for (uint32_t ci = 0; ci < WPW; ++ci) {
                     const uint32_t cc = par + SUBS * ci;
@@ -412,9 +405,9 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                 const bool last = kb + 1U == R;
                 // ================= first epilogue: T from D =================
                 {
-                    uint32_t mwords[4] = {0, 0, 0, 0};
+                    uint32_t mwords[WPW] = {0, 0};
                     if (BWD) load_words(args.bits_t + k * args.bits_stride + bits_row, mwords);
-                    uint32_t words[4] = {0, 0, 0, 0};  // the first WPW are used
+                    uint32_t words[WPW] = {0, 0};
                     stage_bias(2U * k);
                     if (!warp_wait(&mma_done[0], uses & 1U)) { ok = false; break; }
                     tc_fence_after();
@@ -442,9 +435,9 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
                 }
                 // ================= second epilogue: new S =================
                 {
-                    uint32_t mwords[4] = {0, 0, 0, 0};
+                    uint32_t mwords[WPW] = {0, 0};
                     if (BWD) load_words(args.bits_s + k * args.bits_stride + bits_row, mwords);
-                    uint32_t words[4] = {0, 0, 0, 0};  // the first WPW are used
+                    uint32_t words[WPW] = {0, 0};
                     stage_bias(2U * k + 1U);
                     if (!warp_wait(&mma_done[1], uses & 1U)) { ok = false; break; }
                     tc_fence_after();

@@ -103,87 +103,6 @@ struct GemmCfg {
     static_assert(SMEM_BYTES <= 232448, "shared memory budget");
 };
 
-namespace detail {
-
-__device__ __forceinline__ void store_f16x32(__half* dst, const float (&v)[32], uint32_t valid, bool vec_ok, bool bf16) {
-    if (valid == 32 && vec_ok) {
-        uint4* p = reinterpret_cast<uint4*>(dst);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            uint4 u;
-            u.x = ptx::pack_operand_pair(v[q * 8 + 0], v[q * 8 + 1], bf16);
-            u.y = ptx::pack_operand_pair(v[q * 8 + 2], v[q * 8 + 3], bf16);
-            u.z = ptx::pack_operand_pair(v[q * 8 + 4], v[q * 8 + 5], bf16);
-            u.w = ptx::pack_operand_pair(v[q * 8 + 6], v[q * 8 + 7], bf16);
-            p[q] = u;
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-            if (static_cast<uint32_t>(j) < valid) reinterpret_cast<uint16_t*>(dst)[j] = ptx::to_operand(v[j], bf16);
-    }
-}
-
-__device__ __forceinline__ void store_f32x32(float* dst, const float (&v)[32], uint32_t valid, bool vec_ok) {
-    if (valid == 32 && vec_ok) {
-        float4* p = reinterpret_cast<float4*>(dst);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) p[q] = make_float4(v[q * 4], v[q * 4 + 1], v[q * 4 + 2], v[q * 4 + 3]);
-    } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-            if (static_cast<uint32_t>(j) < valid) dst[j] = v[j];
-    }
-}
-
-__device__ __forceinline__ void load_f32x32(const float* src, float (&v)[32], uint32_t valid, bool vec_ok) {
-    if (valid == 32 && vec_ok) {
-        const float4* p = reinterpret_cast<const float4*>(src);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const float4 f = p[q];
-            v[q * 4] = f.x;
-            v[q * 4 + 1] = f.y;
-            v[q * 4 + 2] = f.z;
-            v[q * 4 + 3] = f.w;
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) v[j] = static_cast<uint32_t>(j) < valid ? src[j] : 0.0f;
-    }
-}
-
-// positive-mask from fp16 activations: m[j] = src[j] > 0
-__device__ __forceinline__ uint32_t load_mask32(const __half* src, uint32_t valid, bool vec_ok) {
-    uint32_t bits = 0;
-    if (valid == 32 && vec_ok) {
-        const uint4* p = reinterpret_cast<const uint4*>(src);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint4 u = p[q];
-            const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                // a positive non-zero half has sign 0 and a non-zero magnitude
-                const uint32_t lo = w[e] & 0xFFFFU, hi = w[e] >> 16;
-                if (lo != 0U && (lo & 0x8000U) == 0U) bits |= 1U << (q * 8 + e * 2);
-                if (hi != 0U && (hi & 0x8000U) == 0U) bits |= 1U << (q * 8 + e * 2 + 1);
-            }
-        }
-    } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-            if (static_cast<uint32_t>(j) < valid) {
-                // positive in either 16-bit format: sign clear, magnitude non-zero
-                const uint16_t h = reinterpret_cast<const uint16_t*>(src)[j];
-                if (h != 0U && h < 0x8000U) bits |= 1U << j;
-            }
-    }
-    return bits;
-}
-
-}  // namespace detail
-
 template <class Cfg>
 __global__ void __launch_bounds__(Cfg::THREADS, 1)
 umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const GemmArgs args) {

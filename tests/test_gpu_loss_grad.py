@@ -121,7 +121,7 @@ def _walk_case(oracle, dims, n, seed):
     return shape, w, states, np.ascontiguousarray(lab)
 
 
-# hidden widths the fused residual-tower kernels take (multiples of 32 up to 256), ragged last tiles included
+# hidden widths of the fused residual tower that are multiples of its 32-column chunks, ragged last tiles included
 @pytest.mark.parametrize("dims,n", [((72, 72, 128, 224, 3, 1), 900), ((72, 72, 64, 256, 2, 1), 300), ((72, 72, 64, 96, 5, 3), 260),
                                      ((72, 72, 64, 160, 1, 1), 128)])
 def test_residual_tower_fused(oracle, engine, dims, n):
@@ -131,13 +131,13 @@ def test_residual_tower_fused(oracle, engine, dims, n):
 
 def test_reference_hard_caps(oracle, engine):
     # hd1 4096, hd2 512 are the reference's compile-time caps (native/cuda/mlp_forward.cu:7-9); 29 outputs as in the
-    # depth-classification variant; hd2 > 256 takes the per-layer residual path
+    # depth-classification variant; hd2 > 256 takes the residual tower for pairs of CTAs
     shape, w, states, labels = _walk_case(oracle, (72, 72, 4096, 512, 2, 29), 96, seed=3)
     check_against_oracle(oracle, engine, shape, w * 0.3, states, labels)
 
 
 def test_residual_tower_layered_matches_fused(oracle, engine, monkeypatch):
-    # the per-layer GEMM path (taken for other widths) on a width both paths accept
+    # the per-layer GEMM path (batch normalisation's) and the fused one on the same model
     shape, w, states, labels = _walk_case(oracle, (72, 72, 64, 64, 3, 1), 500, seed=5)
     loss_f, grad_f = run_engine(engine, shape, w, states, labels)
     monkeypatch.setenv("MGT_RESIDUAL_PATH", "layered")
@@ -256,7 +256,7 @@ def test_bfloat16_operands(oracle, dims, n):
 
 
 def test_wide_deep_variant_bf16_cross_entropy(oracle):
-    # hd1 4096, hd2 512 (the reference's compile-time caps, per-layer residual path), 29 per-depth logits, bfloat16, cross-entropy
+    # hd1 4096, hd2 512 (the reference's compile-time caps, residual tower for pairs of CTAs), 29 per-depth logits, bfloat16, cross-entropy
     shape, w, states, labels = _options_case(oracle, (72, 72, 4096, 512, 2, 29), 96, seed=23, scale=0.01)
     _check_option_case(oracle, shape, w, states, labels, bf16=True, cross_entropy=True, tol=8e-3)
 
