@@ -82,6 +82,7 @@ SgemmKernel(const __grid_constant__ SgemmArgs a) {
     constexpr uint32_t NT = (BM / TM) * (BN / TN);
     constexpr uint32_t QA = BM * BK / 4 / NT, QB = BN * BK / 4 / NT;  // float4 loads per thread and chunk
     constexpr uint32_t LDA = BM + 4, LDB = BN + 4;
+    constexpr int VW = TN < 4 ? TN : 4, NV = TN / VW;  // a thread's columns: NV vectors of VW
     static_assert(QA >= 1 && QB >= 1 && QA * NT * 4 == BM * BK && QB * NT * 4 == BN * BK && BK % 16 == 0, "whole quads per thread");
     __shared__ __align__(16) float As[KG][2][BK][LDA];
     __shared__ __align__(16) float Bs[KG][2][BK][LDB];
@@ -163,10 +164,16 @@ SgemmKernel(const __grid_constant__ SgemmArgs a) {
                 av[2 * i + 1] = v.y;
             }
 #pragma unroll
-            for (int j = 0; j < TN / 4; ++j) {
-                // (a thread's columns lie in quads BN / (TN / 4) apart: the warp reads consecutive quads)
-                const float4 v = *reinterpret_cast<const float4*>(&Bs[group_k][buf][k][(j * (BN / (TN / 4)) + tx * 4U) ^ (TB ? k & 8U : 0U)]);
-                bv[4 * j] = v.x; bv[4 * j + 1] = v.y; bv[4 * j + 2] = v.z; bv[4 * j + 3] = v.w;
+            for (int j = 0; j < NV; ++j) {
+                // (a thread's vectors lie BN / NV columns apart: the warp reads consecutive ones)
+                const float* b = &Bs[group_k][buf][k][(j * (BN / NV) + tx * VW) ^ (TB ? k & 8U : 0U)];
+                if constexpr (VW == 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(b);
+                    bv[4 * j] = v.x; bv[4 * j + 1] = v.y; bv[4 * j + 2] = v.z; bv[4 * j + 3] = v.w;
+                } else {
+                    const float2 v = *reinterpret_cast<const float2*>(b);
+                    bv[2 * j] = v.x; bv[2 * j + 1] = v.y;
+                }
             }
 #pragma unroll
             for (int j = 0; j < TN; ++j) {
@@ -211,28 +218,29 @@ SgemmKernel(const __grid_constant__ SgemmArgs a) {
         const uint32_t m = m0 + ty * TM + i;
         if (m >= a.M) break;
 #pragma unroll
-        for (int jq = 0; jq < TN / 4; ++jq) {
-            const uint32_t n = n0 + jq * (BN / (TN / 4)) + tx * 4U;
+        for (int jq = 0; jq < NV; ++jq) {
+            const uint32_t n = n0 + jq * (BN / NV) + tx * VW;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
+            for (int e = 0; e < VW; ++e) {
                 if (n + e >= a.N) continue;
-                float x = v[i][jq * 4 + e];
+                float x = v[i][jq * VW + e];
                 if (!partial) {
                     if (a.bias != nullptr) x += __ldg(a.bias + n + e);
                     if (a.add != nullptr) x += a.add[static_cast<uint64_t>(m) * a.ld_add + n + e];
                     if (a.relu != 0U) x = fmaxf(x, 0.0f);
                     if (a.mask != nullptr) x = __ldg(a.mask + static_cast<uint64_t>(m) * a.ld_mask + n + e) > 0.0f ? x : 0.0f;
-                    cs[jq * 4 + e] += x;
+                    cs[jq * VW + e] += x;
                 }
-                v[i][jq * 4 + e] = x;
+                v[i][jq * VW + e] = x;
             }
             float* dst = C + static_cast<uint64_t>(m) * ldc + n;
-            if (vec_c && n + 4U <= a.N) {
-                *reinterpret_cast<float4*>(dst) = make_float4(v[i][jq * 4], v[i][jq * 4 + 1], v[i][jq * 4 + 2], v[i][jq * 4 + 3]);
+            if (vec_c && n + VW <= a.N) {
+                if constexpr (VW == 4) *reinterpret_cast<float4*>(dst) = make_float4(v[i][jq * 4], v[i][jq * 4 + 1], v[i][jq * 4 + 2], v[i][jq * 4 + 3]);
+                else *reinterpret_cast<float2*>(dst) = make_float2(v[i][jq * 2], v[i][jq * 2 + 1]);
             } else {
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (n + e < a.N) dst[e] = v[i][jq * 4 + e];
+                for (int e = 0; e < VW; ++e)
+                    if (n + e < a.N) dst[e] = v[i][jq * VW + e];
             }
         }
     }
@@ -243,9 +251,9 @@ SgemmKernel(const __grid_constant__ SgemmArgs a) {
         static_assert(kRowGroups * BN <= KG * 2 * BK * LDB, "column sums fit the operand buffer");
         if (KG > 1) asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory"); else __syncthreads();  // (with KG > 1 only the first group is still here)
 #pragma unroll
-        for (int jq = 0; jq < TN / 4; ++jq)
+        for (int jq = 0; jq < NV; ++jq)
 #pragma unroll
-            for (int e = 0; e < 4; ++e) red[ty * BN + jq * (BN / (TN / 4)) + tx * 4U + e] = cs[jq * 4 + e];
+            for (int e = 0; e < VW; ++e) red[ty * BN + jq * (BN / NV) + tx * VW + e] = cs[jq * VW + e];
         if (KG > 1) asm volatile("bar.sync 1, %0;" ::"n"(NT) : "memory"); else __syncthreads();
         for (uint32_t c = tid; c < BN; c += NT) {
             if (n0 + c >= a.N) break;
@@ -261,8 +269,8 @@ SgemmKernel(const __grid_constant__ SgemmArgs a) {
 // tile is what takes the time, so small tiles. Gradients split K over four groups of threads there. The forward product (neither
 // operand transposed) adds in the order of k whatever its tile: its results decide the ReLUs, and every other order opens or
 // closes one here and there, which moves the gradient by up to 1e-4, where a gradient product's own order moves it by 1e-7. So one
-// K group, and chunks of 64 to keep loads in flight (a step of 1 024 samples, hd1 256, hd2 64, 2 blocks 186 us with four groups,
-// 195 us like this).
+// K group, chunks of 64 to keep loads in flight and 4 x 2 results a thread for a shorter turn (a step of 1 024 samples, hd1 256,
+// hd2 64, 2 blocks: 186 us with four groups, 195 us with 4 x 4 results, 190 us like this).
 enum class SgemmTile { kLarge, kMiddle, kSmall };
 inline uint32_t SgemmTileRows(SgemmTile t) { return t == SgemmTile::kLarge ? 128U : (t == SgemmTile::kMiddle ? 64U : 32U); }
 inline SgemmTile PickSgemmTile(uint32_t M, uint32_t N, uint64_t batches, uint32_t sm_count) {
@@ -282,7 +290,7 @@ inline cudaError_t Sgemm(cudaStream_t st, SgemmArgs a, uint32_t groups, SgemmTil
     const dim3 grid((a.N + t - 1) / t, (a.M + t - 1) / t, groups * a.splits);
     if (tile == SgemmTile::kLarge) SgemmKernel<128, 128, 8, 8, 1, 16, TA, TB><<<grid, 256, 0, st>>>(a);
     else if (tile == SgemmTile::kMiddle) SgemmKernel<64, 64, 8, 4, 1, 16, TA, TB><<<grid, 128, 0, st>>>(a);
-    else if constexpr (!TA && !TB) SgemmKernel<32, 32, 4, 4, 1, 64, TA, TB><<<grid, 64, 0, st>>>(a);
+    else if constexpr (!TA && !TB) SgemmKernel<32, 32, 4, 2, 1, 64, TA, TB><<<grid, 128, 0, st>>>(a);
     else SgemmKernel<32, 32, 4, 4, 4, 16, TA, TB><<<grid, 256, 0, st>>>(a);
     return cudaGetLastError();
 }
