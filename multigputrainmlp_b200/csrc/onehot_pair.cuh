@@ -11,10 +11,10 @@
 // Why pairs: with one CTA per tile the kernel is bound by shared-memory bandwidth, not by the tensor cores. A K chunk of 64
 // is 8 MMAs of 128 x 256 x 16 = 1 024 tensor cycles; it reads 96 KB of operands (768 cycles at 128 bytes a cycle), takes in
 // 16 KB by TMA (128) and scatters about a thousand 2-byte stores into the one-hot rows, up to eight to a bank (400): 1 640
-// cycles measured. In a pair each SM reads 64 KB, and synthesises half the rows. p888 at 53 248 samples, forward 0.97 ms
-// and gradient 0.89 ms with one CTA per tile, 0.76 and 0.84 ms in pairs. The forward now spends 1 045 of the ideal 1 024 cycles
-// on a chunk (plus 6 000 a piece for the epilogue, both accumulators being all of tensor memory); the gradient 1 160 of 960,
-// where the scattered stores and the MMAs' operand reads get in each other's way (1 060 without the stores).
+// cycles measured. In a pair each SM reads 64 KB, and synthesises half the rows. p888 at 53 248 samples, forward 0.96 ms
+// and gradient 0.92 ms with one CTA per tile, 0.72 and 0.73 ms in pairs (the latter with the zeroing of the result): 1.96 and
+// 1.92 PFLOP/s executed. What is left beside the MMAs is the epilogue of a piece (6 000 cycles, both accumulators being all of
+// tensor memory) and, in the gradient, scattered stores that get in the way of the MMAs' operand reads.
 //
 // How a pair's work is cut. Forward: the columns of all row tiles form one line and every pair takes an equal stretch of it, in
 // steps of 64 columns, and cuts that into equal pieces of at most 512 (no partly filled last round). Gradient: the K chunks of

@@ -25,8 +25,8 @@
 //
 // What bounds it is the chain of a product - MMAs (1 570 cycles at H 224), hand-over, epilogue, hand-over, about 4 500 together -
 // with one tile at a time, since TMEM has no room for a second. So whatever can wait does: bias values are staged while the MMAs
-// run, sign bits and bias sums are taken after the panels are handed on. p888 (H 224, 16 blocks), forward + backward:
-// 339 + 310 us at 53 248 samples (363 + 317 before), 99 + 88 us at 3 001 (120 + 105).
+// run, sign bits and bias sums are taken after the panels are handed on. p888 (H 224, 16 blocks), forward + backward in a list
+// of launches: 361 + 317 us at 53 248 samples (377 + 338 before), 99 + 88 us at 3 001 (120 + 105).
 #pragma once
 
 #include <cuda.h>
