@@ -415,7 +415,7 @@ onehot_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
         if constexpr (!GRAD) {
             // thread = one column: accumulator t / 128, row t % 128 of this CTA's half
             const uint32_t q = t >> 7, j = t & 127U, row = t;
-            if (V >= 64U) {
+            if (V >= 64U && (reinterpret_cast<uintptr_t>(args.states) & 3U) == 0U) {  // (the classes are fetched as words)
                 // A column's ones sit at k_p = p*V + s[p], increasing in p, and the chunks of a piece are visited in increasing
                 // k, so each column keeps a cursor; with V >= 64 a chunk holds at most two of its ones (plus the all-ones row,
                 // in the last chunk). The places of the NEXT chunk are worked out while the MMAs of the current ones run;
@@ -483,7 +483,8 @@ onehot_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
                     if (have) prepare(c);
                 }
             } else {
-                // few classes: many ones per column and chunk, so a thread writes its whole row
+                // few classes: many ones per column and chunk, so a thread writes its whole row (right for any number of classes, and
+                // for records that do not start at a word)
                 while (ok && pieces.next(p)) {
                     const uint32_t cols = q == 0U ? min(256U, p.cols) : (p.cols > 256U ? p.cols - 256U : 0U);
                     const uint32_t sample = p.n0 + q * 256U + rank * (cols / 2U) + j;

@@ -253,6 +253,32 @@ def test_embedding_forms_on_one_batch(oracle, monkeypatch, dims, n, bf16):
     assert launches["gather"] == launches["onehot"] + 1
 
 
+# states that start anywhere: a caller's own array of 80-byte records has no alignment to keep
+@pytest.mark.parametrize("half_lin", [True, False])
+@pytest.mark.parametrize("form", ["gather", "onehot"])
+def test_states_at_odd_addresses(oracle, monkeypatch, form, half_lin):
+    monkeypatch.setenv("MGT_EMBEDDING_FORM", form)
+    n, c = 333, mgt.CudaMlpShape(72, 72, 200, 24, 1, 1)
+    moves, target = random_puzzle(72, 18, 1)
+    _, states, depth, _ = oracle.random_walks(moves, target, seed=1, epoch=0, step=0, rank=0, k_min=1, k_max=29, samples=n)
+    w = torch.from_numpy((np.random.default_rng(1).standard_normal(c.param_count) * 0.03).astype(np.float32)).to(DEV)
+    floats = mgt.mlp_loss_grad_workspace_floats(c, n, 1, half_lin, half_lin)
+    ws, loss, labels = torch.empty(floats, device=DEV), torch.zeros(1, device=DEV), torch.from_numpy(depth).to(DEV)
+    grads = []
+    engine = mgt.Engine(0)
+    try:
+        for offset in (0, 1, 2):
+            buffer = torch.zeros(n * 80 + 16, dtype=torch.uint8, device=DEV)
+            buffer[offset:offset + n * 80] = torch.from_numpy(states).to(DEV).ravel()
+            grad = torch.full((c.param_count,), float("nan"), device=DEV)
+            assert engine.launch_mlp_loss_grad(c, w, None, buffer[offset:], labels, n, loss, grad, ws, floats, use_half_input_grad=half_lin, use_half_linear=half_lin) == 0
+            assert engine.check()[0] == 0
+            grads.append(grad.cpu().numpy())
+    finally:
+        engine.close()
+    assert np.isfinite(grads[0]).all() and np.array_equal(grads[0], grads[1]) and np.array_equal(grads[0], grads[2])
+
+
 # residual tower for pairs of CTAs (hd2 above 256): unequal halves, a second half of one chunk, whole panels, ragged tiles
 @pytest.mark.parametrize("hd2,n,mirror", [(257, 130, False), (264, 128, True), (320, 129, True), (390, 300, False), (512, 257, True)])
 @pytest.mark.parametrize("bf16", [False, True])
