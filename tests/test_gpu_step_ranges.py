@@ -371,7 +371,7 @@ def test_steps_on_several_streams_do_not_wait_for_each_other(small_step):
     for stream in streams:
         assert other(stream) == 0 and other.result() is not None  # (modules loaded, second streams made)
     with torch.cuda.stream(streams[0]):
-        torch.cuda._sleep(1 << 30)  # half a second
+        torch.cuda._sleep(3 << 30)  # a second and a half
     assert other(streams[0]) == 0
     late = streams[0].record_event()
     assert small_step(streams[1]) == 0
