@@ -70,11 +70,11 @@ struct Workspace {
     uint32_t p_dz;    // pitch (halfs) of dz tensors over H2
     uint32_t p_f32;   // pitch (floats) of the fp32 residual / gradient streams
     uint32_t p_w1, p_w2, p_wout;  // pitches of the internal fp16 weight copy
-    uint64_t off_a1, off_x, off_r1, off_xf, off_dzf, off_dz2, off_dz1t, off_dz1, off_partial, off_head, off_wint, off_dy, off_dyh, off_colsum;
+    uint64_t off_a1, off_x, off_r1, off_xf, off_dzf, off_dz2, off_dz1t, off_dz1, off_partial, off_partial_fc2, off_partial_fc1, off_partial_out, off_head, off_wint, off_dy, off_dyh, off_colsum;
     uint64_t colsum_floats, colsum_slot_floats, dz_stride;
     uint64_t off_bits, bits_stride;  // ReLU sign bits of the residual tower: 2R+1 entries of bits_stride words
     uint64_t x_stride, r1_stride;  // bytes between consecutive blocks' tensors
-    uint64_t partial_floats, head_blocks;
+    uint64_t head_blocks;
     // batch normalisation (only planned when it is on): fp32 pre-activations of the R+1 normalised layers, their saved
     // mean / rstd, partial sums of the reductions, the statistics vector when the caller gives no exchange buffer
     // the embedding layer by gathering rows instead of one-hot GEMMs (sample lists of the table gradient, dz1 as rows of samples)
@@ -150,6 +150,14 @@ EmbeddingForms PickEmbeddingForms(const mgt_mlp_shape_t& s, uint32_t B, uint32_t
     return {4.0 + sums / 8.0e6 < PlanPairForward(s, B, sm).us, 8.0 + B * 0.0019 + sums / 6.7e6 < PlanPairGrad(s, B, sm).us};
 }
 
+// Columns of a product's tile: 224 serves the p888 residual width without padded MMA columns.
+inline uint32_t PickBN(uint32_t n) { return n <= 224 ? 224U : 256U; }
+// K splits of a weight gradient: at most one wave of [128 x 256] tiles.
+inline uint32_t MostSplits(uint32_t M, uint32_t N, uint32_t groups, uint32_t sm_count) {
+    const uint64_t tiles = (uint64_t)((M + 127U) / 128U) * ((N + PickBN(N) - 1U) / PickBN(N)) * groups;
+    return tiles >= sm_count ? 1U : (uint32_t)(sm_count / tiles);
+}
+
 // No term may fall with a larger batch: a caller sizes its scratch for the largest batch and runs smaller ones in it. So what a
 // form of the embedding layer needs is planned whichever form this batch takes (288 bytes a sample of 72 positions). half_ig: the
 // table gradient is the 16-bit one (the fp32 one keeps its lists behind this workspace).
@@ -187,16 +195,12 @@ Workspace PlanWorkspace(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm_count,
     w.p_dz1_rows = (uint32_t)RoundUp(s.hd1, 8);
     w.off_dz1 = take(std::max<uint64_t>(hidden_act_bytes, half_ig ? (uint64_t)B * w.p_dz1_rows * 2 : 0));
     w.off_lists = take(half_ig ? gather::ListWords(B, s.state_len, s.state_value_pad) * 4 : 0);
-    // split-K partials: at most one CTA wave of [128 x 256] fp32 tiles plus slack for tile padding
-    const uint64_t hidden_units = (uint64_t)((s.hd1 + 127) / 128) * ((s.hd2 + 255) / 256);
-    const uint64_t resid_units = (uint64_t)((s.hd2 + 127) / 128) * ((s.hd2 + 255) / 256);
-    const uint64_t hidden_splits = hidden_units >= sm_count ? 1 : sm_count / hidden_units;
-    const uint64_t p1 = hidden_splits * (uint64_t)s.hd1 * s.hd2;
-    const uint64_t group_units = resid_units * (w.R > 0 ? w.R : 1);
-    const uint64_t group_splits = group_units >= sm_count ? 1 : sm_count / group_units;
-    const uint64_t p2 = group_splits * (w.R > 0 ? w.R : 1) * (uint64_t)s.hd2 * s.hd2;
-    w.partial_floats = p1 > p2 ? p1 : p2;
-    w.off_partial = take(w.partial_floats * 4);
+    // split-K partials, of every product until the sums of the step are launched
+    const uint32_t r = w.R > 0 ? w.R : 1;
+    w.off_partial = take((uint64_t)MostSplits(s.hd1, s.hd2, 1, sm_count) * s.hd1 * s.hd2 * 4);
+    w.off_partial_fc2 = take((uint64_t)MostSplits(s.hd2, s.hd2, r, sm_count) * r * s.hd2 * s.hd2 * 4);
+    w.off_partial_fc1 = take((uint64_t)MostSplits(s.hd2, s.hd2, r, sm_count) * r * s.hd2 * s.hd2 * 4);
+    w.off_partial_out = take(s.output_dim > 1 ? (uint64_t)MostSplits(s.hd2, s.output_dim, 1, sm_count) * s.hd2 * s.output_dim * 4 : 0);
     w.head_blocks = kHeadBlocks;
     w.off_head = take((uint64_t)kHeadBlocks * HeadPartialFloats(s) * 4);
     // per-warp column sums: one slot per residual dX GEMM (2R of them)
@@ -462,7 +466,7 @@ mgt_status_t LaunchPair(mgt_engine* e, const CUtensorMap& ta, const CUtensorMap&
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
 }
 
-// Tile configurations. BN = 224 serves the p888 residual width without padded MMA columns.
+// Tile configurations.
 template <int BN, Epi EPI> using CfgFwd = GemmCfg<BN, false, BSource::kTmaMN, EPI, 3, 3>;   // act[K-major] x W[K][N]
 template <int BN, Epi EPI> using CfgDx = GemmCfg<BN, false, BSource::kTmaK, EPI, 3, 3>;     // dz[K-major] x W[N][K]
 // B-stationary forms for reductions of at most 256 (the residual width): weights stay in shared memory
@@ -480,8 +484,6 @@ template <int BN> using CfgDwG = GemmCfg<BN, true, BSource::kTmaMN, Epi::kPartia
 using CfgDbgKK = GemmCfg<256, false, BSource::kTmaK, Epi::kPartialF32, 3, 3>;
 using CfgDbgKM = GemmCfg<256, false, BSource::kTmaMN, Epi::kPartialF32, 3, 3>;
 using CfgDbgMK = GemmCfg<256, true, BSource::kTmaK, Epi::kPartialF32, 3, 3>;
-
-inline uint32_t PickBN(uint32_t n) { return n <= 224 ? 224U : 256U; }
 
 GemmArgs BaseArgs(uint32_t M, uint32_t N, uint32_t K, uint32_t bn_total, uint32_t splits) {
     GemmArgs a{};
@@ -533,132 +535,85 @@ RepackHalfKernel(const float* __restrict__ src, uint8_t* __restrict__ dst, const
     }
 }
 
-// grad[i] = sum over splits (fixed order) of partial[split][i]; loads of eight splits are in flight at once
-__global__ void __launch_bounds__(256)
-ReducePartialsKernel(const float* __restrict__ partial, uint32_t splits, uint64_t count, float* __restrict__ out) {
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
-        float sum = partial[i];
-        uint32_t s = 1;
-        for (; s + 8U <= splits; s += 8U) {
-            float x[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) x[q] = partial[(uint64_t)(s + q) * count + i];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) sum += x[q];
-        }
-        for (; s < splits; ++s) sum += partial[(uint64_t)s * count + i];
-        out[i] = sum;
-    }
-}
-
-// dst[c] = sum over rows r of src[r * row_stride + col_offset + c], in a fixed order: each of 32 row
-// groups adds its rows (r = g, g+32, ...) and the groups are then added 0..31. One CTA per 8 columns,
-// so that a few-hundred-column reduction still spreads over dozens of SMs.
+// Sums over partial results, each in a fixed order: out[group][i] = sum over terms t of src[group][t * stride + i]. The sums of a
+// step that nothing in the step waits for - split-K planes, bias sums of the tiles, what the head's CTAs leave - are collected and
+// go in one launch: as six of 2 to 14 us each, with a gap before it, they were a seventh of the smallest steps (64 samples of hd1 8,
+// hd2 8: 85 us, now 73; 1 024 of hd1 256, hd2 64, 2 blocks: 118, now 103; p888 at 53 248: 3 059, now 3 051).
+// Few items with many terms (kLanes): eight items a CTA, each of 32 lanes adds terms g, g + 32, ... and the lanes are then
+// added 0..31. Many items with few terms: an item (kItem) or four neighbouring ones (kQuad) a thread, terms in order.
+struct SumJob {
+    enum Form : uint32_t { kLanes, kItem, kQuad };
+    const float* src;
+    float* dst;
+    uint64_t src_group, dst_group, stride;  // floats from one group, one term to the next
+    uint64_t items;
+    uint32_t terms, per_group, first_cta;
+    Form form;
+};
+struct SumJobs {
+    static constexpr int kMax = 12;
+    SumJob job[kMax];
+    uint32_t count, ctas;
+};
 constexpr uint32_t kReduceCols = 8;
-__global__ void __launch_bounds__(256)
-ReduceRowsKernel(const float* __restrict__ src, uint32_t rows, uint64_t row_stride, uint32_t col_offset, uint32_t cols, float* __restrict__ dst) {
-    __shared__ float s_part[32][kReduceCols + 1];
-    const uint32_t cl = threadIdx.x & (kReduceCols - 1U), g = threadIdx.x / kReduceCols;
-    const uint32_t c = blockIdx.x * kReduceCols + cl;
-    float sum = 0.0f;
-    if (c < cols) {
-        const float* p = src + col_offset + c;
-        uint32_t r = g;
-        for (; r + 96U < rows; r += 128U) {
-            const float a0 = p[(uint64_t)r * row_stride];
-            const float a1 = p[(uint64_t)(r + 32U) * row_stride];
-            const float a2 = p[(uint64_t)(r + 64U) * row_stride];
-            const float a3 = p[(uint64_t)(r + 96U) * row_stride];
-            sum += a0; sum += a1; sum += a2; sum += a3;
-        }
-        for (; r < rows; r += 32U) sum += p[(uint64_t)r * row_stride];
-    }
-    s_part[g][cl] = sum;
-    __syncthreads();
-    if (g == 0 && c < cols) {
-        float total = s_part[0][cl];
+template <class T>
+__device__ __forceinline__ T SumTerms(const float* src, uint64_t stride, uint32_t terms, uint64_t i) {
+    auto at = [&](uint32_t t) { return __ldg(reinterpret_cast<const T*>(src + t * stride) + i); };
+    auto add = [](float4& x, const float4& y) { x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w; };
+    auto add1 = [](float& x, float y) { x += y; };
+    T sum = at(0);
+    uint32_t t = 1;
+    for (; t + 8U <= terms; t += 8U) {  // eight loads in flight
+        T x[8];
 #pragma unroll
-        for (int q = 1; q < 32; ++q) total += s_part[q][cl];
-        dst[c] = total;
-    }
-}
-
-// The three reductions behind HeadOut1Kernel in one launch: items [0, H2] -> grad W_out and grad b_out (contiguous in the
-// parameter layout), item H2 + 1 -> the loss, items [H2 + 2, 2 H2 + 2) -> the bias gradient of the layer below the head.
-// Same thread-to-row assignment and order of additions as ReduceRowsKernel.
-__global__ void __launch_bounds__(256)
-ReduceHeadKernel(const float* __restrict__ src, uint32_t rows, uint32_t H2, float* __restrict__ grad_out_layer, float* __restrict__ loss,
-                 float* __restrict__ bias_below) {
-    __shared__ float s_part[32][kReduceCols + 1];
-    const uint32_t items = 2U * H2 + 2U;
-    const uint32_t cl = threadIdx.x & (kReduceCols - 1U), g = threadIdx.x / kReduceCols;
-    const uint32_t c = blockIdx.x * kReduceCols + cl;
-    float sum = 0.0f;
-    if (c < items) {
-        const float* p = src + c;
-        uint32_t r = g;
-        for (; r + 96U < rows; r += 128U) {
-            const float a0 = p[(uint64_t)r * items];
-            const float a1 = p[(uint64_t)(r + 32U) * items];
-            const float a2 = p[(uint64_t)(r + 64U) * items];
-            const float a3 = p[(uint64_t)(r + 96U) * items];
-            sum += a0; sum += a1; sum += a2; sum += a3;
-        }
-        for (; r < rows; r += 32U) sum += p[(uint64_t)r * items];
-    }
-    s_part[g][cl] = sum;
-    __syncthreads();
-    if (g == 0 && c < items) {
-        float total = s_part[0][cl];
+        for (uint32_t q = 0; q < 8U; ++q) x[q] = at(t + q);
 #pragma unroll
-        for (int q = 1; q < 32; ++q) total += s_part[q][cl];
-        if (c <= H2) grad_out_layer[c] = total;
-        else if (c == H2 + 1U) *loss = total;
-        else bias_below[c - H2 - 2U] = total;
-    }
-}
-
-// The two reducers above for a stack of problems: blockIdx.y selects the problem.
-__global__ void __launch_bounds__(256)
-ReducePartialsGroupedKernel(const float* __restrict__ partial, uint32_t splits, uint64_t count, float* __restrict__ out, uint64_t out_group_stride) {
-    const float* src = partial + (uint64_t)blockIdx.y * splits * count;
-    float* dst = out + (uint64_t)blockIdx.y * out_group_stride;
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += stride) {
-        float sum = src[i];
-        for (uint32_t s = 1; s < splits; ++s) sum += src[(uint64_t)s * count + i];
-        dst[i] = sum;
-    }
-}
-
-struct ReduceDestinations { uint64_t offset[2 * MGT_MAX_RESIDUAL_BLOCKS]; };  // element offsets into the gradient array
-
-__global__ void __launch_bounds__(256)
-ReduceRowsGroupedKernel(const float* __restrict__ src, uint32_t rows, uint32_t cols, uint64_t slot_stride, float* __restrict__ grad, ReduceDestinations dst) {
-    __shared__ float s_part[32][kReduceCols + 1];
-    const uint32_t cl = threadIdx.x & (kReduceCols - 1U), g = threadIdx.x / kReduceCols;
-    const uint32_t c = blockIdx.x * kReduceCols + cl;
-    float sum = 0.0f;
-    if (c < cols) {
-        const float* p = src + (uint64_t)blockIdx.y * slot_stride + c;
-        uint32_t r = g;
-        for (; r + 96U < rows; r += 128U) {
-            const float a0 = p[(uint64_t)r * cols];
-            const float a1 = p[(uint64_t)(r + 32U) * cols];
-            const float a2 = p[(uint64_t)(r + 64U) * cols];
-            const float a3 = p[(uint64_t)(r + 96U) * cols];
-            sum += a0; sum += a1; sum += a2; sum += a3;
+        for (uint32_t q = 0; q < 8U; ++q) {
+            if constexpr (sizeof(T) == 16) add(sum, x[q]); else add1(sum, x[q]);
         }
-        for (; r < rows; r += 32U) sum += p[(uint64_t)r * cols];
     }
-    s_part[g][cl] = sum;
-    __syncthreads();
-    if (g == 0 && c < cols) {
-        float total = s_part[0][cl];
+    for (; t < terms; ++t) {
+        const T x = at(t);
+        if constexpr (sizeof(T) == 16) add(sum, x); else add1(sum, x);
+    }
+    return sum;
+}
+__global__ void __launch_bounds__(256)
+SumKernel(const __grid_constant__ SumJobs jobs) {
+    __shared__ float s_part[32][kReduceCols + 1];
+    uint32_t at = 0;
+    while (at + 1U < jobs.count && blockIdx.x >= jobs.job[at + 1U].first_cta) ++at;
+    const SumJob& job = jobs.job[at];
+    const uint32_t local = blockIdx.x - job.first_cta, group = local / job.per_group, cta = local - group * job.per_group;
+    const float* src = job.src + group * job.src_group;
+    float* dst = job.dst + group * job.dst_group;
+    if (job.form == SumJob::kLanes) {
+        const uint32_t cl = threadIdx.x & (kReduceCols - 1U), g = threadIdx.x / kReduceCols, c = cta * kReduceCols + cl;
+        float sum = 0.0f;
+        if (c < job.items) {
+            const float* p = src + c;
+            uint32_t r = g;
+            for (; r + 96U < job.terms; r += 128U) {
+                const float a0 = p[r * job.stride], a1 = p[(r + 32U) * job.stride], a2 = p[(r + 64U) * job.stride], a3 = p[(r + 96U) * job.stride];
+                sum += a0; sum += a1; sum += a2; sum += a3;
+            }
+            for (; r < job.terms; r += 32U) sum += p[r * job.stride];
+        }
+        s_part[g][cl] = sum;
+        __syncthreads();
+        if (g == 0 && c < job.items) {
+            float total = s_part[0][cl];
 #pragma unroll
-        for (int q = 1; q < 32; ++q) total += s_part[q][cl];
-        grad[dst.offset[blockIdx.y] + c] = total;
+            for (int q = 1; q < 32; ++q) total += s_part[q][cl];
+            dst[c] = total;
+        }
+        return;
+    }
+    const uint64_t i = cta * 256ULL + threadIdx.x;
+    if (job.form == SumJob::kQuad) {
+        if (i < job.items / 4U) reinterpret_cast<float4*>(dst)[i] = SumTerms<float4>(src, job.stride, job.terms, i);
+    } else if (i < job.items) {
+        dst[i] = SumTerms<float>(src, job.stride, job.terms, i);
     }
 }
 
@@ -666,7 +621,7 @@ ReduceRowsGroupedKernel(const float* __restrict__ src, uint32_t rows, uint32_t c
 // master weights, diff, dy = 2 diff / B, loss term diff^2 / B, dcur = w * dy, then the ReLU mask of
 // the last block. One warp per sample (grid-stride); per-CTA partial sums go to
 // partials[CTA][2*H2+2] = { grad W_out[H2], grad b_out, loss, column sums of dz[H2] } and are added
-// in a fixed order by ReduceRowsKernel.
+// in a fixed order.
 constexpr int kHeadMaxPerLane = MGT_MAX_HD2 / 32;
 __global__ void __launch_bounds__(kHeadThreads)
 HeadOut1Kernel(const float* __restrict__ w_out, const float* __restrict__ b_out, const float* __restrict__ labels, const float* __restrict__ x,
@@ -1022,31 +977,6 @@ HeadOutNKernel(const __grid_constant__ HeadArgs a) {
     }
 }
 
-// The partial rows of the head with several outputs: item 0 -> loss, items [1, H2] -> the bias gradient of the layer below,
-// items (H2, H2 + OUT] -> grad b_out. Same order of additions as ReduceRowsKernel.
-__global__ void __launch_bounds__(256)
-ReduceHeadNKernel(const float* __restrict__ src, uint32_t rows, uint32_t H2, uint32_t row_floats, uint32_t items, float* __restrict__ loss, float* __restrict__ bias_below,
-                  float* __restrict__ grad_b) {
-    __shared__ float s_part[32][kReduceCols + 1];
-    const uint32_t cl = threadIdx.x & (kReduceCols - 1U), g = threadIdx.x / kReduceCols;
-    const uint32_t c = blockIdx.x * kReduceCols + cl;
-    float sum = 0.0f;
-    if (c < items) {
-#pragma unroll 4
-        for (uint32_t r = g; r < rows; r += 32U) sum += src[(uint64_t)r * row_floats + c];
-    }
-    s_part[g][cl] = sum;
-    __syncthreads();
-    if (g == 0 && c < items) {
-        float total = s_part[0][cl];
-#pragma unroll
-        for (int q = 1; q < 32; ++q) total += s_part[q][cl];
-        if (c == 0U) *loss = total;
-        else if (c <= H2) bias_below[c - 1U] = total;
-        else grad_b[c - 1U - H2] = total;
-    }
-}
-
 // grad b_out[o] = sum_b dy[b][o]: one CTA per output, rows dealt to the threads and added in a fixed tree.
 __global__ void __launch_bounds__(256)
 HeadOutNBiasGradKernel(const float* __restrict__ dy, uint32_t B, uint32_t OUT, float* __restrict__ grad_b) {
@@ -1087,10 +1017,64 @@ bool LaunchHeadKernel(int device, uint32_t grid, size_t smem, cudaStream_t st, c
     return true;
 }
 
+// The sums of a step that wait to be launched. Pass() launches them when the caller wants finished ranges on the way or the stages
+// timed (`at_once`), or when kMostWaiting bytes of partial results wait: those are still in L2 then (p888: the planes of a weight
+// gradient are 13 to 16 MB).
+struct Sums {
+    static constexpr uint64_t kMostWaiting = 8ULL << 20;
+    mgt_engine* e;
+    bool at_once;
+    SumJobs jobs{};
+    uint64_t waiting = 0;
+
+    void Add(SumJob j, uint32_t groups) {
+        if (groups == 0U) return;
+        const uint32_t per_cta = j.form == SumJob::kLanes ? kReduceCols : (j.form == SumJob::kQuad ? 1024U : 256U);
+        j.per_group = (uint32_t)((j.items + per_cta - 1U) / per_cta);
+        j.first_cta = jobs.ctas;
+        jobs.ctas += j.per_group * groups;
+        waiting += j.items * j.terms * groups * sizeof(float);
+        jobs.job[jobs.count++] = j;
+    }
+    // dst[i] = sum over `rows` rows of src[r * stride + i]
+    void Rows(const float* src, uint32_t rows, uint64_t stride, uint32_t items, float* dst, uint32_t groups = 1, uint64_t src_group = 0, uint64_t dst_group = 0) {
+        Add({src, dst, src_group, dst_group, stride, items, rows, 0, 0, SumJob::kLanes}, groups);
+    }
+    // dst[group][i] = sum over the group's `splits` planes of `count` floats
+    void Planes(const float* src, uint32_t splits, uint64_t count, float* dst, uint32_t groups = 1, uint64_t dst_group = 0) {
+        const bool quads = ((count | dst_group) & 3ULL) == 0ULL && ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15U) == 0U;
+        Add({src, dst, splits * count, dst_group, count, count, splits, 0, 0, quads ? SumJob::kQuad : SumJob::kItem}, groups);
+    }
+    // what HeadOut1Kernel's CTAs leave: rows of { grad W_out, grad b_out, loss, column sums of dz }
+    void Head(const float* src, uint32_t rows, uint32_t H2, float* grad_out_layer, float* loss, float* bias_below) {
+        const uint32_t width = 2U * H2 + 2U;
+        Rows(src, rows, width, H2 + 1U, grad_out_layer);
+        Rows(src + H2 + 1U, rows, width, 1, loss);
+        if (bias_below != nullptr) Rows(src + H2 + 2U, rows, width, H2, bias_below);
+    }
+    // bias gradients of the tower from its column sums: slot k -> b1_k, slot R + k -> b2_{k-1} (the hidden bias for k = 0)
+    void TowerBiases(const mgt_mlp_shape_t& s, const float* colsum, uint32_t rows, uint64_t slot, float* grad, bool second) {
+        const uint32_t H = s.hd2, R = s.residual_blocks;
+        Rows(colsum, rows, H, H, grad + Fc1B(s, 0), R, slot, BlockParams(s));
+        if (!second) return;
+        Rows(colsum + slot * R, rows, H, H, grad + HiddenBias(s));
+        Rows(colsum + slot * (R + 1ULL), rows, H, H, grad + Fc2B(s, 0), R - 1U, slot, BlockParams(s));
+    }
+    mgt_status_t Pass(cudaStream_t st) { return at_once || waiting > kMostWaiting ? Launch(st) : MGT_OK; }
+    mgt_status_t Launch(cudaStream_t st) {
+        if (jobs.count == 0U) return MGT_OK;
+        SumKernel<<<jobs.ctas, 256, 0, st>>>(jobs);
+        jobs.count = jobs.ctas = 0U;
+        waiting = 0;
+        ++e->launches;
+        return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
+    }
+};
+
 // Output layer with several outputs, its loss and the gradient entering the layer below, enqueued; all gradients of the head
 // except W_out's, which is a product over the batch.
 template <bool kCrossEntropy, bool kF32>
-mgt_status_t LaunchHeadN(mgt_engine* e, cudaStream_t st, const HeadArgs& a, float* loss, float* bias_below, float* grad_b) {
+mgt_status_t LaunchHeadN(mgt_engine* e, cudaStream_t st, const HeadArgs& a, Sums& sums, float* loss, float* bias_below, float* grad_b) {
     const bool tiled = a.OUT <= 64U;
     const uint32_t tiles = tiled ? (a.B + kHeadTile - 1U) / kHeadTile : (a.B + 7U) / 8U;
     const uint32_t grid = tiles < kHeadBlocks ? tiles : kHeadBlocks;
@@ -1100,10 +1084,13 @@ mgt_status_t LaunchHeadN(mgt_engine* e, cudaStream_t st, const HeadArgs& a, floa
     else if (tiled) ok = LaunchHeadKernel<HeadTileKernel<64, kCrossEntropy, kF32>>(e->device, grid, HeadTileSmem<64>(a.H2), st, a);
     else ok = LaunchHeadKernel<HeadOutNKernel<kCrossEntropy, kF32>>(e->device, grid, (kHeadThreads / 32) * a.OUT * sizeof(float), st, a);
     if (!ok) return MGT_CUDA_FAILURE;
-    const uint32_t items = tiled ? 1U + a.H2 + a.OUT : 1U + a.H2;
-    ReduceHeadNKernel<<<(items + kReduceCols - 1U) / kReduceCols, 256, 0, st>>>(a.partials, grid, a.H2, 1U + a.H2 + a.OUT, items, loss, bias_below, grad_b);
-    if (!tiled) HeadOutNBiasGradKernel<<<a.OUT, 256, 0, st>>>(a.dy, a.B, a.OUT, grad_b);
-    e->launches += tiled ? 2 : 3;
+    // the partial rows of the CTAs: { loss, column sums of dz, with up to 64 outputs column sums of dy }
+    const uint32_t width = 1U + a.H2 + a.OUT;
+    sums.Rows(a.partials, grid, width, 1, loss);
+    if (bias_below != nullptr) sums.Rows(a.partials + 1U, grid, width, a.H2, bias_below);
+    if (tiled) sums.Rows(a.partials + 1U + a.H2, grid, width, a.OUT, grad_b);
+    else HeadOutNBiasGradKernel<<<a.OUT, 256, 0, st>>>(a.dy, a.B, a.OUT, grad_b);
+    e->launches += tiled ? 1 : 2;
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
 }
 
@@ -1250,10 +1237,10 @@ BackpropPlan PlanBackprop(const mgt_engine* e, uint32_t M, uint32_t N, uint32_t 
 
 // dX[M x N] = dz[M x K, K-major] * W[N x K, row-major]^T with a backward epilogue that produces the
 // next dz tensor; its fp32 column sums (a bias gradient) go to `colsum` (zeroed by the caller,
-// PlanBackprop().rows rows of N) and, if bias_grad is given, are reduced into bias_grad[N] right away.
+// PlanBackprop().rows rows of N).
 template <Epi EPI>
 mgt_status_t GemmBackpropInput(mgt_engine* e, cudaStream_t st, const __half* dz, uint32_t dz_pitch, const __half* w, uint32_t w_pitch,
-                               uint32_t M, uint32_t N, uint32_t K, GemmArgs epi, float* colsum, float* bias_grad) {
+                               uint32_t M, uint32_t N, uint32_t K, GemmArgs epi, float* colsum) {
     const BackpropPlan p = PlanBackprop(e, M, N, K);
     GemmArgs a = BaseArgs(M, N, K, p.bn, 1);
     a.out_f32 = epi.out_f32; a.ld_f32 = epi.ld_f32; a.out_f16 = epi.out_f16; a.ld_f16 = epi.ld_f16;
@@ -1262,97 +1249,64 @@ mgt_status_t GemmBackpropInput(mgt_engine* e, cudaStream_t st, const __half* dz,
     CUtensorMap ta, tb;
     MGT_MAP(e->Map(&ta, dz, K, M, dz_pitch, 64, 128));
     MGT_MAP(e->Map(&tb, w, K, N, w_pitch, 64, p.bn));
-    if (p.stationary) {
-        MGT_TRY(p.bn == 224 ? LaunchGemm<CfgDxS<224, EPI>>(e, ta, tb, a, st) : LaunchGemm<CfgDxS<256, EPI>>(e, ta, tb, a, st));
-    } else {
-        MGT_TRY(p.bn == 224 ? LaunchGemm<CfgDx<224, EPI>>(e, ta, tb, a, st) : LaunchGemm<CfgDx<256, EPI>>(e, ta, tb, a, st));
-    }
-    if (bias_grad != nullptr) {
-        ReduceRowsKernel<<<(N + kReduceCols - 1) / kReduceCols, 256, 0, st>>>(colsum, p.rows, N, 0, N, bias_grad);
-        ++e->launches;
-    }
-    return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
+    if (p.stationary) return p.bn == 224 ? LaunchGemm<CfgDxS<224, EPI>>(e, ta, tb, a, st) : LaunchGemm<CfgDxS<256, EPI>>(e, ta, tb, a, st);
+    return p.bn == 224 ? LaunchGemm<CfgDx<224, EPI>>(e, ta, tb, a, st) : LaunchGemm<CfgDx<256, EPI>>(e, ta, tb, a, st);
 }
 
 // The weight gradients of all residual blocks for one of the two linear layers in ONE launch:
 // grad_g[in x out] = act_g^T * dz_g for g = 0..groups-1, where act_g / dz_g are slices of two tapes and
-// grad_g lie `grad_group_stride` floats apart. Split-K with a fixed-order reduction.
+// grad_g lie `grad_group_stride` floats apart. Split-K.
 mgt_status_t GemmGradWeightsGrouped(mgt_engine* e, cudaStream_t st, const __half* act_tape, uint32_t act_pitch, uint64_t act_stride_bytes,
                                     const __half* dz_tape, uint32_t dz_pitch, uint64_t dz_stride_bytes, uint32_t groups, uint32_t samples,
-                                    uint32_t in_dim, uint32_t out_dim, float* partial, uint64_t partial_floats, float* grad_first, uint64_t grad_group_stride) {
-    const uint32_t M = in_dim, N = out_dim, K = samples;
-    const uint32_t bn = PickBN(N);
-    GemmArgs a = BaseArgs(M, N, K, bn, 1);
-    const uint64_t tiles = (uint64_t)a.m_tiles * a.n_tiles * groups;
-    uint32_t splits = tiles >= (uint64_t)e->sm_count ? 1U : (uint32_t)(e->sm_count / tiles);
-    const uint64_t per_split = (uint64_t)M * N;
-    if ((uint64_t)splits * groups * per_split > partial_floats) splits = (uint32_t)(partial_floats / (per_split * groups));
-    if (splits < 1) return MGT_CAPACITY_EXCEEDED;
-    a = BaseArgs(M, N, K, bn, splits);
+                                    uint32_t in_dim, uint32_t out_dim, float* partial, Sums& sums, float* grad_first, uint64_t grad_group_stride) {
+    const uint32_t bn = PickBN(out_dim);
+    GemmArgs a = BaseArgs(in_dim, out_dim, samples, bn, MostSplits(in_dim, out_dim, groups, (uint32_t)e->sm_count));
     a.groups = groups;
     a.partial = partial;
     CUtensorMap ta, tb;
-    MGT_MAP(e->Map3D(&ta, act_tape, M, K, groups, act_pitch, act_stride_bytes, 64, 64));
-    MGT_MAP(e->Map3D(&tb, dz_tape, N, K, groups, dz_pitch, dz_stride_bytes, 64, 64));
+    MGT_MAP(e->Map3D(&ta, act_tape, in_dim, samples, groups, act_pitch, act_stride_bytes, 64, 64));
+    MGT_MAP(e->Map3D(&tb, dz_tape, out_dim, samples, groups, dz_pitch, dz_stride_bytes, 64, 64));
     MGT_TRY(bn == 224 ? LaunchGemm<CfgDwG<224>>(e, ta, tb, a, st) : LaunchGemm<CfgDwG<256>>(e, ta, tb, a, st));
-    const dim3 grid(GridFor(per_split, 256, e->sm_count) / (groups > 4 ? 4 : 1) + 1, groups);
-    ReducePartialsGroupedKernel<<<grid, 256, 0, st>>>(partial, a.splits, per_split, grad_first, grad_group_stride);
-    ++e->launches;
-    return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
+    sums.Planes(partial, a.splits, (uint64_t)in_dim * out_dim, grad_first, groups, grad_group_stride);
+    return MGT_OK;
 }
 
-// grad[in x out] = act^T * dz, reduced over the batch with split-K and a fixed-order reduction.
+// grad[in x out] = act^T * dz, reduced over the batch with split-K.
 mgt_status_t GemmGradWeights(mgt_engine* e, cudaStream_t st, const __half* act, uint32_t act_pitch, const __half* dz, uint32_t dz_pitch,
-                             uint32_t samples, uint32_t in_dim, uint32_t out_dim, float* partial, uint64_t partial_floats, float* grad_out) {
-    const uint32_t M = in_dim, N = out_dim, K = samples;
-    const uint32_t bn = PickBN(N);
-    GemmArgs a = BaseArgs(M, N, K, bn, 1);
-    const uint64_t tiles = (uint64_t)a.m_tiles * a.n_tiles;
-    uint32_t splits = tiles >= (uint64_t)e->sm_count ? 1U : (uint32_t)(e->sm_count / tiles);
-    const uint64_t per_split = (uint64_t)M * N;
-    if ((uint64_t)splits * per_split > partial_floats) splits = (uint32_t)(partial_floats / per_split);
-    if (splits < 1) return MGT_CAPACITY_EXCEEDED;
-    a = BaseArgs(M, N, K, bn, splits);
+                             uint32_t samples, uint32_t in_dim, uint32_t out_dim, float* partial, Sums& sums, float* grad_out) {
+    const uint32_t bn = PickBN(out_dim);
+    GemmArgs a = BaseArgs(in_dim, out_dim, samples, bn, MostSplits(in_dim, out_dim, 1, (uint32_t)e->sm_count));
     a.partial = partial;
     CUtensorMap ta, tb;
-    MGT_MAP(e->Map(&ta, act, M, K, act_pitch, 64, 64));
-    MGT_MAP(e->Map(&tb, dz, N, K, dz_pitch, 64, 64));
+    MGT_MAP(e->Map(&ta, act, in_dim, samples, act_pitch, 64, 64));
+    MGT_MAP(e->Map(&tb, dz, out_dim, samples, dz_pitch, 64, 64));
     MGT_TRY(bn == 224 ? LaunchGemm<CfgDw<224>>(e, ta, tb, a, st) : LaunchGemm<CfgDw<256>>(e, ta, tb, a, st));
-    ReducePartialsKernel<<<GridFor(per_split, 256, e->sm_count), 256, 0, st>>>(partial, a.splits, per_split, grad_out);
-    ++e->launches;
-    return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
+    sums.Planes(partial, a.splits, (uint64_t)in_dim * out_dim, grad_out);
+    return MGT_OK;
 }
 
 // grad[in x out] = act^T * dz with the activation stored as actT[in][samples]: a K-major A operand.
 mgt_status_t GemmGradWeightsRows(mgt_engine* e, cudaStream_t st, const __half* act_t, uint32_t act_t_pitch, const __half* dz, uint32_t dz_pitch,
-                                 uint32_t samples, uint32_t in_dim, uint32_t out_dim, float* partial, uint64_t partial_floats, float* grad_out) {
-    const uint32_t M = in_dim, N = out_dim, K = samples;
-    const uint32_t bn = PickBN(N);
-    GemmArgs a = BaseArgs(M, N, K, bn, 1);
-    const uint64_t tiles = (uint64_t)a.m_tiles * a.n_tiles;
-    uint32_t splits = tiles >= (uint64_t)e->sm_count ? 1U : (uint32_t)(e->sm_count / tiles);
-    const uint64_t per_split = (uint64_t)M * N;
-    if ((uint64_t)splits * per_split > partial_floats) splits = (uint32_t)(partial_floats / per_split);
-    if (splits < 1) return MGT_CAPACITY_EXCEEDED;
-    a = BaseArgs(M, N, K, bn, splits);
+                                 uint32_t samples, uint32_t in_dim, uint32_t out_dim, float* partial, Sums& sums, float* grad_out) {
+    const uint32_t bn = PickBN(out_dim);
+    GemmArgs a = BaseArgs(in_dim, out_dim, samples, bn, MostSplits(in_dim, out_dim, 1, (uint32_t)e->sm_count));
     a.partial = partial;
     CUtensorMap ta, tb;
-    MGT_MAP(e->Map(&ta, act_t, K, M, act_t_pitch, 64, 128));
-    MGT_MAP(e->Map(&tb, dz, N, K, dz_pitch, 64, 64));
+    MGT_MAP(e->Map(&ta, act_t, samples, in_dim, act_t_pitch, 64, 128));
+    MGT_MAP(e->Map(&tb, dz, out_dim, samples, dz_pitch, 64, 64));
     MGT_TRY(bn == 224 ? LaunchGemm<CfgDwRows<224>>(e, ta, tb, a, st) : LaunchGemm<CfgDwRows<256>>(e, ta, tb, a, st));
-    ReducePartialsKernel<<<GridFor(per_split, 256, e->sm_count), 256, 0, st>>>(partial, a.splits, per_split, grad_out);
-    ++e->launches;
-    return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
+    sums.Planes(partial, a.splits, (uint64_t)in_dim * out_dim, grad_out);
+    return MGT_OK;
 }
 
 // dxT[N_in x samples] = (W[N_in x K] * dz[samples x K]^T) * [mask bit]: the hidden layer's dX with its wide side as rows; the
 // mask words are the ones the embedding forward wrote beside its activation.
-// Row sums of the result (the bias gradient of the layer below) are reduced into bias_grad[N_in] in a fixed order. With
+// Row sums of the result (the bias gradient of the layer below) go to bias_grad[N_in] with the step's sums. With
 // dx_f32 the result goes there instead, in fp32 and with one row per sample; with dx_rows it goes to dx_t in the operand format
 // with one row per sample.
 mgt_status_t GemmBackpropInputRows(mgt_engine* e, cudaStream_t st, const __half* w, uint32_t w_pitch, const __half* dz, uint32_t dz_pitch, uint32_t samples,
                                    uint32_t in_dim, uint32_t out_dim, uint32_t* mask_bits, uint32_t ld_bits, __half* dx_t, uint32_t t_pitch, float* dx_f32, uint32_t f32_pitch, bool dx_rows, uint32_t dx_rows_pitch, float* rowsum,
-                                   uint64_t rowsum_rows, float* bias_grad) {
+                                   uint64_t rowsum_rows, Sums& sums, float* bias_grad) {
     GemmArgs a = BaseArgs(in_dim, samples, out_dim, CfgDxRows::BN, 1);
     const uint64_t rows = (uint64_t)a.n_tiles * CfgDxRows::EPI_STRIDE;
     if (rows > rowsum_rows) return MGT_CAPACITY_EXCEEDED;
@@ -1362,9 +1316,8 @@ mgt_status_t GemmBackpropInputRows(mgt_engine* e, cudaStream_t st, const __half*
     MGT_MAP(e->Map(&ta, w, out_dim, in_dim, w_pitch, 64, 128));
     MGT_MAP(e->Map(&tb, dz, out_dim, samples, dz_pitch, 64, CfgDxRows::BN));
     MGT_TRY(dx_f32 != nullptr ? LaunchGemm<CfgDxRowsF32>(e, ta, tb, a, st) : (dx_rows ? LaunchGemm<CfgDxRowsF16T>(e, ta, tb, a, st) : LaunchGemm<CfgDxRows>(e, ta, tb, a, st)));
-    ReduceRowsKernel<<<(in_dim + kReduceCols - 1) / kReduceCols, 256, 0, st>>>(rowsum, (uint32_t)rows, in_dim, 0, in_dim, bias_grad);
-    ++e->launches;
-    return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
+    sums.Rows(rowsum, (uint32_t)rows, in_dim, in_dim, bias_grad);
+    return MGT_OK;
 }
 
 // The residual tower in one launch per direction. hd2 up to 256: tower_chain.cuh, a CTA per tile of 128 samples (the tile's
@@ -1407,7 +1360,7 @@ mgt_status_t LaunchChain(mgt_engine* e, cudaStream_t st, const __half* w_first, 
 // gradients of all blocks are two grouped products at the end. Rows are padded to four floats.
 struct Fp32Workspace {
     uint32_t p1, p2;
-    uint64_t a1, x, r1, dz2, dz1t, dz1, dy, head, partial, colsum, colsum_slot, colsum_in, lists, total;  // float offsets
+    uint64_t a1, x, r1, dz2, dz1t, dz1, dy, head, partial, partial_fc2, partial_fc1, partial_out, colsum, colsum_slot, colsum_in, lists, total;  // float offsets
 };
 struct DwPlan {
     fp32path::SgemmTile tile;
@@ -1439,8 +1392,10 @@ Fp32Workspace PlanFp32(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm) {
     w.dy = take((uint64_t)B * s.output_dim);
     w.head = take((uint64_t)kHeadBlocks * HeadPartialFloats(s));
     auto planes = [&](uint32_t M, uint32_t N, uint32_t groups) { return (uint64_t)PlanDw(M, N, B, groups, sm).splits * groups * M * N; };
-    const uint64_t p_hidden = planes(s.hd1, s.hd2, 1), p_block = planes(s.hd2, s.hd2, (uint32_t)r), p_out = planes(s.hd2, s.output_dim, 1);
-    w.partial = take(std::max(p_hidden, std::max(p_block, p_out)));
+    w.partial = take(planes(s.hd1, s.hd2, 1));
+    w.partial_fc2 = take(planes(s.hd2, s.hd2, (uint32_t)r));
+    w.partial_fc1 = take(planes(s.hd2, s.hd2, (uint32_t)r));
+    w.partial_out = take(s.output_dim > 1 ? planes(s.hd2, s.output_dim, 1) : 0);
     w.colsum_slot = (uint64_t)((B + 31U) / 32U) * s.hd2;  // one row per tile of at least 32 samples
     w.colsum = take(w.colsum_slot * 2 * r);
     w.colsum_in = take((uint64_t)((B + 31U) / 32U) * s.hd1);
@@ -1452,7 +1407,7 @@ uint64_t Fp32WorkspaceFloats(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm) 
 
 template <class F>
 mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float* w, const uint8_t* states, const float* labels, uint32_t B, float* loss,
-                            float* grad, float* workspace, bool half_ig, mgt_backward_profile_t* profile, F&& notify, cudaStream_t st) {
+                            float* grad, float* workspace, bool half_ig, bool told, mgt_backward_profile_t* profile, F&& notify, cudaStream_t st) {
     using namespace mgt::fp32path;
     const uint32_t sm = PlanSmCount(e->sm_count);
     const Fp32Workspace ws = PlanFp32(s, B, sm);
@@ -1464,7 +1419,7 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
     auto r1 = [&](uint32_t k) { return base + ws.r1 + bh2 * k; };
     auto dz2 = [&](uint32_t k) { return base + ws.dz2 + bh2 * k; };    // [0] hidden layer, [k + 1] fc2 of block k
     auto dz1t = [&](uint32_t k) { return base + ws.dz1t + bh2 * k; };  // fc1 of block k
-    float *dy = base + ws.dy, *dz1 = base + ws.dz1, *partial = base + ws.partial, *colsum = base + ws.colsum;
+    float *dy = base + ws.dy, *dz1 = base + ws.dz1, *colsum = base + ws.colsum;
     const SgemmTile tile_h2 = PickSgemmTile(B, H2, 1, sm), tile_h1 = PickSgemmTile(B, H1, 1, sm);
     const uint32_t rows_h2 = (B + SgemmTileRows(tile_h2) - 1U) / SgemmTileRows(tile_h2), rows_h1 = (B + SgemmTileRows(tile_h1) - 1U) / SgemmTileRows(tile_h1);
     auto ok = [&]() { return cudaGetLastError() == cudaSuccess; };
@@ -1483,21 +1438,18 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
         ++e->launches;
         return Sgemm<false, true>(st, a, 1, tile) == cudaSuccess;
     };
+    // (the sums of the step in one launch at its end, unless the caller is told of finished ranges or times the stages)
+    Sums sums{e, told};
     // grad_g[M x N] = act_g^T dz_g over the batch
     auto weight_grad = [&](const float* act, uint32_t ld_act, uint64_t act_stride, uint32_t M, const float* dz, uint32_t ld_dz, uint64_t dz_stride, uint32_t N, uint32_t groups,
-                           float* out, uint64_t out_stride) {
+                           float* partial, float* out, uint64_t out_stride) {
         const DwPlan plan = PlanDw(M, N, B, groups, sm);
         SgemmArgs a{};
         a.A = act; a.lda = ld_act; a.stride_a = act_stride; a.B = dz; a.ldb = ld_dz; a.stride_b = dz_stride; a.M = M; a.N = N; a.K = B; a.splits = plan.splits;
         a.C = plan.splits > 1U ? partial : out; a.ldc = N; a.stride_c = out_stride;
         if (Sgemm<true, false>(st, a, groups, plan.tile) != cudaSuccess) return false;
         ++e->launches;
-        if (plan.splits > 1U) {
-            const uint64_t count = (uint64_t)M * N;
-            const dim3 grid(GridFor(count, 256, e->sm_count) / (groups > 4 ? 4 : 1) + 1, groups);
-            ReducePartialsGroupedKernel<<<grid, 256, 0, st>>>(partial, plan.splits, count, out, out_stride);
-            ++e->launches;
-        }
+        if (plan.splits > 1U) sums.Planes(partial, plan.splits, (uint64_t)M * N, out, groups, out_stride);
         return ok();
     };
     StageTimer timer{e, st, profile};
@@ -1517,14 +1469,15 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
     if (OUT == 1U) {
         const uint32_t grid = (B + 7U) / 8U < kHeadBlocks ? (B + 7U) / 8U : kHeadBlocks;
         HeadOut1Kernel<<<grid, kHeadThreads, 0, st>>>(w + OutputWeight(s), w + OutputBias(s), labels, x(R), p2, B, H2, dz2(R), nullptr, 0, base + ws.head, false);
-        ReduceHeadKernel<<<(2 * H2 + 2 + kReduceCols - 1) / kReduceCols, 256, 0, st>>>(base + ws.head, grid, H2, grad + OutputWeight(s), loss, head_bias_dst);
-        e->launches += 2;
+        sums.Head(base + ws.head, grid, H2, grad + OutputWeight(s), loss, head_bias_dst);
+        ++e->launches;
     } else {
         const HeadArgs h{w + OutputWeight(s), OUT, w + OutputBias(s), labels, nullptr, 0, x(R), p2, B, H2, OUT, dy, nullptr, 0, dz2(R), nullptr, 0, base + ws.head, false};
-        MGT_TRY(LaunchHeadN<false, true>(e, st, h, loss, head_bias_dst, grad + OutputBias(s)));
-        if (!weight_grad(x(R), p2, 0, H2, dy, OUT, 0, OUT, 1, grad + OutputWeight(s), 0)) return MGT_CUDA_FAILURE;
+        MGT_TRY(LaunchHeadN<false, true>(e, st, h, sums, loss, head_bias_dst, grad + OutputBias(s)));
+        if (!weight_grad(x(R), p2, 0, H2, dy, OUT, 0, OUT, 1, base + ws.partial_out, grad + OutputWeight(s), 0)) return MGT_CUDA_FAILURE;
     }
     if (!ok()) return MGT_CUDA_FAILURE;
+    MGT_TRY(sums.Pass(st));
     MGT_TRY(notify(OutputWeight(s), (uint64_t)H2 * OUT + OUT));
     if (!timer.Mark(profile ? &profile->output_ms : nullptr)) return MGT_CUDA_FAILURE;
     // input gradients down the tower and through the hidden layer
@@ -1536,15 +1489,10 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
     // The weight gradients of all blocks, bias gradients from the column sums, and then those of the hidden layer come before the
     // table gradient: their ranges are announced as soon as they are enqueued, and a caller's exchange of them runs beside it.
     if (R > 0) {
-        if (!weight_grad(r1(0), p2, bh2, H2, dz2(1), p2, bh2, H2, R, grad + Fc2W(s, 0), BlockParams(s)) ||
-            !weight_grad(x(0), p2, bh2, H2, dz1t(0), p2, bh2, H2, R, grad + Fc1W(s, 0), BlockParams(s))) return MGT_CUDA_FAILURE;
-        ReduceDestinations dst{};
-        for (uint32_t k = 0; k < R; ++k) {
-            dst.offset[k] = Fc1B(s, k);
-            dst.offset[R + k] = k > 0 ? Fc2B(s, k - 1) : HiddenBias(s);
-        }
-        ReduceRowsGroupedKernel<<<dim3((H2 + kReduceCols - 1) / kReduceCols, 2 * R), 256, 0, st>>>(colsum, rows_h2, H2, ws.colsum_slot, grad, dst);
-        ++e->launches;
+        if (!weight_grad(r1(0), p2, bh2, H2, dz2(1), p2, bh2, H2, R, base + ws.partial_fc2, grad + Fc2W(s, 0), BlockParams(s)) ||
+            !weight_grad(x(0), p2, bh2, H2, dz1t(0), p2, bh2, H2, R, base + ws.partial_fc1, grad + Fc1W(s, 0), BlockParams(s))) return MGT_CUDA_FAILURE;
+        sums.TowerBiases(s, colsum, rows_h2, ws.colsum_slot, grad, true);
+        MGT_TRY(sums.Pass(st));
         for (uint32_t rb = R; rb > 0; --rb) {
             MGT_TRY(notify(Fc2W(s, rb - 1U), (uint64_t)H2 * H2 + H2));
             MGT_TRY(notify(Fc1W(s, rb - 1U), (uint64_t)H2 * H2 + H2));
@@ -1552,11 +1500,12 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
     }
     if (!ok() || !timer.Mark(profile ? &profile->residual_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
     if (!backward(dz2(0), w + HiddenWeight(s), H1, nullptr, a1, p1, dz1, base + ws.colsum_in, tile_h1)) return MGT_CUDA_FAILURE;
-    if (!weight_grad(a1, p1, 0, H1, dz2(0), p2, 0, H2, 1, grad + HiddenWeight(s), 0)) return MGT_CUDA_FAILURE;
+    if (!weight_grad(a1, p1, 0, H1, dz2(0), p2, 0, H2, 1, base + ws.partial, grad + HiddenWeight(s), 0)) return MGT_CUDA_FAILURE;
+    MGT_TRY(sums.Pass(st));
     MGT_TRY(notify(HiddenWeight(s), (uint64_t)H1 * H2 + H2));
     // the input-bias gradient sums the fp32 dz1 (mlp_backward.cu:1505)
-    ReduceRowsKernel<<<(H1 + kReduceCols - 1) / kReduceCols, 256, 0, st>>>(base + ws.colsum_in, rows_h1, H1, 0, H1, grad + InputBias(s));
-    ++e->launches;
+    sums.Rows(base + ws.colsum_in, rows_h1, H1, H1, grad + InputBias(s));
+    MGT_TRY(sums.Pass(st));
     if (half_ig) {
         RoundHalfKernel<<<GridFor((uint64_t)B * p1, 256, e->sm_count), 256, 0, st>>>(dz1, (uint64_t)B * p1);
         ++e->launches;
@@ -1564,6 +1513,7 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
     if (!ok() || !timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
     if (EmbeddingGrad(st, states, dz1, p1, B, L, V, H1, reinterpret_cast<uint32_t*>(base + ws.lists), grad) != cudaSuccess) return MGT_CUDA_FAILURE;
     e->launches += 2;
+    MGT_TRY(sums.Launch(st));
     MGT_TRY(notify(0, (uint64_t)L * V * H1 + H1));
     if (!timer.Mark(profile ? &profile->input_grad_ms : nullptr)) return MGT_CUDA_FAILURE;
     return MGT_OK;
@@ -1728,7 +1678,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
             if (ready == nullptr) return MGT_OK;
             return ready(ready_user, id++, off, count, stream_v) == MGT_OK ? MGT_OK : MGT_CUDA_FAILURE;
         };
-        return LaunchFp32Path(e, s, w, reinterpret_cast<const uint8_t*>(states), labels, B, loss, grad, workspace, half_ig != 0, profile, tell,
+        return LaunchFp32Path(e, s, w, reinterpret_cast<const uint8_t*>(states), labels, B, loss, grad, workspace, half_ig != 0, ready != nullptr || profile != nullptr, profile, tell,
                               static_cast<cudaStream_t>(stream_v));
     }
     Workspace ws = PlanWorkspace(s, B, PlanSmCount(e->sm_count), half_ig != 0, bnorm);
@@ -1746,13 +1696,15 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     auto dz_tape = [&](uint32_t k) { return reinterpret_cast<__half*>(base + ws.off_dz2 + ws.dz_stride * k); };   // [0] hidden, [k+1] fc2 of block k
     auto dz1_tape = [&](uint32_t k) { return reinterpret_cast<__half*>(base + ws.off_dz1t + ws.dz_stride * k); };  // fc1 of block k
     __half* dz1_h = reinterpret_cast<__half*>(base + ws.off_dz1);
-    float* partial = reinterpret_cast<float*>(base + ws.off_partial);
     float* head_partial = reinterpret_cast<float*>(base + ws.off_head);
     float* colsum = reinterpret_cast<float*>(base + ws.off_colsum);
     const uint32_t H1 = s.hd1, H2 = s.hd2, R = s.residual_blocks, OUT = s.output_dim, IN = ws.IN;
 
     StageTimer timer{e, st, profile};
     if (!timer.Start()) return MGT_CUDA_FAILURE;
+    // Nothing in the step waits for the sums over partial results: they are a launch at its end.
+    const bool told = ready != nullptr || e->early_fn != nullptr || profile != nullptr;
+    Sums sums{e, told};
     uint32_t ready_id = 0;
     auto notify = [&](uint64_t off, uint64_t count) -> mgt_status_t {
         if (ready == nullptr) return MGT_OK;
@@ -1919,22 +1871,23 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
 
     // ---- output head, loss and the gradient entering the last block (mlp_backward.cu:1327-1364)
     __half* dz_cur = dz_tape(R);   // fp16 copy of the gradient w.r.t. the pre-activation the head feeds
-    // the head also yields the fp32 column sums of dz: the bias gradient of the layer below it
-    float* head_bias_dst = grad + (R > 0 ? Fc2B(s, R - 1) : HiddenBias(s));
+    // the head also yields the fp32 column sums of dz: the bias gradient of the layer below it, unless that is normalised
+    float* head_bias_dst = bnorm ? nullptr : grad + (R > 0 ? Fc2B(s, R - 1) : HiddenBias(s));
     if (OUT == 1U) {
         HeadOut1Kernel<<<kHeadBlocks, kHeadThreads, 0, st>>>(w + OutputWeight(s), w + OutputBias(s), labels, x_f32, ws.p_f32, B, H2, dzf, dz_cur, ws.p_dz, head_partial, e->bf16_now);
-        ReduceHeadKernel<<<(2 * H2 + 2 + kReduceCols - 1) / kReduceCols, 256, 0, st>>>(head_partial, kHeadBlocks, H2, grad + OutputWeight(s), loss, head_bias_dst);
-        e->launches += 2;
+        sums.Head(head_partial, kHeadBlocks, H2, grad + OutputWeight(s), loss, head_bias_dst);
+        ++e->launches;
     } else {
         float* dy = reinterpret_cast<float*>(base + ws.off_dy);
         __half* dy_h = reinterpret_cast<__half*>(base + ws.off_dyh);
         const HeadArgs h{hw.wout, hw.pout, w + OutputBias(s), labels, x_h(R), ws.p_act, x_f32, ws.p_f32, B, H2, OUT, dy, dy_h, ws.p_wout, dzf, dz_cur, ws.p_dz, head_partial, e->bf16_now};
-        MGT_TRY(e->options.loss_kind == MGT_LOSS_CROSS_ENTROPY ? LaunchHeadN<true, false>(e, st, h, loss, head_bias_dst, grad + OutputBias(s))
-                                                               : LaunchHeadN<false, false>(e, st, h, loss, head_bias_dst, grad + OutputBias(s)));
+        MGT_TRY(e->options.loss_kind == MGT_LOSS_CROSS_ENTROPY ? LaunchHeadN<true, false>(e, st, h, sums, loss, head_bias_dst, grad + OutputBias(s))
+                                                               : LaunchHeadN<false, false>(e, st, h, sums, loss, head_bias_dst, grad + OutputBias(s)));
         // grad W_out = x_R^T * dy (16-bit operands, fp32 accumulate, mlp_backward.cu:1349-1354): the split-K weight-gradient GEMM
-        MGT_TRY(GemmGradWeights(e, st, x_h(R), ws.p_act, dy_h, ws.p_wout, B, H2, OUT, partial, ws.partial_floats, grad + OutputWeight(s)));
+        MGT_TRY(GemmGradWeights(e, st, x_h(R), ws.p_act, dy_h, ws.p_wout, B, H2, OUT, reinterpret_cast<float*>(base + ws.off_partial_out), sums, grad + OutputWeight(s)));
     }
     if (cudaGetLastError() != cudaSuccess) return MGT_CUDA_FAILURE;
+    MGT_TRY(sums.Pass(st));
     MGT_TRY(notify(OutputWeight(s), (uint64_t)H2 * OUT + OUT));
     if (!timer.Mark(profile ? &profile->output_ms : nullptr)) return MGT_CUDA_FAILURE;
 
@@ -1957,12 +1910,12 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
         if (bnorm) MGT_TRY(bn_backward(k + 1U, grad + Fc2B(s, k)));  // dz_tape(k + 1) = gradient w.r.t. the fc2 output; dzf goes down the skip path as it is
         GemmArgs d2{};  // dz1 = (dz2 * W2^T) * [r1 > 0]
         d2.mask = r1_h(k); d2.ld_mask = ws.p_act; d2.out_f16 = dz1_tape(k); d2.ld_f16 = ws.p_dz;
-        MGT_TRY(GemmBackpropInput<Epi::kMaskF16>(e, st, dz_tape(k + 1), ws.p_dz, hw.w2[k], hw.p2, B, H2, H2, d2, colsum + ws.colsum_slot_floats * k, nullptr));
+        MGT_TRY(GemmBackpropInput<Epi::kMaskF16>(e, st, dz_tape(k + 1), ws.p_dz, hw.w2[k], hw.p2, B, H2, H2, d2, colsum + ws.colsum_slot_floats * k));
         GemmArgs d1{};  // next dz = (dz1 * W1^T + dz2) * [x_k > 0]: ReLU of the previous block (or of the hidden layer)
         d1.add_f32 = dzf; d1.ld_add = ws.p_f32; d1.out_f32 = dzf; d1.ld_f32 = ws.p_f32; d1.mask = x_h(k); d1.ld_mask = ws.p_act;
         d1.out_f16 = dz_tape(k); d1.ld_f16 = ws.p_dz;
         MGT_TRY(GemmBackpropInput<Epi::kAddMaskF32F16>(e, st, dz1_tape(k), ws.p_dz, hw.w1[k], hw.p2, B, H2, H2, d1,
-                                                        colsum + ws.colsum_slot_floats * (R + k), nullptr));
+                                                        colsum + ws.colsum_slot_floats * (R + k)));
     }
     if (!timer.Mark(profile ? &profile->residual_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
 
@@ -1982,7 +1935,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     // 660 us). Not with callers that are told of finished ranges or time the stages: they rely on the order.
     const uint64_t dx_tiles = (uint64_t)((H1 + 127U) / 128U) * ((B + 255U) / 256U);
     SideBranch branch{e, st};
-    if (dx_tiles < 2ULL * e->sm_count && B <= 16384U && ready == nullptr && e->early_fn == nullptr && profile == nullptr) branch.Fork();
+    if (dx_tiles < 2ULL * e->sm_count && B <= 16384U && !told) branch.Fork();
     cudaStream_t st_dw = branch.open ? branch.side.stream : st;
     uint32_t* order = reinterpret_cast<uint32_t*>(base + ws.off_lists);
     uint32_t* first = order + (uint64_t)s.state_len * B;
@@ -1991,11 +1944,14 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
         ++e->launches;
     };
     if (branch.open && half_ig && ws.gather_grad) sort_classes(branch.side.stream);
+    Sums own{e, true};  // (the sums that wait are launched on the second stream, which does not see the dX product)
+    Sums& dx_sums = branch.open ? own : sums;
     // dz1T = (Wh * dzh^T) * [pre-activation of a1 > 0], the input-bias gradient from its row sums. With --input-grad-fp16 0 the
     // embedding gradient wants dz1 in fp32 (mlp_backward.cu:1433-1504, float one-hot GEMM): the same product of fp16 operands
     // with fp32 accumulation, written unrounded as rows of samples.
     MGT_TRY(GemmBackpropInputRows(e, st, hw.wh, hw.p2, dz_cur, ws.p_dz, B, H1, H2, reinterpret_cast<uint32_t*>(base + ws.off_bits_h1), ws.ld_bits_h1, dz1_h,
-                                  ws.p_bt, half_ig ? nullptr : dz1_f32, p_dz1_f32, half_ig && ws.gather_grad, ws.p_dz1_rows, reinterpret_cast<float*>(base + ws.off_rowsum), ws.rowsum_rows, grad + InputBias(s)));
+                                  ws.p_bt, half_ig ? nullptr : dz1_f32, p_dz1_f32, half_ig && ws.gather_grad, ws.p_dz1_rows, reinterpret_cast<float*>(base + ws.off_rowsum), ws.rowsum_rows, dx_sums, grad + InputBias(s)));
+    MGT_TRY(dx_sums.Pass(st));
     if (!timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
 
     // ---- embedding gradient: grad W_in = onehot^T * dz1  (mlp_backward.cu:1440-1504); the input-bias
@@ -2036,19 +1992,14 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
 
     if (R > 0) {
         // weight gradients of all blocks: two grouped split-K GEMMs (fc2: r1_k^T dz2_k, fc1: x_k^T dz1_k)
-        MGT_TRY(GemmGradWeightsGrouped(e, st_dw, r1_h(0), ws.p_act, ws.r1_stride, dz_tape(1), ws.p_dz, ws.dz_stride, R, B, H2, H2, partial,
-                                       ws.partial_floats, grad + Fc2W(s, 0), BlockParams(s)));
-        MGT_TRY(GemmGradWeightsGrouped(e, st_dw, x_h(0), ws.p_act, ws.x_stride, dz1_tape(0), ws.p_dz, ws.dz_stride, R, B, H2, H2, partial,
-                                       ws.partial_floats, grad + Fc1W(s, 0), BlockParams(s)));
-        // bias gradients: column sums of dz1_k -> b1_k, of the dz each fc1 GEMM produced -> b2_{k-1} (hidden bias for k = 0)
-        ReduceDestinations dst{};
-        for (uint32_t k = 0; k < R; ++k) {
-            dst.offset[k] = Fc1B(s, k);
-            dst.offset[R + k] = k > 0 ? Fc2B(s, k - 1) : HiddenBias(s);
-        }
+        MGT_TRY(GemmGradWeightsGrouped(e, st_dw, r1_h(0), ws.p_act, ws.r1_stride, dz_tape(1), ws.p_dz, ws.dz_stride, R, B, H2, H2,
+                                       reinterpret_cast<float*>(base + ws.off_partial_fc2), sums, grad + Fc2W(s, 0), BlockParams(s)));
+        MGT_TRY(sums.Pass(st_dw));
+        MGT_TRY(GemmGradWeightsGrouped(e, st_dw, x_h(0), ws.p_act, ws.x_stride, dz1_tape(0), ws.p_dz, ws.dz_stride, R, B, H2, H2,
+                                       reinterpret_cast<float*>(base + ws.off_partial_fc1), sums, grad + Fc1W(s, 0), BlockParams(s)));
         // (with batch normalisation b2_k and the hidden bias got their gradients from the normalisation's backward pass)
-        ReduceRowsGroupedKernel<<<dim3((H2 + kReduceCols - 1) / kReduceCols, bnorm ? R : 2 * R), 256, 0, st_dw>>>(colsum, colsum_rows, H2, ws.colsum_slot_floats, grad, dst);
-        ++e->launches;
+        sums.TowerBiases(s, colsum, colsum_rows, ws.colsum_slot_floats, grad, !bnorm);
+        MGT_TRY(sums.Pass(st_dw));
         if (cudaGetLastError() != cudaSuccess) return MGT_CUDA_FAILURE;
         for (uint32_t rb = R; rb > 0; --rb) {
             MGT_TRY(notify(Fc2W(s, rb - 1U), (uint64_t)H2 * H2 + H2));
@@ -2059,7 +2010,8 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
 
     // ---- hidden layer backward, dW part; every kernel that reads the hidden weights was enqueued long before, so a caller
     // may update the range in place as soon as it is announced
-    MGT_TRY(GemmGradWeightsRows(e, st_dw, a1_h, ws.p_bt, dz_cur, ws.p_dz, B, H1, H2, partial, ws.partial_floats, grad + HiddenWeight(s)));
+    MGT_TRY(GemmGradWeightsRows(e, st_dw, a1_h, ws.p_bt, dz_cur, ws.p_dz, B, H1, H2, reinterpret_cast<float*>(base + ws.off_partial), sums, grad + HiddenWeight(s)));
+    MGT_TRY(sums.Launch(st_dw));  // (on the second stream they are done while the table gradient still runs)
     if (!branch.Join()) return MGT_CUDA_FAILURE;
     MGT_TRY(notify(HiddenWeight(s), (uint64_t)H1 * H2 + H2));
     if (!timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
@@ -2107,8 +2059,9 @@ mgt_status_t mgt_debug_gemm(mgt_engine_t* e, const uint16_t* a, uint32_t lda, in
     else r = LaunchGemm<CfgDbgKK>(e, ta, tb, args, st);
     if (r != MGT_OK) return r;
     if (args.splits > 1) {
-        ReducePartialsKernel<<<GridFor((uint64_t)m * n, 256, e->sm_count), 256, 0, st>>>(partial_scratch, args.splits, (uint64_t)m * n, d);
-        if (cudaGetLastError() != cudaSuccess) return MGT_CUDA_FAILURE;
+        Sums sums{e, true};
+        sums.Planes(partial_scratch, args.splits, (uint64_t)m * n, d);
+        MGT_TRY(sums.Launch(st));
     }
     return MGT_OK;
 }
