@@ -2,6 +2,7 @@
 // HBM-bound: 28 bytes (30 with the mirror) per parameter; 16-byte accesses, one per thread and array.
 #include "../../include/mgt_b200.h"
 #include "adamw_math.cuh"
+#include "launch.cuh"
 
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
@@ -9,6 +10,7 @@
 namespace {
 
 constexpr uint32_t kAdamWThreads = 128;
+constexpr uint64_t kOverlapParams = 8ULL << 20;  // a longer update does not notice the gap before it, and its CTAs crowd what still runs
 
 template <bool kMirror>
 __global__ void __launch_bounds__(kAdamWThreads)
@@ -17,6 +19,7 @@ AdamWKernel(mgt_adamw_config_t config, float* __restrict__ w, __half* __restrict
     const mgt::AdamWScalars sc = mgt::MakeAdamWScalars(config.step, config.learning_rate, config.beta1, config.beta2, config.eps, config.weight_decay);
     const uint64_t n4 = config.param_count >> 2;
     const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+    mgt::dependent_begin();
     for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n4; i += stride) {
         float4 wv = reinterpret_cast<float4*>(w)[i];
         const float4 gv = reinterpret_cast<const float4*>(g)[i];
@@ -52,6 +55,7 @@ AdamWKernel(mgt_adamw_config_t config, float* __restrict__ w, __half* __restrict
 }
 
 __global__ void FloatToHalfKernel(const float* __restrict__ src, uint64_t count, __half* __restrict__ dst) {
+    mgt::dependent_begin();
     const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride) dst[i] = __float2half_rn(src[i]);
 }
@@ -92,11 +96,11 @@ static mgt_status_t LaunchAdamW(const mgt_adamw_config_t* config, float* w, uint
     const uint64_t want = (n4 + kAdamWThreads - 1ULL) / kAdamWThreads;
     const uint64_t cap = 1ULL << 30;
     const uint32_t blocks = static_cast<uint32_t>(want < 1 ? 1 : (want < cap ? want : cap));
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const mgt::LaunchOn s(static_cast<cudaStream_t>(stream), config->param_count <= kOverlapParams);
     if (mirror) {
-        AdamWKernel<true><<<blocks, kAdamWThreads, 0, s>>>(*config, w, reinterpret_cast<__half*>(w_half), g, m, v);
+        mgt::Launch(AdamWKernel<true>, blocks, kAdamWThreads, 0, s, *config, w, reinterpret_cast<__half*>(w_half), g, m, v);
     } else {
-        AdamWKernel<false><<<blocks, kAdamWThreads, 0, s>>>(*config, w, nullptr, g, m, v);
+        mgt::Launch(AdamWKernel<false>, blocks, kAdamWThreads, 0, s, *config, w, nullptr, g, m, v);
     }
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
 }
@@ -115,7 +119,7 @@ mgt_status_t mgt_launch_float_to_half(const float* values, uint64_t count, uint1
     const uint64_t want = (count + 255ULL) / 256ULL;
     const uint64_t cap = static_cast<uint64_t>(SmCount()) * 16ULL;
     const uint32_t blocks = static_cast<uint32_t>(want < cap ? want : cap);
-    FloatToHalfKernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(values, count, reinterpret_cast<__half*>(half));
+    mgt::Launch(FloatToHalfKernel, blocks, 256, 0, {static_cast<cudaStream_t>(stream), true}, values, count, reinterpret_cast<__half*>(half));
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
 }
 

@@ -20,6 +20,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "launch.cuh"
 #include "ptx_sm100.cuh"
 
 namespace mgt {
@@ -113,6 +114,7 @@ ColumnMomentsKernel(const float* __restrict__ a, uint32_t ld_a, const float* __r
                     const float* __restrict__ rstd, uint32_t rows, uint32_t H, float* __restrict__ partial) {
     __shared__ float smem[kThreads * 2U * 4U];
     const Owner o = MakeOwner(rows, H);
+    dependent_begin();
     for (uint32_t q = o.q0; q < o.Q; q += o.QT) {
         float acc[2][4] = {};
         float mu[4] = {}, rs[4] = {};
@@ -175,6 +177,7 @@ ReduceMomentsKernel(const float* __restrict__ partial, uint32_t blocks, uint32_t
     const uint32_t c = threadIdx.x % kReduceCols, part = threadIdx.x / kReduceCols;
     const uint32_t h = blockIdx.x * kReduceCols + c;
     const bool ok = h < H;
+    dependent_begin();
     const float s1 = AddPartialRows(partial, blocks, 2ULL * H, h, ok, part, c, smem);
     const float s2 = AddPartialRows(partial + H, blocks, 2ULL * H, h, ok, part, c, smem);
     if (ok && part == 0U) {
@@ -191,6 +194,7 @@ ReduceSumsKernel(const float* __restrict__ partial, uint32_t blocks, uint32_t H,
     const uint32_t c = threadIdx.x % kReduceCols, part = threadIdx.x / kReduceCols;
     const uint32_t h = blockIdx.x * kReduceCols + c;
     const bool ok = h < H;
+    dependent_begin();
     const float s = AddPartialRows(partial, blocks, H, h, ok, part, c, smem);
     if (ok && part == 0U) out[h] = s;
 }
@@ -203,6 +207,7 @@ ApplyForwardKernel(const float* __restrict__ z, uint32_t ld_z, const float* __re
                    float eps, uint32_t rows, uint32_t H, float* __restrict__ x_f32, uint32_t ld_x, uint16_t* __restrict__ x_h, uint32_t ld_h, bool bf16,
                    float* __restrict__ save_mean, float* __restrict__ save_rstd, float* __restrict__ running, float momentum, float unbias) {
     const Owner o = MakeOwner(rows, H);
+    dependent_begin();
     for (uint32_t q = o.q0; q < o.Q; q += o.QT) {
         const uint32_t col = q * 4U, valid = min(4U, H - col);
         float mu[4], msq[4], g[4], bsh[4], rs[4];
@@ -250,6 +255,7 @@ ApplyBackwardKernel(const float* __restrict__ dpre, uint32_t ld_d, const float* 
                     uint16_t* __restrict__ dz_h, uint32_t ld_h, bool bf16, float* __restrict__ partial) {
     __shared__ float smem[kThreads * 4U];
     const Owner o = MakeOwner(rows, H);
+    dependent_begin();
     for (uint32_t q = o.q0; q < o.Q; q += o.QT) {
         const uint32_t col = q * 4U, valid = min(4U, H - col);
         float mu[4], rs[4], g[4], m1[4], m2[4];

@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "launch.cuh"
 #include "ptx_sm100.cuh"
 
 namespace mgt {
@@ -59,6 +60,7 @@ ForwardKernel(const uint8_t* __restrict__ states, const uint16_t* __restrict__ t
     __shared__ uint8_t cls[80][32];
     __shared__ float tile[SPLIT][64][33];
     const uint32_t s0 = blockIdx.x * 32U, h0 = blockIdx.y * 64U, t = threadIdx.x, group = (t >> 3) & 31U, part = t >> 8, sub = t & 7U;
+    dependent_begin();
     for (uint32_t i = t; i < 32U * L; i += kThreads) {
         const uint32_t s = i / L, p = i - s * L;
         cls[p][s] = s0 + s < B ? states[static_cast<uint64_t>(s0 + s) * 80U + p] : 0U;
@@ -108,6 +110,7 @@ SortByClassKernel(const uint8_t* __restrict__ states, uint32_t B, uint32_t V, ui
     const uint32_t p = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31U;
     for (uint32_t v = lane; v < 80U; v += 32U) count[warp][v] = 0U;
     __syncwarp();
+    dependent_begin();
     const uint32_t stretch = ((B + 31U) / 32U + 31U) / 32U * 32U;
     const uint32_t lo = min(B, warp * stretch), hi = min(B, lo + stretch);
     for (uint32_t s = lo; s < hi; s += 32U) {
@@ -159,6 +162,8 @@ GradKernel(const uint32_t* __restrict__ order, const uint32_t* __restrict__ firs
     const uint32_t p = min(row / V, L - 1U), v = row - p * V;
     const bool live = row < L * V;
     const uint32_t h = blockIdx.y * 64U + sub * 8U;
+    dependent_begin();
+    first = after_begin(first);
     const uint32_t lo = live ? __ldg(first + p * (V + 1U) + v) : 0U, hi = live ? __ldg(first + p * (V + 1U) + v + 1U) : 0U;
     const uint32_t* list = order + static_cast<uint64_t>(p) * B;
     const uint32_t mask = 0xFFU << (lane & 24U);  // the eight lanes of this group

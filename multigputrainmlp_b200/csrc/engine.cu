@@ -420,7 +420,7 @@ namespace mgt {
 namespace {
 
 template <class Cfg>
-mgt_status_t LaunchGemm(mgt_engine* e, const CUtensorMap& ta, const CUtensorMap& tb, GemmArgs args, cudaStream_t stream) {
+mgt_status_t LaunchGemm(mgt_engine* e, const CUtensorMap& ta, const CUtensorMap& tb, GemmArgs args, LaunchOn stream) {
     // the opt-in shared-memory size is a per-device attribute of each kernel instantiation
     static std::mutex attr_mu;
     static bool attr_done[64] = {};
@@ -442,13 +442,13 @@ mgt_status_t LaunchGemm(mgt_engine* e, const CUtensorMap& ta, const CUtensorMap&
     }
     args.status = e->status_word;
     args.bf16 = e->bf16_now ? 1U : 0U;
-    umma_gemm_kernel<Cfg><<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(ta, tb, args);
+    Launch(umma_gemm_kernel<Cfg>, grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream, ta, tb, args);
     ++e->launches;
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
 }
 
 template <bool GRAD>
-mgt_status_t LaunchPair(mgt_engine* e, const CUtensorMap& ta, const CUtensorMap& to, PairArgs args, cudaStream_t stream) {
+mgt_status_t LaunchPair(mgt_engine* e, const CUtensorMap& ta, const CUtensorMap& to, PairArgs args, LaunchOn stream) {
     static std::mutex attr_mu;
     static bool attr_done[64] = {};
     if (e->device < 0 || e->device >= 64) return MGT_INVALID_CONFIG;
@@ -461,7 +461,7 @@ mgt_status_t LaunchPair(mgt_engine* e, const CUtensorMap& ta, const CUtensorMap&
     }
     args.status = e->status_word;
     args.bf16 = e->bf16_now ? 1U : 0U;
-    onehot_pair_kernel<GRAD><<<2U * args.workers, PairCfg<GRAD>::THREADS, PairCfg<GRAD>::SMEM_BYTES, stream>>>(ta, to, args);
+    Launch(onehot_pair_kernel<GRAD>, 2U * args.workers, PairCfg<GRAD>::THREADS, PairCfg<GRAD>::SMEM_BYTES, stream, ta, to, args);
     ++e->launches;
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
 }
@@ -511,6 +511,7 @@ struct RepackPlan {
 };
 __global__ void __launch_bounds__(256)
 RepackHalfKernel(const float* __restrict__ src, uint8_t* __restrict__ dst, const __grid_constant__ RepackPlan plan, bool bf16) {
+    dependent_begin();
     const uint64_t total = plan.unit_begin[plan.count];
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     uint32_t i = 0;
@@ -584,6 +585,7 @@ SumKernel(const __grid_constant__ SumJobs jobs) {
     uint32_t at = 0;
     while (at + 1U < jobs.count && blockIdx.x >= jobs.job[at + 1U].first_cta) ++at;
     const SumJob& job = jobs.job[at];
+    dependent_begin();
     const uint32_t local = blockIdx.x - job.first_cta, group = local / job.per_group, cta = local - group * job.per_group;
     const float* src = job.src + group * job.src_group;
     float* dst = job.dst + group * job.dst_group;
@@ -631,7 +633,9 @@ HeadOut1Kernel(const float* __restrict__ w_out, const float* __restrict__ b_out,
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31U;
     const uint32_t warps_total = gridDim.x * (kHeadThreads / 32);
     const float inv_n = 1.0f / static_cast<float>(B);
-    const float bias = *b_out;
+    dependent_begin();
+    w_out = after_begin(w_out);
+    const float bias = *after_begin(b_out);
     float wreg[kHeadMaxPerLane], gacc[kHeadMaxPerLane], dacc[kHeadMaxPerLane];
 #pragma unroll
     for (int q = 0; q < kHeadMaxPerLane; ++q) {
@@ -783,6 +787,7 @@ HeadTileKernel(const __grid_constant__ HeadArgs a) {
     float* xs = ws + (size_t)a.H2 * OP;                // [64 columns][XP]: x of the tile, transposed
     float* ys = xs + 64U * XP;                         // [64 samples][OP]
     const uint32_t t = threadIdx.x, warp = t >> 5, lane = t & 31U;
+    dependent_begin();
     for (uint32_t i = t; i < a.H2 * OP; i += kHeadThreads) {
         const uint32_t j = i / OP, o = i % OP;
         float w = 0.0f;
@@ -926,6 +931,7 @@ HeadOutNKernel(const __grid_constant__ HeadArgs a) {
     extern __shared__ float s_dyn[];  // per warp: OUT floats (logits, then rounded dy)
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31U;
     const uint32_t warps_total = gridDim.x * (kHeadThreads / 32), H2 = a.H2, OUT = a.OUT;
+    dependent_begin();
     float* s_dy = s_dyn + warp * OUT;
     auto weight = [&](uint32_t j, uint32_t o) -> float {
         return kF32 ? static_cast<const float*>(a.w_out)[(uint64_t)j * a.p_wout + o] : ptx::from_operand(static_cast<const uint16_t*>(a.w_out)[(uint64_t)j * a.p_wout + o], a.bf16);
@@ -981,6 +987,7 @@ HeadOutNKernel(const __grid_constant__ HeadArgs a) {
 __global__ void __launch_bounds__(256)
 HeadOutNBiasGradKernel(const float* __restrict__ dy, uint32_t B, uint32_t OUT, float* __restrict__ grad_b) {
     __shared__ float s_sum[256];
+    dependent_begin();
     const uint32_t o = blockIdx.x;
     float sum = 0.0f;
     for (uint32_t b = threadIdx.x; b < B; b += 256U) sum += dy[(uint64_t)b * OUT + o];
@@ -997,7 +1004,7 @@ HeadOutNBiasGradKernel(const float* __restrict__ dy, uint32_t B, uint32_t OUT, f
 // to all that is left beside the kernel's static arrays, never to what this launch needs (another thread's launch may want more
 // at that moment, and a kernel with static arrays needs it set below 48 KB too).
 template <void (*kKernel)(HeadArgs)>
-bool LaunchHeadKernel(int device, uint32_t grid, size_t smem, cudaStream_t st, const HeadArgs& a) {
+bool LaunchHeadKernel(int device, uint32_t grid, size_t smem, LaunchOn st, const HeadArgs& a) {
     static std::mutex attr_mu;
     static size_t most[64] = {};
     if (device < 0 || device >= 64) return false;
@@ -1013,7 +1020,7 @@ bool LaunchHeadKernel(int device, uint32_t grid, size_t smem, cudaStream_t st, c
         }
         if (smem > most[device]) return false;
     }
-    kKernel<<<grid, kHeadThreads, smem, st>>>(a);
+    Launch(kKernel, grid, kHeadThreads, smem, st, a);
     return true;
 }
 
@@ -1060,10 +1067,10 @@ struct Sums {
         Rows(colsum + slot * R, rows, H, H, grad + HiddenBias(s));
         Rows(colsum + slot * (R + 1ULL), rows, H, H, grad + Fc2B(s, 0), R - 1U, slot, BlockParams(s));
     }
-    mgt_status_t Pass(cudaStream_t st) { return at_once || waiting > kMostWaiting ? Launch(st) : MGT_OK; }
-    mgt_status_t Launch(cudaStream_t st) {
+    mgt_status_t Pass(LaunchOn st) { return at_once || waiting > kMostWaiting ? LaunchAll(st) : MGT_OK; }
+    mgt_status_t LaunchAll(LaunchOn st) {
         if (jobs.count == 0U) return MGT_OK;
-        SumKernel<<<jobs.ctas, 256, 0, st>>>(jobs);
+        mgt::Launch(SumKernel, jobs.ctas, 256, 0, st, jobs);
         jobs.count = jobs.ctas = 0U;
         waiting = 0;
         ++e->launches;
@@ -1074,7 +1081,7 @@ struct Sums {
 // Output layer with several outputs, its loss and the gradient entering the layer below, enqueued; all gradients of the head
 // except W_out's, which is a product over the batch.
 template <bool kCrossEntropy, bool kF32>
-mgt_status_t LaunchHeadN(mgt_engine* e, cudaStream_t st, const HeadArgs& a, Sums& sums, float* loss, float* bias_below, float* grad_b) {
+mgt_status_t LaunchHeadN(mgt_engine* e, LaunchOn st, const HeadArgs& a, Sums& sums, float* loss, float* bias_below, float* grad_b) {
     const bool tiled = a.OUT <= 64U;
     const uint32_t tiles = tiled ? (a.B + kHeadTile - 1U) / kHeadTile : (a.B + 7U) / 8U;
     const uint32_t grid = tiles < kHeadBlocks ? tiles : kHeadBlocks;
@@ -1089,7 +1096,7 @@ mgt_status_t LaunchHeadN(mgt_engine* e, cudaStream_t st, const HeadArgs& a, Sums
     sums.Rows(a.partials, grid, width, 1, loss);
     if (bias_below != nullptr) sums.Rows(a.partials + 1U, grid, width, a.H2, bias_below);
     if (tiled) sums.Rows(a.partials + 1U + a.H2, grid, width, a.OUT, grad_b);
-    else HeadOutNBiasGradKernel<<<a.OUT, 256, 0, st>>>(a.dy, a.B, a.OUT, grad_b);
+    else Launch(HeadOutNBiasGradKernel, a.OUT, 256, 0, st, a.dy, a.B, a.OUT, grad_b);
     e->launches += tiled ? 1 : 2;
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
 }
@@ -1189,7 +1196,7 @@ struct StageTimer {
 
 // D = act[M x K, K-major] * W[K x N, row-major] with a forward epilogue.
 template <Epi EPI>
-mgt_status_t GemmForward(mgt_engine* e, cudaStream_t st, const __half* act, uint32_t act_pitch, const __half* w, uint32_t w_pitch,
+mgt_status_t GemmForward(mgt_engine* e, LaunchOn st, const __half* act, uint32_t act_pitch, const __half* w, uint32_t w_pitch,
                          uint32_t M, uint32_t N, uint32_t K, GemmArgs epi) {
     const uint32_t bn = PickBN(N);
     GemmArgs a = BaseArgs(M, N, K, bn, 1);
@@ -1204,7 +1211,7 @@ mgt_status_t GemmForward(mgt_engine* e, cudaStream_t st, const __half* act, uint
 
 // The same product with the activation stored as actT[K][M] (one row per input column): an MN-major A operand.
 template <Epi EPI>
-mgt_status_t GemmForwardRows(mgt_engine* e, cudaStream_t st, const __half* act_t, uint32_t act_t_pitch, const __half* w, uint32_t w_pitch,
+mgt_status_t GemmForwardRows(mgt_engine* e, LaunchOn st, const __half* act_t, uint32_t act_t_pitch, const __half* w, uint32_t w_pitch,
                              uint32_t M, uint32_t N, uint32_t K, GemmArgs epi) {
     const uint32_t bn = PickBN(N);
     GemmArgs a = BaseArgs(M, N, K, bn, 1);
@@ -1239,7 +1246,7 @@ BackpropPlan PlanBackprop(const mgt_engine* e, uint32_t M, uint32_t N, uint32_t 
 // next dz tensor; its fp32 column sums (a bias gradient) go to `colsum` (zeroed by the caller,
 // PlanBackprop().rows rows of N).
 template <Epi EPI>
-mgt_status_t GemmBackpropInput(mgt_engine* e, cudaStream_t st, const __half* dz, uint32_t dz_pitch, const __half* w, uint32_t w_pitch,
+mgt_status_t GemmBackpropInput(mgt_engine* e, LaunchOn st, const __half* dz, uint32_t dz_pitch, const __half* w, uint32_t w_pitch,
                                uint32_t M, uint32_t N, uint32_t K, GemmArgs epi, float* colsum) {
     const BackpropPlan p = PlanBackprop(e, M, N, K);
     GemmArgs a = BaseArgs(M, N, K, p.bn, 1);
@@ -1256,7 +1263,7 @@ mgt_status_t GemmBackpropInput(mgt_engine* e, cudaStream_t st, const __half* dz,
 // The weight gradients of all residual blocks for one of the two linear layers in ONE launch:
 // grad_g[in x out] = act_g^T * dz_g for g = 0..groups-1, where act_g / dz_g are slices of two tapes and
 // grad_g lie `grad_group_stride` floats apart. Split-K.
-mgt_status_t GemmGradWeightsGrouped(mgt_engine* e, cudaStream_t st, const __half* act_tape, uint32_t act_pitch, uint64_t act_stride_bytes,
+mgt_status_t GemmGradWeightsGrouped(mgt_engine* e, LaunchOn st, const __half* act_tape, uint32_t act_pitch, uint64_t act_stride_bytes,
                                     const __half* dz_tape, uint32_t dz_pitch, uint64_t dz_stride_bytes, uint32_t groups, uint32_t samples,
                                     uint32_t in_dim, uint32_t out_dim, float* partial, Sums& sums, float* grad_first, uint64_t grad_group_stride) {
     const uint32_t bn = PickBN(out_dim);
@@ -1272,7 +1279,7 @@ mgt_status_t GemmGradWeightsGrouped(mgt_engine* e, cudaStream_t st, const __half
 }
 
 // grad[in x out] = act^T * dz, reduced over the batch with split-K.
-mgt_status_t GemmGradWeights(mgt_engine* e, cudaStream_t st, const __half* act, uint32_t act_pitch, const __half* dz, uint32_t dz_pitch,
+mgt_status_t GemmGradWeights(mgt_engine* e, LaunchOn st, const __half* act, uint32_t act_pitch, const __half* dz, uint32_t dz_pitch,
                              uint32_t samples, uint32_t in_dim, uint32_t out_dim, float* partial, Sums& sums, float* grad_out) {
     const uint32_t bn = PickBN(out_dim);
     GemmArgs a = BaseArgs(in_dim, out_dim, samples, bn, MostSplits(in_dim, out_dim, 1, (uint32_t)e->sm_count));
@@ -1286,7 +1293,7 @@ mgt_status_t GemmGradWeights(mgt_engine* e, cudaStream_t st, const __half* act, 
 }
 
 // grad[in x out] = act^T * dz with the activation stored as actT[in][samples]: a K-major A operand.
-mgt_status_t GemmGradWeightsRows(mgt_engine* e, cudaStream_t st, const __half* act_t, uint32_t act_t_pitch, const __half* dz, uint32_t dz_pitch,
+mgt_status_t GemmGradWeightsRows(mgt_engine* e, LaunchOn st, const __half* act_t, uint32_t act_t_pitch, const __half* dz, uint32_t dz_pitch,
                                  uint32_t samples, uint32_t in_dim, uint32_t out_dim, float* partial, Sums& sums, float* grad_out) {
     const uint32_t bn = PickBN(out_dim);
     GemmArgs a = BaseArgs(in_dim, out_dim, samples, bn, MostSplits(in_dim, out_dim, 1, (uint32_t)e->sm_count));
@@ -1304,7 +1311,7 @@ mgt_status_t GemmGradWeightsRows(mgt_engine* e, cudaStream_t st, const __half* a
 // Row sums of the result (the bias gradient of the layer below) go to bias_grad[N_in] with the step's sums. With
 // dx_f32 the result goes there instead, in fp32 and with one row per sample; with dx_rows it goes to dx_t in the operand format
 // with one row per sample.
-mgt_status_t GemmBackpropInputRows(mgt_engine* e, cudaStream_t st, const __half* w, uint32_t w_pitch, const __half* dz, uint32_t dz_pitch, uint32_t samples,
+mgt_status_t GemmBackpropInputRows(mgt_engine* e, LaunchOn st, const __half* w, uint32_t w_pitch, const __half* dz, uint32_t dz_pitch, uint32_t samples,
                                    uint32_t in_dim, uint32_t out_dim, uint32_t* mask_bits, uint32_t ld_bits, __half* dx_t, uint32_t t_pitch, float* dx_f32, uint32_t f32_pitch, bool dx_rows, uint32_t dx_rows_pitch, float* rowsum,
                                    uint64_t rowsum_rows, Sums& sums, float* bias_grad) {
     GemmArgs a = BaseArgs(in_dim, samples, out_dim, CfgDxRows::BN, 1);
@@ -1327,7 +1334,7 @@ bool ChainEligible(const mgt_engine* e, const mgt_mlp_shape_t& s) {
 }
 
 template <bool BWD>
-mgt_status_t LaunchChain(mgt_engine* e, cudaStream_t st, const __half* w_first, uint32_t w_pitch, uint64_t w_layer_stride_bytes, uint32_t tape_s_entries,
+mgt_status_t LaunchChain(mgt_engine* e, LaunchOn st, const __half* w_first, uint32_t w_pitch, uint64_t w_layer_stride_bytes, uint32_t tape_s_entries,
                          uint32_t tape_t_entries, ChainArgs a) {
     static std::mutex attr_mu;
     static bool attr_done[64] = {};
@@ -1349,8 +1356,8 @@ mgt_status_t LaunchChain(mgt_engine* e, cudaStream_t st, const __half* w_first, 
     a.status = e->status_word;
     a.bf16 = e->bf16_now ? 1U : 0U;
     const uint32_t units = wide ? (uint32_t)e->sm_count / 2U : (uint32_t)e->sm_count, grid = a.tiles < units ? a.tiles : units;
-    if (wide) tower_wide_kernel<BWD><<<2U * grid, WideCfg::THREADS, WideCfg::SMEM_BYTES, st>>>(tw, ts, tt, a);
-    else tower_chain_kernel<BWD><<<grid, ChainCfg::THREADS, ChainCfg::SMEM_BYTES, st>>>(tw, ts, tt, a);
+    if (wide) Launch(tower_wide_kernel<BWD>, 2U * grid, WideCfg::THREADS, WideCfg::SMEM_BYTES, st, tw, ts, tt, a);
+    else Launch(tower_chain_kernel<BWD>, grid, ChainCfg::THREADS, ChainCfg::SMEM_BYTES, st, tw, ts, tt, a);
     ++e->launches;
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
 }
@@ -1407,7 +1414,7 @@ uint64_t Fp32WorkspaceFloats(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm) 
 
 template <class F>
 mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float* w, const uint8_t* states, const float* labels, uint32_t B, float* loss,
-                            float* grad, float* workspace, bool half_ig, bool told, mgt_backward_profile_t* profile, F&& notify, cudaStream_t st) {
+                            float* grad, float* workspace, bool half_ig, bool told, mgt_backward_profile_t* profile, F&& notify, LaunchOn st) {
     using namespace mgt::fp32path;
     const uint32_t sm = PlanSmCount(e->sm_count);
     const Fp32Workspace ws = PlanFp32(s, B, sm);
@@ -1468,7 +1475,7 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
     float* head_bias_dst = grad + (R > 0 ? Fc2B(s, R - 1) : HiddenBias(s));
     if (OUT == 1U) {
         const uint32_t grid = (B + 7U) / 8U < kHeadBlocks ? (B + 7U) / 8U : kHeadBlocks;
-        HeadOut1Kernel<<<grid, kHeadThreads, 0, st>>>(w + OutputWeight(s), w + OutputBias(s), labels, x(R), p2, B, H2, dz2(R), nullptr, 0, base + ws.head, false);
+        Launch(HeadOut1Kernel, grid, kHeadThreads, 0, st, w + OutputWeight(s), w + OutputBias(s), labels, x(R), p2, B, H2, dz2(R), nullptr, 0, base + ws.head, false);
         sums.Head(base + ws.head, grid, H2, grad + OutputWeight(s), loss, head_bias_dst);
         ++e->launches;
     } else {
@@ -1507,17 +1514,23 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
     sums.Rows(base + ws.colsum_in, rows_h1, H1, H1, grad + InputBias(s));
     MGT_TRY(sums.Pass(st));
     if (half_ig) {
-        RoundHalfKernel<<<GridFor((uint64_t)B * p1, 256, e->sm_count), 256, 0, st>>>(dz1, (uint64_t)B * p1);
+        Launch(RoundHalfKernel, GridFor((uint64_t)B * p1, 256, e->sm_count), 256, 0, st, dz1, (uint64_t)B * p1);
         ++e->launches;
     }
     if (!ok() || !timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
     if (EmbeddingGrad(st, states, dz1, p1, B, L, V, H1, reinterpret_cast<uint32_t*>(base + ws.lists), grad) != cudaSuccess) return MGT_CUDA_FAILURE;
     e->launches += 2;
-    MGT_TRY(sums.Launch(st));
+    MGT_TRY(sums.LaunchAll(st));
     MGT_TRY(notify(0, (uint64_t)L * V * H1 + H1));
     if (!timer.Mark(profile ? &profile->input_grad_ms : nullptr)) return MGT_CUDA_FAILURE;
     return MGT_OK;
 }
+
+// Whether the kernels of a step begin before those ahead of them have ended (launch.cuh): where a step is a row of short kernels.
+// 4 096 samples of hd1 1024 210 -> 200 us, 5 003 of hd1 333 172 -> 157, 1 024 of hd1 256 103 -> 82; 3 001 samples of hd1 2560 make no
+// difference, and with kernels that fill the chip the next one's CTAs are in the way: 9 001 samples of hd1 1000 445 -> 491, 8 192 of
+// hd1 2560 in fp32 4 701 -> 5 230. The many passes of batch normalisation stream and gain at any size (53 248 of hd1 2560 5 884 -> 5 510).
+bool OverlapLaunches(const mgt_mlp_shape_t& s, uint32_t B, bool batch_norm) { return batch_norm || (uint64_t)B * s.hd1 <= 6000000ULL; }
 
 struct HalfWeights {
     const __half* in_table; uint32_t p1;     // [(IN+1)][p1], row IN is the input bias
@@ -1679,12 +1692,12 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
             return ready(ready_user, id++, off, count, stream_v) == MGT_OK ? MGT_OK : MGT_CUDA_FAILURE;
         };
         return LaunchFp32Path(e, s, w, reinterpret_cast<const uint8_t*>(states), labels, B, loss, grad, workspace, half_ig != 0, ready != nullptr || profile != nullptr, profile, tell,
-                              static_cast<cudaStream_t>(stream_v));
+                              {static_cast<cudaStream_t>(stream_v), OverlapLaunches(s, B, false)});
     }
     Workspace ws = PlanWorkspace(s, B, PlanSmCount(e->sm_count), half_ig != 0, bnorm);
     if (e->embedding_form != mgt_engine::kBySize) ws.gather_fwd = ws.gather_grad = e->embedding_form == mgt_engine::kGather;
     if (workspace_floats < (ws.total_bytes + 3) / 4 + (half_ig ? 0 : Fp32TableFloats(s, B))) return MGT_CAPACITY_EXCEEDED;
-    cudaStream_t st = static_cast<cudaStream_t>(stream_v);
+    const LaunchOn st(static_cast<cudaStream_t>(stream_v), OverlapLaunches(s, B, bnorm));
     uint8_t* base = reinterpret_cast<uint8_t*>(RoundUp(reinterpret_cast<uintptr_t>(workspace), 1024));
     float* dz1_f32 = reinterpret_cast<float*>(RoundUp(reinterpret_cast<uintptr_t>(workspace + (ws.total_bytes + 3) / 4), 256));  // behind the tensor-core workspace
     const uint32_t p_dz1_f32 = (uint32_t)RoundUp(s.hd1, 4);
@@ -1728,8 +1741,8 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     };
     // z_tape(layer) -> x_f32 / x_h(layer): x = relu(bn(z)) for the hidden layer, relu(x + bn(z)) for a block
     auto bn_forward = [&](uint32_t layer) -> mgt_status_t {
-        bn::ColumnMomentsKernel<false><<<bn_blocks, bn::kThreads, 0, st>>>(z_tape(layer), ws.p_f32, nullptr, 0, nullptr, nullptr, B, H2, bn_partial);
-        bn::ReduceMomentsKernel<<<bn_reduce_grid, bn_reduce_threads, 0, st>>>(bn_partial, bn_blocks, H2, 1.0f / (float)B, bn_stats, nullptr, nullptr);
+        Launch(bn::ColumnMomentsKernel<false>, bn_blocks, bn::kThreads, 0, st, z_tape(layer), ws.p_f32, nullptr, 0, nullptr, nullptr, B, H2, bn_partial);
+        Launch(bn::ReduceMomentsKernel, bn_reduce_grid, bn_reduce_threads, 0, st, bn_partial, bn_blocks, H2, 1.0f / (float)B, bn_stats, nullptr, nullptr);
         MGT_TRY(bn_exchange());
         const float* gamma = w + bn_base + 2ULL * layer * H2;
         float* running = e->bn_running != nullptr ? e->bn_running + 2ULL * layer * H2 : nullptr;
@@ -1737,11 +1750,11 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
         const float unbias = n > 1.0 ? (float)(n / (n - 1.0)) : 1.0f;
         uint16_t* xh = reinterpret_cast<uint16_t*>(x_h(layer));
         if (layer == 0U) {
-            bn::ApplyForwardKernel<false><<<bn_blocks, bn::kThreads, 0, st>>>(z_tape(layer), ws.p_f32, bn_stats, gamma, gamma + H2, e->options.bn_eps, B, H2, x_f32,
+            Launch(bn::ApplyForwardKernel<false>, bn_blocks, bn::kThreads, 0, st, z_tape(layer), ws.p_f32, bn_stats, gamma, gamma + H2, e->options.bn_eps, B, H2, x_f32,
                                                                              ws.p_f32, xh, ws.p_act, e->bf16_now, bn_mean(layer), bn_rstd(layer), running,
                                                                              e->bn_momentum, unbias);
         } else {
-            bn::ApplyForwardKernel<true><<<bn_blocks, bn::kThreads, 0, st>>>(z_tape(layer), ws.p_f32, bn_stats, gamma, gamma + H2, e->options.bn_eps, B, H2, x_f32,
+            Launch(bn::ApplyForwardKernel<true>, bn_blocks, bn::kThreads, 0, st, z_tape(layer), ws.p_f32, bn_stats, gamma, gamma + H2, e->options.bn_eps, B, H2, x_f32,
                                                                             ws.p_f32, xh, ws.p_act, e->bf16_now, bn_mean(layer), bn_rstd(layer), running,
                                                                             e->bn_momentum, unbias);
         }
@@ -1751,13 +1764,13 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     // dzf (gradient w.r.t. the sum entering the ReLU above the layer) -> dz_tape(layer) = gradient w.r.t. z, plus the
     // gradients of gamma, beta and of the bias inside z
     auto bn_backward = [&](uint32_t layer, float* bias_grad) -> mgt_status_t {
-        bn::ColumnMomentsKernel<true><<<bn_blocks, bn::kThreads, 0, st>>>(dzf, ws.p_f32, z_tape(layer), ws.p_f32, bn_mean(layer), bn_rstd(layer), B, H2, bn_partial);
+        Launch(bn::ColumnMomentsKernel<true>, bn_blocks, bn::kThreads, 0, st, dzf, ws.p_f32, z_tape(layer), ws.p_f32, bn_mean(layer), bn_rstd(layer), B, H2, bn_partial);
         float* dgamma = grad + bn_base + 2ULL * layer * H2;
-        bn::ReduceMomentsKernel<<<bn_reduce_grid, bn_reduce_threads, 0, st>>>(bn_partial, bn_blocks, H2, 1.0f / (float)B, bn_stats, dgamma + H2, dgamma);
+        Launch(bn::ReduceMomentsKernel, bn_reduce_grid, bn_reduce_threads, 0, st, bn_partial, bn_blocks, H2, 1.0f / (float)B, bn_stats, dgamma + H2, dgamma);
         MGT_TRY(bn_exchange());
-        bn::ApplyBackwardKernel<<<bn_blocks, bn::kThreads, 0, st>>>(dzf, ws.p_f32, z_tape(layer), ws.p_f32, bn_mean(layer), bn_rstd(layer), w + bn_base + 2ULL * layer * H2,
+        Launch(bn::ApplyBackwardKernel, bn_blocks, bn::kThreads, 0, st, dzf, ws.p_f32, z_tape(layer), ws.p_f32, bn_mean(layer), bn_rstd(layer), w + bn_base + 2ULL * layer * H2,
                                                                     bn_stats, B, H2, reinterpret_cast<uint16_t*>(dz_tape(layer)), ws.p_dz, e->bf16_now, bn_partial);
-        bn::ReduceSumsKernel<<<bn_reduce_grid, bn_reduce_threads, 0, st>>>(bn_partial, bn_blocks, H2, bias_grad);
+        Launch(bn::ReduceSumsKernel, bn_reduce_grid, bn_reduce_threads, 0, st, bn_partial, bn_blocks, H2, bias_grad);
         e->launches += 4;
         return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
     };
@@ -1791,7 +1804,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
             hw.w2[k] = repack(Fc2W(s, k), H2, H2, ws.p_w2);
         }
         hw.wout = repack(OutputWeight(s), H2, OUT, ws.p_wout);
-        RepackHalfKernel<<<GridFor(plan.unit_begin[plan.count], 256, e->sm_count), 256, 0, st>>>(w, base + ws.off_wint, plan, e->bf16_now);
+        Launch(RepackHalfKernel, GridFor(plan.unit_begin[plan.count], 256, e->sm_count), 256, 0, st, w, base + ws.off_wint, plan, e->bf16_now);
         ++e->launches;
         if (cudaGetLastError() != cudaSuccess) return MGT_CUDA_FAILURE;
     }
@@ -1799,8 +1812,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     // ---- embedding forward: a1 = relu([onehot | 1] * [W_in ; b_in])  (mlp_backward.cu:755-832)
     if (ws.gather_fwd) {
         auto run = [&](auto kernel) {
-            kernel<<<dim3((B + 31U) / 32U, (H1 + 63U) / 64U), 256 * gather::kForwardSplit, 0, st>>>(
-                reinterpret_cast<const uint8_t*>(states), reinterpret_cast<const uint16_t*>(hw.in_table), hw.p1, B, s.state_len, s.state_value_pad, H1,
+            Launch(kernel, dim3((B + 31U) / 32U, (H1 + 63U) / 64U), 256 * gather::kForwardSplit, 0, st, reinterpret_cast<const uint8_t*>(states), reinterpret_cast<const uint16_t*>(hw.in_table), hw.p1, B, s.state_len, s.state_value_pad, H1,
                 reinterpret_cast<uint16_t*>(a1_h), ws.p_bt, reinterpret_cast<uint32_t*>(base + ws.off_bits_h1), ws.ld_bits_h1);
         };
         if (e->bf16_now) run(gather::ForwardKernel<gather::kForwardSplit, true>); else run(gather::ForwardKernel<gather::kForwardSplit, false>);
@@ -1874,7 +1886,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     // the head also yields the fp32 column sums of dz: the bias gradient of the layer below it, unless that is normalised
     float* head_bias_dst = bnorm ? nullptr : grad + (R > 0 ? Fc2B(s, R - 1) : HiddenBias(s));
     if (OUT == 1U) {
-        HeadOut1Kernel<<<kHeadBlocks, kHeadThreads, 0, st>>>(w + OutputWeight(s), w + OutputBias(s), labels, x_f32, ws.p_f32, B, H2, dzf, dz_cur, ws.p_dz, head_partial, e->bf16_now);
+        Launch(HeadOut1Kernel, kHeadBlocks, kHeadThreads, 0, st, w + OutputWeight(s), w + OutputBias(s), labels, x_f32, ws.p_f32, B, H2, dzf, dz_cur, ws.p_dz, head_partial, e->bf16_now);
         sums.Head(head_partial, kHeadBlocks, H2, grad + OutputWeight(s), loss, head_bias_dst);
         ++e->launches;
     } else {
@@ -1932,18 +1944,19 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     // hd1 1000, hd2 200, 8 blocks 510 -> 453 us a step, 1 024 of hd1 256, hd2 64, 2 blocks 134 -> 114, 64 of hd1 8, hd2 8
     // 99 -> 89. With more tiles each kernel has the whole chip anyway, and beyond some 16 000 samples of a small model the
     // gradient's gathers lose more to the shared memory of the GEMMs beside them than they gain (54 025 of hd1 88: 611 ->
-    // 660 us). Not with callers that are told of finished ranges or time the stages: they rely on the order.
+    // 660 us). Nor for the smallest steps, which the
+    // host's calls bound (64 samples of hd1 8: 59 us with, 56 without). Not with callers that are told of finished ranges or time the stages: they rely on the order.
     const uint64_t dx_tiles = (uint64_t)((H1 + 127U) / 128U) * ((B + 255U) / 256U);
     SideBranch branch{e, st};
-    if (dx_tiles < 2ULL * e->sm_count && B <= 16384U && !told) branch.Fork();
-    cudaStream_t st_dw = branch.open ? branch.side.stream : st;
+    if (dx_tiles < 2ULL * e->sm_count && B <= 16384U && (uint64_t)B * H1 >= 65536U && !told) branch.Fork();
+    const LaunchOn st_dw(branch.open ? branch.side.stream : st.stream, st.overlap);
     uint32_t* order = reinterpret_cast<uint32_t*>(base + ws.off_lists);
     uint32_t* first = order + (uint64_t)s.state_len * B;
-    auto sort_classes = [&](cudaStream_t stream) {
-        gather::SortByClassKernel<<<s.state_len, 1024, 0, stream>>>(reinterpret_cast<const uint8_t*>(states), B, s.state_value_pad, order, first);
+    auto sort_classes = [&](LaunchOn stream) {
+        Launch(gather::SortByClassKernel, s.state_len, 1024, 0, stream, reinterpret_cast<const uint8_t*>(states), B, s.state_value_pad, order, first);
         ++e->launches;
     };
-    if (branch.open && half_ig && ws.gather_grad) sort_classes(branch.side.stream);
+    if (branch.open && half_ig && ws.gather_grad) sort_classes(st_dw);
     Sums own{e, true};  // (the sums that wait are launched on the second stream, which does not see the dX product)
     Sums& dx_sums = branch.open ? own : sums;
     // dz1T = (Wh * dzh^T) * [pre-activation of a1 > 0], the input-bias gradient from its row sums. With --input-grad-fp16 0 the
@@ -1963,7 +1976,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     } else if (ws.gather_grad) {
         const bool vec = (H1 & 3U) == 0U && (reinterpret_cast<uintptr_t>(grad) & 15U) == 0U;
         auto run = [&](auto kernel, uint32_t rows_per_cta) {
-            kernel<<<dim3((IN + rows_per_cta - 1U) / rows_per_cta, (H1 + 63U) / 64U), 256, 0, st>>>(order, first, reinterpret_cast<const uint16_t*>(dz1_h), ws.p_dz1_rows, B,
+            Launch(kernel, dim3((IN + rows_per_cta - 1U) / rows_per_cta, (H1 + 63U) / 64U), 256, 0, st, order, first, reinterpret_cast<const uint16_t*>(dz1_h), ws.p_dz1_rows, B,
                                                                                                s.state_len, s.state_value_pad, H1, grad, vec);
         };
         if (!branch.open) sort_classes(st);
@@ -2011,7 +2024,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     // ---- hidden layer backward, dW part; every kernel that reads the hidden weights was enqueued long before, so a caller
     // may update the range in place as soon as it is announced
     MGT_TRY(GemmGradWeightsRows(e, st_dw, a1_h, ws.p_bt, dz_cur, ws.p_dz, B, H1, H2, reinterpret_cast<float*>(base + ws.off_partial), sums, grad + HiddenWeight(s)));
-    MGT_TRY(sums.Launch(st_dw));  // (on the second stream they are done while the table gradient still runs)
+    MGT_TRY(sums.LaunchAll(st_dw));  // (on the second stream they are done while the table gradient still runs)
     if (!branch.Join()) return MGT_CUDA_FAILURE;
     MGT_TRY(notify(HiddenWeight(s), (uint64_t)H1 * H2 + H2));
     if (!timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
@@ -2040,7 +2053,7 @@ mgt_status_t mgt_debug_gemm(mgt_engine_t* e, const uint16_t* a, uint32_t lda, in
                             float* d, uint32_t m, uint32_t n, uint32_t k, uint32_t splits, float* partial_scratch, void* stream) {
     if (e == nullptr || a == nullptr || b == nullptr || d == nullptr || m == 0 || n == 0 || k == 0 || splits == 0) return MGT_INVALID_CONFIG;
     if (splits > 1 && partial_scratch == nullptr) return MGT_INVALID_CONFIG;
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const LaunchOn st(static_cast<cudaStream_t>(stream), false);
     GemmArgs args = BaseArgs(m, n, k, 256, splits);
     // with a single split the accumulator tiles go straight into d, as 16-byte vectors when n is a multiple of 4
     if (args.splits == 1 && (n & 3U) == 0U && (reinterpret_cast<uintptr_t>(d) & 15U) != 0U) return MGT_INVALID_CONFIG;
@@ -2061,7 +2074,7 @@ mgt_status_t mgt_debug_gemm(mgt_engine_t* e, const uint16_t* a, uint32_t lda, in
     if (args.splits > 1) {
         Sums sums{e, true};
         sums.Planes(partial_scratch, args.splits, (uint64_t)m * n, d);
-        MGT_TRY(sums.Launch(st));
+        MGT_TRY(sums.LaunchAll(st));
     }
     return MGT_OK;
 }

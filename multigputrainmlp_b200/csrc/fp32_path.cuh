@@ -11,6 +11,7 @@
 #include <stdint.h>
 
 #include "embedding_gather.cuh"
+#include "launch.cuh"
 
 namespace mgt {
 namespace fp32path {
@@ -147,6 +148,7 @@ SgemmKernel(const __grid_constant__ SgemmArgs a) {
     for (int i = 0; i < TM / 2; ++i)
 #pragma unroll
         for (int j = 0; j < TN; ++j) acc[i][j] = 0ULL;
+    dependent_begin();
     fetch(0);
     stage(0);
     __syncthreads();
@@ -283,15 +285,15 @@ inline bool SgemmAligned(const float* p, uint32_t ld, uint64_t stride) {
     return (reinterpret_cast<uintptr_t>(p) & 15U) == 0U && (ld & 3U) == 0U && (stride & 3ULL) == 0ULL;
 }
 template <bool TA, bool TB>
-inline cudaError_t Sgemm(cudaStream_t st, SgemmArgs a, uint32_t groups, SgemmTile tile) {
+inline cudaError_t Sgemm(LaunchOn st, SgemmArgs a, uint32_t groups, SgemmTile tile) {
     a.vec_a = SgemmAligned(a.A, a.lda, a.stride_a);
     a.vec_b = SgemmAligned(a.B, a.ldb, a.stride_b);
     const uint32_t t = SgemmTileRows(tile);
     const dim3 grid((a.N + t - 1) / t, (a.M + t - 1) / t, groups * a.splits);
-    if (tile == SgemmTile::kLarge) SgemmKernel<128, 128, 8, 8, 1, 16, TA, TB><<<grid, 256, 0, st>>>(a);
-    else if (tile == SgemmTile::kMiddle) SgemmKernel<64, 64, 8, 4, 1, 16, TA, TB><<<grid, 128, 0, st>>>(a);
-    else if constexpr (!TA && !TB) SgemmKernel<32, 32, 4, 2, 1, 64, TA, TB><<<grid, 128, 0, st>>>(a);
-    else SgemmKernel<32, 32, 4, 4, 4, 16, TA, TB><<<grid, 256, 0, st>>>(a);
+    if (tile == SgemmTile::kLarge) Launch(SgemmKernel<128, 128, 8, 8, 1, 16, TA, TB>, grid, 256, 0, st, a);
+    else if (tile == SgemmTile::kMiddle) Launch(SgemmKernel<64, 64, 8, 4, 1, 16, TA, TB>, grid, 128, 0, st, a);
+    else if constexpr (!TA && !TB) Launch(SgemmKernel<32, 32, 4, 2, 1, 64, TA, TB>, grid, 128, 0, st, a);
+    else Launch(SgemmKernel<32, 32, 4, 4, 4, 16, TA, TB>, grid, 256, 0, st, a);
     return cudaGetLastError();
 }
 
@@ -308,6 +310,7 @@ EmbeddingForwardKernel(const uint8_t* __restrict__ states, const float* __restri
     constexpr uint32_t kSamples = 8U * SPW;
     __shared__ uint8_t cls[80][kSamples];  // [position][sample]
     const uint32_t s0 = blockIdx.x * kSamples, warp = threadIdx.x >> 5, lane = threadIdx.x & 31U;
+    dependent_begin();
     for (uint32_t i = threadIdx.x; i < kSamples * L; i += 256U) {
         const uint32_t s = i / L, p = i - s * L;
         cls[p][s] = s0 + s < B ? states[static_cast<uint64_t>(s0 + s) * 80U + p] : 0U;
@@ -344,17 +347,17 @@ EmbeddingForwardKernel(const uint8_t* __restrict__ states, const float* __restri
         else dst[0] = fmaxf(acc[q][0], 0.0f);
     }
 }
-inline cudaError_t EmbeddingForward(cudaStream_t st, const uint8_t* states, const float* w_in, const float* b_in, uint32_t B, uint32_t L, uint32_t V, uint32_t H1,
+inline cudaError_t EmbeddingForward(LaunchOn st, const uint8_t* states, const float* w_in, const float* b_in, uint32_t B, uint32_t L, uint32_t V, uint32_t H1,
                                     float* a1, uint32_t ld, uint32_t sm_count) {
     const bool quads = (H1 & 3U) == 0U && (ld & 3U) == 0U && (reinterpret_cast<uintptr_t>(w_in) & 15U) == 0U;
     const uint32_t col_blocks = (H1 + (quads ? 128U : 32U) - 1U) / (quads ? 128U : 32U);
     // eight samples per warp once that still leaves four CTAs for every SM
     const bool many = static_cast<uint64_t>((B + 63U) / 64U) * col_blocks >= 4ULL * sm_count;
     const dim3 grid(many ? (B + 63U) / 64U : (B + 7U) / 8U, col_blocks);
-    if (quads && many) EmbeddingForwardKernel<8, 4><<<grid, 256, 0, st>>>(states, w_in, b_in, B, L, V, H1, a1, ld);
-    else if (quads) EmbeddingForwardKernel<1, 4><<<grid, 256, 0, st>>>(states, w_in, b_in, B, L, V, H1, a1, ld);
-    else if (many) EmbeddingForwardKernel<8, 1><<<grid, 256, 0, st>>>(states, w_in, b_in, B, L, V, H1, a1, ld);
-    else EmbeddingForwardKernel<1, 1><<<grid, 256, 0, st>>>(states, w_in, b_in, B, L, V, H1, a1, ld);
+    if (quads && many) Launch(EmbeddingForwardKernel<8, 4>, grid, 256, 0, st, states, w_in, b_in, B, L, V, H1, a1, ld);
+    else if (quads) Launch(EmbeddingForwardKernel<1, 4>, grid, 256, 0, st, states, w_in, b_in, B, L, V, H1, a1, ld);
+    else if (many) Launch(EmbeddingForwardKernel<8, 1>, grid, 256, 0, st, states, w_in, b_in, B, L, V, H1, a1, ld);
+    else Launch(EmbeddingForwardKernel<1, 1>, grid, 256, 0, st, states, w_in, b_in, B, L, V, H1, a1, ld);
     return cudaGetLastError();
 }
 
@@ -371,6 +374,8 @@ EmbeddingGradKernel(const uint32_t* __restrict__ order, const uint32_t* __restri
     if (row >= L * V) return;
     const uint32_t p = row / V, v = row - p * V;
     const uint32_t h = (blockIdx.y * 32U + lane) * W;
+    dependent_begin();
+    first = after_begin(first);
     const uint32_t lo = __ldg(first + p * (V + 1U) + v), hi = __ldg(first + p * (V + 1U) + v + 1U);
     const uint32_t* list = order + static_cast<uint64_t>(p) * B;
     float acc[W] = {};
@@ -398,20 +403,21 @@ EmbeddingGradKernel(const uint32_t* __restrict__ order, const uint32_t* __restri
     else dst[0] = acc[0];
 }
 // `lists`: gather::ListWords words of scratch
-inline cudaError_t EmbeddingGrad(cudaStream_t st, const uint8_t* states, const float* dz1, uint32_t ld, uint32_t B, uint32_t L, uint32_t V, uint32_t H1,
+inline cudaError_t EmbeddingGrad(LaunchOn st, const uint8_t* states, const float* dz1, uint32_t ld, uint32_t B, uint32_t L, uint32_t V, uint32_t H1,
                                  uint32_t* lists, float* grad_table) {
     uint32_t* first = lists + static_cast<uint64_t>(L) * B;
-    gather::SortByClassKernel<<<L, 1024, 0, st>>>(states, B, V, lists, first);
+    Launch(gather::SortByClassKernel, L, 1024, 0, st, states, B, V, lists, first);
     const bool quads = (H1 & 3U) == 0U && (ld & 3U) == 0U && (reinterpret_cast<uintptr_t>(grad_table) & 15U) == 0U;
     const uint32_t cols = quads ? 128U : 32U;
     const dim3 grid((L * V + 7U) / 8U, (H1 + cols - 1U) / cols);
-    if (quads) EmbeddingGradKernel<4><<<grid, 256, 0, st>>>(lists, first, dz1, ld, B, L, V, H1, grad_table);
-    else EmbeddingGradKernel<1><<<grid, 256, 0, st>>>(lists, first, dz1, ld, B, L, V, H1, grad_table);
+    if (quads) Launch(EmbeddingGradKernel<4>, grid, 256, 0, st, lists, first, dz1, ld, B, L, V, H1, grad_table);
+    else Launch(EmbeddingGradKernel<1>, grid, 256, 0, st, lists, first, dz1, ld, B, L, V, H1, grad_table);
     return cudaGetLastError();
 }
 
 // fp16 rounding of the embedding-gradient operand (--linear-fp16 0 --input-grad-fp16 1)
 __global__ void RoundHalfKernel(float* __restrict__ x, uint64_t total) {
+    dependent_begin();
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += stride) x[i] = __half2float(__float2half_rn(x[i]));
 }

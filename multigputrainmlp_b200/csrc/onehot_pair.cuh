@@ -25,6 +25,7 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include "launch.cuh"
 #include "ptx_sm100.cuh"
 
 namespace mgt {
@@ -220,6 +221,7 @@ onehot_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
     pair::cluster_sync_all();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_holder;
+    dependent_begin();
     pair::Pieces<GRAD> pieces(args, worker);
     pair::Piece p;
 

@@ -32,6 +32,7 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include "launch.cuh"
 #include "ptx_sm100.cuh"
 
 namespace mgt {
@@ -192,6 +193,7 @@ tower_chain_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_holder;
+    dependent_begin();
 
     if (warp == 0) {
         // ------------------------------- weight stream ------------------------------------

@@ -15,6 +15,7 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include "launch.cuh"
 #include "onehot_pair.cuh"
 #include "ptx_sm100.cuh"
 #include "tower_chain.cuh"
@@ -113,6 +114,7 @@ tower_wide_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_consta
     pair::cluster_sync_all();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_holder;
+    dependent_begin();
     const uint32_t cluster = blockIdx.x >> 1, clusters = gridDim.x >> 1;
 
     if (warp == 0) {

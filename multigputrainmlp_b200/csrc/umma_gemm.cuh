@@ -17,6 +17,7 @@
 #include <cuda.h>
 #include <cuda_fp16.h>
 
+#include "launch.cuh"
 #include "ptx_sm100.cuh"
 
 namespace mgt {
@@ -160,6 +161,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_holder;
+    dependent_begin();
     // unit -> (m tile, n tile, split): splits of one tile are neighbours
     auto group_of = [&](uint32_t unit) { return Cfg::GROUPED ? unit / units_per_group : 0U; };
     auto decode = [&](uint32_t unit, uint32_t& mt, uint32_t& nt, uint32_t& sp) {

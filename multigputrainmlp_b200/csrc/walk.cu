@@ -17,6 +17,7 @@
 // (x mod b = ((hi mod b) * (2^32 mod b) + lo mod b) mod b, each step by a multiply-high with ceil(2^32 / b) and one
 // correction), which is several times cheaper than a 64-bit remainder.
 #include "../../include/mgt_b200.h"
+#include "launch.cuh"
 
 #include <cuda_runtime.h>
 
@@ -102,6 +103,7 @@ RandomWalkKernel(mgt_random_walk_config_t config, uint64_t base_seed, uint64_t e
     const bool drawer = tid < kWalkSamples;
     if (!drawer) {
         constexpr uint32_t kHelpers = kWalkThreads - kWalkSamples;
+        mgt::dependent_begin();
         for (uint32_t i = tid - kWalkSamples; i < kMoveWords; i += kHelpers) {
             const uint32_t mv = i / kStateWords, wd = i - mv * kStateWords;
             const uint32_t given = mv < config.move_count ? reinterpret_cast<const uint32_t*>(moves[mv].v)[wd] : 0U;
@@ -167,6 +169,8 @@ RandomWalkKernel(mgt_random_walk_config_t config, uint64_t base_seed, uint64_t e
                 cur = ahead; ahead = ahead2; plain = plain1; other = other1;
             }
             s_count[tid] = static_cast<uint8_t>(now);
+            // (the moves of the first round are drawn while the kernel ahead still runs: they are a matter of the arguments alone)
+            if (round == 0U) mgt::dependent_begin();
         }
         __syncthreads();
         const bool final_round = round + 1U == rounds;
@@ -226,6 +230,7 @@ RandomWalkKernel(mgt_random_walk_config_t config, uint64_t base_seed, uint64_t e
 __global__ void ExpandScalarLabelsKernel(const float* __restrict__ scalar_labels, uint32_t samples, uint32_t output_dim, float* __restrict__ labels) {
     const uint64_t item = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     const uint64_t total = static_cast<uint64_t>(samples) * output_dim;
+    mgt::dependent_begin();
     if (item >= total) return;
     labels[item] = scalar_labels[item / output_dim];
 }
@@ -260,13 +265,11 @@ mgt_status_t mgt_launch_random_walk(const mgt_random_walk_config_t* config, uint
     }
     // Up to 32 samples for each of 148 SMs a CTA takes 32: one word of positions per thread, the shortest path. Beyond that
     // 128 per CTA, so that the pair table is composed a quarter as often (three CTAs share an SM).
-    cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const mgt::LaunchOn st(static_cast<cudaStream_t>(stream), true);
     if (config->sample_count <= 148U * 32U) {
-        RandomWalkKernel<32><<<(config->sample_count + 31U) / 32U, kWalkThreads, 0, st>>>(
-            *config, base_seed, epoch, step, global_rank, device_moves, device_target, device_states, device_labels, device_meta);
+        mgt::Launch(RandomWalkKernel<32>, (config->sample_count + 31U) / 32U, kWalkThreads, 0, st, *config, base_seed, epoch, step, global_rank, device_moves, device_target, device_states, device_labels, device_meta);
     } else {
-        RandomWalkKernel<128><<<(config->sample_count + 127U) / 128U, kWalkThreads, 0, st>>>(
-            *config, base_seed, epoch, step, global_rank, device_moves, device_target, device_states, device_labels, device_meta);
+        mgt::Launch(RandomWalkKernel<128>, (config->sample_count + 127U) / 128U, kWalkThreads, 0, st, *config, base_seed, epoch, step, global_rank, device_moves, device_target, device_states, device_labels, device_meta);
     }
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
 }
@@ -276,7 +279,7 @@ mgt_status_t mgt_launch_expand_scalar_labels(const float* device_scalar_labels, 
     if (device_scalar_labels == nullptr || device_labels == nullptr || samples == 0 || output_dim == 0) return MGT_INVALID_CONFIG;
     const uint64_t total = static_cast<uint64_t>(samples) * output_dim;
     const uint32_t blocks = static_cast<uint32_t>((total + 255ULL) / 256ULL);
-    ExpandScalarLabelsKernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(device_scalar_labels, samples, output_dim, device_labels);
+    mgt::Launch(ExpandScalarLabelsKernel, blocks, 256, 0, {static_cast<cudaStream_t>(stream), true}, device_scalar_labels, samples, output_dim, device_labels);
     return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
 }
 

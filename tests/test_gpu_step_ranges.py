@@ -363,6 +363,48 @@ def small_step():
     engine.close()
 
 
+# Kernels that begin before the one ahead of them has ended: the same training steps with the device idle before every call, and
+# with foreign kernels between the calls, must end in the same bits.
+@pytest.mark.parametrize("half,batch_norm", [(True, False), (False, False), (True, True)])
+@pytest.mark.parametrize("n", [64, 1500])
+def test_steps_back_to_back(half, batch_norm, n):
+    shape = mgt.CudaMlpShape(72, 72, 256, 40, 2, 1)
+    total = shape.param_count + (mgt.bn_param_count(shape) if batch_norm else 0)
+    first = torch.from_numpy((np.random.default_rng(n).standard_normal(total) * 0.03).astype(np.float32)).to(DEV)
+    moves, target = random_puzzle(72, 18, n)
+    moves, target = torch.from_numpy(moves).to(DEV), torch.from_numpy(target).to(DEV)
+    floats = mgt.mlp_loss_grad_workspace_floats(shape, n, 1, half, half, batch_norm=batch_norm)
+    engine = mgt.Engine(0)
+    results = []
+    try:
+        assert engine.set_train_options(batch_norm=batch_norm) == 0
+        for between in ("idle", "nothing", "kernels"):
+            w, m, v, grad = first.clone(), torch.zeros_like(first), torch.zeros_like(first), torch.zeros_like(first)
+            w_half, loss, depth = w.half(), torch.zeros(1, device=DEV), torch.zeros(n, device=DEV)
+            states, meta = torch.zeros(n, 80, dtype=torch.uint8, device=DEV), torch.zeros(n, 16, dtype=torch.uint8, device=DEV)
+            ws = torch.full((floats,), float("nan"), device=DEV)
+
+            def pause():
+                if between == "idle":
+                    torch.cuda.synchronize()
+                elif between == "kernels":
+                    w.mul_(1.0)
+                    grad.add_(0.0)
+            for step in range(6):
+                assert mgt.launch_random_walk_kernel(mgt.RandomWalkKernelConfig(n, 1, 20), 5, 0, step, 0, moves, target, states, depth, meta) == 0
+                pause()
+                assert engine.launch_mlp_loss_grad(shape, w, w_half, states, depth, n, loss, grad, ws, floats, use_half_input_grad=half, use_half_linear=half) == 0
+                pause()
+                assert mgt.launch_adamw_kernel_with_half_mirror(mgt.AdamWKernelConfig(total, step + 1, 1e-3), w, w_half, grad, m, v) == 0
+                pause()
+            assert engine.check()[0] == 0
+            results.append([t.cpu().numpy() for t in (w, m, v, loss, states)])
+    finally:
+        engine.close()
+    for other in results[1:]:
+        assert all(np.array_equal(a, b) for a, b in zip(other, results[0]))
+
+
 def test_steps_on_several_streams_do_not_wait_for_each_other(small_step):
     other = SmallStep(small_step.engine, 64)
     assert small_step(one_stream=True) == 0
