@@ -188,17 +188,6 @@ ReduceMomentsKernel(const float* __restrict__ partial, uint32_t blocks, uint32_t
     }
 }
 
-__global__ void __launch_bounds__(kReduceCols * kReduceParts)
-ReduceSumsKernel(const float* __restrict__ partial, uint32_t blocks, uint32_t H, float* __restrict__ out) {
-    __shared__ float smem[kReduceCols * kReduceParts];
-    const uint32_t c = threadIdx.x % kReduceCols, part = threadIdx.x / kReduceCols;
-    const uint32_t h = blockIdx.x * kReduceCols + c;
-    const bool ok = h < H;
-    dependent_begin();
-    const float s = AddPartialRows(partial, blocks, H, h, ok, part, c, smem);
-    if (ok && part == 0U) out[h] = s;
-}
-
 // stats = {mean[H], meansq[H]} of the (global) batch -> saved mean/rstd of the layer, running statistics, and
 // x = relu(y) (hidden layer) or x = relu(x + y) (block) in fp32 plus its 16-bit copy.
 template <bool kResidual>

@@ -81,7 +81,7 @@ struct Workspace {
     bool gather_fwd, gather_grad;
     uint32_t p_dz1_rows;
     uint64_t off_lists;
-    uint64_t off_bn_z, bn_z_stride, off_bn_save, off_bn_partial, off_bn_stats;
+    uint64_t off_bn_z, bn_z_stride, off_bn_save, off_bn_partial, off_bn_bias, off_bn_stats;
     uint64_t total_bytes;
 };
 
@@ -225,6 +225,7 @@ Workspace PlanWorkspace(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm_count,
         w.off_bn_z = take(w.bn_z_stride * (w.R + 1));
         w.off_bn_save = take((uint64_t)(w.R + 1) * 2 * s.hd2 * 4);
         w.off_bn_partial = take((uint64_t)bn::kMaxBlocks * 2 * s.hd2 * 4);
+        w.off_bn_bias = take((uint64_t)(w.R + 1) * bn::kMaxBlocks * s.hd2 * 4);
         w.off_bn_stats = take(2ULL * s.hd2 * 4);
     }
     w.total_bytes = off + 1024;  // slack to align the caller's base
@@ -1201,7 +1202,7 @@ mgt_status_t GemmForward(mgt_engine* e, LaunchOn st, const __half* act, uint32_t
     const uint32_t bn = PickBN(N);
     GemmArgs a = BaseArgs(M, N, K, bn, 1);
     a.bias = epi.bias; a.out_f32 = epi.out_f32; a.ld_f32 = epi.ld_f32; a.out_f16 = epi.out_f16; a.ld_f16 = epi.ld_f16;
-    a.add_f32 = epi.add_f32; a.ld_add = epi.ld_add; a.mask = epi.mask; a.ld_mask = epi.ld_mask;
+    a.add_f32 = epi.add_f32; a.ld_add = epi.ld_add; a.mask = epi.mask; a.ld_mask = epi.ld_mask; a.moments = epi.moments;
     CUtensorMap ta, tb;
     MGT_MAP(e->Map(&ta, act, K, M, act_pitch, 64, 128));
     MGT_MAP(e->Map(&tb, w, N, K, w_pitch, 64, 64));
@@ -1216,7 +1217,7 @@ mgt_status_t GemmForwardRows(mgt_engine* e, LaunchOn st, const __half* act_t, ui
     const uint32_t bn = PickBN(N);
     GemmArgs a = BaseArgs(M, N, K, bn, 1);
     a.bias = epi.bias; a.out_f32 = epi.out_f32; a.ld_f32 = epi.ld_f32; a.out_f16 = epi.out_f16; a.ld_f16 = epi.ld_f16;
-    a.add_f32 = epi.add_f32; a.ld_add = epi.ld_add; a.mask = epi.mask; a.ld_mask = epi.ld_mask;
+    a.add_f32 = epi.add_f32; a.ld_add = epi.ld_add; a.mask = epi.mask; a.ld_mask = epi.ld_mask; a.moments = epi.moments;
     CUtensorMap ta, tb;
     MGT_MAP(e->Map(&ta, act_t, M, K, act_t_pitch, 64, 64));
     MGT_MAP(e->Map(&tb, w, N, K, w_pitch, 64, 64));
@@ -1732,6 +1733,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     auto bn_mean = [&](uint32_t layer) { return reinterpret_cast<float*>(base + ws.off_bn_save) + 2ULL * layer * H2; };
     auto bn_rstd = [&](uint32_t layer) { return bn_mean(layer) + H2; };
     float* bn_partial = reinterpret_cast<float*>(base + ws.off_bn_partial);
+    auto bn_bias = [&](uint32_t layer) { return reinterpret_cast<float*>(base + ws.off_bn_bias) + (uint64_t)layer * bn::kMaxBlocks * H2; };  // partial sums of a bias gradient
     float* bn_stats = bnorm && e->bn_exchange_buffer != nullptr ? e->bn_exchange_buffer : reinterpret_cast<float*>(base + ws.off_bn_stats);
     const uint32_t bn_blocks = bn::BlocksFor(B, e->sm_count);
     const uint32_t bn_reduce_grid = (H2 + bn::kReduceCols - 1U) / bn::kReduceCols, bn_reduce_threads = bn::kReduceCols * bn::kReduceParts;
@@ -1739,10 +1741,15 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
         if (e->bn_exchange == nullptr) return MGT_OK;
         return e->bn_exchange(e->bn_exchange_user, bn_stats, 2ULL * H2, stream_v) == MGT_OK ? MGT_OK : MGT_CUDA_FAILURE;
     };
+    // Widths of one tile: the GEMM that makes z leaves its column moments too, as four rows of partial sums a CTA. As a kernel of its
+    // own they read z again: p888 at 53 248 samples 5 524 -> 5 450 us a step. (The moments of the backward pass in the epilogue
+    // of the product before them were tried: it needs z there, and 5 485 us.)
+    const uint32_t bn_rows = 4U * std::min((B + 127U) / 128U, (uint32_t)e->sm_count);
+    const bool bn_fused = H2 <= 256U && bn_rows <= bn::kMaxBlocks;
     // z_tape(layer) -> x_f32 / x_h(layer): x = relu(bn(z)) for the hidden layer, relu(x + bn(z)) for a block
     auto bn_forward = [&](uint32_t layer) -> mgt_status_t {
-        Launch(bn::ColumnMomentsKernel<false>, bn_blocks, bn::kThreads, 0, st, z_tape(layer), ws.p_f32, nullptr, 0, nullptr, nullptr, B, H2, bn_partial);
-        Launch(bn::ReduceMomentsKernel, bn_reduce_grid, bn_reduce_threads, 0, st, bn_partial, bn_blocks, H2, 1.0f / (float)B, bn_stats, nullptr, nullptr);
+        if (!bn_fused) Launch(bn::ColumnMomentsKernel<false>, bn_blocks, bn::kThreads, 0, st, z_tape(layer), ws.p_f32, nullptr, 0, nullptr, nullptr, B, H2, bn_partial);
+        Launch(bn::ReduceMomentsKernel, bn_reduce_grid, bn_reduce_threads, 0, st, bn_partial, bn_fused ? bn_rows : bn_blocks, H2, 1.0f / (float)B, bn_stats, nullptr, nullptr);
         MGT_TRY(bn_exchange());
         const float* gamma = w + bn_base + 2ULL * layer * H2;
         float* running = e->bn_running != nullptr ? e->bn_running + 2ULL * layer * H2 : nullptr;
@@ -1758,20 +1765,19 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
                                                                             ws.p_f32, xh, ws.p_act, e->bf16_now, bn_mean(layer), bn_rstd(layer), running,
                                                                             e->bn_momentum, unbias);
         }
-        e->launches += 3;
+        e->launches += bn_fused ? 2 : 3;
         return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
     };
     // dzf (gradient w.r.t. the sum entering the ReLU above the layer) -> dz_tape(layer) = gradient w.r.t. z, plus the
     // gradients of gamma, beta and of the bias inside z
-    auto bn_backward = [&](uint32_t layer, float* bias_grad) -> mgt_status_t {
+    auto bn_backward = [&](uint32_t layer) -> mgt_status_t {
         Launch(bn::ColumnMomentsKernel<true>, bn_blocks, bn::kThreads, 0, st, dzf, ws.p_f32, z_tape(layer), ws.p_f32, bn_mean(layer), bn_rstd(layer), B, H2, bn_partial);
         float* dgamma = grad + bn_base + 2ULL * layer * H2;
         Launch(bn::ReduceMomentsKernel, bn_reduce_grid, bn_reduce_threads, 0, st, bn_partial, bn_blocks, H2, 1.0f / (float)B, bn_stats, dgamma + H2, dgamma);
         MGT_TRY(bn_exchange());
         Launch(bn::ApplyBackwardKernel, bn_blocks, bn::kThreads, 0, st, dzf, ws.p_f32, z_tape(layer), ws.p_f32, bn_mean(layer), bn_rstd(layer), w + bn_base + 2ULL * layer * H2,
-                                                                    bn_stats, B, H2, reinterpret_cast<uint16_t*>(dz_tape(layer)), ws.p_dz, e->bf16_now, bn_partial);
-        Launch(bn::ReduceSumsKernel, bn_reduce_grid, bn_reduce_threads, 0, st, bn_partial, bn_blocks, H2, bias_grad);
-        e->launches += 4;
+                                                                    bn_stats, B, H2, reinterpret_cast<uint16_t*>(dz_tape(layer)), ws.p_dz, e->bf16_now, bn_bias(layer));
+        e->launches += 3;
         return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_CUDA_FAILURE;
     };
 
@@ -1839,7 +1845,9 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
         epi.bias = w + HiddenBias(s); epi.out_f32 = x_f32; epi.ld_f32 = ws.p_f32; epi.out_f16 = x_h(0); epi.ld_f16 = ws.p_act;
         if (bnorm) {
             epi.out_f32 = z_tape(0);
-            MGT_TRY(GemmForwardRows<Epi::kBiasF32>(e, st, a1_h, ws.p_bt, hw.wh, hw.p2, B, H2, H1, epi));
+            epi.moments = bn_partial;
+            MGT_TRY(bn_fused ? GemmForwardRows<Epi::kBiasF32Moments>(e, st, a1_h, ws.p_bt, hw.wh, hw.p2, B, H2, H1, epi)
+                             : GemmForwardRows<Epi::kBiasF32>(e, st, a1_h, ws.p_bt, hw.wh, hw.p2, B, H2, H1, epi));
             MGT_TRY(bn_forward(0));
         } else {
             MGT_TRY(GemmForwardRows<Epi::kBiasReluF32F16>(e, st, a1_h, ws.p_bt, hw.wh, hw.p2, B, H2, H1, epi));
@@ -1873,7 +1881,9 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
         e2.out_f16 = x_h(k + 1); e2.ld_f16 = ws.p_act;
         if (bnorm) {
             e2.out_f32 = z_tape(k + 1U);
-            MGT_TRY(GemmForward<Epi::kBiasF32>(e, st, r1_h(k), ws.p_act, hw.w2[k], hw.p2, B, H2, H2, e2));
+            e2.moments = bn_partial;
+            MGT_TRY(bn_fused ? GemmForward<Epi::kBiasF32Moments>(e, st, r1_h(k), ws.p_act, hw.w2[k], hw.p2, B, H2, H2, e2)
+                             : GemmForward<Epi::kBiasF32>(e, st, r1_h(k), ws.p_act, hw.w2[k], hw.p2, B, H2, H2, e2));
             MGT_TRY(bn_forward(k + 1U));
             continue;
         }
@@ -1919,15 +1929,14 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     }
     for (uint32_t rb = R; rb > 0 && !chain; --rb) {
         const uint32_t k = rb - 1U;
-        if (bnorm) MGT_TRY(bn_backward(k + 1U, grad + Fc2B(s, k)));  // dz_tape(k + 1) = gradient w.r.t. the fc2 output; dzf goes down the skip path as it is
+        if (bnorm) MGT_TRY(bn_backward(k + 1U));  // dz_tape(k + 1) = gradient w.r.t. the fc2 output; dzf goes down the skip path as it is
         GemmArgs d2{};  // dz1 = (dz2 * W2^T) * [r1 > 0]
         d2.mask = r1_h(k); d2.ld_mask = ws.p_act; d2.out_f16 = dz1_tape(k); d2.ld_f16 = ws.p_dz;
         MGT_TRY(GemmBackpropInput<Epi::kMaskF16>(e, st, dz_tape(k + 1), ws.p_dz, hw.w2[k], hw.p2, B, H2, H2, d2, colsum + ws.colsum_slot_floats * k));
         GemmArgs d1{};  // next dz = (dz1 * W1^T + dz2) * [x_k > 0]: ReLU of the previous block (or of the hidden layer)
         d1.add_f32 = dzf; d1.ld_add = ws.p_f32; d1.out_f32 = dzf; d1.ld_f32 = ws.p_f32; d1.mask = x_h(k); d1.ld_mask = ws.p_act;
         d1.out_f16 = dz_tape(k); d1.ld_f16 = ws.p_dz;
-        MGT_TRY(GemmBackpropInput<Epi::kAddMaskF32F16>(e, st, dz1_tape(k), ws.p_dz, hw.w1[k], hw.p2, B, H2, H2, d1,
-                                                        colsum + ws.colsum_slot_floats * (R + k)));
+        MGT_TRY(GemmBackpropInput<Epi::kAddMaskF32F16>(e, st, dz1_tape(k), ws.p_dz, hw.w1[k], hw.p2, B, H2, H2, d1, colsum + ws.colsum_slot_floats * (R + k)));
     }
     if (!timer.Mark(profile ? &profile->residual_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
 
@@ -1938,7 +1947,13 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
 
     // ---- hidden layer backward, dX part (mlp_backward.cu:1417-1438): dz_tape(0) = dcur * [x0 > 0]
     dz_cur = dz_tape(0);
-    if (bnorm) MGT_TRY(bn_backward(0, grad + HiddenBias(s)));
+    if (bnorm) {
+        MGT_TRY(bn_backward(0));
+        // the gradients of the biases in front of the normalisations, of all layers
+        sums.Rows(bn_bias(0), bn_blocks, H2, H2, grad + HiddenBias(s));
+        sums.Rows(bn_bias(1), bn_blocks, H2, H2, grad + Fc2B(s, 0), R, (uint64_t)bn::kMaxBlocks * H2, BlockParams(s));
+        MGT_TRY(sums.Pass(st));
+    }
     // Small batches: the weight gradients run beside the dX products and the embedding gradient, on the second stream. Neither
     // branch fills the SMs there (the dX product has fewer than two tiles an SM), and every launch is a gap: 9 001 samples of
     // hd1 1000, hd2 200, 8 blocks 510 -> 453 us a step, 1 024 of hd1 256, hd2 64, 2 blocks 134 -> 114, 64 of hd1 8, hd2 8

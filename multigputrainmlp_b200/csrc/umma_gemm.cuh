@@ -32,6 +32,7 @@ enum class Epi : int {
     kAddMaskF32F16,        // v = (acc + add) * [mask > 0]; out_f32 = v (may alias add); out_f16 = v
     kPartialF32,           // partial[split][m][n] = acc
     kBiasF32,              // out_f32 = acc + bias                 (a pre-activation kept in fp32: input of batch normalisation)
+    kBiasF32Moments,       // the same, with the sums and the sums of squares of its columns in `moments`
     kMaskRowsumF16,        // out_f16[m][n] = acc * [bit n of bits[m]]; rowsum[(n tile, warp of the quadrant)][m] = sum over the warp's columns
     kMaskRowsumF32,        // the same values unrounded and transposed: out_f32[n][m] (the lanes of a warp write 32 neighbouring columns of one row)
     kMaskRowsumF16T,       // ... in the operand format: out_f16[n][m]
@@ -55,6 +56,9 @@ struct GemmArgs {
     // (bias gradients): row (blockIdx.x * 8 + epilogue warp) of colsum[gridDim.x * 8][N] accumulates
     // what that warp handled. The buffer must be zero before the launch.
     float* colsum;
+    // kBiasF32Moments: row (blockIdx.x * 4 + TMEM lane quadrant) of moments[gridDim.x * 4][2][N] gets what the quadrant's warps
+    // handled; one N tile, every slot of a launch is written (no zeroing needed)
+    float* moments;
     // kMaskRowsumF16: fp32 row sums of the masked values, one partial row of M floats per (N tile, warp of a lane quadrant):
     // rowsum[(n_tile * EPI_WARPS / 4 + w)][m]; every slot of a launch is written (no zeroing needed)
     float* rowsum;
@@ -91,9 +95,10 @@ struct GemmCfg {
     static constexpr int EPI_STRIDE = EPI_WARPS_ / 4;  // ... and take every EPI_STRIDE-th 32-column chunk
     static constexpr int THREADS = 64 + 32 * EPI_WARPS;
     static constexpr int EPI_TILE_PITCH = 36;
-    // per epilogue warp: a padded 32x32 fp32 tile, 32 words of ReLU-mask bits and four rows of column-sum accumulators
+    static constexpr bool MOMENTS = EPI_ == Epi::kBiasF32Moments;
+    // per epilogue warp: a padded 32x32 fp32 tile, 32 words of ReLU-mask bits and four rows of column-sum accumulators (eight for moments)
     // (the row-sum epilogues write from registers and need no staging)
-    static constexpr int EPI_WARP_BYTES = (EPI_ == Epi::kMaskRowsumF16 || EPI_ == Epi::kMaskRowsumF32 || EPI_ == Epi::kMaskRowsumF16T) ? 0 : (32 * EPI_TILE_PITCH * 4 + 128 + 4 * 32 * 4);
+    static constexpr int EPI_WARP_BYTES = (EPI_ == Epi::kMaskRowsumF16 || EPI_ == Epi::kMaskRowsumF32 || EPI_ == Epi::kMaskRowsumF16T) ? 0 : (32 * EPI_TILE_PITCH * 4 + 128 + (MOMENTS ? 8 : 4) * 32 * 4);
     static constexpr int EPI_STAGE_BYTES = EPI_WARPS * EPI_WARP_BYTES;
     static constexpr int SMEM_BYTES = 1024 + SA_ * A_STAGE_BYTES + SB_ * B_STAGE_BYTES + 256 + EPI_STAGE_BYTES;
     static_assert(BN_ % 16 == 0 && BN_ >= 16 && BN_ <= 256, "UMMA N");
@@ -366,7 +371,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             // instruction. The global operands of a chunk (residual/skip values, ReLU mask source, bias) are
             // requested one chunk ahead - for the first chunk of a tile before the tile's MMAs have even finished -
             // so their latency is off the critical path. Ragged shapes take a scalar form without prefetch.
-            constexpr bool kPlainF32 = Cfg::EPI == Epi::kBiasF32;  // fp32 out only: no ReLU, no 16-bit copy
+            constexpr bool kPlainF32 = Cfg::EPI == Epi::kBiasF32 || Cfg::MOMENTS;  // fp32 out only: no ReLU, no 16-bit copy
             constexpr bool kHasBias = Cfg::EPI == Epi::kBiasReluF16 || Cfg::EPI == Epi::kBiasReluF32F16 || Cfg::EPI == Epi::kBiasResReluF32F16 || kPlainF32;
             constexpr bool kHasAdd = Cfg::EPI == Epi::kBiasResReluF32F16 || Cfg::EPI == Epi::kAddMaskF32F16;
             constexpr bool kHasMask = Cfg::EPI == Epi::kMaskF16 || Cfg::EPI == Epi::kAddMaskF32F16;
@@ -380,9 +385,9 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
             // read-modify-write per chunk
             float* col_acc = reinterpret_cast<float*>(mask_words + 32);
             constexpr bool kColsumLocal = Cfg::BSTAT && kHasMask && BN / (32 * Cfg::EPI_STRIDE) <= 4;
-            if (kColsumLocal) {
+            if (kColsumLocal || Cfg::MOMENTS) {
 #pragma unroll
-                for (int i = 0; i < 4; ++i) col_acc[i * 32 + lane] = 0.0f;
+                for (int i = 0; i < (Cfg::MOMENTS ? 8 : 4); ++i) col_acc[i * 32 + lane] = 0.0f;
                 __syncwarp();
             }
             const uint32_t r4 = lane >> 3, c4 = (lane & 7U) * 4U;  // fp32 vectors: 4 rows x 8 lanes
@@ -540,6 +545,17 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                                 if (col_ok) reinterpret_cast<uint16_t*>(args.out_f16)[static_cast<uint64_t>(m_base + rr) * args.ld_f16 + n0 + lane] = to_operand(tile[rr * TP + lane], args.bf16 != 0U);
                         }
                     }
+                    if constexpr (Cfg::MOMENTS) {
+                        float s1 = 0.0f, s2 = 0.0f;  // column `lane` of the staged tile, rows in order
+#pragma unroll 8
+                        for (uint32_t rr = 0; rr < 32U; ++rr) {
+                            const float x = rr < rows_ok ? tile[rr * TP + lane] : 0.0f;
+                            s1 += x;
+                            s2 += x * x;
+                        }
+                        col_acc[(cc / Cfg::EPI_STRIDE) * 64 + lane] += s1;  // this lane is the only user of the slots
+                        col_acc[(cc / Cfg::EPI_STRIDE) * 64 + 32 + lane] += s2;
+                    }
                     if constexpr (kHasMask) {
                         if (args.colsum != nullptr) {
                             float total = 0.0f;  // column `lane` of the staged tile, rows in order
@@ -557,6 +573,16 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                 }
                 tc_fence_before();
                 mbar_arrive(&acc_empty[ab]);
+            }
+            if (Cfg::MOMENTS) {
+                float* row = args.moments + (static_cast<uint64_t>(blockIdx.x) * 4U + quad) * 2U * args.N;
+                for (int cc = static_cast<int>(chunk_parity); cc < BN / 32; cc += Cfg::EPI_STRIDE) {
+                    const uint32_t n = cc * 32 + lane;
+                    if (n < args.N) {
+                        row[n] = col_acc[(cc / Cfg::EPI_STRIDE) * 64 + lane];
+                        row[args.N + n] = col_acc[(cc / Cfg::EPI_STRIDE) * 64 + 32 + lane];
+                    }
+                }
             }
             if (kColsumLocal && args.colsum != nullptr && blockIdx.x < total_units) {
                 const uint32_t nt = blockIdx.x % args.n_tiles;  // the N tile of every unit of this CTA

@@ -117,6 +117,8 @@ CASES = [
     ((6, 8, 9, 7, 2, 11), 40, False, False, True),
     ((72, 72, 96, 224, 2, 29), 300, True, True, False),       # bfloat16 + cross-entropy
     ((72, 72, 64, 32, 0, 1), 128, False, False, False),       # no residual blocks: the hidden layer's normalisation alone
+    ((6, 8, 32, 256, 1, 1), 300, False, False, True),         # the widest layer whose GEMM leaves the moments of its columns
+    ((6, 8, 32, 264, 1, 1), 300, False, False, True),         # ... and one that is wider
 ]
 
 
