@@ -15,6 +15,7 @@
 #include "batch_norm.cuh"
 #include "embedding_gather.cuh"
 #include "fp32_path.cuh"
+#include "fp32_tower.cuh"
 #include "onehot_pair.cuh"
 #include "tower_chain.cuh"
 #include "tower_wide.cuh"
@@ -1368,8 +1369,13 @@ mgt_status_t LaunchChain(mgt_engine* e, LaunchOn st, const __half* w_first, uint
 // gradients of all blocks are two grouped products at the end. Rows are padded to four floats.
 struct Fp32Workspace {
     uint32_t p1, p2;
-    uint64_t a1, x, r1, dz2, dz1t, dz1, dy, head, partial, partial_fc2, partial_fc1, partial_out, colsum, colsum_slot, colsum_in, lists, total;  // float offsets
+    uint64_t a1, x, r1, dz2, dz1t, dz1, dy, head, partial, partial_fc2, partial_fc1, partial_out, colsum, colsum_slot, colsum_in, bits, bits_entry, tower_w, lists, total;  // float offsets
 };
+// The blocks in one launch per direction (fp32_tower.cuh): widths up to 128, up to 256 with 4 096 samples. A CTA streams every matrix
+// through one warp, which is the longest part of wide ones with few samples to a CTA (ms a step, by layers and fused: 64 samples of
+// hd2 256, 10 blocks 0.57, 0.80; 1 500 of hd2 161, 31 blocks 1.95, 2.17; 2 500 of hd2 510, 8 blocks 3.26, 4.33; but 2 000 of hd2 128, 30
+// blocks 1.44, 1.30; 20 000 of hd2 240, 5 blocks 4.09, 3.71; 30 000 of hd2 18, 20 blocks 1.75, 1.24; 300 of hd2 8, 32 blocks 0.90, 0.20).
+bool FusedFp32Tower(const mgt_mlp_shape_t& s, uint32_t B) { return s.residual_blocks > 0 && (s.hd2 <= 128U || (s.hd2 <= 256U && B >= 4096U)); }
 struct DwPlan {
     fp32path::SgemmTile tile;
     uint32_t splits;
@@ -1404,9 +1410,13 @@ Fp32Workspace PlanFp32(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm) {
     w.partial_fc2 = take(planes(s.hd2, s.hd2, (uint32_t)r));
     w.partial_fc1 = take(planes(s.hd2, s.hd2, (uint32_t)r));
     w.partial_out = take(s.output_dim > 1 ? planes(s.hd2, s.output_dim, 1) : 0);
-    w.colsum_slot = (uint64_t)((B + 31U) / 32U) * s.hd2;  // one row per tile of at least 32 samples
+    const bool fused = FusedFp32Tower(s, B);
+    w.colsum_slot = (fused ? fp32path::TowerSumRows(B) : (uint64_t)((B + 31U) / 32U)) * s.hd2;  // one row per tile of at least 32 samples, 8 in the tower
     w.colsum = take(w.colsum_slot * 2 * r);
     w.colsum_in = take((uint64_t)((B + 31U) / 32U) * s.hd1);
+    w.bits_entry = fp32path::TowerBitWords(B, s.hd2);
+    w.bits = take(fused ? w.bits_entry * 2 * r : 0);
+    w.tower_w = take(fused ? 2 * r * (uint64_t)w.p2 * w.p2 : 0);  // (the tower's matrices padded, where it cannot take them as they lie)
     w.lists = take(gather::ListWords(B, s.state_len, s.state_value_pad));
     w.total = off + 64;
     return w;
@@ -1430,6 +1440,17 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
     float *dy = base + ws.dy, *dz1 = base + ws.dz1, *colsum = base + ws.colsum;
     const SgemmTile tile_h2 = PickSgemmTile(B, H2, 1, sm), tile_h1 = PickSgemmTile(B, H1, 1, sm);
     const uint32_t rows_h2 = (B + SgemmTileRows(tile_h2) - 1U) / SgemmTileRows(tile_h2), rows_h1 = (B + SgemmTileRows(tile_h1) - 1U) / SgemmTileRows(tile_h1);
+    const bool fused = FusedFp32Tower(s, B);
+    const TowerPlan tower = fused ? PlanTower(B, H2, sm) : TowerPlan{};
+    TowerArgs tower_args{};
+    tower_args.B = B; tower_args.H = H2; tower_args.R = R; tower_args.pitch = p2;
+    tower_args.w = w + Fc1W(s, 0); tower_args.ld_w = H2; tower_args.w_step = BlockParams(s) / 2;
+    tower_args.bias = w + Fc1B(s, 0); tower_args.bias_step = BlockParams(s) / 2;
+    const bool pad_tower = fused && ((H2 & 3U) != 0U || (reinterpret_cast<uintptr_t>(tower_args.w) & 15U) != 0U);
+    if (pad_tower) { tower_args.w = base + ws.tower_w; tower_args.ld_w = p2; tower_args.w_step = (uint64_t)p2 * p2; }
+    tower_args.tape_stride = bh2;
+    tower_args.bits = reinterpret_cast<uint32_t*>(base + ws.bits); tower_args.entry_stride = ws.bits_entry;
+    tower_args.status = e->status_word;
     auto ok = [&]() { return cudaGetLastError() == cudaSuccess; };
     // out[B x N] = act[B x K] W[K x N] + bias, ReLU (with the residual added before it)
     auto forward = [&](const float* act, uint32_t ld_act, uint32_t K, const float* weight, const float* bias, const float* res, float* out) {
@@ -1463,12 +1484,22 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
     StageTimer timer{e, st, profile};
     if (!timer.Start()) return MGT_CUDA_FAILURE;
 
+    if (pad_tower) {
+        Launch(PadMatricesKernel, dim3((p2 + 7U) / 8U, 2U * R), 256, 0, st, w + Fc1W(s, 0), BlockParams(s) / 2, H2, p2, base + ws.tower_w);
+        ++e->launches;
+    }
     if (EmbeddingForward(st, states, w, w + InputBias(s), B, L, V, H1, a1, p1, sm) != cudaSuccess) return MGT_CUDA_FAILURE;
     ++e->launches;
     if (!timer.Mark(profile ? &profile->input_forward_ms : nullptr)) return MGT_CUDA_FAILURE;
     if (!forward(a1, p1, H1, w + HiddenWeight(s), w + HiddenBias(s), nullptr, x(0))) return MGT_CUDA_FAILURE;
     if (!timer.Mark(profile ? &profile->hidden_forward_ms : nullptr)) return MGT_CUDA_FAILURE;
-    for (uint32_t k = 0; k < R; ++k) {
+    if (fused) {
+        TowerArgs t = tower_args;
+        t.state_tape = x(0); t.inner_tape = r1(0);
+        if (LaunchTower<false>(e->device, st, tower, t) != cudaSuccess) return MGT_CUDA_FAILURE;
+        ++e->launches;
+    }
+    for (uint32_t k = 0; k < R && !fused; ++k) {
         if (!forward(x(k), p2, H2, w + Fc1W(s, k), w + Fc1B(s, k), nullptr, r1(k)) || !forward(r1(k), p2, H2, w + Fc2W(s, k), w + Fc2B(s, k), x(k), x(k + 1U))) return MGT_CUDA_FAILURE;
     }
     if (!timer.Mark(profile ? &profile->residual_forward_ms : nullptr)) return MGT_CUDA_FAILURE;
@@ -1489,7 +1520,13 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
     MGT_TRY(notify(OutputWeight(s), (uint64_t)H2 * OUT + OUT));
     if (!timer.Mark(profile ? &profile->output_ms : nullptr)) return MGT_CUDA_FAILURE;
     // input gradients down the tower and through the hidden layer
-    for (uint32_t rb = R; rb > 0; --rb) {
+    if (fused) {
+        TowerArgs t = tower_args;
+        t.state_tape = dz2(0); t.inner_tape = dz1t(0); t.colsum = colsum; t.colsum_slot = ws.colsum_slot;
+        if (LaunchTower<true>(e->device, st, tower, t) != cudaSuccess) return MGT_CUDA_FAILURE;
+        ++e->launches;
+    }
+    for (uint32_t rb = R; rb > 0 && !fused; --rb) {
         const uint32_t k = rb - 1U;
         if (!backward(dz2(k + 1U), w + Fc2W(s, k), H2, nullptr, r1(k), p2, dz1t(k), colsum + ws.colsum_slot * k, tile_h2) ||
             !backward(dz1t(k), w + Fc1W(s, k), H2, dz2(k + 1U), x(k), p2, dz2(k), colsum + ws.colsum_slot * (R + k), tile_h2)) return MGT_CUDA_FAILURE;
@@ -1499,7 +1536,7 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
     if (R > 0) {
         if (!weight_grad(r1(0), p2, bh2, H2, dz2(1), p2, bh2, H2, R, base + ws.partial_fc2, grad + Fc2W(s, 0), BlockParams(s)) ||
             !weight_grad(x(0), p2, bh2, H2, dz1t(0), p2, bh2, H2, R, base + ws.partial_fc1, grad + Fc1W(s, 0), BlockParams(s))) return MGT_CUDA_FAILURE;
-        sums.TowerBiases(s, colsum, rows_h2, ws.colsum_slot, grad, true);
+        sums.TowerBiases(s, colsum, fused ? tower.tiles : rows_h2, ws.colsum_slot, grad, true);
         MGT_TRY(sums.Pass(st));
         for (uint32_t rb = R; rb > 0; --rb) {
             MGT_TRY(notify(Fc2W(s, rb - 1U), (uint64_t)H2 * H2 + H2));
@@ -1531,7 +1568,8 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
 // 4 096 samples of hd1 1024 210 -> 200 us, 5 003 of hd1 333 172 -> 157, 1 024 of hd1 256 103 -> 82; 3 001 samples of hd1 2560 make no
 // difference, and with kernels that fill the chip the next one's CTAs are in the way: 9 001 samples of hd1 1000 445 -> 491, 8 192 of
 // hd1 2560 in fp32 4 701 -> 5 230. The many passes of batch normalisation stream and gain at any size (53 248 of hd1 2560 5 884 -> 5 510).
-bool OverlapLaunches(const mgt_mlp_shape_t& s, uint32_t B, bool batch_norm) { return batch_norm || (uint64_t)B * s.hd1 <= 6000000ULL; }
+// The fp32 products fill the chip sooner: 3 000 samples of hd1 1001, hd2 301 2 427 -> 2 997 us, 1 024 of hd1 256, hd2 64 175 -> 148.
+bool OverlapLaunches(const mgt_mlp_shape_t& s, uint32_t B, bool batch_norm, bool fp32) { return batch_norm || (uint64_t)B * s.hd1 <= (fp32 ? 1000000ULL : 6000000ULL); }
 
 struct HalfWeights {
     const __half* in_table; uint32_t p1;     // [(IN+1)][p1], row IN is the input bias
@@ -1693,12 +1731,12 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
             return ready(ready_user, id++, off, count, stream_v) == MGT_OK ? MGT_OK : MGT_CUDA_FAILURE;
         };
         return LaunchFp32Path(e, s, w, reinterpret_cast<const uint8_t*>(states), labels, B, loss, grad, workspace, half_ig != 0, ready != nullptr || profile != nullptr, profile, tell,
-                              {static_cast<cudaStream_t>(stream_v), OverlapLaunches(s, B, false)});
+                              {static_cast<cudaStream_t>(stream_v), OverlapLaunches(s, B, false, true)});
     }
     Workspace ws = PlanWorkspace(s, B, PlanSmCount(e->sm_count), half_ig != 0, bnorm);
     if (e->embedding_form != mgt_engine::kBySize) ws.gather_fwd = ws.gather_grad = e->embedding_form == mgt_engine::kGather;
     if (workspace_floats < (ws.total_bytes + 3) / 4 + (half_ig ? 0 : Fp32TableFloats(s, B))) return MGT_CAPACITY_EXCEEDED;
-    const LaunchOn st(static_cast<cudaStream_t>(stream_v), OverlapLaunches(s, B, bnorm));
+    const LaunchOn st(static_cast<cudaStream_t>(stream_v), OverlapLaunches(s, B, bnorm, false));
     uint8_t* base = reinterpret_cast<uint8_t*>(RoundUp(reinterpret_cast<uintptr_t>(workspace), 1024));
     float* dz1_f32 = reinterpret_cast<float*>(RoundUp(reinterpret_cast<uintptr_t>(workspace + (ws.total_bytes + 3) / 4), 256));  // behind the tensor-core workspace
     const uint32_t p_dz1_f32 = (uint32_t)RoundUp(s.hd1, 4);

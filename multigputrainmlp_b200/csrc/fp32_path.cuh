@@ -21,7 +21,7 @@ namespace fp32path {
 //   TA = false: A is [M][lda] (K contiguous)     TA = true: A is [K][lda] (M contiguous)
 //   TB = false: B is [K][ldb] (N contiguous)     TB = true: B is [N][ldb] (K contiguous)
 // blockIdx.z = group * splits + split: groups are equal problems `stride_*` floats apart, splits share K. With splits > 1
-// the result is a plane of partial sums, added up in order by ReducePartialsGroupedKernel; otherwise the epilogue applies,
+// the result is a plane of partial sums, added up in order with the sums of the step; otherwise the epilogue applies,
 // each step optional:   v = relu((acc + bias[n] + add[m][n])) * [mask[m][n] > 0]   and column sums of v per tile row.
 struct SgemmArgs {
     const float* A;

@@ -114,6 +114,14 @@ def test_fp32_linears_over_tiles(oracle, dims, n):
     loss_grad_case(oracle, dims, n, flags=(False, False), tol=1e-5, section_tol=2e-5)
 
 
+# The fp32 tower as it is cut for different batches and widths: 32, 64, 128, 224 and 256 columns a warp, one to four warps side by
+# side, stages of 8 to 32, ends of tiles, matrices that have to be padded; and layer by layer. The oracle adds the samples one after the other in
+# fp32, each sum to n 2^-24 of its terms at worst.
+@pytest.mark.parametrize("hd2,n", [(224, 8201), (250, 8190), (96, 16390), (128, 2999), (117, 1021), (16, 40001), (200, 1021), (301, 700), (9, 64)])
+def test_fp32_tower_cuts(oracle, hd2, n):
+    loss_grad_case(oracle, (6, 4, 16, hd2, 1, 1), n, flags=(False, False), tol=1e-5 + n * 2.0 ** -24, section_tol=2e-5 + n * 2.0 ** -24)
+
+
 def multiply_in_order(x, w):
     """x w in fp32, one multiply-add after the other along k (the product of two floats is exact in double)."""
     acc = np.zeros((x.shape[0], w.shape[1]), np.float32)
