@@ -102,12 +102,6 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* map, int
         ::"r"(ptx::smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(x), "r"(y)
         : "memory");
 }
-// 2-D tiled TMA store from this CTA's shared memory (bulk-group completion); what lies outside the tensor is clipped
-__device__ __forceinline__ void tma_store_2d(const void* map, const void* smem_src, int32_t x, int32_t y) {
-    asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%2, %3}], [%1];"
-                 ::"l"(reinterpret_cast<uint64_t>(map)), "r"(ptx::smem_u32(smem_src)), "r"(x), "r"(y)
-                 : "memory");
-}
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_holder, uint32_t columns) {
     asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(ptx::smem_u32(smem_holder)), "r"(columns) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
@@ -343,7 +337,7 @@ onehot_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_const
                         fence_proxy_async_smem();
                         __syncwarp();
                         if (lane == 0) {
-                            pair::tma_store_2d(&tma_out, tile, static_cast<int32_t>(at), static_cast<int32_t>(p.mt * 256U + rank * 128U + quad * 32U));
+                            tma_store_2d(&tma_out, tile, static_cast<int32_t>(at), static_cast<int32_t>(p.mt * 256U + rank * 128U + quad * 32U));
                             bulk_commit_group();
                         }
                     }

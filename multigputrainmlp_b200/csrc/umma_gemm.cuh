@@ -34,6 +34,7 @@ enum class Epi : int {
     kBiasF32,              // out_f32 = acc + bias                 (a pre-activation kept in fp32: input of batch normalisation)
     kBiasF32Moments,       // the same, with the sums and the sums of squares of its columns in `moments`
     kMaskRowsumF16,        // out_f16[m][n] = acc * [bit n of bits[m]]; rowsum[(n tile, warp of the quadrant)][m] = sum over the warp's columns
+    kMaskRowsumF16Tma,     // the same result by TMA stores through shared memory
     kMaskRowsumF32,        // the same values unrounded and transposed: out_f32[n][m] (the lanes of a warp write 32 neighbouring columns of one row)
     kMaskRowsumF16T,       // ... in the operand format: out_f16[n][m]
 };
@@ -97,10 +98,12 @@ struct GemmCfg {
     static constexpr int EPI_TILE_PITCH = 36;
     static constexpr bool MOMENTS = EPI_ == Epi::kBiasF32Moments;
     // per epilogue warp: a padded 32x32 fp32 tile, 32 words of ReLU-mask bits and four rows of column-sum accumulators (eight for moments)
-    // (the row-sum epilogues write from registers and need no staging)
-    static constexpr int EPI_WARP_BYTES = (EPI_ == Epi::kMaskRowsumF16 || EPI_ == Epi::kMaskRowsumF32 || EPI_ == Epi::kMaskRowsumF16T) ? 0 : (32 * EPI_TILE_PITCH * 4 + 128 + (MOMENTS ? 8 : 4) * 32 * 4);
+    // (the row-sum epilogues without TMA stores write from registers and need no staging)
+    static constexpr bool TMA_OUT = EPI_ == Epi::kMaskRowsumF16Tma;  // two 32 x 32 tiles of the output per epilogue warp
+    static constexpr int EPI_OFFSET = TMA_OUT ? 1024 : 256;          // behind the barriers; a swizzled tile starts on 512 bytes
+    static constexpr int EPI_WARP_BYTES = TMA_OUT ? 2 * 2048 : (EPI_ == Epi::kMaskRowsumF16 || EPI_ == Epi::kMaskRowsumF32 || EPI_ == Epi::kMaskRowsumF16T) ? 0 : (32 * EPI_TILE_PITCH * 4 + 128 + (MOMENTS ? 8 : 4) * 32 * 4);
     static constexpr int EPI_STAGE_BYTES = EPI_WARPS * EPI_WARP_BYTES;
-    static constexpr int SMEM_BYTES = 1024 + SA_ * A_STAGE_BYTES + SB_ * B_STAGE_BYTES + 256 + EPI_STAGE_BYTES;
+    static constexpr int SMEM_BYTES = 1024 + SA_ * A_STAGE_BYTES + SB_ * B_STAGE_BYTES + EPI_OFFSET + EPI_STAGE_BYTES;
     static_assert(BN_ % 16 == 0 && BN_ >= 16 && BN_ <= 256, "UMMA N");
     static_assert(BN_ % 32 == 0, "epilogue drains 32 columns at a time");
     static_assert(EPI_WARPS_ == 8 || EPI_WARPS_ == 16, "epilogue warps");
@@ -111,7 +114,7 @@ struct GemmCfg {
 
 template <class Cfg>
 __global__ void __launch_bounds__(Cfg::THREADS, 1)
-umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const GemmArgs args) {
+umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const __grid_constant__ CUtensorMap tma_out, const GemmArgs args) {
     using namespace ptx;
     constexpr int BM = Cfg::BM, BN = Cfg::BN, SA = Cfg::SA, SB = Cfg::SB;
     // equal rings of A and B advance together: one barrier pair a stage
@@ -133,7 +136,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     uint64_t* acc_empty = acc_full + ACC_BUFS;
     uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_empty + ACC_BUFS);
     volatile int* cta_abort = reinterpret_cast<volatile int*>(tmem_holder + 1);
-    float* epi_stage = reinterpret_cast<float*>(b_ring + SB * Cfg::B_STAGE_BYTES + 256);
+    float* epi_stage = reinterpret_cast<float*>(b_ring + SB * Cfg::B_STAGE_BYTES + Cfg::EPI_OFFSET);
 
     const uint32_t warp = threadIdx.x >> 5;
     const uint32_t lane = threadIdx.x & 31U;
@@ -157,6 +160,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         fence_barrier_init();
         prefetch_tensormap(&tma_a);
         prefetch_tensormap(&tma_b);
+        if (Cfg::TMA_OUT) prefetch_tensormap(&tma_out);
     }
     if (warp == 1) {
         tmem_alloc(tmem_holder, 512);
@@ -285,11 +289,17 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         const uint32_t chunk_parity = ew >> 2;
         uint32_t unit_iter = 0;
         bool ok = true;
-        if constexpr (Cfg::EPI == Epi::kMaskRowsumF16 || Cfg::EPI == Epi::kMaskRowsumF32 || Cfg::EPI == Epi::kMaskRowsumF16T) {
+        if constexpr (Cfg::TMA_OUT || Cfg::EPI == Epi::kMaskRowsumF16 || Cfg::EPI == Epi::kMaskRowsumF32 || Cfg::EPI == Epi::kMaskRowsumF16T) {
             // D and the output have a row per TMEM lane and the warp's 32 columns side by side in that row: 64 bytes per lane,
             // written as four 16-byte vectors straight from registers; the mask of a chunk is one word per lane; the row
             // sum is a sum over the lane's own registers. (Full 32-byte sectors; whole rows per warp are not needed.)
+            // TMA_OUT: a warp turns 32 rows x 32 columns into the operand format in a shared-memory tile of its own and a TMA store writes it,
+            // while the next chunk goes into the other tile: a lane storing its 64 bytes straight from registers touches 32 lines per
+            // instruction, and the load/store unit then bounds a CTA with more than one unit (a step of p888 at 53 248 samples
+            // 3 044 -> 2 999 us, with batch normalisation 5 463 -> 5 395).
             const bool vec_ok = (args.ld_f16 & 7U) == 0U;
+            [[maybe_unused]] uint8_t* tiles = reinterpret_cast<uint8_t*>(epi_stage) + ew * Cfg::EPI_WARP_BYTES;
+            [[maybe_unused]] uint32_t stores = 0;
             constexpr int CPW = (BN / 32 + Cfg::EPI_STRIDE - 1) / Cfg::EPI_STRIDE;  // chunks of a unit per warp
             // the mask words of a unit do not depend on its MMAs: those of the NEXT unit are requested while this one is drained
             auto request = [&](uint32_t unit, uint32_t (&words)[CPW]) {
@@ -341,6 +351,27 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                                 else reinterpret_cast<uint16_t*>(args.out_f16)[static_cast<uint64_t>(n0 + j) * args.ld_f16 + m] = to_operand(v[j], args.bf16 != 0U);
                             }
                         }
+                    } else if (Cfg::TMA_OUT) {
+                        // (rows past M and columns past N are outside the map)
+                        uint8_t* tile = tiles + (stores & 1U) * 2048U;
+                        if (lane == 0) bulk_wait_read_but_one();  // the store before last has read this tile
+                        __syncwarp();
+#pragma unroll
+                        for (uint32_t q = 0; q < 4U; ++q) {
+                            uint4 u;
+                            u.x = pack_operand_pair(v[8 * q + 0], v[8 * q + 1], args.bf16 != 0U);
+                            u.y = pack_operand_pair(v[8 * q + 2], v[8 * q + 3], args.bf16 != 0U);
+                            u.z = pack_operand_pair(v[8 * q + 4], v[8 * q + 5], args.bf16 != 0U);
+                            u.w = pack_operand_pair(v[8 * q + 6], v[8 * q + 7], args.bf16 != 0U);
+                            *reinterpret_cast<uint4*>(tile + lane * 64U + ((q ^ ((lane >> 1) & 3U)) << 4)) = u;  // 64-byte swizzle
+                        }
+                        fence_proxy_async_smem();
+                        __syncwarp();
+                        if (lane == 0) {
+                            tma_store_2d(&tma_out, tile, static_cast<int32_t>(n0), static_cast<int32_t>(mt * BM + quad * 32U));
+                            bulk_commit_group();
+                        }
+                        ++stores;
                     } else if (m_ok) {
                         uint16_t* dst = reinterpret_cast<uint16_t*>(args.out_f16) + static_cast<uint64_t>(m) * args.ld_f16 + n0;
                         if (vec) {
@@ -364,6 +395,7 @@ umma_gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
                 tc_fence_before();
                 mbar_arrive(&acc_empty[ab]);
             }
+            if (Cfg::TMA_OUT && lane == 0) bulk_wait_all();  // the stores read this CTA's shared memory until they complete
         } else {
             // Row-major tensors: a TMEM lane holds one row, but global memory wants a warp on whole rows. Each warp
             // stages operands and results through its own padded 32x32 fp32 tile in shared memory, so that every

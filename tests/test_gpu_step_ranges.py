@@ -295,6 +295,13 @@ def test_wide_residual_tower(oracle, hd2, n, mirror, bf16):
                    section_tol=2e-2 if bf16 else 3e-3)
 
 
+# The hidden layer's input gradient by TMA stores (more tiles than SMs): ragged last rows and columns, one to four K chunks
+@pytest.mark.parametrize("hd1,hd2,n", [(1000, 64, 10001), (300, 129, 25700)])
+def test_hidden_input_gradient_stores(oracle, monkeypatch, hd1, hd2, n):
+    monkeypatch.setenv("MGT_EMBEDDING_FORM", "onehot")
+    loss_grad_case(oracle, (8, 8, hd1, hd2, 1, 1), n, mirror=False)
+
+
 # weight gradients on the second stream beside the table gradient, by gathering (its sort on that stream too) and by the one-hot
 # product; the last call of a case runs on one stream and has to give the same bits
 @pytest.mark.parametrize("dims,n", [((72, 72, 896, 40, 2, 1), 96), ((72, 72, 897, 40, 2, 1), 96), ((54, 6, 1024, 64, 1, 3), 513), ((72, 72, 1032, 33, 0, 1), 257)])
