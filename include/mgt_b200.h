@@ -341,6 +341,13 @@ mgt_status_t mgt_debug_gemm(mgt_engine_t* engine, const uint16_t* a, uint32_t ld
                             const uint16_t* b, uint32_t ldb, int32_t b_mn_major, float* d, uint32_t m, uint32_t n,
                             uint32_t k, uint32_t splits, float* partial_scratch, void* stream);
 
+/* `jobs` sums over partial results through the kernel that ends a training step, for the parity tests:
+ * dst[j][i] = src[j][0][i] + ... + src[j][terms - 1][i], i < items. planes: summed in order, one item (or four
+ * neighbours, where items and both addresses are multiples of four floats) a thread; else by 32 lanes, each
+ * adding every 32nd term in order, and the lanes then in order. No counterpart in the reference. */
+mgt_status_t mgt_debug_sums(mgt_engine_t* engine, const float* src, uint32_t terms, uint32_t items, uint32_t jobs,
+                            int32_t planes, float* dst, void* stream);
+
 /* Split-K GEMM that allocates nothing. No counterpart in the reference.
  *
  * Same computation and arguments as mgt_debug_gemm, for callers that cannot obtain device memory

@@ -50,4 +50,5 @@ def _declare(lib: C.CDLL) -> None:
     lib.mgt_launch_adamw.argtypes = [vp, vp, vp, vp, vp, vp]
     lib.mgt_launch_adamw_with_half_mirror.argtypes = [vp, vp, vp, vp, vp, vp, vp]
     lib.mgt_launch_float_to_half.argtypes = [vp, u64, vp, vp]
+    lib.mgt_debug_sums.argtypes = [vp, vp, u32, u32, u32, i32, vp, vp]
     lib.mgt_debug_gemm.argtypes = [vp, vp, u32, i32, vp, u32, i32, vp, u32, u32, u32, u32, vp, vp]

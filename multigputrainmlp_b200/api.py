@@ -265,6 +265,9 @@ class Engine:
         return int(self._lib.mgt_debug_gemm(self.handle, _ptr(a), lda, int(a_mn_major), _ptr(b), ldb, int(b_mn_major), _ptr(d),
                                             m, n, k, splits, _ptr(partial), _stream(stream)))
 
+    def debug_sums(self, src, terms, items, jobs, planes, dst, stream=None) -> int:
+        return int(self._lib.mgt_debug_sums(self.handle, _ptr(src), terms, items, jobs, int(planes), _ptr(dst), _stream(stream)))
+
 
 def validate_adamw_kernel_config(config: AdamWKernelConfig) -> int:
     cfg = config.c()

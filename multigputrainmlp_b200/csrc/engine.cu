@@ -1029,16 +1029,21 @@ bool LaunchHeadKernel(int device, uint32_t grid, size_t smem, LaunchOn st, const
 
 // The sums of a step that wait to be launched. Pass() launches them when the caller wants finished ranges on the way or the stages
 // timed (`at_once`), or when kMostWaiting bytes of partial results wait: those are still in L2 then (p888: the planes of a weight
-// gradient are 13 to 16 MB).
+// gradient are 13 to 16 MB). Sums that find the list full launch what waits first; whether that worked is told by the next
+// Pass() or LaunchAll(). They go to the stream `on`, which every kernel that left the partial results has to be ahead of.
 struct Sums {
     static constexpr uint64_t kMostWaiting = 8ULL << 20;
     mgt_engine* e;
     bool at_once;
+    LaunchOn on;
     SumJobs jobs{};
     uint64_t waiting = 0;
+    mgt_status_t full = MGT_OK;  // of the launches that made room
 
     void Add(SumJob j, uint32_t groups) {
         if (groups == 0U) return;
+        if (jobs.count == SumJobs::kMax && full == MGT_OK) full = LaunchAll();
+        if (full != MGT_OK) return;
         const uint32_t per_cta = j.form == SumJob::kLanes ? kReduceCols : (j.form == SumJob::kQuad ? 1024U : 256U);
         j.per_group = (uint32_t)((j.items + per_cta - 1U) / per_cta);
         j.first_cta = jobs.ctas;
@@ -1070,10 +1075,10 @@ struct Sums {
         Rows(colsum + slot * R, rows, H, H, grad + HiddenBias(s));
         Rows(colsum + slot * (R + 1ULL), rows, H, H, grad + Fc2B(s, 0), R - 1U, slot, BlockParams(s));
     }
-    mgt_status_t Pass(LaunchOn st) { return at_once || waiting > kMostWaiting ? LaunchAll(st) : MGT_OK; }
-    mgt_status_t LaunchAll(LaunchOn st) {
-        if (jobs.count == 0U) return MGT_OK;
-        mgt::Launch(SumKernel, jobs.ctas, 256, 0, st, jobs);
+    mgt_status_t Pass() { return at_once || waiting > kMostWaiting ? LaunchAll() : full; }
+    mgt_status_t LaunchAll() {
+        if (full != MGT_OK || jobs.count == 0U) return full;
+        mgt::Launch(SumKernel, jobs.ctas, 256, 0, on, jobs);
         jobs.count = jobs.ctas = 0U;
         waiting = 0;
         ++e->launches;
@@ -1479,7 +1484,7 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
         return Sgemm<false, true>(st, a, 1, tile) == cudaSuccess;
     };
     // (the sums of the step in one launch at its end, unless the caller is told of finished ranges or times the stages)
-    Sums sums{e, told};
+    Sums sums{e, told, st};
     // grad_g[M x N] = act_g^T dz_g over the batch
     auto weight_grad = [&](const float* act, uint32_t ld_act, uint64_t act_stride, uint32_t M, const float* dz, uint32_t ld_dz, uint64_t dz_stride, uint32_t N, uint32_t groups,
                            float* partial, float* out, uint64_t out_stride) {
@@ -1527,7 +1532,7 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
         if (!weight_grad(x(R), p2, 0, H2, dy, OUT, 0, OUT, 1, base + ws.partial_out, grad + OutputWeight(s), 0)) return MGT_CUDA_FAILURE;
     }
     if (!ok()) return MGT_CUDA_FAILURE;
-    MGT_TRY(sums.Pass(st));
+    MGT_TRY(sums.Pass());
     MGT_TRY(notify(OutputWeight(s), (uint64_t)H2 * OUT + OUT));
     if (!timer.Mark(profile ? &profile->output_ms : nullptr)) return MGT_CUDA_FAILURE;
     // input gradients down the tower and through the hidden layer
@@ -1548,7 +1553,7 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
         if (!weight_grad(r1(0), p2, bh2, H2, dz2(1), p2, bh2, H2, R, base + ws.partial_fc2, grad + Fc2W(s, 0), BlockParams(s)) ||
             !weight_grad(x(0), p2, bh2, H2, dz1t(0), p2, bh2, H2, R, base + ws.partial_fc1, grad + Fc1W(s, 0), BlockParams(s))) return MGT_CUDA_FAILURE;
         sums.TowerBiases(s, colsum, fused ? tower.tiles : rows_h2, ws.colsum_slot, grad, true);
-        MGT_TRY(sums.Pass(st));
+        MGT_TRY(sums.Pass());
         for (uint32_t rb = R; rb > 0; --rb) {
             MGT_TRY(notify(Fc2W(s, rb - 1U), (uint64_t)H2 * H2 + H2));
             MGT_TRY(notify(Fc1W(s, rb - 1U), (uint64_t)H2 * H2 + H2));
@@ -1557,11 +1562,11 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
     if (!ok() || !timer.Mark(profile ? &profile->residual_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
     if (!backward(dz2(0), w + HiddenWeight(s), H1, nullptr, a1, p1, dz1, base + ws.colsum_in, tile_h1)) return MGT_CUDA_FAILURE;
     if (!weight_grad(a1, p1, 0, H1, dz2(0), p2, 0, H2, 1, base + ws.partial, grad + HiddenWeight(s), 0)) return MGT_CUDA_FAILURE;
-    MGT_TRY(sums.Pass(st));
+    MGT_TRY(sums.Pass());
     MGT_TRY(notify(HiddenWeight(s), (uint64_t)H1 * H2 + H2));
     // the input-bias gradient sums the fp32 dz1 (mlp_backward.cu:1505)
     sums.Rows(base + ws.colsum_in, rows_h1, H1, H1, grad + InputBias(s));
-    MGT_TRY(sums.Pass(st));
+    MGT_TRY(sums.Pass());
     if (half_ig) {
         Launch(RoundHalfKernel, GridFor((uint64_t)B * p1, 256, e->sm_count), 256, 0, st, dz1, (uint64_t)B * p1);
         ++e->launches;
@@ -1569,7 +1574,7 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
     if (!ok() || !timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
     if (EmbeddingGrad(st, states, dz1, p1, B, L, V, H1, reinterpret_cast<uint32_t*>(base + ws.lists), grad) != cudaSuccess) return MGT_CUDA_FAILURE;
     e->launches += 2;
-    MGT_TRY(sums.LaunchAll(st));
+    MGT_TRY(sums.LaunchAll());
     MGT_TRY(notify(0, (uint64_t)L * V * H1 + H1));
     if (!timer.Mark(profile ? &profile->input_grad_ms : nullptr)) return MGT_CUDA_FAILURE;
     return MGT_OK;
@@ -1767,7 +1772,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     if (!timer.Start()) return MGT_CUDA_FAILURE;
     // Nothing in the step waits for the sums over partial results: they are a launch at its end.
     const bool told = ready != nullptr || e->early_fn != nullptr || profile != nullptr;
-    Sums sums{e, told};
+    Sums sums{e, told, st};
     uint32_t ready_id = 0;
     auto notify = [&](uint64_t off, uint64_t count) -> mgt_status_t {
         if (ready == nullptr) return MGT_OK;
@@ -1958,7 +1963,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
         MGT_TRY(GemmGradWeights(e, st, x_h(R), ws.p_act, dy_h, ws.p_wout, B, H2, OUT, reinterpret_cast<float*>(base + ws.off_partial_out), sums, grad + OutputWeight(s)));
     }
     if (cudaGetLastError() != cudaSuccess) return MGT_CUDA_FAILURE;
-    MGT_TRY(sums.Pass(st));
+    MGT_TRY(sums.Pass());
     MGT_TRY(notify(OutputWeight(s), (uint64_t)H2 * OUT + OUT));
     if (!timer.Mark(profile ? &profile->output_ms : nullptr)) return MGT_CUDA_FAILURE;
 
@@ -2001,7 +2006,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
         // the gradients of the biases in front of the normalisations, of all layers
         sums.Rows(bn_bias(0), bn_blocks, H2, H2, grad + HiddenBias(s));
         sums.Rows(bn_bias(1), bn_blocks, H2, H2, grad + Fc2B(s, 0), R, (uint64_t)bn::kMaxBlocks * H2, BlockParams(s));
-        MGT_TRY(sums.Pass(st));
+        MGT_TRY(sums.Pass());
     }
     // Small batches: the weight gradients run beside the dX products and the embedding gradient, on the second stream. Neither
     // branch fills the SMs there (the dX product has fewer than two tiles an SM), and every launch is a gap: 9 001 samples of
@@ -2021,14 +2026,15 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
         ++e->launches;
     };
     if (branch.open && half_ig && ws.gather_grad) sort_classes(st_dw);
-    Sums own{e, true};  // (the sums that wait are launched on the second stream, which does not see the dX product)
+    sums.on = st_dw;
+    Sums own{e, true, st};  // (the sums that wait are launched on the second stream, which does not see the dX product)
     Sums& dx_sums = branch.open ? own : sums;
     // dz1T = (Wh * dzh^T) * [pre-activation of a1 > 0], the input-bias gradient from its row sums. With --input-grad-fp16 0 the
     // embedding gradient wants dz1 in fp32 (mlp_backward.cu:1433-1504, float one-hot GEMM): the same product of fp16 operands
     // with fp32 accumulation, written unrounded as rows of samples.
     MGT_TRY(GemmBackpropInputRows(e, st, hw.wh, hw.p2, dz_cur, ws.p_dz, B, H1, H2, reinterpret_cast<uint32_t*>(base + ws.off_bits_h1), ws.ld_bits_h1, dz1_h,
                                   ws.p_bt, half_ig ? nullptr : dz1_f32, p_dz1_f32, half_ig && ws.gather_grad, ws.p_dz1_rows, reinterpret_cast<float*>(base + ws.off_rowsum), ws.rowsum_rows, dx_sums, grad + InputBias(s)));
-    MGT_TRY(dx_sums.Pass(st));
+    MGT_TRY(dx_sums.Pass());
     if (!timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
 
     // ---- embedding gradient: grad W_in = onehot^T * dz1  (mlp_backward.cu:1440-1504); the input-bias
@@ -2071,12 +2077,12 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
         // weight gradients of all blocks: two grouped split-K GEMMs (fc2: r1_k^T dz2_k, fc1: x_k^T dz1_k)
         MGT_TRY(GemmGradWeightsGrouped(e, st_dw, r1_h(0), ws.p_act, ws.r1_stride, dz_tape(1), ws.p_dz, ws.dz_stride, R, B, H2, H2,
                                        reinterpret_cast<float*>(base + ws.off_partial_fc2), sums, grad + Fc2W(s, 0), BlockParams(s)));
-        MGT_TRY(sums.Pass(st_dw));
+        MGT_TRY(sums.Pass());
         MGT_TRY(GemmGradWeightsGrouped(e, st_dw, x_h(0), ws.p_act, ws.x_stride, dz1_tape(0), ws.p_dz, ws.dz_stride, R, B, H2, H2,
                                        reinterpret_cast<float*>(base + ws.off_partial_fc1), sums, grad + Fc1W(s, 0), BlockParams(s)));
         // (with batch normalisation b2_k and the hidden bias got their gradients from the normalisation's backward pass)
         sums.TowerBiases(s, colsum, colsum_rows, ws.colsum_slot_floats, grad, !bnorm);
-        MGT_TRY(sums.Pass(st_dw));
+        MGT_TRY(sums.Pass());
         if (cudaGetLastError() != cudaSuccess) return MGT_CUDA_FAILURE;
         for (uint32_t rb = R; rb > 0; --rb) {
             MGT_TRY(notify(Fc2W(s, rb - 1U), (uint64_t)H2 * H2 + H2));
@@ -2088,7 +2094,7 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     // ---- hidden layer backward, dW part; every kernel that reads the hidden weights was enqueued long before, so a caller
     // may update the range in place as soon as it is announced
     MGT_TRY(GemmGradWeightsRows(e, st_dw, a1_h, ws.p_bt, dz_cur, ws.p_dz, B, H1, H2, reinterpret_cast<float*>(base + ws.off_partial), sums, grad + HiddenWeight(s)));
-    MGT_TRY(sums.LaunchAll(st_dw));  // (on the second stream they are done while the table gradient still runs)
+    MGT_TRY(sums.LaunchAll());  // (on the second stream they are done while the table gradient still runs)
     if (!branch.Join()) return MGT_CUDA_FAILURE;
     MGT_TRY(notify(HiddenWeight(s), (uint64_t)H1 * H2 + H2));
     if (!timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
@@ -2136,11 +2142,22 @@ mgt_status_t mgt_debug_gemm(mgt_engine_t* e, const uint16_t* a, uint32_t lda, in
     else r = LaunchGemm<CfgDbgKK>(e, ta, tb, args, st);
     if (r != MGT_OK) return r;
     if (args.splits > 1) {
-        Sums sums{e, true};
+        Sums sums{e, true, st};
         sums.Planes(partial_scratch, args.splits, (uint64_t)m * n, d);
-        MGT_TRY(sums.LaunchAll(st));
+        MGT_TRY(sums.LaunchAll());
     }
     return MGT_OK;
+}
+
+mgt_status_t mgt_debug_sums(mgt_engine_t* e, const float* src, uint32_t terms, uint32_t items, uint32_t jobs, int32_t planes, float* dst, void* stream) {
+    if (e == nullptr || src == nullptr || dst == nullptr || terms == 0 || items == 0 || jobs == 0) return MGT_INVALID_CONFIG;
+    Sums sums{e, false, {static_cast<cudaStream_t>(stream), false}};
+    for (uint32_t j = 0; j < jobs; ++j) {
+        const float* at = src + (uint64_t)j * terms * items;
+        if (planes) sums.Planes(at, terms, items, dst + (uint64_t)j * items);
+        else sums.Rows(at, terms, items, items, dst + (uint64_t)j * items);
+    }
+    return sums.LaunchAll();
 }
 
 }  // extern "C"

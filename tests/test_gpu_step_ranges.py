@@ -185,6 +185,27 @@ def test_fp32_table_gradient(oracle, dims, n, mirror):
     loss_grad_case(oracle, dims, n, flags=(False, True), mirror=mirror)
 
 
+# sums over partial results: lists up to, at and beyond what one launch takes, terms around the 32 lanes and the eight loads in
+# flight, items that are no whole CTA and no whole quads; bit for bit in the documented order
+@pytest.mark.parametrize("planes", [False, True])
+@pytest.mark.parametrize("jobs,terms,items", [(1, 1, 1), (2, 33, 9), (12, 131, 40), (13, 9, 1028), (40, 160, 263)])
+def test_sums_of_partial_results(planes, jobs, terms, items):
+    src = np.random.default_rng(jobs).standard_normal((jobs, terms, items)).astype(np.float32)
+    dst = torch.full((jobs * items,), float("nan"), device=DEV)
+    engine = mgt.Engine(0)
+    try:
+        assert engine.debug_sums(torch.from_numpy(src).to(DEV), terms, items, jobs, planes, dst) == 0
+    finally:
+        engine.close()
+    want = np.zeros((jobs, items), np.float32)
+    for lane in range(1 if planes else min(32, terms)):
+        part = np.zeros((jobs, items), np.float32)
+        for t in range(lane, terms, 1 if planes else 32):
+            part += src[:, t]
+        want += part
+    assert np.array_equal(dst.cpu().numpy().reshape(jobs, items), want)
+
+
 # output head: the widths of its tile (16, 32, 64) and the per-sample form beyond them, tiles of 64 samples
 @pytest.mark.parametrize("outputs,hd2,n", [(2, 16, 64), (16, 300, 65), (17, 40, 63), (32, 272, 200), (33, 24, 130), (64, 512, 70), (65, 48, 96)])
 @pytest.mark.parametrize("cross_entropy", [False, True])
