@@ -210,14 +210,17 @@ TowerKernel(const __grid_constant__ TowerArgs a) {
         const uint32_t rg = warp / CG, cg = warp - rg * CG;
         const uint32_t col0 = cg * NJ * 32U + lane;                       // this lane's columns: col0 + 32 j
         const uint32_t row0 = blockIdx.x * 8U * W + rg * 8U;
-        // sign words: this lane keeps word `lane` and word 32 + lane of the warp's 8 x NJ, counted row by row
+        // sign words: this lane keeps word `lane` and word 32 + lane of the warp's 8 x NJ, counted row by row. Rows past the batch have
+        // none: a unit counts as closed there in the backward pass, whatever the forward pass made of their zeros (weights without
+        // bound make NaN of them, which must not get into the column sums).
         constexpr uint32_t kWords = 8U * NJ;
+        const bool word0 = lane < kWords && row0 + lane / NJ < a.B, word1 = 32U + lane < kWords && row0 + (32U + lane) / NJ < a.B;
         auto word_at = [&](uint32_t entry, uint32_t i) -> uint32_t* {
             return a.bits + entry * a.entry_stride + static_cast<uint64_t>(row0 + i / NJ) * a.words + cg * NJ + i % NJ;
         };
         auto store_words = [&](uint32_t entry, uint32_t w0, uint32_t w1) {
-            if (lane < kWords) *word_at(entry, lane) = w0;
-            if (32U + lane < kWords) *word_at(entry, 32U + lane) = w1;
+            if (word0) *word_at(entry, lane) = w0;
+            if (word1) *word_at(entry, 32U + lane) = w1;
         };
         // the CG warps that share rows meet here after an epilogue (with column sums all warps of the CTA do)
         auto meet = [&]() {
@@ -266,8 +269,8 @@ TowerKernel(const __grid_constant__ TowerArgs a) {
             uint32_t m0 = 0, m1 = 0;
             if (BWD) {
                 const uint32_t entry = second ? R + k : k;
-                if (lane < kWords) m0 = *word_at(entry, lane);
-                if (32U + lane < kWords) m1 = *word_at(entry, 32U + lane);
+                if (word0) m0 = *word_at(entry, lane);
+                if (word1) m1 = *word_at(entry, 32U + lane);
             } else {
                 const float* b = a.bias + matrix(p) * a.bias_step;
 #pragma unroll

@@ -122,6 +122,40 @@ def test_fp32_tower_cuts(oracle, hd2, n):
     loss_grad_case(oracle, (6, 4, 16, hd2, 1, 1), n, flags=(False, False), tol=1e-5 + n * 2.0 ** -24, section_tol=2e-5 + n * 2.0 ** -24)
 
 
+# A weight without bound behind a unit that no sample opens: its products with the samples are NaN before a ReLU that closes on
+# them and before masks that are zero, so that all gradients are those of the same model with that weight 0. Nor may the rows of the tower's
+# last tile that are no samples bring it into the bias gradients: there the unit would be open.
+@pytest.mark.parametrize("hd2,n", [(24, 61), (128, 1003), (224, 4099)])
+def test_fp32_tower_rows_past_the_batch(hd2, n):
+    c = mgt.CudaMlpShape(6, 4, 16, hd2, 2, 1)
+    rng = np.random.default_rng(hd2)
+    w = (rng.standard_normal(c.param_count) * 0.03).astype(np.float32)
+    hidden = 24 * 16 + 16
+    w[hidden + 16 * hd2:hidden + 17 * hd2] = 1.0  # hidden bias: every activation positive
+    first = hidden + 17 * hd2                     # W1_0, b1_0, W2_0, b2_0
+    second = first + hd2 * hd2 + hd2
+    w[first:first + hd2 * hd2].reshape(hd2, hd2)[:, 0] = -1.0
+    w[first + hd2 * hd2] = 0.5                    # unit 0 of the first block: open where the activations are zero, and only there
+    w[second + hd2 * hd2 + 3] = -1000.0           # unit 3 behind it: closed
+    states = torch.from_numpy(rng.integers(0, 4, (n, 80), dtype=np.uint8)).to(DEV)
+    labels, loss = torch.ones(n, device=DEV), torch.zeros(1, device=DEV)
+    floats = mgt.mlp_loss_grad_workspace_floats(c, n, 1, False, False)
+    ws = torch.empty(floats, device=DEV)
+    grads = []
+    engine = mgt.Engine(0)
+    try:
+        for value in (0.0, np.inf):
+            w[second + 3] = value                 # from unit 0 to unit 3
+            grad = torch.full((c.param_count,), float("nan"), device=DEV)
+            assert engine.launch_mlp_loss_grad(c, torch.from_numpy(w).to(DEV), None, states, labels, n, loss, grad, ws, floats, use_half_input_grad=False,
+                                               use_half_linear=False) == 0
+            assert engine.check()[0] == 0
+            grads.append(grad.cpu().numpy())
+    finally:
+        engine.close()
+    assert np.isfinite(grads[0]).all() and np.array_equal(grads[1], grads[0])
+
+
 def multiply_in_order(x, w):
     """x w in fp32, one multiply-add after the other along k (the product of two floats is exact in double)."""
     acc = np.zeros((x.shape[0], w.shape[1]), np.float32)
