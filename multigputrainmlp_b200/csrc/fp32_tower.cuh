@@ -64,6 +64,8 @@ inline size_t TowerSmem(uint32_t H, uint32_t W, uint32_t padded, uint32_t chunk,
     const size_t rows = (H + 15U) / 16U * 16U;
     return (2U * rows * (8U * W + 4U) + stages * static_cast<size_t>(padded) * (chunk + 4U) + 2U * W * padded) * sizeof(float) + kTowerBarBytes;
 }
+// words of sign bits of a sample
+inline uint32_t TowerSampleWords(uint32_t H) { return H <= 128U || H > 224U ? (H + 31U) / 32U : 7U; }
 // Picks the cut with the least estimated time: rounds of the chip x (cycles a k x H + 3 000 for epilogue and waits of a product). The
 // cycles of a k are measured: those of one warp on its scheduler, and what every further one adds.
 inline TowerPlan PlanTower(uint32_t B, uint32_t H, uint32_t sm) {
@@ -73,6 +75,7 @@ inline TowerPlan PlanTower(uint32_t B, uint32_t H, uint32_t sm) {
     double best_cost = 1e30;
     for (const Width& width : kWidths) {
         const uint32_t nj = width.nj, cg = (H + 32U * nj - 1U) / (32U * nj), padded = cg * nj * 32U;
+        if (nj >= 7U && (cg > 1U || nj > TowerSampleWords(H))) continue;  // (never the best; a sample has TowerSampleWords words)
         for (uint32_t w = 1U; w <= 8U; ++w) {
             if ((w * cg + 1U) * 32U > TowerThreads(nj)) break;
             // the deepest stages of which three fit, or two of eight
@@ -93,8 +96,8 @@ inline TowerPlan PlanTower(uint32_t B, uint32_t H, uint32_t sm) {
     }
     return best;
 }
-// words of sign bits of one entry, and rows of column sums of one slot, for any plan; neither falls with a larger batch
-inline uint64_t TowerBitWords(uint32_t B, uint32_t H) { return (static_cast<uint64_t>(B) + 64U) * ((H + 31U) / 32U + 7U); }
+// words of one entry of sign bits, and rows of column sums of one slot, for any plan: neither falls with a larger batch
+inline uint64_t TowerBitWords(uint32_t B, uint32_t H) { return static_cast<uint64_t>(B) * TowerSampleWords(H); }
 inline uint64_t TowerSumRows(uint32_t B) { return (static_cast<uint64_t>(B) + 7U) / 8U; }
 
 __device__ __forceinline__ void CopyAsync16(float* dst, const float* src) {
@@ -210,11 +213,13 @@ TowerKernel(const __grid_constant__ TowerArgs a) {
         const uint32_t rg = warp / CG, cg = warp - rg * CG;
         const uint32_t col0 = cg * NJ * 32U + lane;                       // this lane's columns: col0 + 32 j
         const uint32_t row0 = blockIdx.x * 8U * W + rg * 8U;
-        // sign words: this lane keeps word `lane` and word 32 + lane of the warp's 8 x NJ, counted row by row. Rows past the batch have
-        // none: a unit counts as closed there in the backward pass, whatever the forward pass made of their zeros (weights without
-        // bound make NaN of them, which must not get into the column sums).
+        // sign words: this lane keeps word `lane` and word 32 + lane of the warp's 8 x NJ, counted row by row. Columns past the width
+        // have none (but with one warp of 224 or 256 columns: asking there too costs that kernel 1 %), nor have rows past the batch: a
+        // unit counts as closed there in the backward pass, whatever the forward pass made of their zeros (weights without bound make
+        // NaN of them, which must not get into the column sums).
         constexpr uint32_t kWords = 8U * NJ;
-        const bool word0 = lane < kWords && row0 + lane / NJ < a.B, word1 = 32U + lane < kWords && row0 + (32U + lane) / NJ < a.B;
+        auto has_word = [&](uint32_t i) { return i < kWords && row0 + i / NJ < a.B && (NJ >= 7 || cg * NJ + i % NJ < a.words); };
+        const bool word0 = has_word(lane), word1 = has_word(32U + lane);
         auto word_at = [&](uint32_t entry, uint32_t i) -> uint32_t* {
             return a.bits + entry * a.entry_stride + static_cast<uint64_t>(row0 + i / NJ) * a.words + cg * NJ + i % NJ;
         };
@@ -390,7 +395,7 @@ inline cudaError_t LaunchTower(int device, LaunchOn st, const TowerPlan& plan, T
     a.col_groups = plan.col_groups;
     a.chunk = plan.chunk;
     a.stages = plan.stages;
-    a.words = plan.col_groups * plan.nj;
+    a.words = TowerSampleWords(a.H);
     switch (plan.nj) {
         case 1: return TowerRun<1, BWD>(device, st, a, plan);
         case 2: return TowerRun<2, BWD>(device, st, a, plan);

@@ -49,6 +49,16 @@ def test_host_side_validation_without_gpu():
     assert mgt.validate_adamw_kernel_config(mgt.AdamWKernelConfig(8, 1, 1e-3, weight_decay=-1.0)) == 1
 
 
+def test_scratch_of_the_fp32_tower():
+    # what a step all in fp32 keeps of a sample: activations and gradients of every layer, a sign bit and an eighth of a bias sum for each
+    # unit of the tower, its place in the sample lists; and the planes of the weight gradients besides
+    import multigputrainmlp_b200 as mgt
+    for h1, h2, blocks, batch, words in ((64, 8, 32, 100000, 1), (64, 72, 16, 60000, 3), (64, 136, 8, 30000, 7), (2560, 224, 16, 8192, 7)):
+        values = 2 * h1 + (4 * blocks + 2) * h2 + 2 * blocks * (words + h2 / 8) + (h1 + h2) / 32 + 73
+        floats = mgt.mlp_loss_grad_workspace_floats(mgt.CudaMlpShape(72, 72, h1, h2, blocks, 1), batch, 1, False, False)
+        assert batch * values < floats <= batch * values + 80 * (h1 * h2 + 2 * blocks * h2 * h2)
+
+
 def test_workspace_never_shrinks_with_the_batch():
     # scratch sized for the largest batch has to do for every smaller one, on both sides of every rule that picks a kernel by size
     import multigputrainmlp_b200 as mgt
