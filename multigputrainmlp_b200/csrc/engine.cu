@@ -1097,7 +1097,12 @@ mgt_status_t LaunchHeadN(mgt_engine* e, LaunchOn st, const HeadArgs& a, Sums& su
     if (a.OUT <= 16U) ok = LaunchHeadKernel<HeadTileKernel<16, kCrossEntropy, kF32>>(e->device, grid, HeadTileSmem<16>(a.H2), st, a);
     else if (a.OUT <= 32U) ok = LaunchHeadKernel<HeadTileKernel<32, kCrossEntropy, kF32>>(e->device, grid, HeadTileSmem<32>(a.H2), st, a);
     else if (tiled) ok = LaunchHeadKernel<HeadTileKernel<64, kCrossEntropy, kF32>>(e->device, grid, HeadTileSmem<64>(a.H2), st, a);
-    else ok = LaunchHeadKernel<HeadOutNKernel<kCrossEntropy, kF32>>(e->device, grid, (kHeadThreads / 32) * a.OUT * sizeof(float), st, a);
+    else {
+        // With more than a CTA an SM not before the kernel ahead has ended: this one has its weights through L1, and a CTA that begins beside a
+        // tower's keeps the split of the SM that the tower asked for, all shared memory (8 433 samples, hd2 256: 128 outputs 2 671 us a step,
+        // 1 634 like this; 70 outputs 732, 550; 2 000 samples 240, 241; but 500 samples, hd2 64 103, 105).
+        ok = LaunchHeadKernel<HeadOutNKernel<kCrossEntropy, kF32>>(e->device, grid, (kHeadThreads / 32) * a.OUT * sizeof(float), {st.stream, st.overlap && grid <= (uint32_t)e->sm_count}, a);
+    }
     if (!ok) return MGT_CUDA_FAILURE;
     // the partial rows of the CTAs: { loss, column sums of dz, with up to 64 outputs column sums of dy }
     const uint32_t width = 1U + a.H2 + a.OUT;
