@@ -1589,8 +1589,18 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
 // 4 096 samples of hd1 1024 210 -> 200 us, 5 003 of hd1 333 172 -> 157, 1 024 of hd1 256 103 -> 82; 3 001 samples of hd1 2560 make no
 // difference, and with kernels that fill the chip the next one's CTAs are in the way: 9 001 samples of hd1 1000 445 -> 491, 8 192 of
 // hd1 2560 in fp32 4 701 -> 5 230. The many passes of batch normalisation stream and gain at any size (53 248 of hd1 2560 5 884 -> 5 510).
-// The fp32 products fill the chip sooner: 3 000 samples of hd1 1001, hd2 301 2 427 -> 2 997 us, 1 024 of hd1 256, hd2 64 175 -> 148.
-bool OverlapLaunches(const mgt_mlp_shape_t& s, uint32_t B, bool batch_norm, bool fp32) { return batch_norm || (uint64_t)B * s.hd1 <= (fp32 ? 1000000ULL : 6000000ULL); }
+bool OverlapLaunches(const mgt_mlp_shape_t& s, uint32_t B, bool batch_norm) { return batch_norm || (uint64_t)B * s.hd1 <= 6000000ULL; }
+// All in fp32 the kernels have their operands through L1, and lose some of it to the shared memory of the next one, as soon as a
+// product has more than one or two tiles for an SM. Counted in tiles of 32 x 32, of the products by hd1 (the input gradient) and of those
+// by hd2 (the blocks): us a step without and with, by samples / hd1 / hd2 / blocks. Few tiles: 250 / 512 / 64 / 4 176 -> 153; 128 / 1000 /
+// 192 / 6 373 -> 322; 1 000 / 256 / 192 / 6 400 -> 379. Too many by hd1: 256 / 1000 / 128 / 4 265 -> 292; 102 / 2500 / 192 / 6 470 -> 534;
+// by hd2: 2 000 / 64 / 128 / 4 223 -> 249; 3 800 / 64 / 256 / 6 899 -> 1 099; 320 / 400 / 400 / 6 528 -> 558. A narrow hd2 leaves the chip
+// emptier: 512 / 1000 / 24 / 4 173 -> 149, 1 000 / 512 / 64 / 4 193 -> 184, but 8 000 / 64 / 24 / 4 170 -> 177.
+bool OverlapFp32Launches(const mgt_mlp_shape_t& s, uint32_t B) {
+    auto tiles = [&](uint32_t n) { return (uint64_t)((B + 31U) / 32U) * ((n + 31U) / 32U); };
+    const uint64_t by_hd1 = s.hd2 <= 32U || (s.hd2 <= 64U && s.hd1 <= 512U) ? 518U : (s.hd1 <= 512U ? 256U : 160U);
+    return tiles(s.hd1) <= by_hd1 && tiles(s.hd2) <= (s.hd2 <= 320U ? 200U : 112U);
+}
 
 struct HalfWeights {
     const __half* in_table; uint32_t p1;     // [(IN+1)][p1], row IN is the input bias
@@ -1752,12 +1762,12 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
             return ready(ready_user, id++, off, count, stream_v) == MGT_OK ? MGT_OK : MGT_CUDA_FAILURE;
         };
         return LaunchFp32Path(e, s, w, reinterpret_cast<const uint8_t*>(states), labels, B, loss, grad, workspace, half_ig != 0, ready != nullptr || profile != nullptr, profile, tell,
-                              {static_cast<cudaStream_t>(stream_v), OverlapLaunches(s, B, false, true)});
+                              {static_cast<cudaStream_t>(stream_v), OverlapFp32Launches(s, B)});
     }
     Workspace ws = PlanWorkspace(s, B, PlanSmCount(e->sm_count), half_ig != 0, bnorm);
     if (e->embedding_form != mgt_engine::kBySize) ws.gather_fwd = ws.gather_grad = e->embedding_form == mgt_engine::kGather;
     if (workspace_floats < (ws.total_bytes + 3) / 4 + (half_ig ? 0 : Fp32TableFloats(s, B))) return MGT_CAPACITY_EXCEEDED;
-    const LaunchOn st(static_cast<cudaStream_t>(stream_v), OverlapLaunches(s, B, bnorm, false));
+    const LaunchOn st(static_cast<cudaStream_t>(stream_v), OverlapLaunches(s, B, bnorm));
     uint8_t* base = reinterpret_cast<uint8_t*>(RoundUp(reinterpret_cast<uintptr_t>(workspace), 1024));
     float* dz1_f32 = reinterpret_cast<float*>(RoundUp(reinterpret_cast<uintptr_t>(workspace + (ws.total_bytes + 3) / 4), 256));  // behind the tensor-core workspace
     const uint32_t p_dz1_f32 = (uint32_t)RoundUp(s.hd1, 4);
