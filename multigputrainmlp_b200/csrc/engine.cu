@@ -1392,11 +1392,26 @@ struct Fp32Workspace {
     uint32_t p1, p2;
     uint64_t a1, x, r1, dz2, dz1t, dz1, dy, head, partial, partial_fc2, partial_fc1, partial_out, colsum, colsum_slot, colsum_in, bits, bits_entry, tower_w, lists, total;  // float offsets
 };
-// The blocks in one launch per direction (fp32_tower.cuh): widths up to 128, up to 256 with 4 096 samples. A CTA streams every matrix
-// through one warp, which is the longest part of wide ones with few samples to a CTA (ms a step, by layers and fused: 64 samples of
-// hd2 256, 10 blocks 0.57, 0.80; 1 500 of hd2 161, 31 blocks 1.95, 2.17; 2 500 of hd2 510, 8 blocks 3.26, 4.33; but 2 000 of hd2 128, 30
-// blocks 1.44, 1.30; 20 000 of hd2 240, 5 blocks 4.09, 3.71; 30 000 of hd2 18, 20 blocks 1.75, 1.24; 300 of hd2 8, 32 blocks 0.90, 0.20).
-bool FusedFp32Tower(const mgt_mlp_shape_t& s, uint32_t B) { return s.residual_blocks > 0 && (s.hd2 <= 128U || (s.hd2 <= 256U && B >= 4096U)); }
+// The blocks in one launch per direction (fp32_tower.cuh). Widths up to 128: always (us a step, by layers and fused: 1 000 samples of hd2
+// 128, 16 blocks 680, 490; 30 000 of hd2 128, 8 blocks 1 960, 1 800; 300 of hd2 8, 32 blocks 900, 200). Up to 256: a CTA streams every
+// matrix through one warp, which is the longest part with few samples to a CTA (2 000 samples, 6 blocks, hd2 160 441, 365; 192 440, 416; 224
+// 526, 573; 256 598, 654; 2 500 of hd2 160 466, 426; 224 765, 668; 256 812, 752). From there on it is the faster form while one round of the
+// chip takes all samples (8 blocks: 5 000 of hd2 160 920, 690; 7 000 of hd2 240 1 531, 1 426). Beyond, both go in steps, the tower of 32 to
+// 56 samples an SM, the products of a tile an SM, and an estimate of both decides (hd2 224: 9 500 2 013, 2 420; 12 000 2 393, 2 507; 20 000
+// 4 468, 3 573; hd2 160: 9 500 1 372, 1 257; 12 000 1 506, 1 699). Of 119 steps of 8 400 to 42 000 samples it took the slower form for
+// 10, by 4.6 % at most. Wider ones are products of their own (2 500 of hd2 510, 8 blocks 3 260, 4 330).
+constexpr uint32_t kFusedFp32Batch = 2500U;
+// whether any batch of up to B samples is fused: scratch is planned by this
+bool MayFuseFp32Tower(const mgt_mlp_shape_t& s, uint32_t B) { return s.residual_blocks > 0 && (s.hd2 <= 128U || (s.hd2 <= 256U && B >= kFusedFp32Batch)); }
+bool FusedFp32Tower(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm) {
+    if (!MayFuseFp32Tower(s, B)) return false;
+    if (s.hd2 <= 128U) return true;
+    const fp32path::TowerPlan plan = fp32path::PlanTower(B, s.hd2, sm);
+    if (plan.rounds == 1U) return true;
+    auto each = [&](uint32_t t) { return ((uint64_t)((B + t - 1U) / t) * ((s.hd2 + t - 1U) / t) + sm - 1U) / sm; };  // tiles for the fullest SM
+    const bool large = fp32path::PickSgemmTile(B, s.hd2, 1, sm) == fp32path::SgemmTile::kLarge;
+    return plan.us < (large ? 20.0 + 0.130 * s.hd2 * (double)each(128U) : 13.2 + 0.0284 * s.hd2 * (double)each(64U));
+}
 struct DwPlan {
     fp32path::SgemmTile tile;
     uint32_t splits;
@@ -1431,7 +1446,7 @@ Fp32Workspace PlanFp32(const mgt_mlp_shape_t& s, uint32_t B, uint32_t sm) {
     w.partial_fc2 = take(planes(s.hd2, s.hd2, (uint32_t)r));
     w.partial_fc1 = take(planes(s.hd2, s.hd2, (uint32_t)r));
     w.partial_out = take(s.output_dim > 1 ? planes(s.hd2, s.output_dim, 1) : 0);
-    const bool fused = FusedFp32Tower(s, B);
+    const bool fused = MayFuseFp32Tower(s, B);
     w.colsum_slot = (fused ? fp32path::TowerSumRows(B) : (uint64_t)((B + 31U) / 32U)) * s.hd2;  // one row per tile of at least 32 samples, 8 in the tower
     w.colsum = take(w.colsum_slot * 2 * r);
     w.colsum_in = take((uint64_t)((B + 31U) / 32U) * s.hd1);
@@ -1461,7 +1476,7 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
     float *dy = base + ws.dy, *dz1 = base + ws.dz1, *colsum = base + ws.colsum;
     const SgemmTile tile_h2 = PickSgemmTile(B, H2, 1, sm), tile_h1 = PickSgemmTile(B, H1, 1, sm);
     const uint32_t rows_h2 = (B + SgemmTileRows(tile_h2) - 1U) / SgemmTileRows(tile_h2), rows_h1 = (B + SgemmTileRows(tile_h1) - 1U) / SgemmTileRows(tile_h1);
-    const bool fused = FusedFp32Tower(s, B);
+    const bool fused = FusedFp32Tower(s, B, sm);
     const TowerPlan tower = fused ? PlanTower(B, H2, sm) : TowerPlan{};
     TowerArgs tower_args{};
     tower_args.B = B; tower_args.H = H2; tower_args.R = R; tower_args.pitch = p2;

@@ -56,6 +56,8 @@ struct TowerArgs {
 struct TowerPlan {
     uint32_t nj, row_groups, col_groups, tiles, chunk, stages;
     size_t smem;
+    uint32_t rounds;  // of the chip, a tile to every place that an SM has for one
+    double us;        // what a product of all samples takes in that many rounds, as measured (widths of 129 to 256)
 };
 constexpr uint32_t kTowerSmem = 227U * 1024U, kTowerBarBytes = 128U;
 inline uint32_t TowerThreads(uint32_t nj) { return nj >= 7U ? 256U : 512U; }          // of a CTA at most
@@ -67,10 +69,11 @@ inline size_t TowerSmem(uint32_t H, uint32_t W, uint32_t padded, uint32_t chunk,
 // words of sign bits of a sample
 inline uint32_t TowerSampleWords(uint32_t H) { return H <= 128U || H > 224U ? (H + 31U) / 32U : 7U; }
 // Picks the cut with the least estimated time: rounds of the chip x (cycles a k x H + 3 000 for epilogue and waits of a product). The
-// cycles of a k are measured: those of one warp on its scheduler, and what every further one adds.
+// cycles of a k are measured: those of one warp on its scheduler, and what every further one adds. So is the time of a round, for
+// 100 units in us, with one warp on a scheduler and with more: by the steps of two rounds and more in the list at FusedFp32Tower.
 inline TowerPlan PlanTower(uint32_t B, uint32_t H, uint32_t sm) {
-    struct Width { uint32_t nj; double alone, each; };
-    constexpr Width kWidths[] = {{1U, 20.0, 20.0}, {2U, 46.0, 26.0}, {4U, 66.0, 45.0}, {7U, 78.0, 71.0}, {8U, 88.0, 81.0}};
+    struct Width { uint32_t nj; double alone, each, round_alone, round; };
+    constexpr Width kWidths[] = {{1U, 20.0, 20.0, 8.3, 8.3}, {2U, 46.0, 26.0, 8.3, 8.3}, {4U, 66.0, 45.0, 12.1, 12.1}, {7U, 78.0, 71.0, 8.4, 10.8}, {8U, 88.0, 81.0, 10.0, 13.2}};
     TowerPlan best{};
     double best_cost = 1e30;
     for (const Width& width : kWidths) {
@@ -90,7 +93,7 @@ inline TowerPlan PlanTower(uint32_t B, uint32_t H, uint32_t sm) {
             const double cost = rounds * (std::max(width.alone, width.each * ((warps * resident + 3U) / 4U)) * H + 3000.0 * resident);
             if (cost < best_cost) {
                 best_cost = cost;
-                best = {nj, w, cg, tiles, chunk, stages, smem};
+                best = {nj, w, cg, tiles, chunk, stages, smem, rounds, rounds * (H / 100.0) * (warps * resident <= 4U ? width.round_alone : width.round)};
             }
         }
     }
