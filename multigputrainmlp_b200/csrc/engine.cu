@@ -1592,7 +1592,7 @@ mgt_status_t LaunchFp32Path(mgt_engine* e, const mgt_mlp_shape_t& s, const float
         ++e->launches;
     }
     if (!ok() || !timer.Mark(profile ? &profile->hidden_backward_ms : nullptr)) return MGT_CUDA_FAILURE;
-    if (EmbeddingGrad(st, states, dz1, p1, B, L, V, H1, reinterpret_cast<uint32_t*>(base + ws.lists), grad) != cudaSuccess) return MGT_CUDA_FAILURE;
+    if (EmbeddingGrad(st, states, dz1, p1, B, L, V, H1, reinterpret_cast<uint32_t*>(base + ws.lists), false, grad) != cudaSuccess) return MGT_CUDA_FAILURE;
     e->launches += 2;
     MGT_TRY(sums.LaunchAll());
     MGT_TRY(notify(0, (uint64_t)L * V * H1 + H1));
@@ -2049,13 +2049,18 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     SideBranch branch{e, st};
     if (dx_tiles < 2ULL * e->sm_count && B <= 16384U && (uint64_t)B * H1 >= 65536U && !told) branch.Fork();
     const LaunchOn st_dw(branch.open ? branch.side.stream : st.stream, st.overlap);
-    uint32_t* order = reinterpret_cast<uint32_t*>(base + ws.off_lists);
+    uint32_t* order = half_ig ? reinterpret_cast<uint32_t*>(base + ws.off_lists) : reinterpret_cast<uint32_t*>(dz1_f32 + (uint64_t)B * p_dz1_f32);
     uint32_t* first = order + (uint64_t)s.state_len * B;
     auto sort_classes = [&](LaunchOn stream) {
         Launch(gather::SortByClassKernel, s.state_len, 1024, 0, stream, reinterpret_cast<const uint8_t*>(states), B, s.state_value_pad, order, first);
         ++e->launches;
     };
-    if (branch.open && half_ig && ws.gather_grad) sort_classes(st_dw);
+    // The sort of a gathered table gradient goes first on the second stream. Behind the dX product it finds no room beside the weight
+    // gradients there (registers), and the table gradient waits for them: fp32 table, 2 blocks, samples / hd1 / hd2 16 384 / 64 / 32 184 us
+    // a step on one stream's order, 210 with launches that overlap, 180 like this; 6 000 / 256 / 96 172, 166, 150. With longer gathers, which leave
+    // the weight gradients no room in turn, it costs more than it saves: 10 000 / 512 / 200, 6 blocks 364 -> 387; 16 384 / 512 / 96 352 -> 392.
+    const bool sort_aside = branch.open && (half_ig ? ws.gather_grad : H1 <= 256U || (H1 <= 512U && B <= 4096U));
+    if (sort_aside) sort_classes(st_dw);
     sums.on = st_dw;
     Sums own{e, true, st};  // (the sums that wait are launched on the second stream, which does not see the dX product)
     Sums& dx_sums = branch.open ? own : sums;
@@ -2069,18 +2074,18 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
 
     // ---- embedding gradient: grad W_in = onehot^T * dz1  (mlp_backward.cu:1440-1504); the input-bias
     // gradient (mlp_backward.cu:1505) is the column sum written by the GEMM above
+    if (sort_aside && !branch.Tie(1, branch.side.stream, st)) return MGT_CUDA_FAILURE;  // (of the branch only the sort is enqueued yet)
     if (!half_ig) {
         if (fp32path::EmbeddingGrad(st, reinterpret_cast<const uint8_t*>(states), dz1_f32, p_dz1_f32, B, s.state_len, s.state_value_pad, H1,
-                                    reinterpret_cast<uint32_t*>(dz1_f32 + (uint64_t)B * p_dz1_f32), grad) != cudaSuccess) return MGT_CUDA_FAILURE;
-        e->launches += 2;
+                                    order, sort_aside, grad) != cudaSuccess) return MGT_CUDA_FAILURE;
+        e->launches += sort_aside ? 1 : 2;
     } else if (ws.gather_grad) {
         const bool vec = (H1 & 3U) == 0U && (reinterpret_cast<uintptr_t>(grad) & 15U) == 0U;
         auto run = [&](auto kernel, uint32_t rows_per_cta) {
             Launch(kernel, dim3((IN + rows_per_cta - 1U) / rows_per_cta, (H1 + 63U) / 64U), 256, 0, st, order, first, reinterpret_cast<const uint16_t*>(dz1_h), ws.p_dz1_rows, B,
                                                                                                s.state_len, s.state_value_pad, H1, grad, vec);
         };
-        if (!branch.open) sort_classes(st);
-        else if (!branch.Tie(1, branch.side.stream, st)) return MGT_CUDA_FAILURE;  // (of the branch only the sort is enqueued yet)
+        if (!sort_aside) sort_classes(st);
         // a group of lanes per table row, four groups where that leaves fewer than 16 warps for an SM
         const bool few = (uint64_t)IN * ((H1 + 63U) / 64U) < 64ULL * e->sm_count;
         if (few) { if (e->bf16_now) run(gather::GradKernel<4, true>, 8U); else run(gather::GradKernel<4, false>, 8U); }

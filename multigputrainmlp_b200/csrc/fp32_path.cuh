@@ -402,11 +402,11 @@ EmbeddingGradKernel(const uint32_t* __restrict__ order, const uint32_t* __restri
     if (W == 4) *reinterpret_cast<float4*>(dst) = make_float4(acc[0], acc[1 % W], acc[2 % W], acc[3 % W]);
     else dst[0] = acc[0];
 }
-// `lists`: gather::ListWords words of scratch
+// `lists`: gather::ListWords words of scratch; `sorted`: gather::SortByClassKernel has left its lists there
 inline cudaError_t EmbeddingGrad(LaunchOn st, const uint8_t* states, const float* dz1, uint32_t ld, uint32_t B, uint32_t L, uint32_t V, uint32_t H1,
-                                 uint32_t* lists, float* grad_table) {
+                                 uint32_t* lists, bool sorted, float* grad_table) {
     uint32_t* first = lists + static_cast<uint64_t>(L) * B;
-    Launch(gather::SortByClassKernel, L, 1024, 0, st, states, B, V, lists, first);
+    if (!sorted) Launch(gather::SortByClassKernel, L, 1024, 0, st, states, B, V, lists, first);
     const bool quads = (H1 & 3U) == 0U && (ld & 3U) == 0U && (reinterpret_cast<uintptr_t>(grad_table) & 15U) == 0U;
     const uint32_t cols = quads ? 128U : 32U;
     const dim3 grid((L * V + 7U) / 8U, (H1 + cols - 1U) / cols);

@@ -213,8 +213,10 @@ def test_fp32_forward_adds_in_order(oracle, dims):
         engine.close()
 
 
-# fp32 table gradient behind fp16 linears: classes without samples, one class per position, many samples per class
-@pytest.mark.parametrize("dims,n,mirror", [((72, 72, 36, 40, 1, 1), 45, True), ((54, 6, 130, 64, 2, 1), 1000, True), ((16, 1, 33, 24, 1, 2), 257, False)])
+# fp32 table gradient behind fp16 linears: classes without samples, one class per position, many samples per class; its sort on the
+# second stream (hd1 up to 256, up to 512 with 4 096 samples) and on the caller's
+@pytest.mark.parametrize("dims,n,mirror", [((72, 72, 36, 40, 1, 1), 45, True), ((54, 6, 130, 64, 2, 1), 1000, True), ((16, 1, 33, 24, 1, 2), 257, False),
+                                           ((20, 12, 256, 40, 2, 1), 4100, True), ((20, 12, 512, 24, 3, 1), 300, False), ((20, 12, 260, 24, 3, 1), 4100, True), ((20, 12, 516, 24, 3, 1), 300, True)])
 def test_fp32_table_gradient(oracle, dims, n, mirror):
     loss_grad_case(oracle, dims, n, flags=(False, True), mirror=mirror)
 
