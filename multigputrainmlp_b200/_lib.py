@@ -43,6 +43,8 @@ def _declare(lib: C.CDLL) -> None:
     lib.mgt_engine_check.argtypes = [vp, vp, C.POINTER(i32)]
     lib.mgt_engine_launch_count.restype = u64
     lib.mgt_engine_launch_count.argtypes = [vp]
+    lib.mgt_engine_fork_count.restype = u64
+    lib.mgt_engine_fork_count.argtypes = [vp]
     lib.mgt_mlp_loss_grad_workspace_floats.restype = u64
     lib.mgt_mlp_loss_grad_workspace_floats.argtypes = [vp, u32, u32, i32, i32]
     lib.mgt_launch_mlp_loss_grad.argtypes = [vp, vp, vp, vp, vp, vp, u32, vp, vp, vp, u64, u32, u32, i32, i32, vp, vp, vp, vp, u32]

@@ -218,6 +218,10 @@ class Engine:
     def launch_count(self) -> int:
         return int(self._lib.mgt_engine_launch_count(self.handle))
 
+    @property
+    def fork_count(self) -> int:
+        return int(self._lib.mgt_engine_fork_count(self.handle))
+
     def check(self, stream=None):
         code = C.c_int32(0)
         st = int(self._lib.mgt_engine_check(self.handle, _stream(stream), C.byref(code)))

@@ -354,6 +354,7 @@ struct mgt_engine {
     size_t side_turn = 0;
     std::mutex side_mu;    // of the two above; and an event is recorded and waited for in one piece
     uint64_t launches = 0;  // kernels launched through this engine (host-side count)
+    uint64_t forks = 0;     // passes of which a part ran on a second stream
     bool layered_tower = false;  // MGT_RESIDUAL_PATH=layered: per-layer GEMMs instead of the fused residual-tower kernels (both are tested)
     enum { kBySize, kGather, kOneHot } embedding_form = kBySize;  // MGT_EMBEDDING_FORM=gather|onehot: one form of the embedding layer for all sizes (both are tested)
     mgt_gradient_ready_fn early_fn = nullptr;  // mgt_engine_set_early_range_hook
@@ -1161,6 +1162,7 @@ struct SideBranch {
             const unsigned long long held = CaptureOf(side.stream);
             ok = held == 0 || held == capture;
             open = ok && TieLocked(0, main, side.stream);
+            e->forks += open ? 1U : 0U;
         }
         if (!open) cudaGetLastError();
         return open;
@@ -1694,6 +1696,7 @@ mgt_status_t mgt_engine_destroy(mgt_engine_t* e) {
 }
 
 uint64_t mgt_engine_launch_count(const mgt_engine_t* e) { return e == nullptr ? 0 : e->launches; }
+uint64_t mgt_engine_fork_count(const mgt_engine_t* e) { return e == nullptr ? 0 : e->forks; }
 
 mgt_status_t mgt_engine_check(mgt_engine_t* e, void* stream, int32_t* out_device_code) {
     if (e == nullptr) return MGT_INVALID_CONFIG;
@@ -2040,14 +2043,19 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
     }
     // Small batches: the weight gradients run beside the dX products and the embedding gradient, on the second stream. Neither
     // branch fills the SMs there (the dX product has fewer than two tiles an SM), and every launch is a gap: 9 001 samples of
-    // hd1 1000, hd2 200, 8 blocks 510 -> 453 us a step, 1 024 of hd1 256, hd2 64, 2 blocks 134 -> 114, 64 of hd1 8, hd2 8
-    // 99 -> 89. With more tiles each kernel has the whole chip anyway, and beyond some 16 000 samples of a small model the
-    // gradient's gathers lose more to the shared memory of the GEMMs beside them than they gain (54 025 of hd1 88: 611 ->
-    // 660 us). Nor for the smallest steps, which the
-    // host's calls bound (64 samples of hd1 8: 59 us with, 56 without). Not with callers that are told of finished ranges or time the stages: they rely on the order.
+    // hd1 1000, hd2 200, 8 blocks 510 -> 453 us a step, 1 024 of hd1 256, hd2 64, 2 blocks 91 -> 82. With more tiles each kernel has the
+    // whole chip anyway, and beyond some 16 000 samples of a small model the gradient's gathers lose more to the shared memory of the
+    // GEMMs beside them than they gain (54 025 of hd1 88: 611 -> 660 us).
+    // The fork is six calls more for the host, which bounds the shortest steps: whatever runs beside what, they take 61 to 66 us with it
+    // (by host). So not where the chain of kernels is shorter than that. It grows with the blocks and, from some thousand samples x hd1
+    // on, with the embedding layer; without and with the fork, samples / hd1 / hd2: no blocks 500 / 64 / 16 51, 57; one 64 / 8 / 8 60, 66,
+    // 300 / 16 / 16 65, 66, 64 / 256 / 16 67, 66, 1 000 / 32 / 16 70, 66; two 64 / 8 / 16 61, 67, 64 / 64 / 16 67, 62, 256 / 8 / 16 69, 62,
+    // 1 024 / 56 / 16 76, 66; four 64 / 8 / 64 71, 66, 256 / 64 / 64 84, 76, 3 000 / 16 / 64 96, 87; 24 256 / 8 / 256 427, 415.
+    // Not with callers that are told of finished ranges or time the stages: they rely on the order.
     const uint64_t dx_tiles = (uint64_t)((H1 + 127U) / 128U) * ((B + 255U) / 256U);
+    constexpr uint64_t kLeast[] = {65536U, 16384U, 2048U, 0U};  // samples x hd1, by the number of blocks
     SideBranch branch{e, st};
-    if (dx_tiles < 2ULL * e->sm_count && B <= 16384U && (uint64_t)B * H1 >= 65536U && !told) branch.Fork();
+    if (dx_tiles < 2ULL * e->sm_count && B <= 16384U && (uint64_t)B * H1 >= kLeast[std::min(R, 3U)] && !told) branch.Fork();
     const LaunchOn st_dw(branch.open ? branch.side.stream : st.stream, st.overlap);
     uint32_t* order = half_ig ? reinterpret_cast<uint32_t*>(base + ws.off_lists) : reinterpret_cast<uint32_t*>(dz1_f32 + (uint64_t)B * p_dz1_f32);
     uint32_t* first = order + (uint64_t)s.state_len * B;

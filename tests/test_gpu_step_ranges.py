@@ -47,9 +47,9 @@ def test_walk_rounds_and_edges(oracle, n, k_min, k_max, state_len, move_count):
     assert np.array_equal(meta.cpu().numpy().view(WALK_META_DTYPE).reshape(-1), want_meta)
 
 
-def loss_grad_case(oracle, dims, n, *, seed=1, scale=0.03, mirror=True, options=None, flags=(True, True), tol=1e-3, section_tol=3e-3, coherent=False):
+def loss_grad_case(oracle, dims, n, *, seed=1, scale=0.03, mirror=True, options=None, flags=(True, True), tol=1e-3, section_tol=3e-3, forks=None):
     """One loss + gradient launch on a walk batch against the oracle's model of the same data flow, whole and by section. The last
-    of four calls has a callback, which keeps all work on the caller's stream; the first three may use a second one."""
+    of four calls has a callback, which keeps all work on the caller's stream; the first three may use a second one (`forks`: have to, may not)."""
     shape = MlpShape(*dims)
     length, values = shape.state_len, shape.state_value_pad
     moves, target = random_puzzle(length, 18, seed)
@@ -77,6 +77,7 @@ def loss_grad_case(oracle, dims, n, *, seed=1, scale=0.03, mirror=True, options=
             assert st == 0 and engine.check()[0] == 0
             launches = engine.launch_count - before
             results.append((float(loss.item()), grad.cpu().numpy()))
+        assert forks is None or engine.fork_count == (3 if forks else 0)
     finally:
         engine.close()
     for other in results[1:]:
@@ -365,7 +366,14 @@ def test_hidden_input_gradient_stores(oracle, monkeypatch, hd1, hd2, n):
 @pytest.mark.parametrize("form", ["gather", "onehot"])
 def test_weight_gradients_beside_the_embedding_gradient(oracle, monkeypatch, dims, n, form):
     monkeypatch.setenv("MGT_EMBEDDING_FORM", form)
-    loss_grad_case(oracle, dims, n, scale=0.02)
+    loss_grad_case(oracle, dims, n, scale=0.02, forks=True)
+
+
+# ... where that begins, by the number of blocks
+@pytest.mark.parametrize("blocks,hd1,n,forks", [(0, 255, 256, False), (0, 256, 256, True), (1, 127, 128, False), (1, 128, 128, True), (2, 31, 66, False), (2, 32, 64, True), (3, 8, 64, True),
+                                                (3, 8, 16385, False)])
+def test_steps_that_fork(oracle, blocks, hd1, n, forks):
+    loss_grad_case(oracle, (12, 6, hd1, 24, blocks, 1), n, forks=forks)
 
 
 # Bias sums of the backward tower with two and three tiles to a CTA (or pair), whose products follow one another into the same
@@ -402,7 +410,8 @@ def test_tower_bias_sums_over_tiles(oracle, monkeypatch, hd2, n):
 
 
 class SmallStep:
-    """Loss + gradient of a batch that the library spreads over two streams, with scratch of its own."""
+    """Loss + gradient of a batch that the library spreads over two streams, with scratch of its own. Every call has to have done so,
+    unless it asks for one stream."""
 
     def __init__(self, engine, n=96, dims=(72, 72, 256, 40, 2, 1)):
         rng = np.random.default_rng(n)
@@ -414,9 +423,12 @@ class SmallStep:
         self.ws = torch.empty(self.floats, device=DEV)
         torch.cuda.synchronize()
 
-    def __call__(self, stream=None, one_stream=False):
-        return self.engine.launch_mlp_loss_grad(self.shape, self.w, None, self.states, self.labels, self.n, self.loss, self.grad, self.ws, self.floats, stream=stream,
-                                                gradient_ready=(lambda *a: 0) if one_stream else None)
+    def __call__(self, stream=None, one_stream=False, forks=1):
+        before = self.engine.fork_count
+        status = self.engine.launch_mlp_loss_grad(self.shape, self.w, None, self.states, self.labels, self.n, self.loss, self.grad, self.ws, self.floats, stream=stream,
+                                                  gradient_ready=(lambda *a: 0) if one_stream else None)
+        assert self.engine.fork_count - before == (0 if one_stream else forks)
+        return status
 
     def result(self):
         torch.cuda.synchronize()
@@ -520,6 +532,8 @@ def test_two_captures_at_once(small_step):
     assert other(one_stream=True) == 0 and small_step(one_stream=True) == 0
     want_other, want = other.result(), small_step.result()
     streams, graphs = [torch.cuda.Stream() for _ in range(2)], [torch.cuda.CUDAGraph() for _ in range(2)]
+    assert small_step(streams[0]) == 0 and other(streams[1]) == 0  # (second streams made)
+    assert np.array_equal(small_step.result(), want) and np.array_equal(other.result(), want_other)
     with torch.cuda.stream(streams[0]):
         graphs[0].capture_begin(capture_error_mode="relaxed")
         assert small_step(streams[0]) == 0
@@ -544,7 +558,7 @@ def test_first_step_of_an_engine_under_capture():
     want = step.result()
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
-        assert step() == 0
+        assert step(forks=0) == 0
     graph.replay()
     assert np.array_equal(step.result(), want)
     for held in holders + [step]:
