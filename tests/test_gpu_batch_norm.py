@@ -119,6 +119,7 @@ CASES = [
     ((72, 72, 64, 32, 0, 1), 128, False, False, False),       # no residual blocks: the hidden layer's normalisation alone
     ((6, 8, 32, 256, 1, 1), 300, False, False, True),         # the widest layer whose GEMM leaves the moments of its columns
     ((6, 8, 32, 264, 1, 1), 300, False, False, True),         # ... and one that is wider
+    ((8, 8, 32, 40, 1, 1), 37965, False, False, True),        # CTAs that add the moments of two and three tiles, the last one ragged
 ]
 
 

@@ -47,9 +47,10 @@ def test_walk_rounds_and_edges(oracle, n, k_min, k_max, state_len, move_count):
     assert np.array_equal(meta.cpu().numpy().view(WALK_META_DTYPE).reshape(-1), want_meta)
 
 
-def loss_grad_case(oracle, dims, n, *, seed=1, scale=0.03, mirror=True, options=None, flags=(True, True), tol=1e-3, section_tol=3e-3, forks=None):
+def loss_grad_case(oracle, dims, n, *, seed=1, scale=0.03, mirror=True, options=None, flags=(True, True), tol=1e-3, section_tol=3e-3, forks=None, slices=None):
     """One loss + gradient launch on a walk batch against the oracle's model of the same data flow, whole and by section. The last
-    of four calls has a callback, which keeps all work on the caller's stream; the first three may use a second one (`forks`: have to, may not)."""
+    of four calls has a callback, which keeps all work on the caller's stream; the first three may use a second one (`forks`: have to, may not).
+    slices: the oracle, which adds the samples one after the other, gets that many at a time and its results are added in double."""
     shape = MlpShape(*dims)
     length, values = shape.state_len, shape.state_value_pad
     moves, target = random_puzzle(length, 18, seed)
@@ -87,6 +88,12 @@ def loss_grad_case(oracle, dims, n, *, seed=1, scale=0.03, mirror=True, options=
         st, want_loss, want, _ = oracle.loss_grad_ex(shape, w, states, labels, half_linear=half_lin, half_input_grad=half_ig, **(options or {}))
     elif half_lin:
         st, want_loss, want = oracle.loss_grad_mixed(shape, w, states, labels)
+    elif slices:
+        st, want_loss, want = 0, 0.0, np.zeros(shape.param_count)
+        for lo in range(0, n, slices):
+            some, some_loss, some_grad = oracle.loss_grad(shape, w, states[lo:lo + slices], labels[lo:lo + slices])
+            share = min(slices, n - lo) / n
+            st, want_loss, want = st | some, want_loss + share * some_loss, want + share * some_grad.astype(np.float64)
     else:
         st, want_loss, want = oracle.loss_grad(shape, w, states, labels)
     assert st == 0 and np.isfinite(got).all()
@@ -115,12 +122,34 @@ def test_fp32_linears_over_tiles(oracle, dims, n):
     loss_grad_case(oracle, dims, n, flags=(False, False), tol=1e-5, section_tol=2e-5)
 
 
-# The fp32 tower as it is cut for different batches and widths: 32, 64, 128, 224 and 256 columns a warp, one to four warps side by
-# side, stages of 8 to 32, ends of tiles, matrices that have to be padded; and layer by layer. The oracle adds the samples one after the other in
-# fp32, each sum to n 2^-24 of its terms at worst.
-@pytest.mark.parametrize("hd2,n", [(224, 8201), (250, 8190), (96, 16390), (128, 2999), (117, 1021), (16, 40001), (200, 1021), (301, 700), (9, 64)])
-def test_fp32_tower_cuts(oracle, hd2, n):
-    loss_grad_case(oracle, (6, 4, 16, hd2, 1, 1), n, flags=(False, False), tol=1e-5 + n * 2.0 ** -24, section_tol=2e-5 + n * 2.0 ** -24)
+# The fp32 tower as it is cut for different batches and widths: one warp of 32, 64, 128, 224 or 256 columns, up to four of 32 and of 64
+# side by side and two of 128; stages of 8, 16 and 32; one round of the chip and more; ends of tiles, matrices that have to be padded. Blocks that
+# hand their signs, the ring of weights and the column sums' two places on to one another. And layer by layer, the widths of 129 to 256
+# too: with few samples, and where the products' tiles fill the chip better than another round of the tower's.
+@pytest.mark.parametrize("hd2,n,blocks", [(4, 70, 3), (9, 64, 3), (40, 300, 3), (72, 301, 3), (117, 1021, 3), (60, 12001, 2), (128, 2999, 2), (136, 2600, 2), (200, 3301, 2), (5, 20001, 2), (96, 16390, 2),
+                                          (16, 40001, 2), (160, 7001, 2), (224, 4201, 2), (224, 8201, 1), (250, 4100, 2), (250, 8190, 1), (136, 9500, 1), (200, 1021, 2), (250, 2499, 2), (224, 9501, 1), (301, 700, 2)])
+def test_fp32_tower_cuts(oracle, hd2, n, blocks):
+    loss_grad_case(oracle, (6, 4, 16, hd2, blocks, 1), n, flags=(False, False), tol=1e-5, section_tol=2e-5, slices=1000)
+
+
+# ... and which widths and batches take it: a block more is then no launch more, else it is four products more
+@pytest.mark.parametrize("hd2,n,fused", [(8, 33, True), (128, 70, True), (129, 2499, False), (129, 2500, True), (160, 9500, True), (160, 12000, False), (224, 8200, True), (224, 9500, False), (224, 20000, True),
+                                         (256, 2500, True), (257, 2600, False)])
+def test_fp32_tower_or_layers(hd2, n, fused):
+    states, labels, loss = torch.zeros(n, 80, dtype=torch.uint8, device=DEV), torch.ones(n, device=DEV), torch.zeros(1, device=DEV)
+    launches = []
+    engine = mgt.Engine(0)
+    try:
+        for blocks in (1, 2):
+            c = mgt.CudaMlpShape(4, 4, 16, hd2, blocks, 1)
+            w, floats = torch.zeros(c.param_count, device=DEV), mgt.mlp_loss_grad_workspace_floats(c, n, 1, False, False)
+            before = engine.launch_count
+            assert engine.launch_mlp_loss_grad(c, w, None, states, labels, n, loss, torch.empty_like(w), torch.empty(floats, device=DEV), floats, use_half_input_grad=False,
+                                               use_half_linear=False, gradient_ready=lambda *a: 0) == 0
+            launches.append(engine.launch_count - before)
+    finally:
+        engine.close()
+    assert launches[1] - launches[0] == (0 if fused else 4)
 
 
 # A weight without bound behind a unit that no sample opens: its products with the samples are NaN before a ReLU that closes on
@@ -546,6 +575,54 @@ def test_two_captures_at_once(small_step):
     for graph in graphs:
         graph.replay()
     assert np.array_equal(small_step.result(), want) and np.array_equal(other.result(), want_other)
+
+
+# Steps as a graph: kernels that begin before the one ahead of them has ended, behind forks and joins, and behind the memsets of a one-hot
+# product with shared tiles and of the layered tower of batch normalisation. Two steps in a graph, replayed three times.
+@pytest.mark.parametrize("dims,n,flags,form,batch_norm", [((72, 72, 256, 40, 2, 1), 1500, (True, True), "gather", False), ((72, 72, 2560, 24, 1, 1), 130, (True, True), "onehot", False),
+                                                          ((72, 72, 256, 40, 2, 3), 300, (True, True), "gather", True), ((72, 72, 256, 300, 2, 1), 300, (True, True), "onehot", True),
+                                                          ((72, 72, 256, 300, 2, 29), 300, (False, True), "gather", False), ((72, 72, 256, 40, 2, 1), 1000, (False, False), "gather", False)])
+def test_captured_steps(monkeypatch, dims, n, flags, form, batch_norm):
+    monkeypatch.setenv("MGT_EMBEDDING_FORM", form)
+    c = mgt.CudaMlpShape(*dims)
+    total = c.param_count + (mgt.bn_param_count(c) if batch_norm else 0)
+    rng = np.random.default_rng(n)
+    first = torch.from_numpy((rng.standard_normal(total) * 0.03).astype(np.float32)).to(DEV)
+    states = torch.from_numpy(rng.integers(0, 72, (n, 80), dtype=np.uint8)).to(DEV)
+    labels, loss, grad = torch.ones(n * dims[5], device=DEV), torch.zeros(1, device=DEV), torch.zeros(total, device=DEV)
+    floats = mgt.mlp_loss_grad_workspace_floats(c, n, 1, *flags, batch_norm=batch_norm)
+    w, m, v, ws = first.clone(), torch.zeros_like(first), torch.zeros_like(first), torch.full((floats,), float("nan"), device=DEV)
+    stream, graph, engine = torch.cuda.Stream(), torch.cuda.CUDAGraph(), mgt.Engine(0)
+    forks = 2 if flags[1] else 0
+
+    def two_steps():
+        for _ in range(2):
+            assert engine.launch_mlp_loss_grad(c, w, None, states, labels, n, loss, grad, ws, floats, use_half_input_grad=flags[0], use_half_linear=flags[1], stream=stream) == 0
+            assert mgt.launch_adamw_kernel(mgt.AdamWKernelConfig(total, 1, 1e-3), w, grad, m, v, stream=stream) == 0
+
+    def finish():
+        torch.cuda.synchronize()
+        assert engine.check()[0] == 0
+        result = [t.cpu().numpy() for t in (w, m, v, grad, loss)]
+        for t, start in ((w, first), (m, 0.0), (v, 0.0), (grad, float("nan"))):
+            t.copy_(start) if isinstance(start, torch.Tensor) else t.fill_(start)
+        torch.cuda.synchronize()
+        return result
+    try:
+        assert engine.set_train_options(batch_norm=batch_norm) == 0
+        torch.cuda.synchronize()
+        for _ in range(3):
+            two_steps()
+        want = finish()
+        assert np.isfinite(want[0]).all() and engine.fork_count == 3 * forks
+        with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+            two_steps()
+        assert engine.fork_count == 4 * forks
+        for _ in range(3):
+            graph.replay()
+        assert all(np.array_equal(a, b) for a, b in zip(finish(), want))
+    finally:
+        engine.close()
 
 
 def test_first_step_of_an_engine_under_capture():
