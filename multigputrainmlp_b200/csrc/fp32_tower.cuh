@@ -48,23 +48,24 @@ struct TowerArgs {
     float* colsum;              // backward: slot j at colsum + j * colsum_slot, one row of H per CTA
     uint64_t colsum_slot;
     uint32_t row_groups, col_groups;  // W and CG
-    uint32_t chunk, stages;     // depth of a weight stage (a multiple of 8) and their number
+    uint32_t chunk, stages;     // depth of a weight stage (a multiple of 8) and their number: kTowerStages, but as a constant it makes the kernel
+                                // slower (p888 at 8 192 samples 3 670 -> 3 748 us a step)
     int* status;
 };
 
 // How a batch is cut. Columns of a warp: 32 NJ; the more, the fewer shared-memory reads a multiply-add needs, but the fewer warps.
 struct TowerPlan {
-    uint32_t nj, row_groups, col_groups, tiles, chunk, stages;
+    uint32_t nj, row_groups, col_groups, tiles, chunk;
     size_t smem;
     uint32_t rounds;  // of the chip, a tile to every place that an SM has for one
     double us;        // what a product of all samples takes in that many rounds, as measured (widths of 129 to 256)
 };
-constexpr uint32_t kTowerSmem = 227U * 1024U, kTowerBarBytes = 128U;
+constexpr uint32_t kTowerSmem = 227U * 1024U, kTowerBarBytes = 128U, kTowerStages = 3U;
 inline uint32_t TowerThreads(uint32_t nj) { return nj >= 7U ? 256U : 512U; }          // of a CTA at most
 inline uint32_t TowerResidentThreads(uint32_t nj) { return nj <= 2U ? 1024U : TowerThreads(nj); }  // of an SM, by registers
-inline size_t TowerSmem(uint32_t H, uint32_t W, uint32_t padded, uint32_t chunk, uint32_t stages) {
+inline size_t TowerSmem(uint32_t H, uint32_t W, uint32_t padded, uint32_t chunk) {
     const size_t rows = (H + 15U) / 16U * 16U;
-    return (2U * rows * (8U * W + 4U) + stages * static_cast<size_t>(padded) * (chunk + 4U) + 2U * W * padded) * sizeof(float) + kTowerBarBytes;
+    return (2U * rows * (8U * W + 4U) + kTowerStages * static_cast<size_t>(padded) * (chunk + 4U) + 2U * W * padded) * sizeof(float) + kTowerBarBytes;
 }
 // words of sign bits of a sample
 inline uint32_t TowerSampleWords(uint32_t H) { return H <= 128U || H > 224U ? (H + 31U) / 32U : 7U; }
@@ -81,19 +82,16 @@ inline TowerPlan PlanTower(uint32_t B, uint32_t H, uint32_t sm) {
         if (nj >= 7U && (cg > 1U || nj > TowerSampleWords(H))) continue;  // (never the best; a sample has TowerSampleWords words)
         for (uint32_t w = 1U; w <= 8U; ++w) {
             if ((w * cg + 1U) * 32U > TowerThreads(nj)) break;
-            // the deepest stages of which three fit, or two of eight
-            uint32_t chunk = 32U, stages = 3U;
-            while (chunk > 8U && (TowerSmem(H, w, padded, chunk, stages) > kTowerSmem || chunk >= 2U * H)) chunk /= 2U;
-            if (TowerSmem(H, w, padded, chunk, stages) > kTowerSmem) stages = 2U;
-            const size_t smem = TowerSmem(H, w, padded, chunk, stages);
-            if (smem > kTowerSmem) continue;
+            uint32_t chunk = 32U;  // the deepest stages of which three fit (of eight k they do for every width up to 256)
+            while (chunk > 8U && (TowerSmem(H, w, padded, chunk) > kTowerSmem || chunk >= 2U * H)) chunk /= 2U;
+            const size_t smem = TowerSmem(H, w, padded, chunk);
             const uint32_t tiles = (B + 8U * w - 1U) / (8U * w), warps = w * cg;
             const uint32_t resident = std::max<uint32_t>(1U, std::min<uint32_t>({static_cast<uint32_t>(kTowerSmem / (smem + 1024U)), TowerResidentThreads(nj) / (warps * 32U + 32U), tiles / sm}));
             const uint32_t rounds = (tiles + sm * resident - 1U) / (sm * resident);
             const double cost = rounds * (std::max(width.alone, width.each * ((warps * resident + 3U) / 4U)) * H + 3000.0 * resident);
             if (cost < best_cost) {
                 best_cost = cost;
-                best = {nj, w, cg, tiles, chunk, stages, smem, rounds, rounds * (H / 100.0) * (warps * resident <= 4U ? width.round_alone : width.round)};
+                best = {nj, w, cg, tiles, chunk, smem, rounds, rounds * (H / 100.0) * (warps * resident <= 4U ? width.round_alone : width.round)};
             }
         }
     }
@@ -397,7 +395,7 @@ inline cudaError_t LaunchTower(int device, LaunchOn st, const TowerPlan& plan, T
     a.row_groups = plan.row_groups;
     a.col_groups = plan.col_groups;
     a.chunk = plan.chunk;
-    a.stages = plan.stages;
+    a.stages = kTowerStages;
     a.words = TowerSampleWords(a.H);
     switch (plan.nj) {
         case 1: return TowerRun<1, BWD>(device, st, a, plan);
