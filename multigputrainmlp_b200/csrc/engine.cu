@@ -542,8 +542,9 @@ RepackHalfKernel(const float* __restrict__ src, uint8_t* __restrict__ dst, const
 
 // Sums over partial results, each in a fixed order: out[group][i] = sum over terms t of src[group][t * stride + i]. The sums of a
 // step that nothing in the step waits for - split-K planes, bias sums of the tiles, what the head's CTAs leave - are collected and
-// go in one launch: as six of 2 to 14 us each, with a gap before it, they were a seventh of the smallest steps (64 samples of hd1 8,
-// hd2 8: 85 us, now 73; 1 024 of hd1 256, hd2 64, 2 blocks: 118, now 103; p888 at 53 248: 3 059, now 3 051).
+// go in one launch: as six of 2 to 14 us each, with a gap before it, they were a seventh of the smallest steps (us a step with six, with
+// one, and with one since launches overlap too: 64 samples of hd1 8, hd2 8 85, 73, 56; 1 024 of hd1 256, hd2 64, 2 blocks 118, 103, 82;
+// p888 at 53 248 3 059, 3 051, where they do not overlap).
 // Few items with many terms (kLanes): eight items a CTA, each of 32 lanes adds terms g, g + 32, ... and the lanes are then
 // added 0..31. Many items with few terms: an item (kItem) or four neighbouring ones (kQuad) a thread, terms in order.
 struct SumJob {
@@ -776,9 +777,9 @@ __device__ __forceinline__ void HeadLossRow(const HeadArgs& a, uint32_t b, float
 // Up to 64 outputs: a CTA takes 64 samples at a time. Forward as a small register-tiled product (a thread: four samples x
 // OP / 16 outputs) from x staged 64 columns at a time and the weights staged once; the loss by a warp per sample; backward
 // with a thread per hidden column, its OP weights in registers, so that dy is read as broadcast vectors and rows of dz are
-// written whole. Bound by HBM: x in the operand format and in fp32 (the ReLU mask), dz in both. One warp per sample with a
-// scalar read of x and of a weight for every multiply-add was bound by the load pipe: 1.83 ms at batch 131 072, hd2 512, 29
-// outputs, now 0.70 ms.
+// written whole. Bound by the multiply-adds of both products on the CUDA cores and the shared-memory reads that feed them: 0.68 ms at
+// batch 131 072, hd2 512, 29 outputs, where the 0.8 GB it moves (x in the operand format and in fp32 for the ReLU mask, dz in
+// both) take 0.13. One warp per sample with a scalar read of x and of a weight for every multiply-add took 1.83 ms.
 constexpr uint32_t kHeadTile = 64;
 template <int OP>
 constexpr size_t HeadTileSmem(uint32_t H2) { return ((size_t)H2 * OP + 64U * (kHeadTile + 4U) + kHeadTile * OP) * sizeof(float); }
@@ -1829,8 +1830,8 @@ mgt_status_t mgt_launch_mlp_loss_grad(mgt_engine_t* e, const mgt_mlp_shape_t* sh
         return e->bn_exchange(e->bn_exchange_user, bn_stats, 2ULL * H2, stream_v) == MGT_OK ? MGT_OK : MGT_CUDA_FAILURE;
     };
     // Widths of one tile: the GEMM that makes z leaves its column moments too, as four rows of partial sums a CTA. As a kernel of its
-    // own they read z again: p888 at 53 248 samples 5 524 -> 5 450 us a step. (The moments of the backward pass in the epilogue
-    // of the product before them were tried: it needs z there, and 5 485 us.)
+    // own they read z again: p888 at 53 248 samples 5 485 -> 5 415 us a step. (The moments of the backward pass in the epilogue of
+    // the product before them as well: it needs z there, and 5 485 us again.)
     const uint32_t bn_rows = 4U * std::min((B + 127U) / 128U, (uint32_t)e->sm_count);
     const bool bn_fused = H2 <= 256U && bn_rows <= bn::kMaxBlocks;
     // z_tape(layer) -> x_f32 / x_h(layer): x = relu(bn(z)) for the hidden layer, relu(x + bn(z)) for a block

@@ -1,11 +1,12 @@
 // Kernel launches that may begin before the kernel ahead of them in the stream has ended (programmatic dependent launch).
 //
-// Every kernel of this library sets itself up (barriers, tensor memory, shared memory), then calls dependent_begin() before it touches
-// global memory: that waits until the kernels ahead are complete and their writes visible, and lets the next kernel of the stream
-// be set up in turn. As a kernel lets the next one in only after its own wait, at most two kernels of a stream are on the chip, and
+// Every kernel of a training step (not those of comm.cu, which exchange gradients) sets itself up (barriers, tensor memory, shared
+// memory), then calls dependent_begin() before it touches global memory: that waits until the kernels ahead are complete and their
+// writes visible, and lets the next kernel of the stream be set up in turn. As a kernel lets the next one in only after its own wait, at most two kernels of a stream are on the chip, and
 // a kernel that is not launched this way (another library's, a copy, an exchange kernel) is ordered as ever.
 // What it saves is the gap between two launches, 1 to 2 us, and the set-up, 1 to 3 us. What it costs: the CTAs of the next kernel take
-// shared memory from the L1 of a kernel that still runs, and SMs from the other stream. See OverlapLaunches in engine.cu for where it pays.
+// shared memory from the L1 of a kernel that still runs, find little of it themselves beside one that asked for all shared memory, and
+// take SMs from the other stream. See OverlapLaunches and OverlapFp32Launches in engine.cu for where it pays.
 #pragma once
 
 #include <cuda_runtime.h>
