@@ -63,7 +63,7 @@ def test_workspace_never_shrinks_with_the_batch():
     # scratch sized for the largest batch has to do for every smaller one, on both sides of every rule that picks a kernel by size
     import multigputrainmlp_b200 as mgt
     spans = [((72, 72, 2560, 224, 16, 1), range(3500, 3800)), ((72, 72, 1000, 200, 8, 29), range(7200, 7600)), ((54, 54, 512, 64, 2, 1), range(16600, 16800)),
-             ((54, 6, 1024, 256, 4, 1), range(1, 4000, 37)), ((72, 72, 333, 77, 3, 1), range(1, 40000, 401)), ((16, 1, 33, 24, 0, 2), range(1, 300))]
+             ((54, 6, 1024, 256, 4, 1), range(1, 4000, 37)), ((72, 72, 333, 77, 3, 1), range(1, 40000, 401)), ((16, 16, 64, 224, 4, 1), range(2400, 2600, 7)), ((16, 1, 33, 24, 0, 2), range(1, 300))]
     for dims, batches in spans:
         shape = mgt.CudaMlpShape(*dims)
         for half_ig, half_lin, bn in ((True, True, False), (False, True, False), (True, True, True), (False, False, False), (True, False, False)):
